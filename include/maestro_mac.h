@@ -94,8 +94,9 @@ typedef struct mac_opts {
     int inner_vcycles;      /* mixed precision: FP32 V-cycles per FP64 refinement step (>= 1;
                                default 3; the most per step when adaptive_inner is on); the
                                FP64 residual is formed once per step                          */
-    int coarse_tail;        /* 1 (default): the levels small enough for shared memory and the
-                               bottom solve run as one single-CTA kernel (same arithmetic)     */
+    int coarse_tail;        /* 1 (default): the levels small enough for a thread-block cluster's
+                               shared memory and the bottom solve run as one kernel (same
+                               arithmetic)                                                     */
     int adaptive_inner;     /* mixed precision, 1 (default): after each step the next step runs
                                only as many inner V-cycles (<= inner_vcycles) as the contraction
                                just observed predicts the tolerance needs; 0: always

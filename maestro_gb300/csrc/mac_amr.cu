@@ -711,6 +711,7 @@ struct GpuExec : GpuMl<double> {
         // mixed precision: the FP32 level-0 operator of the inner cycles' coarse correction
         if (!rc && c->o.precision == MAC_PREC_MIXED) rc = setup_fp32_copies(c);
         if (!rc) rc = setup_coarse_levels(c);
+        if (!rc) rc = wait_bottom_inverse(c);   // the level-0 cycles below read it
         singular = c->singular;
         return rc;
     }

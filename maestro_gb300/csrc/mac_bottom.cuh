@@ -1,5 +1,5 @@
-// Bottom solver of the multigrid (coarsest level, natural layout, FP64): device code shared by
-// the bottom kernel (mac_kernels.cu) and the single-CTA tail V-cycle (mac_tail.cu).
+// Bottom solver of the multigrid in one CTA (coarsest level, natural layout, FP64), for levels too
+// large for the cluster solver's shared memory (mac_tail.cu).
 // FBoxLib's default MAC bottom solve (Docs/mg/mg.tex:221-249): nub red/black Gauss-Seidel sweeps,
 // BiCGStab to bottom_eps, nub sweeps; here BiCGStab is Jacobi preconditioned.
 #pragma once
@@ -14,63 +14,7 @@ struct BotView {
     const double *bx, *by, *bz, *dg, *idg;
 };
 
-// Synchronisation policies of the bottom solver.  Sync128<NAMED>: 128 threads (four warps, so
-// the four FP64 units of the SM share the work), work item p of a loop handled by warp p % 4
-// (item permutation), reductions: xor-shuffle within each warp, then the four warp sums in a fixed
-// order -- every thread gets the same value.  NAMED: barrier 1 over the first 128 threads of a
-// larger CTA, else __syncthreads (a 128-thread CTA).  CtaSync: any CTA size, natural item order.
-template <bool NAMED>
-struct Sync128 {
-    static __device__ __forceinline__ void sync() {
-        if (NAMED)
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-        else
-            __syncthreads();
-    }
-    static __device__ __forceinline__ int tid() {
-        const int t = threadIdx.x;
-        return 4 * (t & 31) + (t >> 5);
-    }
-    static __device__ __forceinline__ int nt() { return 128; }
-    static __device__ double sum(double v, double* sm) {
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
-        sync();
-        const double r = (sm[0] + sm[1]) + (sm[2] + sm[3]);
-        sync();
-        return r;
-    }
-    // two sums at once (one pair of barriers)
-    static __device__ void sum2(double& a, double& b, double* sm) {
-        for (int o = 16; o > 0; o >>= 1) {
-            a += __shfl_xor_sync(0xffffffffu, a, o);
-            b += __shfl_xor_sync(0xffffffffu, b, o);
-        }
-        if ((threadIdx.x & 31) == 0) {
-            sm[threadIdx.x >> 5] = a;
-            sm[4 + (threadIdx.x >> 5)] = b;
-        }
-        sync();
-        a = (sm[0] + sm[1]) + (sm[2] + sm[3]);
-        b = (sm[4] + sm[5]) + (sm[6] + sm[7]);
-        sync();
-    }
-    // maximum of unsigned 64-bit keys (integer pipe)
-    static __device__ unsigned long long umax(unsigned long long v, double* sm) {
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
-            v = w > v ? w : v;
-        }
-        unsigned long long* u = reinterpret_cast<unsigned long long*>(sm);
-        if ((threadIdx.x & 31) == 0) u[threadIdx.x >> 5] = v;
-        sync();
-        unsigned long long r = u[0];
-        for (int w = 1; w < 4; ++w) r = u[w] > r ? u[w] : r;
-        sync();
-        return r;
-    }
-};
-
+// Synchronisation policy of the one-CTA bottom solver: any CTA size, natural item order.
 struct CtaSync {
     static __device__ __forceinline__ void sync() { __syncthreads(); }
     static __device__ __forceinline__ int tid() { return threadIdx.x; }

@@ -34,7 +34,7 @@
 namespace mac {
 
 constexpr int kMaxLevels = 32;
-constexpr int kBottomMaxCells = 65536;   // single-CTA bottom solver limit
+constexpr int kBottomMaxCells = 65536;   // bottom solver limit
 constexpr int kBotScrPerCell = 18;       // bottom solver scratch: 14 doubles + 7 ints per cell
 
 #define MAC_CUDA_TRY(expr)                                   \
@@ -313,7 +313,8 @@ struct mac_ctx {
     cudaEvent_t aux_ev[2] = {nullptr, nullptr};   // [0] operators ready, [1] inverse done
     bool inv_pending = false;                     // the main stream still has to wait on aux_ev[1]
     int tail_start[2] = {-1, -1};                 // first tail level (FP64, FP32); -1: none
-    size_t tail_smem[2] = {0, 0};
+    int tail_nc = 16;                             // CTAs of the tail cluster
+    bool bottom_cluster = false;                  // the bottom alone fits the cluster
     double ktime_ms[8] = {};
     int ktime_launches[8] = {};
 
@@ -384,14 +385,19 @@ void launch_bottom(const Dims& d, const LevelArrays<double>& a64, Tio* x, const 
                    double* scratch, bool singular, int nub, double eps, int max_iter,
                    int* iter_counter, cudaStream_t s);
 
-int prepare_kernels();
-
-// ---- single-CTA tail V-cycle (mac_tail.cu) --------------------------------------------------
+// ---- cluster tail V-cycle (mac_tail.cu) -----------------------------------------------------
+// nlev == 0: the bottom alone (f0 and e0 in its natural layout, e0 the initial guess)
 constexpr int kTailMaxLevels = 8;
 constexpr int kTailSmemMax = 200 * 1024;
+struct TailGeo {
+    int repl, rpc;                        // held whole by every CTA; rows a CTA
+    int two;                              // two pairs of cells a thread
+    int off;                              // byte offset in shared memory
+    unsigned mcpc, mn1, mhn0;             // reciprocals of rpc n0, n1, n0 / 2
+};
 template <typename T>
 struct TailParams {
-    int nlev;                             // tail levels above the bottom
+    int nlev;                             // tail levels above the bottom (0: the bottom alone)
     Dims lev[kTailMaxLevels];             // their dimensions (checkerboard-split in global memory)
     const T* bx[kTailMaxLevels];
     const T* by[kTailMaxLevels];
@@ -400,7 +406,7 @@ struct TailParams {
     const T* idg[kTailMaxLevels];
     Dims bottom;                          // bottom level (natural layout, FP64 operator)
     const double *bbx, *bby, *bbz, *bdg, *bidg;
-    const T* f0;                          // right-hand side of the first tail level
+    const T* f0;                          // right-hand side of the first tail level (or the bottom)
     T* e0;                                // its correction (output)
     BcDesc bc;
     int nu1, nu2, nub, singular, bottom_max_iter;
@@ -408,12 +414,16 @@ struct TailParams {
     int* iters;
     const double* binv;                   // dense (pseudo-)inverse of the bottom; null: BiCGStab
     T omega;                              // relaxation weight of the half-sweeps (1: Gauss-Seidel)
+    TailGeo geo[kTailMaxLevels];          // plan (launch_tail)
+    int bottom_off, bottom_m;             // bottom: byte offset, cells a CTA
+    unsigned bottom_mm;                   // reciprocal of bottom_m
 };
+// whether nl levels and the bottom (exact: solved by its inverse) fit a cluster of nc CTAs
 template <typename T>
-size_t tail_smem_bytes(const Dims* lev, int nl, const Dims& bottom);
+bool tail_fits(const Dims* lev, int nl, const Dims& bottom, bool exact, int nc);
 template <typename T>
-void launch_tail(const TailParams<T>& P, size_t smem, cudaStream_t s);
-int prepare_tail_kernels();
+void launch_tail(TailParams<T>& P, int nc, cudaStream_t s);   // (fills P's plan)
+int prepare_tail_kernels(int* nc);
 // exact bottom solve of the FP32 V-cycle: bottoms of at most kDenseBottomMax cells, row r of the
 // inverse applied by kDenseSeg lanes of a warp
 constexpr int kDenseBottomMax = 64;
@@ -427,6 +437,7 @@ int setup_coarse_levels(mac_ctx* c);
 // the exact bottom's (pseudo-)inverse, on the side stream once the bottom operator is built
 // (no-op unless the FP32 V-cycle uses it); run_solve orders the V-cycles after it
 int issue_bottom_inverse(mac_ctx* c);
+int wait_bottom_inverse(mac_ctx* c);
 int setup_fp32_copies(mac_ctx* c);
 // phi_nat (optional): the initial guess in natural layout, moved into the level-0 phi in the same pass
 int setup_rhs(mac_ctx* c, const double* macrhs, bool have_beta0, const double* phi_nat = nullptr);

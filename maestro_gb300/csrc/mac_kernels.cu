@@ -106,7 +106,7 @@ k_gsrb(Dims d, int colour, T* __restrict__ us, const T* __restrict__ uo, const T
     T acc = arms<T>(fs[q], q, nb, uo, bxs, bys, bzs, bxo, byo, bzo);
     if (SOR) {
         const T old = us[q];
-        us[q] = fmaT(omega, acc * ids[q] - old, old);
+        us[q] = fmaT(omega, fmaT(acc, ids[q], -old), old);
     } else {
         us[q] = acc * ids[q];
     }
@@ -629,40 +629,19 @@ k_first_resid_zero(int n, double* __restrict__ f, const double* __restrict__ mea
     if (threadIdx.x == 0 && m) atomicMax(maxbits, m);
 }
 
-// ---- single-CTA FP64 bottom solver (natural layout): device code in mac_bottom.cuh -------------
+// ---- FP64 bottom solver of levels too large for the cluster's shared memory (natural layout):
+// one CTA, vectors in global scratch; device code in mac_bottom.cuh ------------------------------
 constexpr int kBottomThreads = 1024;
-constexpr int kBottomSmemCells = 1024;   // 7 + kBotScrPerCell doubles per cell: 204,800 B
 
-// SMEM: the five operator arrays and the nine work vectors live in dynamic shared memory
-// (levels of up to kBottomSmemCells cells, 128 threads), else in global scratch (1024 threads).
-template <typename Tio, bool SMEM>
+template <typename Tio>
 __global__ void __launch_bounds__(kBottomThreads)
-k_bottom(BotView vin, Tio* __restrict__ xio, const Tio* __restrict__ fio, double* __restrict__ gscr,
+k_bottom(BotView v, Tio* __restrict__ xio, const Tio* __restrict__ fio, double* __restrict__ scr,
          int singular, int nub, double eps, int max_iter, int* __restrict__ iters) {
     pdl_wait();
     pdl_trigger();
     __shared__ double sm[33];
-    extern __shared__ double dsm[];
-    const int N = vin.N;
-    BotView v = vin;
-    double* scr = gscr;
+    const int N = v.N;
     const int tid = threadIdx.x, nt = blockDim.x;
-    if (SMEM) {
-        double* ops = dsm;
-        for (int c = tid; c < N; c += nt) {
-            ops[c] = vin.bx[c];
-            ops[N + c] = vin.by[c];
-            ops[2 * N + c] = vin.bz[c];
-            ops[3 * N + c] = vin.dg[c];
-            ops[4 * N + c] = vin.idg[c];
-        }
-        v.bx = ops;
-        v.by = ops + N;
-        v.bz = ops + 2 * N;
-        v.dg = ops + 3 * N;
-        v.idg = ops + 4 * N;
-        scr = dsm + 5 * N;
-    }
     double* x = scr;
     double* f = scr + N;
     for (int c = tid; c < N; c += nt) {
@@ -670,11 +649,7 @@ k_bottom(BotView vin, Tio* __restrict__ xio, const Tio* __restrict__ fio, double
         f[c] = (double)fio[c];
     }
     __syncthreads();
-    int count;
-    if (SMEM)
-        count = bottom_body<Sync128<false>>(v, x, f, scr + 2 * N, sm, singular, nub, eps, max_iter);
-    else
-        count = bottom_body<CtaSync>(v, x, f, scr + 2 * N, sm, singular, nub, eps, max_iter);
+    const int count = bottom_body<CtaSync>(v, x, f, scr + 2 * N, sm, singular, nub, eps, max_iter);
     __syncthreads();
     for (int c = tid; c < N; c += nt) xio[c] = (Tio)x[c];
     if (tid == 0 && iters) atomicAdd(iters, count);
@@ -814,27 +789,8 @@ void launch_bottom(const Dims& d, const LevelArrays<double>& a64, Tio* x, const 
     v.bz = a64.bz;
     v.dg = a64.diag;
     v.idg = a64.invdiag;
-    // small levels: 128 threads, operator and vectors in shared memory; large: one 1024-thread
-    // CTA on global scratch
-    const size_t smem = (size_t)(7 + kBotScrPerCell) * d.ncell * sizeof(double);
-    if (d.ncell <= kBottomSmemCells)
-        launch_chain(k_bottom<Tio, true>, dim3(1), dim3(128), smem, s, v, x, f, scratch,
-                   singular ? 1 : 0, nub, eps, max_iter, iter_counter);
-    else
-        launch_chain(k_bottom<Tio, false>, dim3(1), dim3(kBottomThreads), 0, s, v, x, f, scratch,
-                   singular ? 1 : 0, nub, eps, max_iter, iter_counter);
-}
-
-// Opt the shared-memory bottom solver into more than 48 KB of dynamic shared memory (called once
-// per context, outside any stream capture).
-int prepare_kernels() {
-    const int bytes = (7 + kBotScrPerCell) * kBottomSmemCells * (int)sizeof(double);
-    if (cudaFuncSetAttribute(k_bottom<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
-        cudaFuncSetAttribute(k_bottom<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        return MAC_ERR_CUDA;
-    }
-    return MAC_OK;
+    launch_chain(k_bottom<Tio>, dim3(1), dim3(kBottomThreads), 0, s, v, x, f, scratch,
+                 singular ? 1 : 0, nub, eps, max_iter, iter_counter);
 }
 
 template void launch_gsrb<double>(const Dims&, int, LevelArrays<double>&, cudaStream_t, double);

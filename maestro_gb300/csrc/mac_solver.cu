@@ -173,14 +173,15 @@ void vcycle(mac_ctx* c, int l) {
     // rest on plain Gauss-Seidel half-sweeps
     const T omega = std::is_same<T, float>::value ? T(c->o.inner_omega) : T(1);
     const bool gs = omega == T(1);
-    if (l == c->nlevels - 1) {
+    const bool bottom = l == c->nlevels - 1;
+    if (bottom && !c->bottom_cluster) {
         launch_bottom<T>(L.d, L.a64, a.phi, a.f, c->bottom_scratch, c->singular, o.nub,
                          o.bottom_eps, o.bottom_max_iter, c->red.counters, c->stream);
         ++c->issued;
         return;
     }
     const int tslot = std::is_same<T, float>::value ? 1 : 0;
-    if (o.coarse_tail && l == c->tail_start[tslot]) {
+    if (bottom || (o.coarse_tail && l == c->tail_start[tslot])) {
         TailParams<T> tp;
         tp.nlev = c->nlevels - 1 - l;
         for (int q = 0; q < tp.nlev; ++q) {
@@ -212,7 +213,7 @@ void vcycle(mac_ctx* c, int l) {
         tp.iters = c->red.counters;
         tp.binv = std::is_same<T, float>::value && exact_bottom(c) ? c->bot_inv : nullptr;
         tp.omega = omega;
-        launch_tail<T>(tp, c->tail_smem[tslot], c->stream);
+        launch_tail<T>(tp, c->tail_nc, c->stream);
         ++c->issued;
         return;
     }
@@ -496,14 +497,7 @@ int run_solve(mac_ctx* c, mac_stats* st) {
         if (c->o.fused_sweep && c->otf && fused_plan(c) && !c->e_alt &&
             (rc = alloc_arr(c, &c->e_alt, (size_t)F.d.ncell)))
             return rc;
-        if (exact_bottom(c)) {
-            if (!c->inv_pending) {   // (a caller that built the levels some other way)
-                int rc2 = issue_bottom_inverse(c);
-                if (rc2) return rc2;
-            }
-            MAC_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->aux_ev[1], 0));
-            c->inv_pending = false;
-        }
+        if ((rc = wait_bottom_inverse(c))) return rc;
     }
     MAC_CUDA_TRY(cudaMemcpyAsync(c->red.h_scalars, c->red.scalars, 8 * sizeof(double),
                                  cudaMemcpyDeviceToHost, c->stream));
@@ -720,21 +714,26 @@ int ctx_alloc(mac_ctx* c) {
         }
     const Level& B = c->lev[c->nlevels - 1];
     if (B.d.ncell > kBottomMaxCells) return MAC_ERR_UNSUPPORTED;
-    // single-CTA tail plans: from the first level >= 1 that is small enough (FP32 <= 4096 cells,
-    // FP64 <= 512: one SM's FP64 rate) and whose tail fits in shared memory
+    // Cluster tail plans: from the first level >= 1 with at most 32768 cells (FP32) / 16384 (FP64)
+    // that fits the cluster.  The limits are where a half-sweep on the cluster's 16 SMs stops being
+    // shorter than a kernel launch over the whole chip (2-3 us): FP64 by the 16 SMs' issue rate,
+    // FP32 by two pairs of cells a thread.
+    c->bottom_cluster = tail_fits<double>(nullptr, 0, B.d, false, c->tail_nc);
+    const bool small_bottom = B.d.ncell <= kDenseBottomMax;
     for (int slot = 0; slot < 2; ++slot) {
-        const int limit = slot ? 4096 : 512;
+        const int limit = slot ? 32768 : 16384;
         c->tail_start[slot] = -1;
-        if (B.d.ncell > 4096) continue;
         for (int l = 1; l < c->nlevels - 1; ++l) {
-            if (c->lev[l].d.ncell > limit || c->nlevels - 1 - l > kTailMaxLevels) continue;
+            const int nl = c->nlevels - 1 - l;
+            if (c->lev[l].d.ncell > limit || nl > kTailMaxLevels) continue;
             Dims ds[kTailMaxLevels];
-            for (int q = 0; q < c->nlevels - 1 - l; ++q) ds[q] = c->lev[l + q].d;
-            const size_t bytes = slot ? tail_smem_bytes<float>(ds, c->nlevels - 1 - l, B.d)
-                                      : tail_smem_bytes<double>(ds, c->nlevels - 1 - l, B.d);
-            if (bytes > (size_t)kTailSmemMax) continue;
+            for (int q = 0; q < nl; ++q) ds[q] = c->lev[l + q].d;
+            bool fits = true;
+            for (int ex = 0; ex <= (small_bottom ? 1 : 0); ++ex)
+                fits = fits && (slot ? tail_fits<float>(ds, nl, B.d, ex, c->tail_nc)
+                                     : tail_fits<double>(ds, nl, B.d, ex, c->tail_nc));
+            if (!fits) continue;
             c->tail_start[slot] = l;
-            c->tail_smem[slot] = bytes;
             break;
         }
     }
@@ -982,6 +981,16 @@ int issue_bottom_inverse(mac_ctx* c) {
     c->inv_pending = true;
     return MAC_OK;
 }
+int wait_bottom_inverse(mac_ctx* c) {
+    if (c->o.precision != MAC_PREC_MIXED || !exact_bottom(c)) return MAC_OK;
+    if (!c->inv_pending) {   // (a caller that built the levels some other way)
+        int rc = issue_bottom_inverse(c);
+        if (rc) return rc;
+    }
+    MAC_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->aux_ev[1], 0));
+    c->inv_pending = false;
+    return MAC_OK;
+}
 int load_beta0(mac_ctx* c, int ptr_kind, const double* b0, const double* b0e) {
     return load_beta0_impl(c, ptr_kind, b0, b0e);
 }
@@ -1091,8 +1100,7 @@ int mac_ctx_create(mac_ctx** out, const mac_geom* g, const mac_opts* o, void* cu
         delete c;
         return MAC_ERR_UNSUPPORTED;
     }
-    rc = prepare_kernels();
-    if (!rc) rc = prepare_tail_kernels();
+    rc = prepare_tail_kernels(&c->tail_nc);
     if (!rc) rc = ctx_alloc(c);
     if (rc) {
         ctx_free(c);

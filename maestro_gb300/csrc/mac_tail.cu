@@ -1,116 +1,321 @@
-// Single-CTA "tail" of the V-cycle: every level from the first one small enough to live in
-// shared memory down to the bottom solve runs inside one kernel, so the smallest levels no
-// longer pay one kernel launch per half-sweep.  The arithmetic is the multi-kernel V-cycle's,
-// operation for operation (same fused-multiply-add order per cell, same child order in the
-// restriction, same separable trilinear prolongation, the same single-warp bottom solve), so the
-// result is bitwise the same; only the data lives in shared memory in natural layout.
+// Cluster "tail" of the V-cycle: every level from the first one small enough down to the bottom
+// solve runs inside one kernel, on one thread-block cluster whose CTAs share the levels through
+// distributed shared memory, so the small levels pay a cluster barrier instead of a kernel launch
+// per half-sweep.  The arithmetic is the multi-kernel V-cycle's, operation for operation (same
+// fused-multiply-add order per cell, same child order in the restriction, same separable
+// trilinear prolongation, the same bottom solver), so the result is bitwise the same.
+//
+// What bounds it: latency.  On GB300 a cluster barrier takes ~380 cycles (256 threads a CTA), a
+// dependent distributed-shared-memory load ~240, a block barrier 20-80, and an SM sub-partition
+// issues one FP64 warp instruction per 64 cycles; a launch-chained half-sweep kernel takes 2-3 us.
+// So
+//  * a level's rows are spread over all CTAs; a thread owns one or two pairs of x-neighbours (one
+//    cell of each colour) for a whole visit of the level, their operator, right-hand side and
+//    neighbour addresses in registers; only e and the defects are in (distributed) shared memory;
+//  * levels of at most kReplCells<T> cells and the exactly solved bottom are computed by every CTA
+//    alone: block barriers only (above that the FP64 rate, or the work, of one SM costs more than
+//    the cluster barriers saved);
+//  * the first red half-sweep of a level starts from a zero correction, so it reads no neighbour.
+// Measured against the one-CTA tail and bottom it replaces (whole calls): 128^2 FP64 1427 -> 1116
+// us, 64^3 mixed 1316 -> 1131 us, 160x96x112 FP64 (a bottom of 3360 cells, 14 bottom solves) 20.8 ->
+// 7.1 ms, 256^3 mixed 6.99 -> 6.87 ms.
 #include "mac_internal.cuh"
 #include "mac_bottom.cuh"
 
 namespace mac {
 namespace {
 
-constexpr int kTailThreads = 1024;
+constexpr int kInvThreads = 1024;
+constexpr int kClusterMax = 16;          // CTAs of the tail cluster (16: opt-in size; fallback 8)
+constexpr int kTailMaxThreads = 512;
+constexpr int kTailItems = 2;            // pairs of cells a thread at most
+constexpr int kOps = 17;                 // operator values of a pair in shared memory
+template <typename T>
+constexpr int kReplCells = sizeof(T) == 4 ? 512 : 128;
 
 __device__ __forceinline__ double fmaT2(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float fmaT2(float a, float b, float c) { return fmaf(a, b, c); }
 
+// x / d for x d < 2^32 with m = floor(2^32 / d) + 1 (d > 1; d == 1 is m = 0)
+__host__ __device__ __forceinline__ unsigned div_magic(unsigned d) {
+    return d > 1 ? (unsigned)(0x100000000ull / d) + 1u : 0u;
+}
+__device__ __forceinline__ unsigned fdiv(unsigned x, unsigned m) { return m ? __umulhi(x, m) : x; }
+
+// ---- cluster primitives -----------------------------------------------------------------------
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ unsigned cluster_size() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::
+                     : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() {
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned smem_u32(const void* p) {
+    return (unsigned)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ unsigned mapa(unsigned a, unsigned cta) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(cta));
+    return r;
+}
+__device__ __forceinline__ float ld_cluster(unsigned a, float) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ double ld_cluster(unsigned a, double) {
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void st_cluster(unsigned a, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void st_cluster(unsigned a, double v) {
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void sync_level(bool repl) {
+    if (repl)
+        __syncthreads();
+    else
+        cluster_sync();
+}
+
+// A level as this CTA sees it: its share of the rows (row = j + n1 k), or all of them (repl).
+struct Geo {
+    int n0, n1, n2, rz, hn0;
+    int row0, rows, repl;
+    unsigned cpc, mcpc, mn1, mhn0;
+    unsigned ea, ra;   // shared addresses of e and r, index i + n0 (row - row0)
+    int pairs;         // pairs per CTA: stride of the operator arrays
+    int nops;          // byte offset of the operator arrays in the dynamic shared memory
+};
 template <typename T>
-struct TailLevel {
-    int n0, n1, n2, N, rz;
-    T *e, *f, *bx, *by, *bz, *dg, *idg;   // shared memory, natural layout
+__device__ __forceinline__ Geo geo_of(const TailParams<T>& P, int l, unsigned rank, unsigned smem) {
+    const TailGeo& q = P.geo[l];
+    const Dims& D = P.lev[l];
+    Geo g;
+    g.n0 = D.n0;
+    g.n1 = D.n1;
+    g.n2 = D.n2;
+    g.rz = D.rz;
+    g.hn0 = D.n0 >> 1;
+    g.repl = q.repl;
+    const int R = D.n1 * D.n2;
+    g.row0 = q.repl ? 0 : min(R, (int)rank * q.rpc);
+    g.rows = min(R - g.row0, q.rpc);
+    g.cpc = q.rpc * D.n0;
+    g.mcpc = q.mcpc;
+    g.mn1 = q.mn1;
+    g.mhn0 = q.mhn0;
+    g.ea = smem + q.off;
+    g.ra = g.ea + g.cpc * (unsigned)sizeof(T);
+    g.pairs = q.rpc * g.hn0;
+    g.nops = q.off + 2 * (int)(g.cpc * sizeof(T));
+    return g;
+}
+
+// Shared (cluster) address of entry lin of an array of the level (its local address: base).
+template <typename T>
+__device__ __forceinline__ unsigned addr_of(const Geo& g, unsigned base, unsigned lin) {
+    if (g.repl) return base + lin * (unsigned)sizeof(T);
+    const unsigned cta = fdiv(lin, g.mcpc);
+    return mapa(base + (lin - cta * g.cpc) * (unsigned)sizeof(T), cta);
+}
+
+// A pair of x-neighbours of one row; index s: 0 the colour-0 cell, 1 the colour-1 cell.
+template <typename T>
+struct Pair {
+    bool on;
+    int p;              // position (0: cell 2h, 1: cell 2h + 1) of the colour-0 cell
+    T c[2][6];          // low/high face coefficients: x-, x+, y-, y+, z-, z+
+    T id[2], f[2], e[2];
+    unsigned own, xm[2], xp[2];   // shared addresses: cell 2h of e; the x-neighbours outside ...
+    unsigned row[4];    // cell 2h of the rows y-, y+, z-, z+ (cluster addresses)
 };
 
+// Operator arrays of a pair (stride g.pairs): bx of cells 2h, 2h+1, 2h+2, then by, by+, bz, bz+,
+// 1/diag, diag, f of the two cells.
+enum { kBx = 0, kBy = 3, kByp = 5, kBz = 7, kBzp = 9, kId = 11, kDg = 13, kF = 15 };
+
+template <typename T, bool Z3>
+__device__ __forceinline__ void load_pair(Pair<T>& q, const Geo& g, const T* ops, int t) {
+    q.on = t < g.rows * g.hn0;
+    if (!q.on) return;
+    const int lr = fdiv(t, g.mhn0), h = t - lr * g.hn0;
+    const int row = g.row0 + lr, k = fdiv(row, g.mn1), j = row - k * g.n1;
+    const int p = (j + k) & 1;
+    q.p = p;
+    const int S = g.pairs;
+    const T* o = ops + t;
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        const int a = s ? 1 - p : p;   // position of the colour-s cell
+        q.c[s][0] = o[(kBx + a) * S];
+        q.c[s][1] = o[(kBx + a + 1) * S];
+        q.c[s][2] = o[(kBy + a) * S];
+        q.c[s][3] = o[(kByp + a) * S];
+        q.c[s][4] = o[(kBz + a) * S];
+        q.c[s][5] = o[(kBzp + a) * S];
+        q.id[s] = o[(kId + a) * S];
+        q.f[s] = o[(kF + a) * S];
+    }
+    constexpr unsigned z = sizeof(T);
+    const unsigned base = g.ea + (unsigned)(lr * g.n0) * z;
+    q.own = base + 2 * h * z;
+    const unsigned lo = base + (h == 0 ? g.n0 - 1 : 2 * h - 1) * z;          // left of cell 2h
+    const unsigned hi = base + (h == g.hn0 - 1 ? 0 : 2 * h + 2) * z;         // right of cell 2h+1
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        const int a = s ? 1 - p : p;
+        q.xm[s] = a ? q.own : lo;
+        q.xp[s] = a ? hi : q.own + z;
+    }
+    const int jm = j == 0 ? g.n1 - 1 : j - 1, jp = j == g.n1 - 1 ? 0 : j + 1;
+    const int km = k == 0 ? g.n2 - 1 : k - 1, kp = k == g.n2 - 1 ? 0 : k + 1;
+    q.row[0] = addr_of<T>(g, g.ea, 2 * h + g.n0 * (jm + g.n1 * k));
+    q.row[1] = addr_of<T>(g, g.ea, 2 * h + g.n0 * (jp + g.n1 * k));
+    if (Z3) {
+        q.row[2] = addr_of<T>(g, g.ea, 2 * h + g.n0 * (j + g.n1 * km));
+        q.row[3] = addr_of<T>(g, g.ea, 2 * h + g.n0 * (j + g.n1 * kp));
+    }
+}
+
 template <typename T>
-__device__ __forceinline__ T arms_nat(T acc, const TailLevel<T>& L, const T* __restrict__ u, int i,
-                                      int j, int k, int c) {
-    const int im = i == 0 ? L.n0 - 1 : i - 1, ip = i == L.n0 - 1 ? 0 : i + 1;
-    const int jm = j == 0 ? L.n1 - 1 : j - 1, jp = j == L.n1 - 1 ? 0 : j + 1;
-    const int km = k == 0 ? L.n2 - 1 : k - 1, kp = k == L.n2 - 1 ? 0 : k + 1;
-    const int cxm = im + L.n0 * (j + L.n1 * k), cxp = ip + L.n0 * (j + L.n1 * k);
-    const int cym = i + L.n0 * (jm + L.n1 * k), cyp = i + L.n0 * (jp + L.n1 * k);
-    const int czm = i + L.n0 * (j + L.n1 * km), czp = i + L.n0 * (j + L.n1 * kp);
-    acc = fmaT2(L.bx[c], u[cxm], acc);
-    acc = fmaT2(L.bx[cxp], u[cxp], acc);
-    acc = fmaT2(L.by[c], u[cym], acc);
-    acc = fmaT2(L.by[cyp], u[cyp], acc);
-    acc = fmaT2(L.bz[c], u[czm], acc);
-    acc = fmaT2(L.bz[czp], u[czp], acc);
+__device__ __forceinline__ void sts(unsigned a, T v);
+template <>
+__device__ __forceinline__ void sts<float>(unsigned a, float v) {
+    asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+template <>
+__device__ __forceinline__ void sts<double>(unsigned a, double v) {
+    asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+
+// acc + the six arms (x-, x+, y-, y+, z-, z+) of the pair's colour-s cell; a 2-D level has no z arm
+template <typename T, bool Z3>
+__device__ __forceinline__ T arms(T acc, const Pair<T>& q, int s) {
+    const unsigned o = (s ? 1 - q.p : q.p) * (unsigned)sizeof(T);
+    const T u0 = ld_cluster(q.xm[s], T(0)), u1 = ld_cluster(q.xp[s], T(0));
+    const T u2 = ld_cluster(q.row[0] + o, T(0)), u3 = ld_cluster(q.row[1] + o, T(0));
+    T u4 = T(0), u5 = T(0);
+    if (Z3) {
+        u4 = ld_cluster(q.row[2] + o, T(0));
+        u5 = ld_cluster(q.row[3] + o, T(0));
+    }
+    acc = fmaT2(q.c[s][0], u0, acc);
+    acc = fmaT2(q.c[s][1], u1, acc);
+    acc = fmaT2(q.c[s][2], u2, acc);
+    acc = fmaT2(q.c[s][3], u3, acc);
+    if (Z3) {
+        acc = fmaT2(q.c[s][4], u4, acc);
+        acc = fmaT2(q.c[s][5], u5, acc);
+    }
     return acc;
 }
 
-// Thread layout over an (nx, rows) index space: tx strides x, ty strides the rows (row =
-// j + n1 k, decoded incrementally), so no per-cell integer division.
-struct Lanes {
-    int tx, ty, TX, RY;
-};
-__device__ __forceinline__ Lanes lanes(int nx) {
-    Lanes q;
-    q.TX = nx < 32 ? nx : 32;
-    q.tx = threadIdx.x % q.TX;
-    q.ty = threadIdx.x / q.TX;
-    q.RY = blockDim.x / q.TX;
-    return q;
-}
-
 template <typename T>
-__device__ __noinline__ void tail_sweep(const TailLevel<T>& L, T omega) {
-    const int hn0 = L.n0 >> 1, rows = L.n1 * L.n2;
-    const Lanes q = lanes(hn0);
-    for (int colour = 0; colour < 2; ++colour) {
-        if (q.ty < q.RY) {
-            int j = q.ty % L.n1, k = q.ty / L.n1;
-            const int dj = q.RY % L.n1, dk = q.RY / L.n1;
-            for (int row = q.ty; row < rows; row += q.RY) {
-                const int s = (colour + j + k) & 1;
-                for (int h = q.tx; h < hn0; h += q.TX) {
-                    const int i = 2 * h + s;
-                    const int c = i + L.n0 * row;
-                    const T acc = arms_nat<T>(L.f[c], L, L.e, i, j, k, c);
-                    if (omega != T(1))
-                        L.e[c] = fmaT2(omega, acc * L.idg[c] - L.e[c], L.e[c]);
-                    else
-                        L.e[c] = acc * L.idg[c];
-                }
-                j += dj;
-                k += dk;
-                if (j >= L.n1) {
-                    j -= L.n1;
-                    ++k;
-                }
+__device__ __forceinline__ void store_e(const Pair<T>& q, int s) {
+    sts<T>(q.own + (s ? 1 - q.p : q.p) * (unsigned)sizeof(T), q.e[s]);
+}
+
+// nu sweeps.  zero: from e = 0 -- the first colour-0 half-sweep has no arm that contributes.
+// (A predicated-off FP64 instruction still takes its pipe's 64 cycles: the dimension is a template
+// parameter, and FP64 levels are never over-relaxed.)
+template <typename T, int K, bool Z3>
+__device__ __forceinline__ void sweeps(Pair<T> (&q)[K], const Geo& g, int nu, T omega, bool zero) {
+    const bool sor = sizeof(T) == 4 && omega != T(1);
+    if (zero) {
+#pragma unroll
+        for (int m = 0; m < K; ++m) {
+            q[m].e[0] = q[m].e[1] = T(0);
+            if (nu == 0 && q[m].on) {
+                store_e(q[m], 0);
+                store_e(q[m], 1);
             }
         }
-        __syncthreads();
+        if (nu == 0) sync_level(g.repl);
+    }
+    for (int it = 0; it < nu; ++it) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+#pragma unroll
+            for (int m = 0; m < K; ++m) {
+                if (!q[m].on) continue;
+                T acc = q[m].f[s];
+                if (!(zero && it == 0 && s == 0)) acc = arms<T, Z3>(acc, q[m], s);
+                if (sor)
+                    q[m].e[s] = fmaT2(omega, fmaT2(acc, q[m].id[s], -q[m].e[s]), q[m].e[s]);
+                else
+                    q[m].e[s] = acc * q[m].id[s];
+                store_e(q[m], s);
+            }
+            sync_level(g.repl);
+        }
     }
 }
 
-// defect of level F restricted into out[coarse natural index] (as T, then converted to To)
-template <typename T, typename To>
-__device__ __noinline__ void tail_restrict(const TailLevel<T>& F, int cn0, int cn1, int cn2, To* out,
-                              bool red_only) {
-    const Lanes ln = lanes(cn0);
-    const int rows = cn1 * cn2;
-    for (int crow = ln.ty; ln.ty < ln.RY && crow < rows; crow += ln.RY)
-    for (int I = ln.tx; I < cn0; I += ln.TX) {
-        const int J = crow % cn1, K = crow / cn1;
-        const int q = I + cn0 * crow;
-        T sum = T(0);
-        for (int b = 0; b < F.rz; ++b) {
-            for (int a = 0; a < 2; ++a) {
-                const int j = 2 * J + a;
-                const int k = F.rz == 2 ? 2 * K + b : K;
-                for (int colour = 0; colour < (red_only ? 1 : 2); ++colour) {
-                    const int i = 2 * I + ((colour + j + k) & 1);
-                    const int c = i + F.n0 * (j + F.n1 * k);
-                    T r = fmaT2(-F.dg[c], F.e[c], F.f[c]);
-                    r = arms_nat<T>(r, F, F.e, i, j, k, c);
-                    sum += r;
-                }
-            }
+// One level down: sweeps from e = 0 and the defects (colour 0 only after a plain Gauss-Seidel
+// black half-sweep) into r.
+template <typename T, int K, bool Z3>
+__device__ __forceinline__ void visit_down(const TailParams<T>& P, int l, unsigned rank, unsigned char* sm,
+                                        bool red_only) {
+    const Geo g = geo_of<T>(P, l, rank, smem_u32(sm));
+    const T* ops = reinterpret_cast<const T*>(sm + g.nops);
+    Pair<T> q[K];
+#pragma unroll
+    for (int m = 0; m < K; ++m) load_pair<T, Z3>(q[m], g, ops, threadIdx.x + m * blockDim.x);
+    sweeps<T, K, Z3>(q, g, P.nu1, P.omega, true);
+    const unsigned dr = g.ra - g.ea;
+#pragma unroll
+    for (int m = 0; m < K; ++m) {
+        if (!q[m].on) continue;
+        for (int s = 0; s < (red_only ? 1 : 2); ++s) {
+            const int a = s ? 1 - q[m].p : q[m].p;
+            const T dg = ops[(kDg + a) * g.pairs + threadIdx.x + m * blockDim.x];
+            const T e = s ? q[m].e[1] : q[m].e[0], f = s ? q[m].f[1] : q[m].f[0];
+            const T r0 = fmaT2(-dg, e, f);
+            const T r = s ? arms<T, Z3>(r0, q[m], 1) : arms<T, Z3>(r0, q[m], 0);
+            sts<T>(q[m].own + dr + a * (unsigned)sizeof(T), r);
         }
-        out[q] = (To)(sum * (T)(1.0 / (4 * F.rz)));
     }
-    __syncthreads();
+    sync_level(g.repl);
+}
+
+// the restricted defect of coarse cell (I, J, K): the mean of its children's, in the order of the
+// multi-kernel restriction
+template <typename T, bool Z3>
+__device__ __forceinline__ T restricted(const Geo& F, int I, int J, int K, bool red_only) {
+    constexpr int rz = Z3 ? 2 : 1;
+    T v[8];
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {
+            if (b >= rz) continue;
+            const int j = 2 * J + a, k = Z3 ? 2 * K + b : K, s = (j + k) & 1;
+            const unsigned at = addr_of<T>(F, F.ra, 2 * I + F.n0 * (j + F.n1 * k));
+            v[(b * 2 + a) * 2] = ld_cluster(at + s * (unsigned)sizeof(T), T(0));
+            if (!red_only) v[(b * 2 + a) * 2 + 1] = ld_cluster(at + (1 - s) * (unsigned)sizeof(T), T(0));
+        }
+    T sum = T(0);
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+        if ((q >> 2) < rz && !(red_only && (q & 1))) sum += v[q];
+    return sum * (T)(1.0 / (4 * rz));
 }
 
 template <typename T>
@@ -131,244 +336,572 @@ __device__ __forceinline__ void nb_w(int q, int n, int blo, int bhi, int& qm, in
     }
 }
 
-// e_fine += trilinear interpolation of the coarse correction ec (natural, cn0 x cn1 x cn2)
-// black_only: colour-1 children only (post-smoothing follows; see k_prolong_add)
+// Where the coarse correction lies: level l + 1's e, or the bottom's (own CTA, or M cells a CTA).
 template <typename T>
-__device__ __noinline__ void tail_prolong(const TailLevel<T>& F, const T* ec, int cn0, int cn1, int cn2,
-                             const BcDesc& bc, bool black_only) {
-    const bool z2 = F.rz == 2;
-    const Lanes ln = lanes(cn0);
-    const int rows = cn1 * cn2;
-    for (int crow = ln.ty; ln.ty < ln.RY && crow < rows; crow += ln.RY)
-    for (int I = ln.tx; I < cn0; I += ln.TX) {
-        const int J = crow % cn1, K = crow / cn1;
-        int xs[3], ys[3], zs[3];
-        T wxm, wxp, wym, wyp, wzm = T(0), wzp = T(0);
-        xs[1] = I;
-        ys[1] = J;
-        zs[1] = K;
-        nb_w<T>(I, cn0, bc.lo[0], bc.hi[0], xs[0], xs[2], wxm, wxp);
-        nb_w<T>(J, cn1, bc.lo[1], bc.hi[1], ys[0], ys[2], wym, wyp);
-        if (z2) nb_w<T>(K, cn2, bc.lo[2], bc.hi[2], zs[0], zs[2], wzm, wzp);
-        T Yv[3][2][2];
-        for (int a = 0; a < 3; ++a) {
-            const int X = xs[a];
-            T Zv[3][2];
-            for (int b = 0; b < 3; ++b) {
-                const int Y = ys[b];
-                const T c0 = ec[X + cn0 * (Y + cn1 * K)];
-                if (z2) {
-                    const T t = T(0.75) * c0;
-                    Zv[b][0] = fmaT2(wzm, ec[X + cn0 * (Y + cn1 * zs[0])], t);
-                    Zv[b][1] = fmaT2(wzp, ec[X + cn0 * (Y + cn1 * zs[2])], t);
-                } else {
-                    Zv[b][0] = c0;
-                    Zv[b][1] = c0;
-                }
-            }
-            for (int zc = 0; zc < 2; ++zc) {
-                const T t = T(0.75) * Zv[1][zc];
-                Yv[a][0][zc] = fmaT2(wym, Zv[0][zc], t);
-                Yv[a][1][zc] = fmaT2(wyp, Zv[2][zc], t);
-            }
-        }
-        for (int zc = 0; zc < (z2 ? 2 : 1); ++zc) {
-            for (int yc = 0; yc < 2; ++yc) {
-                const T t = T(0.75) * Yv[1][yc][zc];
-                const int j = 2 * J + yc;
-                const int k = z2 ? 2 * K + zc : K;
-                const int base = F.n0 * (j + F.n1 * k) + 2 * I;
-                const int c0 = (yc + zc) & 1;   // colour of child 2I
-                if (!black_only || c0) F.e[base] += fmaT2(wxm, Yv[0][yc][zc], t);
-                if (!black_only || !c0) F.e[base + 1] += fmaT2(wxp, Yv[2][yc][zc], t);
-            }
-        }
+struct Coarse {
+    Geo g;
+    unsigned base;
+    __device__ __forceinline__ T operator()(int c) const {
+        return ld_cluster(addr_of<T>(g, base, (unsigned)c), T(0));
     }
-    __syncthreads();
+};
+
+// One level up: e += trilinear interpolation of the coarse correction, then the sweeps.
+// black_only: colour-1 cells only (plain Gauss-Seidel post-smoothing follows; see k_prolong_add).
+template <typename T, int K, bool Z3>
+__device__ __forceinline__ void visit_up(const TailParams<T>& P, int l, unsigned rank, unsigned char* sm,
+                                      const Coarse<T>& ec, int cn1, int cn2, bool black_only) {
+    const Geo g = geo_of<T>(P, l, rank, smem_u32(sm));
+    const T* ops = reinterpret_cast<const T*>(sm + g.nops);
+    const int cn0 = g.hn0;
+    // a row's pairs lie in one warp: the neighbouring coarse columns come from its lanes
+    const bool lanes = cn0 <= 32 && (cn0 & (cn0 - 1)) == 0;
+    Pair<T> q[K];
+#pragma unroll
+    for (int m = 0; m < K; ++m) {
+        const int t = threadIdx.x + m * blockDim.x;
+        load_pair<T, Z3>(q[m], g, ops, t);
+        const int tt = q[m].on ? t : 0;   // (idle lanes stay for the shuffles)
+        const int lr = fdiv(tt, g.mhn0), I = tt - lr * g.hn0;
+        const int row = min(g.row0 + lr, g.n1 * g.n2 - 1);   // (a CTA may own no row)
+        const int k = fdiv(row, g.mn1), j = row - k * g.n1;
+        const int J = j >> 1, Kc = Z3 ? k >> 1 : k;
+        int xs[3], qq[2];
+        T wx[2], w[2];
+        xs[1] = I;
+        nb_w<T>(I, cn0, P.bc.lo[0], P.bc.hi[0], xs[0], xs[2], wx[0], wx[1]);
+        nb_w<T>(J, cn1, P.bc.lo[1], P.bc.hi[1], qq[0], qq[1], w[0], w[1]);
+        const int Yn = j & 1 ? qq[1] : qq[0];
+        const T wy = j & 1 ? w[1] : w[0];
+        int Zn = Kc;
+        T wz = T(0);
+        if (Z3) {
+            nb_w<T>(Kc, cn2, P.bc.lo[2], P.bc.hi[2], qq[0], qq[1], w[0], w[1]);
+            Zn = k & 1 ? qq[1] : qq[0];
+            wz = k & 1 ? w[1] : w[0];
+        }
+        const int r00 = cn0 * (J + cn1 * Kc), r10 = cn0 * (Yn + cn1 * Kc);
+        const int r01 = cn0 * (J + cn1 * Zn), r11 = cn0 * (Yn + cn1 * Zn);
+        // coarse column X interpolated in z, then y
+        auto column = [&](int X) -> T {
+            T zc = ec(X + r00), zn = ec(X + r10);
+            if (Z3) {
+                const T pc = ec(X + r01), pn = ec(X + r11);
+                zc = fmaT2(wz, pc, T(0.75) * zc);
+                zn = fmaT2(wz, pn, T(0.75) * zn);
+            }
+            return fmaT2(wy, zn, T(0.75) * zc);
+        };
+        T Y[3];
+        Y[1] = column(I);
+        if (lanes) {
+            const int l0 = (threadIdx.x & 31) - I;
+            Y[0] = __shfl_sync(0xffffffffu, Y[1], l0 + xs[0]);
+            Y[2] = __shfl_sync(0xffffffffu, Y[1], l0 + xs[2]);
+        } else {
+            Y[0] = column(xs[0]);
+            Y[2] = column(xs[2]);
+        }
+        if (!q[m].on) continue;
+        const T mid = T(0.75) * Y[1];
+        const T d0 = fmaT2(wx[0], Y[0], mid), d1 = fmaT2(wx[1], Y[2], mid);   // cells 2I, 2I + 1
+        const int p = q[m].p;
+        const unsigned z = sizeof(T);
+        const T e0 = ld_cluster(q[m].own + p * z, T(0)), e1 = ld_cluster(q[m].own + (1 - p) * z, T(0));
+        q[m].e[0] = black_only ? e0 : e0 + (p ? d1 : d0);
+        q[m].e[1] = e1 + (p ? d0 : d1);
+        if (!black_only) store_e(q[m], 0);
+        store_e(q[m], 1);
+    }
+    sync_level(g.repl);
+    sweeps<T, K, Z3>(q, g, P.nu2, P.omega, false);
 }
 
 // Asynchronous 4/8-byte global -> shared copy (cp.async); completed by cp_async_wait().
 template <typename T>
 __device__ __forceinline__ void cp_async(T* dst, const T* src) {
     static_assert(sizeof(T) == 4 || sizeof(T) == 8, "4 or 8 bytes");
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
-                     (unsigned)__cvta_generic_to_shared(dst)),
-                 "l"(src), "n"(sizeof(T))
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src),
+                 "n"(sizeof(T))
                  : "memory");
 }
 __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.commit_group;\ncp.async.wait_all;" ::: "memory");
 }
 
-// Visit every cell of a checkerboard-split level once: fn(g, c) with g the split-layout
-// (global) index and c the natural (shared-memory) index; rows decoded incrementally, no
-// per-cell integer division.
-template <class Fn>
-__device__ __forceinline__ void for_split_cells(const Dims& D, Fn fn) {
-    const Lanes q = lanes(D.hn0);
-    if (q.ty >= q.RY) return;
-    const int rows = D.n1 * D.n2;
-    int j = q.ty % D.n1, k = q.ty / D.n1;
-    const int dj = q.RY % D.n1, dk = q.RY / D.n1;
-    for (int row = q.ty; row < rows; row += q.RY) {
-        for (int colour = 0; colour < 2; ++colour) {
-            const int s = (colour + j + k) & 1;
-            for (int h = q.tx; h < D.hn0; h += q.TX)
-                fn(colour * D.half + row * D.hn0 + h, 2 * h + s + D.n0 * row);
+// ---- bottom: Gauss-Seidel sweeps and BiCGStab over the cluster -------------------------------
+// The coarsest level's cells in linear order, M consecutive ones a CTA, one a thread: its operator
+// row, its entries of every vector and its neighbours' addresses are registers; x and y, which
+// neighbours read, are in distributed shared memory.  nub red/black sweeps, Jacobi-preconditioned
+// BiCGStab reducing ||f - A x||_inf by eps, nub sweeps (FBoxLib's bottom, Docs/mg/mg.tex:221-249)
+// with f_c / diag_c + sum_n gc_n x_n as the Gauss-Seidel update (gc_n = a_n / diag).  A warp's
+// cells have one colour (odd rows excepted), so a half-sweep issues half the FP64 instructions.
+struct ClBottom {
+    int N;
+    bool on, odd;            // a cell here; a periodic extent is odd (same-colour neighbours)
+    int colour;
+    unsigned nb[6];          // cluster addresses of the neighbours' x
+    unsigned xa, yoff;       // own x; byte distance from x to y
+    double gc[6], dg, id;
+};
+
+// Cluster-wide sums v[0..NS) and the maximum of the key in a fixed order; fin(sums, key, out)
+// forms the scalars that follow from them in one thread a CTA (an FP64 instruction costs a
+// sub-partition 64 cycles for every warp that issues it).  Every thread gets R.out.  The slots
+// alternate between calls, so one is rewritten only after a later cluster barrier.
+struct ClReduce {
+    double ws[4][kTailMaxThreads];
+    unsigned long long wk[kTailMaxThreads];
+    double slot[2][5][kClusterMax];
+    double tot[5];
+    double out[4];
+};
+template <int NS, class Fin>
+__device__ __forceinline__ void cl_reduce(ClReduce& R, int& parity, const double (&v)[NS],
+                                          unsigned long long key, int nw, Fin fin) {
+    static_assert(NS <= 4, "four sums");
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (w < nw) {
+#pragma unroll
+        for (int s = 0; s < NS; ++s) R.ws[s][threadIdx.x] = v[s];
+        R.wk[threadIdx.x] = key;
+    }
+    __syncthreads();
+    const unsigned nc = cluster_size(), rank = cluster_rank();
+    constexpr int kw = NS < 4 ? NS : 0;   // the warp that takes the key
+    if (w < NS) {
+        double s = R.ws[w][lane];
+        for (int i = 1; i < nw; ++i) s += R.ws[w][32 * i + lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane < (int)nc) st_cluster(mapa(smem_u32(&R.slot[parity][w][rank]), lane), s);
+    }
+    if (w == kw) {
+        unsigned long long k = R.wk[lane];
+        for (int i = 1; i < nw; ++i) {
+            const unsigned long long q = R.wk[32 * i + lane];
+            k = q > k ? q : k;
         }
-        j += dj;
-        k += dk;
-        if (j >= D.n1) {
-            j -= D.n1;
-            ++k;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long q = __shfl_xor_sync(0xffffffffu, k, o);
+            k = q > k ? q : k;
+        }
+        if (lane < (int)nc)
+            st_cluster(mapa(smem_u32(&R.slot[parity][4][rank]), lane), __longlong_as_double((long long)k));
+    }
+    cluster_sync();
+    if (w < NS) {
+        double s = lane < (int)nc ? R.slot[parity][w][lane] : 0.0;
+#pragma unroll
+        for (int o = kClusterMax / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) R.tot[w] = s;
+    }
+    if (w == kw) {
+        unsigned long long k =
+            lane < (int)nc ? (unsigned long long)__double_as_longlong(R.slot[parity][4][lane]) : 0ull;
+#pragma unroll
+        for (int o = kClusterMax / 2; o > 0; o >>= 1) {
+            const unsigned long long q = __shfl_xor_sync(0xffffffffu, k, o);
+            k = q > k ? q : k;
+        }
+        if (lane == 0) R.tot[4] = __longlong_as_double((long long)k);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) fin(R.tot, R.tot[4], R.out);
+    __syncthreads();
+    parity ^= 1;
+}
+
+__device__ __forceinline__ double cl_gsum(const ClBottom& B, unsigned off, double s, bool neg) {
+    double u[6];
+#pragma unroll
+    for (int n = 0; n < 6; ++n) u[n] = ld_cluster(B.nb[n] + off, 0.0);
+#pragma unroll
+    for (int n = 0; n < 6; ++n) s = fma(neg ? -B.gc[n] : B.gc[n], u[n], s);
+    return s;
+}
+
+// nu red/black sweeps on x (register x, published).  Where a periodic extent is odd, same-colour
+// cells neighbour each other: they are updated from each other's old values.
+__device__ __forceinline__ double cl_gsrb(const ClBottom& B, double fi, double x, int nu) {
+    for (int it = 0; it < 2 * nu; ++it) {
+        const bool act = B.on && B.colour == (it & 1);
+        if (act) x = cl_gsum(B, 0, fi, false);
+        if (B.odd) cluster_sync();
+        if (act) sts<double>(B.xa, x);
+        cluster_sync();
+    }
+    return x;
+}
+
+// Solves for x (in: the guess, already published at B.xa by every owner); f's mean comes off when
+// singular.  Every CTA of the cluster runs the same control flow.
+__device__ __noinline__ double cl_solve(const ClBottom& bottom, ClReduce& R, double f, double x, int nw,
+                                        int singular, int nub, double eps, int max_iter, int* iters) {
+    const ClBottom B = bottom;   // (registers)
+    int parity = 0;
+    const unsigned ya = B.xa + B.yoff;
+    {
+        const double v[1] = {B.on ? f : 0.0};
+        cl_reduce<1>(R, parity, v, 0ull, nw, [&](const double* t, double, double* o) {
+            o[0] = singular ? t[0] / B.N : 0.0;
+        });   // (its barrier also publishes x)
+    }
+    if (singular && B.on) f -= R.out[0];
+    const double fi = B.on ? f * B.id : 0.0;
+    x = cl_gsrb(B, fi, x, nub);
+    double r = 0.0, dx = 0.0;
+    if (B.on) {
+        r = f - B.dg * cl_gsum(B, 0, x, true);
+        dx = B.dg * x;
+    }
+    const double rh = r;
+    double p = 0.0, vv = 0.0, rho, beta, omega = 1.0, alpha = 1.0, tol, low;
+    {
+        const double v[2] = {B.on ? r * r : 0.0, B.on ? fma(f, f, dx * dx) : 0.0};
+        // [0] rho = (rh, r) and the first beta (rho_old = alpha = omega = 1); [1] ||r||;  [2] the
+        // rounding level of f - A x: a residual that small (the sweeps alone solved the bottom, or
+        // a singular one's right-hand side keeps a rounded mean) cannot be reduced further, and
+        // iterating on it only adds noise to x
+        cl_reduce<2>(R, parity, v, abs_key(r), nw, [&](const double* t, double k, double* o) {
+            o[0] = t[0];
+            o[1] = k;
+            o[2] = 2e-15 * sqrt(t[1]);
+        });
+        rho = beta = R.out[0];
+        low = R.out[2];
+        tol = fmax(eps * R.out[1], low);
+    }
+    int count = 0;
+    if (R.out[1] > low) {
+        for (int it = 0; it < max_iter && rho != 0.0; ++it) {
+            ++count;
+            double y = 0.0, s = 0.0, t = 0.0;
+            if (B.on) {
+                p = fma(beta, fma(-omega, vv, p), r);
+                y = p * B.id;
+                sts<double>(ya, y);
+            }
+            cluster_sync();
+            if (B.on) vv = B.dg * cl_gsum(B, B.yoff, y, true);
+            // (rh, v); ||r|| of the step before: its test costs one operator application after
+            // convergence instead of a reduction every iteration
+            const double v1[1] = {B.on ? rh * vv : 0.0};
+            cl_reduce<1>(R, parity, v1, abs_key(r), nw, [&](const double* q, double k, double* o) {
+                o[0] = q[0] == 0.0 ? 0.0 : rho * recip_nr(q[0]);
+                o[1] = k;
+                o[2] = q[0];
+            });
+            if (R.out[1] <= tol || R.out[2] == 0.0) break;
+            alpha = R.out[0];
+            if (B.on) {
+                s = fma(-alpha, vv, r);
+                x = fma(alpha, y, x);
+                y = s * B.id;
+                sts<double>(ya, y);
+            }
+            cluster_sync();
+            if (B.on) t = B.dg * cl_gsum(B, B.yoff, y, true);
+            double v4[4] = {0.0, 0.0, 0.0, 0.0};
+            if (B.on) {
+                v4[0] = t * s;
+                v4[1] = t * t;
+                v4[2] = rh * s;
+                v4[3] = rh * t;
+            }
+            // omega = (t, s) / (t, t); (rh, r_new) = (rh, s) - omega (rh, t); the next beta
+            cl_reduce<4>(R, parity, v4, abs_key(s), nw, [&](const double* q, double k, double* o) {
+                const double w = q[1] > 0.0 ? q[0] * recip_nr(q[1]) : 0.0;
+                const double rn = fma(-w, q[3], q[2]);
+                o[0] = w;
+                o[1] = k;
+                o[2] = rn;
+                o[3] = (rn * alpha) * recip_nr(rho * w);
+            });
+            if (R.out[1] <= tol) break;
+            omega = R.out[0];
+            rho = R.out[2];
+            beta = R.out[3];
+            if (B.on) {
+                x = fma(omega, y, x);
+                r = fma(-omega, t, s);
+            }
+            if (omega == 0.0) break;
         }
     }
+    if (B.on) sts<double>(B.xa, x);
+    cluster_sync();
+    *iters = count;
+    return cl_gsrb(B, fi, x, nub);
 }
+
+__host__ __device__ __forceinline__ size_t pad16(size_t b) { return (b + 15) & ~(size_t)15; }
+// bottom cells per CTA (even: pairs of cells) and the threads they take (colours in warps of
+// their own)
+__host__ __device__ __forceinline__ int bottom_cells(int N, int nc) { return 2 * ((N + 2 * nc - 1) / (2 * nc)); }
+__host__ __device__ __forceinline__ int bottom_threads(int M) { return 2 * ((M / 2 + 31) / 32 * 32); }
 
 }  // namespace
 
 template <typename T>
-__global__ void __launch_bounds__(kTailThreads)
-k_tail(TailParams<T> P) {
+__global__ void __launch_bounds__(kTailMaxThreads)
+k_tail(const __grid_constant__ TailParams<T> P) {
     extern __shared__ __align__(16) unsigned char tail_smem[];
+    __shared__ ClReduce R;
+    __shared__ double smean;
     const int tid = threadIdx.x, nt = blockDim.x;
+    const unsigned rank = cluster_rank(), nc = cluster_size();
+    const bool z3 = P.bottom.n2 > 1 || (P.nlev > 0 && P.lev[0].n2 > 1);
     const int nl = P.nlev;   // non-bottom tail levels
-    TailLevel<T> L[kTailMaxLevels];
-    // carve shared memory: per non-bottom level 7 arrays of T, then the bottom's operator (5 N),
-    // x, f and scratch (kBotScrPerCell N) doubles
-    size_t off = 0;
-    for (int l = 0; l < nl; ++l) {
-        const int N = P.lev[l].ncell;
-        T* base = reinterpret_cast<T*>(tail_smem + off);
-        L[l].n0 = P.lev[l].n0;
-        L[l].n1 = P.lev[l].n1;
-        L[l].n2 = P.lev[l].n2;
-        L[l].N = N;
-        L[l].rz = P.lev[l].rz;
-        L[l].e = base;
-        L[l].f = base + N;
-        L[l].bx = base + 2 * N;
-        L[l].by = base + 3 * N;
-        L[l].bz = base + 4 * N;
-        L[l].dg = base + 5 * N;
-        L[l].idg = base + 6 * N;
-        off += ((size_t)7 * N * sizeof(T) + 15) & ~(size_t)15;
-    }
-    double* bsm = reinterpret_cast<double*>(tail_smem + off);
-    const Dims BD = P.bottom;
+    const Dims& BD = P.bottom;
     const int NB = BD.ncell;
-    // load the operators (split layout in global memory -> natural in shared memory).  They are
-    // built before the solve starts (and the host waits for that), so their copies are issued
-    // before the wait on the preceding kernel and overlap its last part; only the restricted
-    // defect f0 comes from that kernel.
+    const bool exact = P.binv != nullptr;
+    const unsigned sbase = smem_u32(tail_smem);
+    cluster_arrive();   // (waited for below: every CTA runs before another touches its memory)
+    // bottom's shared memory.  exact: the inverse, f, then the solution as T; else x, y (M cells
+    // each), then the solution as T
+    const int M = P.bottom_m;
+    double* bsm = reinterpret_cast<double*>(tail_smem + P.bottom_off);
+    double *binv = bsm, *fb = bsm + (size_t)NB * NB;
+    T* eb = reinterpret_cast<T*>(exact ? fb + NB : bsm + 2 * M);
+    // load the operators (split layout in global memory -> a pair's arrays in shared memory, read
+    // back by the same thread).  They are built before the solve starts (and the host waits for
+    // that), so their copies are issued before the wait on the preceding kernel and overlap its
+    // last part; only the restricted defect f0 comes from that kernel.
     for (int l = 0; l < nl; ++l) {
-        const TailLevel<T>& Ll = L[l];
-        const T *gbx = P.bx[l], *gby = P.by[l], *gbz = P.bz[l], *gdg = P.dg[l], *gidg = P.idg[l];
-        for_split_cells(P.lev[l], [&](int g, int c) {
-            cp_async(Ll.bx + c, gbx + g);
-            cp_async(Ll.by + c, gby + g);
-            cp_async(Ll.bz + c, gbz + g);
-            cp_async(Ll.dg + c, gdg + g);
-            cp_async(Ll.idg + c, gidg + g);
-            Ll.e[c] = T(0);
-        });
+        const Geo g = geo_of<T>(P, l, rank, sbase);
+        const Dims& D = P.lev[l];
+        T* ops = reinterpret_cast<T*>(tail_smem + g.nops);
+        const T *gbx = P.bx[l], *gby = P.by[l], *gbz = P.bz[l], *gdg = P.dg[l], *gid = P.idg[l];
+        const int S = g.pairs;
+        for (int t = tid; t < g.rows * g.hn0; t += nt) {
+            const int lr = fdiv(t, g.mhn0), h = t - lr * g.hn0;
+            const int row = g.row0 + lr, k = fdiv(row, g.mn1), j = row - k * g.n1;
+            const int rp = j == g.n1 - 1 ? row - j : row + 1;                      // row of j + 1
+            const int rz = k == g.n2 - 1 ? j : row + g.n1;                         // row of k + 1
+            // split index of (2h + a) in a row of colour parity c: half ((a + c) & 1), column h
+            const int c = (j + k) & 1, cp = (rp - fdiv(rp, g.mn1) * g.n1 + k) & 1;
+            const int cz = (j + (k == g.n2 - 1 ? 0 : k + 1)) & 1;
+            const int i0 = row * D.hn0 + h, ip = rp * D.hn0 + h, iz = rz * D.hn0 + h;
+            const int hn = h == g.hn0 - 1 ? 0 : h + 1;
+            T* o = ops + t;
+            cp_async(o + (kBx + 2) * S, gbx + c * D.half + row * D.hn0 + hn);
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+                const int q = ((a + c) & 1) * D.half + i0;
+                cp_async(o + (kBx + a) * S, gbx + q);
+                cp_async(o + (kBy + a) * S, gby + q);
+                cp_async(o + (kByp + a) * S, gby + ((a + cp) & 1) * D.half + ip);
+                cp_async(o + (kBz + a) * S, gbz + q);
+                cp_async(o + (kBzp + a) * S, gbz + ((a + cz) & 1) * D.half + iz);
+                cp_async(o + (kId + a) * S, gid + q);
+                cp_async(o + (kDg + a) * S, gdg + q);
+            }
+        }
     }
-    BotView v;
-    v.n0 = BD.n0;
-    v.n1 = BD.n1;
-    v.n2 = BD.n2;
-    v.N = NB;
-    double* ops = bsm;
-    for (int c = tid; c < NB; c += nt) {
-        cp_async(ops + c, P.bbx + c);
-        cp_async(ops + NB + c, P.bby + c);
-        cp_async(ops + 2 * NB + c, P.bbz + c);
-        cp_async(ops + 3 * NB + c, P.bdg + c);
-        cp_async(ops + 4 * NB + c, P.bidg + c);
+    ClBottom B;
+    int bc = 0;   // the thread's bottom cell
+    if (exact) {
+        for (int q = tid; q < NB * NB; q += nt) cp_async(binv + q, P.binv + q);
+    } else {
+        // pair q of the CTA's cells: colour 0 to thread q, the other one to the upper half
+        const int c0 = min(NB, (int)rank * M), m = min(NB - c0, M), half = bottom_threads(M) / 2;
+        const int up = tid >= half, q = tid - (up ? half : 0);
+        auto colour = [&](int c) {
+            const int row = c / BD.n0;
+            return (c - row * BD.n0 + row % BD.n1 + row / BD.n1) & 1;
+        };
+        int lm = 2 * q + up;
+        if (2 * q + 1 < m && colour(c0 + 2 * q) == 1 && colour(c0 + 2 * q + 1) == 0) lm = 2 * q + 1 - up;
+        B.N = NB;
+        B.on = tid < 2 * half && lm < m;
+        B.odd = (BD.n0 & 1 && P.bc.lo[0] == MAC_BC_PER) || (BD.n1 & 1 && P.bc.lo[1] == MAC_BC_PER) ||
+                (BD.n2 > 1 && BD.n2 & 1 && P.bc.lo[2] == MAC_BC_PER);
+        B.yoff = M * 8u;
+        B.xa = smem_u32(bsm) + (B.on ? lm : 0) * 8u;
+        B.colour = 0;
+        if (B.on) {
+            const int c = bc = c0 + lm;
+            const int row = c / BD.n0, i = c - row * BD.n0, k = row / BD.n1, j = row - k * BD.n1;
+            const int im = i == 0 ? BD.n0 - 1 : i - 1, ip = i == BD.n0 - 1 ? 0 : i + 1;
+            const int jm = j == 0 ? BD.n1 - 1 : j - 1, jp = j == BD.n1 - 1 ? 0 : j + 1;
+            const int km = k == 0 ? BD.n2 - 1 : k - 1, kp = k == BD.n2 - 1 ? 0 : k + 1;
+            const int nb[6] = {im + BD.n0 * row, ip + BD.n0 * row, i + BD.n0 * (jm + BD.n1 * k),
+                               i + BD.n0 * (jp + BD.n1 * k), i + BD.n0 * (j + BD.n1 * km),
+                               i + BD.n0 * (j + BD.n1 * kp)};
+            const double id = P.bidg[c];
+            const double w[6] = {P.bbx[c], P.bbx[nb[1]], P.bby[c], P.bby[nb[3]], P.bbz[c], P.bbz[nb[5]]};
+            B.colour = (i + j + k) & 1;
+            B.id = id;
+            B.dg = P.bdg[c];
+#pragma unroll
+            for (int n = 0; n < 6; ++n) {
+                const unsigned cta = fdiv(nb[n], P.bottom_mm);
+                B.gc[n] = w[n] * id;
+                B.nb[n] = mapa(smem_u32(bsm) + (nb[n] - cta * M) * 8u, cta);
+            }
+        }
     }
     pdl_wait();
     pdl_trigger();
-    {
-        const T* gf = P.f0;
-        T* sf = L[0].f;
-        for_split_cells(P.lev[0], [&](int g, int c) { cp_async(sf + c, gf + g); });
+    double bf = 0.0, bx = 0.0;   // the bottom cell's right-hand side and solution
+    if (nl > 0) {
+        const Geo g = geo_of<T>(P, 0, rank, sbase);
+        const Dims& D = P.lev[0];
+        T* ops = reinterpret_cast<T*>(tail_smem + g.nops);
+        for (int t = tid; t < g.rows * g.hn0; t += nt) {
+            const int lr = fdiv(t, g.mhn0), h = t - lr * g.hn0;
+            const int row = g.row0 + lr, k = fdiv(row, g.mn1), j = row - k * g.n1;
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+                cp_async(ops + (kF + a) * g.pairs + t,
+                         P.f0 + ((a + j + k) & 1) * D.half + row * D.hn0 + h);
+        }
+    } else if (exact) {
+        for (int c = tid; c < NB; c += nt) fb[c] = (double)P.f0[c];
+    } else if (B.on) {
+        bf = (double)P.f0[bc];
+        bx = (double)P.e0[bc];
     }
     cp_async_wait();
-    v.bx = ops;
-    v.by = ops + NB;
-    v.bz = ops + 2 * NB;
-    v.dg = ops + 3 * NB;
-    v.idg = ops + 4 * NB;
-    double* xb = bsm + 5 * NB;
-    double* fb = bsm + 6 * NB;
-    double* wb = bsm + 7 * NB;
     __syncthreads();
-    // down the V
+    cluster_wait();
+    // down the V.  red-only defect / black-only prolongation rest on plain Gauss-Seidel half-sweeps
+    const bool gs = P.omega == T(1);
+    const bool red = gs && P.nu1 > 0, black = gs && P.nu2 > 0;
     for (int l = 0; l < nl; ++l) {
-        for (int s = 0; s < P.nu1; ++s) tail_sweep<T>(L[l], P.omega);
-        // red-only defect / black-only prolongation rest on plain Gauss-Seidel half-sweeps
-        const bool gs = P.omega == T(1);
-        if (l + 1 < nl) {
-            tail_restrict<T, T>(L[l], L[l + 1].n0, L[l + 1].n1, L[l + 1].n2, L[l + 1].f,
-                                gs && P.nu1 > 0);
+        if (z3) {
+            if (P.geo[l].two)
+                visit_down<T, 2, true>(P, l, rank, tail_smem, red);
+            else
+                visit_down<T, 1, true>(P, l, rank, tail_smem, red);
         } else {
-            tail_restrict<T, double>(L[l], BD.n0, BD.n1, BD.n2, fb, gs && P.nu1 > 0);
+            visit_down<T, 1, false>(P, l, rank, tail_smem, red);
+        }
+        const Geo F = geo_of<T>(P, l, rank, sbase);
+        auto coarse_f = [&](int I, int J, int K) -> T {
+            return z3 ? restricted<T, true>(F, I, J, K, red) : restricted<T, false>(F, I, J, K, red);
+        };
+        if (l + 1 < nl || exact) {
+            // the next level's right-hand side.  One held by every CTA below one that is spread
+            // out: each CTA restricts its share and writes it to all of them (reading every
+            // defect sixteen times took 8000 cycles for 8^3 cells, this 1500).
+            const bool lev = l + 1 < nl;
+            const Geo C = geo_of<T>(P, lev ? l + 1 : l, rank, sbase);
+            const int n0 = lev ? C.n0 : BD.n0, n1 = lev ? C.n1 : BD.n1;
+            const int all = lev ? C.rows * C.n0 : NB;
+            const bool push = !F.repl && (!lev || C.repl);
+            const int share = push ? (all + (int)nc - 1) / (int)nc : all;
+            const int first = push ? (int)rank * share : 0, last = min(all, first + share);
+            for (int t = first + tid; t < last; t += nt) {
+                const int lrow = t / n0, i = t - lrow * n0;
+                const int row = (lev ? C.row0 : 0) + lrow, K = row / n1, J = row - K * n1;
+                const T v = coarse_f(i, J, K);
+                const unsigned a = lev ? sbase + C.nops + ((kF + (i & 1)) * C.pairs + lrow * C.hn0 + (i >> 1)) * (unsigned)sizeof(T)
+                                       : smem_u32(fb) + t * 8u;
+                if (push) {
+                    for (unsigned c = 0; c < nc; ++c) {
+                        if (lev)
+                            st_cluster(mapa(a, c), v);
+                        else
+                            st_cluster(mapa(a, c), (double)v);
+                    }
+                } else if (lev) {
+                    sts<T>(a, v);
+                } else {
+                    sts<double>(a, (double)v);
+                }
+            }
+            sync_level(!push);
+        } else if (B.on) {
+            const int row = bc / BD.n0, K = row / BD.n1;
+            bf = (double)coarse_f(bc - row * BD.n0, row - K * BD.n1, K);
         }
     }
-    // bottom, FP64 (input rhs rounded through T as in the multi-kernel path)
+    // bottom, FP64 (input rhs rounded through T as in the multi-kernel path); its solution is
+    // handed up as T
     int count = 0;
-    __shared__ double sm_red[33];
-    if (P.binv) {
+    Coarse<T> cb;
+    cb.base = smem_u32(eb);
+    cb.g.repl = exact;
+    cb.g.cpc = M;
+    cb.g.mcpc = P.bottom_mm;
+    if (exact) {
         // exact solve by the precomputed (pseudo-)inverse: x = B^-1 (f - mean f) (the mean comes
-        // off for a singular operator, whose constant mode B^-1 only scales)
+        // off for a singular operator, whose constant mode B^-1 only scales), by every CTA
         if (P.singular) {
             if (tid < 32) {
                 double s = 0.0;
                 for (int c = tid; c < NB; c += 32) s += fb[c];
                 for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                if (tid == 0) sm_red[32] = s / NB;
+                if (tid == 0) smean = s / NB;
             }
             __syncthreads();
-            const double mean = sm_red[32];
+            const double mean = smean;
             for (int c = tid; c < NB; c += nt) fb[c] -= mean;
             __syncthreads();
         }
-        // row r of B^-1 by kDenseSeg lanes of one warp (NB <= kDenseBottomMax: one pass)
-        const int r = tid / kDenseSeg, sg = tid % kDenseSeg;
-        double acc = 0.0;
-        if (r < NB)
-            for (int c = sg; c < NB; c += kDenseSeg) acc = fma(__ldg(P.binv + (size_t)r * NB + c), fb[c], acc);
-        for (int o = kDenseSeg / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (r < NB && sg == 0) xb[r] = acc;
+        // row r of B^-1 by kDenseSeg lanes of one warp, the rows spread over the CTAs, each written
+        // to all of them (one CTA's FP64 rate makes 64 rows 4000 cycles)
+        const int sg = tid % kDenseSeg, share = (NB + (int)nc - 1) / (int)nc;
+        const int first = (int)rank * share, last = min(NB, first + share);
+        for (int r0 = first; r0 < last; r0 += nt / kDenseSeg) {
+            const int r = r0 + tid / kDenseSeg;
+            if (r0 + (tid & ~31) / kDenseSeg >= last) continue;   // (whole warps)
+            double acc = 0.0;
+            if (r < last)
+                for (int c = sg; c < NB; c += kDenseSeg) acc = fma(binv[r * NB + c], fb[c], acc);
+            for (int o = kDenseSeg / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (r < last && sg < (int)nc) st_cluster(mapa(smem_u32(eb + r), sg), (T)acc);
+        }
+        cluster_sync();
     } else {
-        for (int c = tid; c < NB; c += nt) xb[c] = 0.0;
-        __syncthreads();
-        if (tid < 128)
-            count = bottom_body<Sync128<true>>(v, xb, fb, wb, sm_red, P.singular, P.nub,
-                                               P.bottom_eps, P.bottom_max_iter);
+        if (B.on) sts<double>(B.xa, bx);
+        bx = cl_solve(B, R, bf, bx, bottom_threads(M) / 32, P.singular, P.nub, P.bottom_eps,
+                      P.bottom_max_iter, &count);
+        if (B.on) eb[bc - (int)rank * M] = (T)bx;
+        cluster_sync();
     }
-    __syncthreads();
-    // the bottom solution is handed up as T, like the multi-kernel path's bottom output
-    T* eb = reinterpret_cast<T*>(wb);
-    for (int c = tid; c < NB; c += nt) eb[c] = (T)xb[c];
-    __syncthreads();
     // up the V
     for (int l = nl - 1; l >= 0; --l) {
-        const bool gs = P.omega == T(1);
-        if (l + 1 < nl)
-            tail_prolong<T>(L[l], L[l + 1].e, L[l + 1].n0, L[l + 1].n1, L[l + 1].n2, P.bc,
-                            gs && P.nu2 > 0);
-        else
-            tail_prolong<T>(L[l], eb, BD.n0, BD.n1, BD.n2, P.bc, gs && P.nu2 > 0);
-        for (int s = 0; s < P.nu2; ++s) tail_sweep<T>(L[l], P.omega);
+        int cn1 = BD.n1, cn2 = BD.n2;
+        Coarse<T> ec = cb;
+        if (l + 1 < nl) {
+            ec.g = geo_of<T>(P, l + 1, rank, sbase);
+            ec.base = ec.g.ea;
+            cn1 = ec.g.n1;
+            cn2 = ec.g.n2;
+        }
+        if (z3) {
+            if (P.geo[l].two)
+                visit_up<T, 2, true>(P, l, rank, tail_smem, ec, cn1, cn2, black);
+            else
+                visit_up<T, 1, true>(P, l, rank, tail_smem, ec, cn1, cn2, black);
+        } else {
+            visit_up<T, 1, false>(P, l, rank, tail_smem, ec, cn1, cn2, black);
+        }
     }
-    // hand the correction of the first tail level back (its split layout)
-    {
-        const T* e = L[0].e;
-        T* ge = P.e0;
-        for_split_cells(P.lev[0], [&](int g, int c) { ge[g] = e[c]; });
+    // hand the correction back: of the first tail level (its split layout), or the bottom's
+    if (nl > 0) {
+        const Geo g = geo_of<T>(P, 0, rank, sbase);
+        const Dims& D = P.lev[0];
+        const T* e = reinterpret_cast<const T*>(tail_smem + P.geo[0].off);
+        if (!g.repl || rank == 0)
+            for (int t = tid; t < g.rows * g.n0; t += nt) {
+                const int pr = t >> 1, a = t & 1;
+                const int lr = fdiv(pr, g.mhn0), h = pr - lr * g.hn0;
+                const int row = g.row0 + lr, k = fdiv(row, g.mn1), j = row - k * g.n1;
+                P.e0[((a + j + k) & 1) * D.half + row * D.hn0 + h] = e[t];
+            }
+    } else if (exact) {
+        if (rank == 0)
+            for (int c = tid; c < NB; c += nt) P.e0[c] = eb[c];
+    } else if (B.on) {
+        P.e0[bc] = (T)bx;
     }
-    if (tid == 0 && P.iters) atomicAdd(P.iters, count);
+    if (tid == 0 && rank == 0 && P.iters) atomicAdd(P.iters, count);
+    cluster_sync();   // no CTA leaves while another may read its shared memory
 }
 
 // (Pseudo-)inverse of the bottom operator for the exact bottom solve of the FP32 V-cycle: the
@@ -381,9 +914,9 @@ k_tail(TailParams<T> P) {
 // each thread owning fixed elements of the packed triangle so that warps stay full (GB300 issues
 // FP64 instructions per warp, whatever the number of active lanes).  FP64, shared memory, one
 // CTA, once per solve (on a side stream, overlapping the right-hand-side setup).
-constexpr int kInvPerThread = (kDenseBottomMax * (kDenseBottomMax + 1) / 2 + kTailThreads - 1) / kTailThreads;
+constexpr int kInvPerThread = (kDenseBottomMax * (kDenseBottomMax + 1) / 2 + kInvThreads - 1) / kInvThreads;
 
-__global__ void __launch_bounds__(kTailThreads)
+__global__ void __launch_bounds__(kInvThreads)
 k_bottom_inverse(Dims D, const double* __restrict__ bx, const double* __restrict__ by,
                  const double* __restrict__ bz, const double* __restrict__ dg, int singular,
                  double* __restrict__ out) {
@@ -461,33 +994,116 @@ k_bottom_inverse(Dims D, const double* __restrict__ bx, const double* __restrict
 
 void launch_bottom_inverse(const Dims& d, const double* bx, const double* by, const double* bz,
                            const double* dg, bool singular, double* out, cudaStream_t s) {
-    k_bottom_inverse<<<1, kTailThreads, 0, s>>>(d, bx, by, bz, dg, singular ? 1 : 0, out);
+    k_bottom_inverse<<<1, kInvThreads, 0, s>>>(d, bx, by, bz, dg, singular ? 1 : 0, out);
 }
 
+// Fills P's plan (rows a CTA, shared-memory offsets) for a cluster of nc CTAs; returns the dynamic
+// shared memory of a CTA, or 0 when the levels or the bottom do not fit.  *threads: of a CTA.
 template <typename T>
-size_t tail_smem_bytes(const Dims* lev, int nl, const Dims& bottom) {
+static size_t plan_tail(TailParams<T>& P, int nc, int* threads) {
     size_t off = 0;
-    for (int l = 0; l < nl; ++l) off += ((size_t)7 * lev[l].ncell * sizeof(T) + 15) & ~(size_t)15;
-    return off + (size_t)(7 + kBotScrPerCell) * bottom.ncell * sizeof(double);
+    int most = 0;   // pairs of the widest level
+    for (int l = 0; l < P.nlev; ++l) {
+        const Dims& D = P.lev[l];
+        TailGeo& q = P.geo[l];
+        const int R0 = D.n1 * D.n2;
+        q.repl = D.ncell <= kReplCells<T>;
+        q.rpc = q.repl ? R0 : (R0 + nc - 1) / nc;
+        q.mcpc = div_magic(q.rpc * D.n0);
+        q.mn1 = div_magic(D.n1);
+        q.mhn0 = div_magic(D.n0 >> 1);
+        q.off = (int)off;
+        const int pairs = q.rpc * (D.n0 >> 1);
+        most = pairs > most ? pairs : most;
+        off += pad16((size_t)(2 * q.rpc * D.n0 + kOps * pairs) * sizeof(T));
+        if (off > (size_t)kTailSmemMax || pairs > (D.n2 > 1 ? kTailItems : 1) * kTailMaxThreads) return 0;
+    }
+    const size_t N = P.bottom.ncell;
+    P.bottom_off = (int)off;
+    P.bottom_m = bottom_cells(P.bottom.ncell, nc);
+    P.bottom_mm = div_magic(P.bottom_m);
+    const bool exact = P.binv != nullptr;
+    if (exact)
+        off += (N * N + N) * sizeof(double) + N * sizeof(T);
+    else
+        off += P.bottom_m * (2 * sizeof(double) + sizeof(T));
+    const int need = exact ? 256 : bottom_threads(P.bottom_m);
+    if (off > (size_t)kTailSmemMax || need > kTailMaxThreads) return 0;
+    // a pair a thread up to 512 threads (a cluster barrier costs 380 cycles with 256 threads, 470
+    // with 512, 600 with 1024), then two
+    int t = 128;
+    while (t < kTailMaxThreads && (t < most || t < need)) t *= 2;
+    for (int l = 0; l < P.nlev; ++l) P.geo[l].two = P.geo[l].rpc * (P.lev[l].n0 >> 1) > t;
+    *threads = t;
+    return off;
 }
 
 template <typename T>
-void launch_tail(const TailParams<T>& P, size_t smem, cudaStream_t s) {
-    launch_chain(k_tail<T>, dim3(1), dim3(kTailThreads), smem, s, P);
+bool tail_fits(const Dims* lev, int nl, const Dims& bottom, bool exact, int nc) {
+    if (nl > kTailMaxLevels) return false;
+    TailParams<T> P;
+    P.nlev = nl;
+    for (int l = 0; l < nl; ++l) P.lev[l] = lev[l];
+    P.bottom = bottom;
+    static const double some = 0.0;
+    P.binv = exact ? &some : nullptr;
+    int t;
+    return plan_tail<T>(P, nc, &t) > 0;
 }
 
-int prepare_tail_kernels() {
-    if (cudaFuncSetAttribute(k_tail<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmemMax) != cudaSuccess ||
-        cudaFuncSetAttribute(k_tail<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmemMax) != cudaSuccess) {
-        cudaGetLastError();
-        return MAC_ERR_CUDA;
+template <typename T>
+void launch_tail(TailParams<T>& P, int nc, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    int threads = 0;
+    cfg.dynamicSmemBytes = plan_tail<T>(P, nc, &threads);
+    cfg.gridDim = dim3(nc);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = nc;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    cudaLaunchKernelEx(&cfg, k_tail<T>, P);
+}
+
+// Opts the tail kernels into their shared memory and cluster size; *nc: the CTAs of a cluster.
+int prepare_tail_kernels(int* nc) {
+    const void* kern[2] = {(const void*)k_tail<float>, (const void*)k_tail<double>};
+    *nc = kClusterMax;
+    for (const void* k : kern) {
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmemMax) != cudaSuccess ||
+            cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaGetLastError();
+            return MAC_ERR_CUDA;
+        }
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kClusterMax);
+        cfg.blockDim = dim3(kTailMaxThreads);
+        cfg.dynamicSmemBytes = kTailSmemMax;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = kClusterMax;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            *nc = 8;   // the portable size
+        }
     }
     return MAC_OK;
 }
 
-template size_t tail_smem_bytes<float>(const Dims*, int, const Dims&);
-template size_t tail_smem_bytes<double>(const Dims*, int, const Dims&);
-template void launch_tail<float>(const TailParams<float>&, size_t, cudaStream_t);
-template void launch_tail<double>(const TailParams<double>&, size_t, cudaStream_t);
+template bool tail_fits<float>(const Dims*, int, const Dims&, bool, int);
+template bool tail_fits<double>(const Dims*, int, const Dims&, bool, int);
+template void launch_tail<float>(TailParams<float>&, int, cudaStream_t);
+template void launch_tail<double>(TailParams<double>&, int, cudaStream_t);
 
 }  // namespace mac
