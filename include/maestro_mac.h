@@ -111,9 +111,9 @@ typedef struct mac_opts {
     int inner_nu1, inner_nu2; /* mixed precision: red/black sweeps down / up the inner FP32
                                V-cycles (default 2 / 1; -1: nu1 / nu2); the FP64 V-cycle always
                                uses nu1 / nu2                                                  */
-    int inner_exact_bottom; /* mixed precision, 1 (default): the inner V-cycles solve a bottom of
-                               at most 64 cells exactly, by its dense FP64 (pseudo-)inverse
-                               formed once per solve; 0: FP64 BiCGStab as the FP64 V-cycle     */
+    int inner_exact_bottom; /* 1 (default): the V-cycles (FP64 and inner) solve a bottom of at most
+                               64 cells exactly, by its dense FP64 (pseudo-)inverse formed once
+                               per solve (needs coarse_tail); 0: FP64 BiCGStab to bottom_eps   */
     double inner_omega;     /* mixed precision: relaxation weight of the inner V-cycles'
                                red/black half-sweeps, 0 < omega < 2 (default 1.25; 1:
                                Gauss-Seidel)                                                   */

@@ -311,7 +311,8 @@ struct mac_ctx {
     double* bot_inv = nullptr;                    // dense bottom (pseudo-)inverse (small bottoms)
     cudaStream_t aux = nullptr;                   // side stream of the bottom inverse
     cudaEvent_t aux_ev[2] = {nullptr, nullptr};   // [0] operators ready, [1] inverse done
-    bool inv_pending = false;                     // the main stream still has to wait on aux_ev[1]
+    int inv_state = 0;                            // 0: none for this operator; 1: the main stream
+                                                  // still has to wait on aux_ev[1]; 2: usable
     int tail_start[2] = {-1, -1};                 // first tail level (FP64, FP32); -1: none
     int tail_nc = 16;                             // CTAs of the tail cluster
     bool bottom_cluster = false;                  // the bottom alone fits the cluster
@@ -435,7 +436,7 @@ void launch_bottom_inverse(const Dims& d, const double* bx, const double* by, co
 int setup_fine_coefficients(mac_ctx* c, const double* beta0, const double* beta0e);
 int setup_coarse_levels(mac_ctx* c);
 // the exact bottom's (pseudo-)inverse, on the side stream once the bottom operator is built
-// (no-op unless the FP32 V-cycle uses it); run_solve orders the V-cycles after it
+// (no-op unless the V-cycles use it), and the main stream's wait for it before the V-cycles
 int issue_bottom_inverse(mac_ctx* c);
 int wait_bottom_inverse(mac_ctx* c);
 int setup_fp32_copies(mac_ctx* c);

@@ -145,8 +145,8 @@ bool fused_sweeps(const mac_ctx* c) {
     return c->otf && c->o.fused_sweep && c->e_alt != nullptr && fused_plan(c);
 }
 
-// The FP32 V-cycle's bottom solved exactly by the dense (pseudo-)inverse (small bottoms, run
-// through the tail kernel); the FP64 V-cycle keeps BiCGStab.
+// The bottom solved exactly by the dense (pseudo-)inverse (small bottoms, run through the tail
+// kernel).
 bool exact_bottom(const mac_ctx* c) {
     return c->o.inner_exact_bottom && c->o.coarse_tail && c->bot_inv != nullptr;
 }
@@ -211,7 +211,7 @@ void vcycle(mac_ctx* c, int l) {
         tp.bottom_max_iter = o.bottom_max_iter;
         tp.bottom_eps = o.bottom_eps;
         tp.iters = c->red.counters;
-        tp.binv = std::is_same<T, float>::value && exact_bottom(c) ? c->bot_inv : nullptr;
+        tp.binv = exact_bottom(c) ? c->bot_inv : nullptr;
         tp.omega = omega;
         launch_tail<T>(tp, c->tail_nc, c->stream);
         ++c->issued;
@@ -497,8 +497,8 @@ int run_solve(mac_ctx* c, mac_stats* st) {
         if (c->o.fused_sweep && c->otf && fused_plan(c) && !c->e_alt &&
             (rc = alloc_arr(c, &c->e_alt, (size_t)F.d.ncell)))
             return rc;
-        if ((rc = wait_bottom_inverse(c))) return rc;
     }
+    if (int rc = wait_bottom_inverse(c)) return rc;
     MAC_CUDA_TRY(cudaMemcpyAsync(c->red.h_scalars, c->red.scalars, 8 * sizeof(double),
                                  cudaMemcpyDeviceToHost, c->stream));
     MAC_CUDA_TRY(cudaMemcpyAsync(c->red.h_counters, c->red.counters, 4 * sizeof(int),
@@ -738,7 +738,7 @@ int ctx_alloc(mac_ctx* c) {
         }
     }
     rc |= alloc_arr(c, &c->bottom_scratch, (size_t)(2 + kBotScrPerCell) * B.d.ncell);
-    if (c->tail_start[1] >= 0 && B.d.ncell <= kDenseBottomMax)
+    if (B.d.ncell <= kDenseBottomMax)
         rc |= alloc_arr(c, &c->bot_inv, (size_t)B.d.ncell * B.d.ncell);
     for (int d = 0; d < c->dm; ++d) {
         const size_t nf = (size_t)(c->n[0] + (d == 0)) * (c->n[1] + (d == 1)) * (c->n[2] + (d == 2));
@@ -967,9 +967,9 @@ void report_call(const mac_ctx* c, const char* what, const mac_stats* st) { repo
 int issue_bottom_inverse(mac_ctx* c) {
     // an inverse issued by a call that stopped before its solve may still read the operator the
     // main stream is about to rebuild
-    if (c->inv_pending) MAC_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->aux_ev[1], 0));
-    c->inv_pending = false;
-    if (c->o.precision != MAC_PREC_MIXED || !exact_bottom(c)) return MAC_OK;
+    if (c->inv_state == 1) MAC_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->aux_ev[1], 0));
+    c->inv_state = 0;
+    if (!exact_bottom(c)) return MAC_OK;
     const Level& B = c->lev[c->nlevels - 1];
     MAC_CUDA_TRY(cudaEventRecord(c->aux_ev[0], c->stream));
     MAC_CUDA_TRY(cudaStreamWaitEvent(c->aux, c->aux_ev[0], 0));
@@ -978,17 +978,17 @@ int issue_bottom_inverse(mac_ctx* c) {
     MAC_CUDA_TRY(cudaGetLastError());
     ++c->issued;
     MAC_CUDA_TRY(cudaEventRecord(c->aux_ev[1], c->aux));
-    c->inv_pending = true;
+    c->inv_state = 1;
     return MAC_OK;
 }
 int wait_bottom_inverse(mac_ctx* c) {
-    if (c->o.precision != MAC_PREC_MIXED || !exact_bottom(c)) return MAC_OK;
-    if (!c->inv_pending) {   // (a caller that built the levels some other way)
+    if (!exact_bottom(c) || c->inv_state == 2) return MAC_OK;
+    if (c->inv_state == 0) {   // (a caller that built the levels some other way)
         int rc = issue_bottom_inverse(c);
         if (rc) return rc;
     }
     MAC_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->aux_ev[1], 0));
-    c->inv_pending = false;
+    c->inv_state = 2;
     return MAC_OK;
 }
 int load_beta0(mac_ctx* c, int ptr_kind, const double* b0, const double* b0e) {

@@ -904,7 +904,7 @@ k_tail(const __grid_constant__ TailParams<T> P) {
     cluster_sync();   // no CTA leaves while another may read its shared memory
 }
 
-// (Pseudo-)inverse of the bottom operator for the exact bottom solve of the FP32 V-cycle: the
+// (Pseudo-)inverse of the bottom operator for the exact bottom solve of the V-cycles: the
 // dense N x N matrix of A x = diag x - sum_n a_n x_n (N <= kDenseBottomMax, natural layout; a
 // periodic arm that wraps onto the same neighbour twice adds up), plus sigma 1 1^T with sigma =
 // mean(diag) / N when A is singular (constant null space: B^-1 f = A^+ f for f of zero mean).
