@@ -34,35 +34,314 @@ constexpr int kMixedInner = 2;        // FP32 multi-level V-cycles per FP64 step
 #define AMR_LOOP(N) for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx < (N); \
                          idx += (long)gridDim.x * blockDim.x)
 
-template <typename T>
-__global__ void k_defect(Geo G, amr::LevT<T> L, amr::LevT<T> C, const T* u, const T* cu,
-                         const T* f, T* r, long N) {
-    AMR_LOOP(N) amr::defect_cell(G, L, C, idx, u, cu, f, r);
+// ---- cell kernels of one level ---------------------------------------------------------------
+//
+// One thread per cell (or cell of one colour) of a plane of the array box, planes along
+// blockIdx.z, the row by one multiplication (Plane).  Two more bits of the level's mask, set with
+// the hierarchy, choose the cell function: kFull (a region cell whose neighbours are all region
+// cells: the plain stencil at constant offsets), kNear (a region cell whose neighbours lie in the
+// array box without a wrap; without coarse data a coarse-fine side only adds to the diagonal).  The
+// other region cells (at domain faces; with coarse data also the kNear ones) take the general
+// functions of mac_amr.cuh, by list in extra planes of the grid: inline, one or two of them in
+// every row made half of all warps run both forms (53 us a defect of 130^3 cells).  They run the same operations in the same order, except
+// that the FP64 stencil takes differences, which needs 15 instead of 20 FP64 instructions (the
+// FP64 pipe binds it: 2.2 M cells took 127 us, with 40 us of memory traffic) and FP64 Gauss-Seidel
+// multiplies by recip_nr.  With the general function for every cell (64-bit indices, divisions,
+// six mask tests) the FP32 sweep ran at 0.23 of HBM, 38 us a colour, the defect 83 us.
+constexpr unsigned char kFull = 4;
+constexpr unsigned char kNear = 8;
+
+struct Plane {
+    unsigned m0;   // reciprocal of the row length (0: divide)
+};
+__device__ __forceinline__ unsigned row_of(unsigned t, unsigned e, Plane P) {
+    return P.m0 ? __umulhi(t, P.m0) : t / e;
+}
+// floor(2^32 / e) + 1 is exact for t e < 2^32, t < e rows
+inline Plane plane(long e, long rows) {
+    Plane P;
+    P.m0 = e > 1 && e * e * rows < (1L << 32) ? (unsigned)(0x100000000ull / (unsigned long long)e) + 1u : 0u;
+    return P;
+}
+inline dim3 plane_grid(long cells, int planes) {
+    return dim3((unsigned)((cells + kThreads - 1) / kThreads), 1, (unsigned)planes);
 }
 
-// One colour of a sweep: one thread per cell of that colour (N = amr::colour_threads).
+// Cells taken by list: the extra planes' threads in order.
+struct Rest {
+    const int* list;
+    int n;
+};
+__device__ __forceinline__ int rest_index(int planes, const Rest& R) {
+    const unsigned t = ((blockIdx.z - (unsigned)planes) * gridDim.x + blockIdx.x) * kThreads + threadIdx.x;
+    return t < (unsigned)R.n ? R.list[t] : -1;
+}
+inline dim3 plane_grid(long cells, int planes, int rest) {
+    dim3 g = plane_grid(cells, planes);
+    const long slice = (long)g.x * kThreads;
+    g.z += (unsigned)((rest + slice - 1) / slice);
+    return g;
+}
+
+// A cell of plane k of the box: index, row r = j + ext1 k, and whether the plane has it.
+struct Cell {
+    unsigned q, r, i, j, k;
+};
 template <typename T>
-__global__ void k_gsrb(Geo G, amr::LevT<T> L, int colour, T* u, const T* f, long N) {
-    AMR_LOOP(N) {
-        const long c = amr::colour_cell(L, idx, colour);
-        if (c >= 0) amr::gsrb_cell(G, L, c, colour, u, f);
+__device__ __forceinline__ bool plane_cell(const amr::LevT<T>& L, Plane P, unsigned k, Cell& c) {
+    const unsigned e0 = L.ext[0], e1 = L.ext[1], t = blockIdx.x * kThreads + threadIdx.x;
+    c.j = row_of(t, e0, P);
+    c.i = t - c.j * e0;
+    c.k = k;
+    c.r = c.j + e1 * k;
+    c.q = c.i + e0 * c.r;
+    return t < e0 * e1 && k < (unsigned)L.ext[2];
+}
+// One cell of the colour a thread: half a row each.
+template <typename T>
+__device__ __forceinline__ bool colour_plane_cell(const amr::LevT<T>& L, Plane P, int colour, unsigned k,
+                                                  Cell& c) {
+    const unsigned e0 = L.ext[0], e1 = L.ext[1], hw = (e0 + 1) / 2;
+    const unsigned t = blockIdx.x * kThreads + threadIdx.x;
+    c.j = row_of(t, hw, P);
+    c.k = k;
+    c.r = c.j + e1 * k;
+    c.i = 2 * (t - c.j * hw) + ((colour + L.lo[0] + L.lo[1] + c.j + L.lo[2] + k) & 1);
+    c.q = c.i + e0 * c.r;
+    return t < hw * e1 && c.i < e0 && k < (unsigned)L.ext[2];
+}
+
+// (Explicit rounding: the FP32 cycles give the general functions' results bit for bit, and with
+// them the constant that a closed domain's phi picks up from FP32 rounding.)
+__device__ __forceinline__ float mulT(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mulT(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float addT(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double addT(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float fmaT(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fmaT(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float recip(float x) { return 1.f / x; }
+__device__ __forceinline__ double recip(double x) { return recip_nr(x); }
+
+// A cell's stencil, loaded before its mask is known (one memory latency a cell instead of two; a
+// neighbour index outside the box is clamped, its value unused): face coefficients and neighbours
+// x-, x+, y-, y+, z-, z+.
+template <typename T>
+struct Stencil {
+    T b[6], u[6], uc, f;
+    unsigned n[6];
+    unsigned char m;
+};
+template <typename T>
+__device__ __forceinline__ void load_stencil(const Geo& G, const amr::LevT<T>& L, const Cell& c, const T* u,
+                                             const T* __restrict__ f, Stencil<T>& A) {
+    const unsigned e0 = L.ext[0], pl = e0 * (unsigned)L.ext[1], last = pl * (unsigned)L.ext[2] - 1;
+    const unsigned f0 = c.q + c.r, f1 = c.q + e0 * c.k;
+    A.m = L.mask[c.q];
+    A.n[0] = c.q - (c.q >= 1u);
+    A.n[1] = min(c.q + 1, last);
+    A.n[2] = c.q >= e0 ? c.q - e0 : 0u;
+    A.n[3] = min(c.q + e0, last);
+    A.b[0] = L.b[0][f0];
+    A.b[1] = L.b[0][f0 + 1];
+    A.b[2] = L.b[1][f1];
+    A.b[3] = L.b[1][f1 + e0];
+    A.uc = u[c.q];
+    A.f = f[c.q];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) A.u[n] = u[A.n[n]];
+    if (G.dm > 2) {
+        A.n[4] = c.q >= pl ? c.q - pl : 0u;
+        A.n[5] = min(c.q + pl, last);
+        A.b[4] = L.b[2][c.q];
+        A.b[5] = L.b[2][c.q + pl];
+        A.u[4] = u[A.n[4]];
+        A.u[5] = u[A.n[5]];
+    }
+}
+
+// cell_op with zero coarse data on a kFull or kNear cell (see amr::cell_op).
+template <typename T>
+__device__ __forceinline__ void near_op(const Geo& G, const amr::LevT<T>& L, const Stencil<T>& A, T& diag,
+                                        T& off) {
+    diag = 0;
+    off = 0;
+#pragma unroll
+    for (int n = 0; n < 6; ++n) {
+        if (n >= 2 * G.dm) break;
+        const T w = mulT(A.b[n], (T)L.ih2[n >> 1]);
+        if ((A.m & kFull) || (L.mask[A.n[n]] & amr::kIn)) {
+            diag = addT(diag, w);
+            off = fmaT(w, A.u[n], off);
+        } else {
+            diag = fmaT((T)(2.0 / 3.0), w, diag);
+        }
     }
 }
 
 template <typename T>
-__global__ void k_reflux(Geo G, amr::LevT<T> F, amr::LevT<T> C, const T* uf, const T* uc, T* res,
-                         long N) {
-    AMR_LOOP(N) amr::reflux_cell(G, F, C, idx, uf, uc, res);
+__device__ __forceinline__ void defect_near(const Geo& G, const amr::LevT<T>& L, const Stencil<T>& A,
+                                            unsigned q, bool cu, T* __restrict__ r) {
+    if (!(A.m & amr::kIn)) {
+        r[q] = 0;
+    } else if (std::is_same<T, double>::value && (A.m & kFull)) {
+        T s = A.f;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            if (d >= G.dm) break;
+            T t = A.b[2 * d] * (A.u[2 * d] - A.uc);
+            t = fma(A.b[2 * d + 1], A.u[2 * d + 1] - A.uc, t);
+            s = fma((T)L.ih2[d], t, s);
+        }
+        r[q] = s;
+    } else if ((A.m & kFull) || ((A.m & kNear) && !cu)) {
+        T dg, off;
+        near_op(G, L, A, dg, off);
+        r[q] = addT(A.f, -fmaT(dg, A.uc, -off));
+    }
 }
 
 template <typename T>
-__global__ void k_restrict(Geo G, amr::LevT<T> F, amr::LevT<T> C, const T* fine, T* crse, long N) {
-    AMR_LOOP(N) amr::restrict_cell(G, F, C, idx, fine, crse);
+__device__ __forceinline__ void gsrb_near(const Geo& G, const amr::LevT<T>& L, const Stencil<T>& A,
+                                          unsigned q, T* u) {
+    if (!(A.m & amr::kIn)) return;
+    if (std::is_same<T, double>::value && (A.m & kFull)) {
+        T dg = 0, s = A.f;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            if (d >= G.dm) break;
+            T t = A.b[2 * d] * A.u[2 * d];
+            t = fma(A.b[2 * d + 1], A.u[2 * d + 1], t);
+            dg = fma((T)L.ih2[d], A.b[2 * d] + A.b[2 * d + 1], dg);
+            s = fma((T)L.ih2[d], t, s);
+        }
+        u[q] = s * recip(dg);
+    } else if (A.m & (kFull | kNear)) {
+        T dg, off;
+        near_op<T>(G, L, A, dg, off);
+        u[q] = (A.f + off) / dg;
+    }
 }
 
+// Two planes a thread: twice the loads in flight.
+constexpr int kPlanes = 2;
+inline int plane_blocks(int planes) { return (planes + kPlanes - 1) / kPlanes; }
+
 template <typename T>
-__global__ void k_prolong(Geo G, amr::LevT<T> F, amr::LevT<T> C, const T* uc, T* uf, long N) {
-    AMR_LOOP(N) amr::prolong_cell(G, F, C, idx, uc, uf);
+__global__ void __launch_bounds__(kThreads)
+k_defect(Geo G, amr::LevT<T> L, amr::LevT<T> C, Plane P, Rest R, const T* __restrict__ u,
+         const T* __restrict__ cu, const T* __restrict__ f, T* __restrict__ r) {
+    const int nz = (L.ext[2] + kPlanes - 1) / kPlanes;
+    if (blockIdx.z >= (unsigned)nz) {
+        const int q = rest_index(nz, R);
+        if (q >= 0) amr::defect_cell(G, L, C, (long)q, u, cu, f, r);
+        return;
+    }
+    Cell c[kPlanes];
+    Stencil<T> A[kPlanes];
+    bool on[kPlanes];
+#pragma unroll
+    for (int p = 0; p < kPlanes; ++p) {
+        on[p] = plane_cell(L, P, kPlanes * blockIdx.z + p, c[p]);
+        if (on[p]) load_stencil(G, L, c[p], u, f, A[p]);
+    }
+#pragma unroll
+    for (int p = 0; p < kPlanes; ++p)
+        if (on[p]) defect_near(G, L, A[p], c[p].q, cu != nullptr, r);
+}
+
+// One colour of a sweep, zero coarse data.
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+k_gsrb(Geo G, amr::LevT<T> L, Plane P, Rest R, int colour, T* u, const T* __restrict__ f) {
+    const int nz = (L.ext[2] + kPlanes - 1) / kPlanes;
+    if (blockIdx.z >= (unsigned)nz) {
+        const int q = rest_index(nz, R);
+        if (q >= 0) amr::gsrb_cell(G, L, (long)q, colour, u, f);
+        return;
+    }
+    Cell c[kPlanes];
+    Stencil<T> A[kPlanes];
+    bool on[kPlanes];
+#pragma unroll
+    for (int p = 0; p < kPlanes; ++p) {
+        on[p] = colour_plane_cell(L, P, colour, kPlanes * blockIdx.z + p, c[p]);
+        if (on[p]) load_stencil(G, L, c[p], u, f, A[p]);
+    }
+#pragma unroll
+    for (int p = 0; p < kPlanes; ++p)
+        if (on[p]) gsrb_near(G, L, A[p], c[p].q, u);
+}
+
+// The coarse cells that take a reflux, by list (a scan of the coarse level's mask took 67 us at
+// 128^3 for 25 thousand cells).
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+k_reflux(Geo G, amr::LevT<T> F, amr::LevT<T> C, const T* uf, const T* uc, T* res, const int* list, int n) {
+    const int t = blockIdx.x * kThreads + threadIdx.x;
+    if (t < n) amr::reflux_cell(G, F, C, (long)list[t], uf, uc, res);
+}
+
+// Covered coarse cells, by list (coarse cell, first child): the mean of the children.
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+k_restrict(Geo G, amr::LevT<T> F, const T* __restrict__ fine, T* __restrict__ crse,
+           const int2* __restrict__ list, int n) {
+    const int t = blockIdx.x * kThreads + threadIdx.x;
+    if (t >= n) return;
+    const int2 q = list[t];
+    const unsigned e0 = F.ext[0], pl = e0 * F.ext[1];
+    T s = 0;
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+        if (a >= (1 << G.dm)) break;
+        s += fine[(unsigned)q.y + (a & 1) + (a & 2 ? e0 : 0u) + (a & 4 ? pl : 0u)];
+    }
+    crse[q.x] = s / (T)(1 << G.dm);
+}
+
+// Multilinear interpolation to the region cells, 0 elsewhere (amr::prolong_cell): the coarse
+// neighbours of a cell away from the domain faces at constant offsets.
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+k_prolong(Geo G, amr::LevT<T> F, amr::LevT<T> C, Plane P, const T* __restrict__ uc, T* __restrict__ uf) {
+    Cell c;
+    if (!plane_cell(F, P, blockIdx.z, c)) return;
+    const unsigned char m = F.mask[c.q];
+    if (!(m & amr::kIn)) {
+        uf[c.q] = 0;
+        return;
+    }
+    const int g[3] = {F.lo[0] + (int)c.i, F.lo[1] + (int)c.j, F.lo[2] + (int)blockIdx.z};
+    bool in = true;
+    int at[3], st[3];
+    const int sz[3] = {1, C.ext[0], C.ext[0] * C.ext[1]};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        at[d] = d < G.dm ? (g[d] >> 1) - C.lo[d] : 0;
+        const int o = d < G.dm ? (g[d] & 1 ? 1 : -1) : 0;
+        st[d] = o * sz[d];
+        in = in && at[d] + o >= 0 && at[d] + o < C.ext[d];
+    }
+    if (!in) {
+        amr::prolong_cell(G, F, C, (long)c.q, uc, uf);
+        return;
+    }
+    const T* b = uc + (at[0] + at[1] * sz[1] + at[2] * sz[2]);
+    T s = 0;
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+        if (a >= (1 << G.dm)) break;
+        T w = 1;
+        int o = 0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            if (d >= G.dm) break;
+            w *= (a >> d) & 1 ? (T)0.25 : (T)0.75;
+            o += (a >> d) & 1 ? st[d] : 0;
+        }
+        s += w * b[o];
+    }
+    uf[c.q] = s;
 }
 
 template <typename T>
@@ -75,92 +354,125 @@ __global__ void k_add_region(amr::LevT<T> L, T* phi, const T* uu, long N) {
     AMR_LOOP(N) if (amr::in_region(L, idx)) phi[idx] += uu[idx];
 }
 
-// Per-block partials over the cells of one level: [0] sum of vol * x, [1] max |x|, [2] NaN
-// count, [3] volume.  valid_only: valid cells (kIn without kCov), else every region cell.
-template <typename T>
+// Per-block partials over the cells of one level: [0] vol * sum of x, [1] max |x|, [2] NaN
+// count (an integer's bits), [3] volume.  valid_only: valid cells (kIn without kCov), else every region cell.
+// SUM: with the sum and the volume (a maximum alone issues no FP64 instruction).
+template <typename T, bool SUM>
 __global__ void k_reduce(amr::LevT<T> L, const T* x, double vol, int valid_only, double* part,
                          long N) {
-    // Only the volume-weighted sum is FP64 arithmetic: the NaN test and the maximum of |x| work
-    // on the IEEE bits (for non-negative doubles the unsigned order of the bits is the numeric
-    // order), the cells are counted as integers and the volume is vol x count, a float's
-    // widening takes the integer pipe: GB300's FP64 pipe is the narrow one.
-    __shared__ double s_sum[kThreads / 32], s_vol[kThreads / 32];
-    __shared__ unsigned long long s_max[kThreads / 32], s_nan[kThreads / 32];
+    // Only the sum is FP64 arithmetic: the NaN test and the maximum of |x| work on the IEEE bits
+    // (for non-negative doubles the unsigned order of the bits is the numeric order), the cells
+    // are counted as integers, the volume multiplies once, a float's widening takes the integer
+    // pipe: GB300's FP64 pipe is the narrow one.  Eight cells' loads are in flight a thread (one at
+    // a time the 2.2 M cells of a 130^3 box took 28 us).
+    __shared__ double s_sum[kThreads / 32];
+    __shared__ unsigned long long s_max[kThreads / 32], s_nan[kThreads / 32], s_cnt[kThreads / 32];
+    constexpr int kU = 8;
     double sum = 0.0;
     unsigned long long mx = 0, nan = 0, cnt = 0;
-    AMR_LOOP(N) {
-        const bool take = valid_only ? amr::is_valid(L, idx) : amr::in_region(L, idx);
-        if (!take) continue;
-        double a;
-        if (std::is_same<T, float>::value)
-            a = to_double((float)x[idx]);
-        else
-            a = (double)x[idx];
-        const unsigned long long b = (unsigned long long)__double_as_longlong(a) & 0x7fffffffffffffffull;
-        if (b > 0x7ff0000000000000ull) {
-            ++nan;
-            continue;
+    const unsigned char want = amr::kIn, sel = valid_only ? (amr::kIn | amr::kCov) : amr::kIn;
+    for (long base = (long)blockIdx.x * kThreads * kU; base < N; base += (long)gridDim.x * kThreads * kU) {
+        T v[kU];
+        unsigned char m[kU];
+#pragma unroll
+        for (int q = 0; q < kU; ++q) {
+            const long idx = base + q * kThreads + threadIdx.x;
+            m[q] = idx < N ? L.mask[idx] : 0;
+            v[q] = idx < N ? x[idx] : T(0);
         }
-        sum = fma(vol, a, sum);
-        mx = b > mx ? b : mx;
-        ++cnt;
+#pragma unroll
+        for (int q = 0; q < kU; ++q) {
+            if ((m[q] & sel) != want) continue;
+            double a;
+            if (std::is_same<T, float>::value)
+                a = to_double((float)v[q]);
+            else
+                a = (double)v[q];
+            const unsigned long long b = (unsigned long long)__double_as_longlong(a) & 0x7fffffffffffffffull;
+            if (b > 0x7ff0000000000000ull) {
+                ++nan;
+                continue;
+            }
+            if (SUM) sum += a;
+            mx = b > mx ? b : mx;
+            ++cnt;
+        }
     }
-    double v = vol * (double)cnt;
     for (int o = 16; o > 0; o >>= 1) {
-        sum += __shfl_down_sync(0xffffffffu, sum, o);
+        if (SUM) sum += __shfl_down_sync(0xffffffffu, sum, o);
         const unsigned long long m = __shfl_down_sync(0xffffffffu, mx, o);
         mx = m > mx ? m : mx;
         nan += __shfl_down_sync(0xffffffffu, nan, o);
-        v += __shfl_down_sync(0xffffffffu, v, o);
+        cnt += __shfl_down_sync(0xffffffffu, cnt, o);
     }
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (lane == 0) {
         s_sum[w] = sum;
         s_max[w] = mx;
         s_nan[w] = nan;
-        s_vol[w] = v;
+        s_cnt[w] = cnt;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int q = 1; q < kThreads / 32; ++q) {
-            sum += s_sum[q];
+            if (SUM) sum += s_sum[q];
             mx = s_max[q] > mx ? s_max[q] : mx;
             nan += s_nan[q];
-            v += s_vol[q];
+            cnt += s_cnt[q];
         }
         double* p = part + 4 * blockIdx.x;
-        p[0] = sum;
+        const double v = SUM ? vol * (double)cnt : 0.0;
+        p[0] = SUM ? vol * sum : 0.0;
         p[1] = __longlong_as_double((long long)mx);
-        p[2] = (double)nan;
+        p[2] = __longlong_as_double((long long)nan);
         p[3] = v;
     }
 }
 
 // out[0] sum, out[1] max, out[2] NaN count, out[3] volume, out[4] mean = sum / volume; one
 // block, fixed order (deterministic).
-__global__ void k_reduce_finish(const double* part, int nparts, double* out) {
-    __shared__ double s[4][kThreads];
-    double a[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int q = threadIdx.x; q < nparts; q += blockDim.x) {
-        a[0] += part[4 * q];
-        a[1] = fmax(a[1], part[4 * q + 1]);
-        a[2] += part[4 * q + 2];
-        a[3] += part[4 * q + 3];
+__global__ void __launch_bounds__(kThreads)
+k_reduce_finish(const double* part, int nparts, double* out) {
+    __shared__ double s[2][kThreads / 32];
+    __shared__ unsigned long long sm[2][kThreads / 32];
+    double sum = 0.0, vol = 0.0;
+    unsigned long long mx = 0, nan = 0;
+    for (int q = threadIdx.x; q < nparts; q += kThreads) {
+        const double2 a = reinterpret_cast<const double2*>(part)[2 * q];
+        const double2 b = reinterpret_cast<const double2*>(part)[2 * q + 1];
+        const unsigned long long m = (unsigned long long)__double_as_longlong(a.y);
+        sum += a.x;
+        vol += b.y;
+        mx = m > mx ? m : mx;
+        nan += (unsigned long long)__double_as_longlong(b.x);
     }
-    for (int k = 0; k < 4; ++k) s[k][threadIdx.x] = a[k];
+    for (int o = 16; o > 0; o >>= 1) {
+        sum += __shfl_down_sync(0xffffffffu, sum, o);
+        vol += __shfl_down_sync(0xffffffffu, vol, o);
+        const unsigned long long m = __shfl_down_sync(0xffffffffu, mx, o);
+        mx = m > mx ? m : mx;
+        nan += __shfl_down_sync(0xffffffffu, nan, o);
+    }
+    const int w = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) {
+        s[0][w] = sum;
+        s[1][w] = vol;
+        sm[0][w] = mx;
+        sm[1][w] = nan;
+    }
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) {
-            s[0][threadIdx.x] += s[0][threadIdx.x + w];
-            s[1][threadIdx.x] = fmax(s[1][threadIdx.x], s[1][threadIdx.x + w]);
-            s[2][threadIdx.x] += s[2][threadIdx.x + w];
-            s[3][threadIdx.x] += s[3][threadIdx.x + w];
-        }
-        __syncthreads();
-    }
     if (threadIdx.x == 0) {
-        for (int k = 0; k < 4; ++k) out[k] = s[k][0];
-        out[4] = s[3][0] > 0.0 ? s[0][0] / s[3][0] : 0.0;
+        for (int q = 1; q < kThreads / 32; ++q) {
+            sum += s[0][q];
+            vol += s[1][q];
+            mx = sm[0][q] > mx ? sm[0][q] : mx;
+            nan += sm[1][q];
+        }
+        out[0] = sum;
+        out[1] = __longlong_as_double((long long)mx);
+        out[2] = (double)nan;
+        out[3] = vol;
+        out[4] = vol > 0.0 ? sum / vol : 0.0;
     }
 }
 
@@ -174,33 +486,135 @@ __global__ void k_sub_scalar(amr::LevT<T> L, T* x, const double* m, int valid_on
     }
 }
 
-__global__ void k_scale_b0(Geo G, Lev L, int d, double* u, const double* b0, const double* b0e,
-                           int mult, long N) {
-    AMR_LOOP(N) {
-        int f[3];
-        amr::face_coords(L, d, idx, f);
-        const double bb = amr::beta0_of_face(G, d, f, b0, b0e);
-        u[idx] = mult ? u[idx] * bb : u[idx] / bb;
+// Level-0 arrays, natural layout <-> the one-level solver's, less *mean (null: 0); in: the
+// correction starts from zero.
+template <typename T>
+__global__ void k_level0_in(Dims d, const T* __restrict__ src, const double* mean, T* __restrict__ f,
+                            T* __restrict__ phi) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = blockIdx.z;
+    if (i >= d.n0 || j >= d.n1) return;
+    const int q = level_index(d, i, j, k);
+    const T v = src[i + d.n0 * (j + d.n1 * k)];
+    f[q] = mean ? v - (T)*mean : v;
+    phi[q] = T(0);
+}
+template <typename T>
+__global__ void k_level0_out(Dims d, const T* __restrict__ phi, const double* mean, T* __restrict__ e) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = blockIdx.z;
+    if (i >= d.n0 || j >= d.n1) return;
+    const T v = phi[level_index(d, i, j, k)];
+    e[i + d.n0 * (j + d.n1 * k)] = mean ? v - (T)*mean : v;
+}
+
+// ---- face kernels: one thread per face of a plane of the array box, planes along blockIdx.z ----
+struct Face {
+    unsigned q, f[3];     // index; box coordinates
+    unsigned hi, lo;      // the cells on either side, when both are in the box (two)
+    bool two;
+};
+__device__ __forceinline__ bool plane_face(const Lev& L, int d, Plane P, Face& c) {
+    const unsigned m0 = L.ext[0] + (d == 0), m1 = L.ext[1] + (d == 1);
+    const unsigned t = blockIdx.x * kThreads + threadIdx.x;
+    if (t >= m0 * m1) return false;
+    c.f[1] = row_of(t, m0, P);
+    c.f[0] = t - c.f[1] * m0;
+    c.f[2] = blockIdx.z;
+    c.q = t + m0 * m1 * c.f[2];
+    const unsigned e0 = L.ext[0], e1 = L.ext[1];
+    c.hi = c.f[0] + e0 * (c.f[1] + e1 * c.f[2]);
+    c.lo = c.hi - (d == 0 ? 1u : d == 1 ? e0 : e0 * e1);
+    c.two = c.f[d] >= 1 && c.f[d] < (unsigned)L.ext[d];
+    return true;
+}
+inline dim3 face_grid(const Lev& L, int d) {
+    return plane_grid((long)(L.ext[0] + (d == 0)) * (L.ext[1] + (d == 1)), L.ext[2] + (d == 2));
+}
+inline Plane face_plane(const Lev& L, int d) { return plane(L.ext[0] + (d == 0), L.ext[1] + (d == 1)); }
+
+// Whether the face borders a region cell (amr::face_in_level).
+__device__ __forceinline__ bool face_used(const Geo& G, const Lev& L, int d, const Face& c) {
+    if (c.two) return (L.mask[c.hi] | L.mask[c.lo]) & amr::kIn;
+    int f[3];
+    amr::face_coords(L, d, (long)c.q, f);
+    return amr::face_in_level(G, L, d, f);
+}
+
+__global__ void __launch_bounds__(kThreads)
+k_scale_b0(Geo G, Lev L, int d, Plane P, double* u, const double* b0, const double* b0e, int mult) {
+    Face c;
+    if (!plane_face(L, d, P, c)) return;
+    const int r = L.lo[G.va] + (int)(G.va == 2 ? c.f[2] : c.f[1]);
+    const double bb = d == G.va ? b0e[r] : b0[r];
+    u[c.q] *= mult ? bb : recip_nr(bb);
+}
+
+// Coarse faces away from covered cells keep their values.
+__global__ void __launch_bounds__(kThreads)
+k_edge_restrict(Geo G, Lev F, Lev C, int d, Plane P, double* uc, const double* uf) {
+    Face c;
+    if (!plane_face(C, d, P, c)) return;
+    if (c.two && !((C.mask[c.hi] | C.mask[c.lo]) & amr::kCov)) return;
+    amr::edge_restrict_face(G, F, C, d, (long)c.q, uc, uf);
+}
+
+// rh = -(div(beta0 U) - macrhs) on region cells (U already holds beta0 U), 0 elsewhere.
+__global__ void __launch_bounds__(kThreads)
+k_divergence(Geo G, Lev L, Plane P, const double* __restrict__ u0, const double* __restrict__ u1,
+             const double* __restrict__ u2, const double* __restrict__ macrhs, double* __restrict__ rh) {
+    Cell c;
+    if (!plane_cell(L, P, blockIdx.z, c)) return;
+    if (!(L.mask[c.q] & amr::kIn)) {
+        rh[c.q] = 0.0;
+        return;
     }
+    const unsigned e0 = L.ext[0], f0 = c.q + c.r, f1 = c.q + e0 * blockIdx.z;
+    double s = macrhs ? macrhs[c.q] : 0.0;
+    s = fma(-L.ih[0], u0[f0 + 1] - u0[f0], s);
+    s = fma(-L.ih[1], u1[f1 + e0] - u1[f1], s);
+    if (G.dm > 2) s = fma(-L.ih[2], u2[c.q + e0 * L.ext[1]] - u2[c.q], s);
+    rh[c.q] = s;
 }
 
-__global__ void k_edge_restrict(Geo G, Lev F, Lev C, int d, double* uc, const double* uf, long N) {
-    AMR_LOOP(N) amr::edge_restrict_face(G, F, C, d, idx, uc, uf);
+// Solver coefficient of a face of the level (amr::coeff_face).
+__global__ void __launch_bounds__(kThreads)
+k_coeff(Geo G, Lev L, int d, Plane P, const double* __restrict__ rho, const double* __restrict__ b0,
+        const double* __restrict__ b0e, int alt, double* __restrict__ beta) {
+    Face c;
+    if (!plane_face(L, d, P, c)) return;
+    if (!c.two) {
+        amr::coeff_face(G, L, d, (long)c.q, rho, b0, b0e, alt, beta);
+        return;
+    }
+    if (!((L.mask[c.hi] | L.mask[c.lo]) & amr::kIn)) return;
+    double v = 2.0 * recip_nr(rho[c.hi] + rho[c.lo]);
+    if (b0) {
+        const int r = L.lo[G.va] + (int)(G.va == 2 ? c.f[2] : c.f[1]);
+        const double bb = d == G.va ? b0e[r] : b0[r];
+        v *= bb;
+        if (alt) v *= bb;
+    }
+    beta[c.q] = v;
 }
 
-__global__ void k_divergence(Geo G, Lev L, const double* u0, const double* u1, const double* u2,
-                             const double* macrhs, double* rh, long N) {
-    AMR_LOOP(N) amr::divergence_cell(G, L, idx, u0, u1, u2, macrhs, rh);
-}
-
-__global__ void k_coeff(Geo G, Lev L, int d, const double* rho, const double* b0,
-                        const double* b0e, int alt, double* beta, long N) {
-    AMR_LOOP(N) amr::coeff_face(G, L, d, idx, rho, b0, b0e, alt, beta);
-}
-
-__global__ void k_correct(Geo G, Lev L, Lev C, int d, const double* phi, const double* cphi,
-                          const double* beta, double* u, long N) {
-    AMR_LOOP(N) amr::correct_face(G, L, C, d, idx, phi, cphi, beta, u);
+// beta0 U -= beta G phi on a face of the level (amr::correct_face).
+__global__ void __launch_bounds__(kThreads)
+k_correct(Geo G, Lev L, Lev C, int d, Plane P, const double* phi, const double* cphi,
+          const double* beta, double* u) {
+    Face c;
+    if (!plane_face(L, d, P, c)) return;
+    if (c.two) {
+        const int n = (L.mask[c.hi] & amr::kIn) + (L.mask[c.lo] & amr::kIn);
+        if (n == 0) return;
+        if (n == 2 * amr::kIn) {
+            u[c.q] = fma(-beta[c.q] * L.ih[d], phi[c.hi] - phi[c.lo], u[c.q]);
+            return;
+        }
+    }
+    amr::correct_face(G, L, C, d, (long)c.q, phi, cphi, beta, u);
 }
 
 // A density that is not positive and finite on a cell the level's faces read (its region and
@@ -226,21 +640,32 @@ __global__ void k_check_rho(Geo G, Lev L, const double* rho, int* flag, long N) 
 
 // The caller's whole-level-domain arrays <-> the level's box arrays (back: the level's own faces
 // and region cells only).
-__global__ void k_full_to_box_faces(Lev L, int d, const double* full, double* box, long N) {
-    AMR_LOOP(N) box[idx] = full[amr::full_face(L, d, idx)];
+__device__ __forceinline__ size_t full_face(const Lev& L, int d, const Face& c) {
+    const size_t m0 = L.n[0] + (d == 0), m1 = L.n[1] + (d == 1);
+    return (c.f[0] + L.lo[0]) + m0 * ((c.f[1] + L.lo[1]) + m1 * (size_t)(c.f[2] + L.lo[2]));
 }
-__global__ void k_full_to_box_cells(Lev L, const double* full, double* box, long N) {
-    AMR_LOOP(N) box[idx] = full[amr::full_cell(L, idx)];
+__device__ __forceinline__ size_t full_cell(const Lev& L, const Cell& c) {
+    return (c.i + L.lo[0]) + (size_t)L.n[0] * ((c.j + L.lo[1]) + (size_t)L.n[1] * (blockIdx.z + L.lo[2]));
 }
-__global__ void k_box_to_full_faces(Geo G, Lev L, int d, const double* box, double* full, long N) {
-    AMR_LOOP(N) {
-        int f[3];
-        amr::face_coords(L, d, idx, f);
-        if (amr::face_in_level(G, L, d, f)) full[amr::full_face(L, d, idx)] = box[idx];
-    }
+__global__ void __launch_bounds__(kThreads)
+k_full_to_box_faces(Lev L, int d, Plane P, const double* __restrict__ full, double* __restrict__ box) {
+    Face c;
+    if (plane_face(L, d, P, c)) box[c.q] = full[full_face(L, d, c)];
 }
-__global__ void k_box_to_full_cells(Lev L, const double* box, double* full, long N) {
-    AMR_LOOP(N) if (amr::in_region(L, idx)) full[amr::full_cell(L, idx)] = box[idx];
+__global__ void __launch_bounds__(kThreads)
+k_full_to_box_cells(Lev L, Plane P, const double* __restrict__ full, double* __restrict__ box) {
+    Cell c;
+    if (plane_cell(L, P, blockIdx.z, c)) box[c.q] = full[full_cell(L, c)];
+}
+__global__ void __launch_bounds__(kThreads)
+k_box_to_full_faces(Geo G, Lev L, int d, Plane P, const double* __restrict__ box, double* __restrict__ full) {
+    Face c;
+    if (plane_face(L, d, P, c) && face_used(G, L, d, c)) full[full_face(L, d, c)] = box[c.q];
+}
+__global__ void __launch_bounds__(kThreads)
+k_box_to_full_cells(Lev L, Plane P, const double* __restrict__ box, double* __restrict__ full) {
+    Cell c;
+    if (plane_cell(L, P, blockIdx.z, c) && (L.mask[c.q] & amr::kIn)) full[full_cell(L, c)] = box[c.q];
 }
 
 __global__ void k_sync_periodic_faces(Geo G, Lev L, int d, double* u, long N) {
@@ -313,6 +738,14 @@ struct AmrState {
         float* buf32[amr::kNumBufs] = {};
         double* phi_user = nullptr;   // the caller's phi of this call (aliases buf kPhi)
         long ncell = 0;
+        // cells of the next coarser level: those that take this level's reflux; the covered ones
+        // with their first child
+        int* reflux = nullptr;
+        int2* cover = nullptr;
+        int nreflux = 0, ncover = 0;
+        // this level's region cells that are not kNear (nrest), then those that are not kFull
+        int* rest = nullptr;
+        int nrest = 0, nrest_cu = 0;
     };
     std::vector<LevelStore> L;
     // per-box (fab) calls: level arrays of the inputs, fab tables, host-pointer staging
@@ -376,7 +809,7 @@ int amr_alloc(AmrState* A, T** p, size_t n) {
 int build_masks(const mac_ctx* c, int nlev, const int* nboxes, const int* box_lo,
                 const int* box_hi, std::vector<std::vector<unsigned char>>& masks,
                 std::vector<std::vector<int>>& boxes, std::vector<Lev>& geom) {
-    const int dm = c->dm;
+    const int dm = c->dm;   // (the masks' kFull and kNear bits: classify)
     masks.assign(nlev, {});
     boxes.assign(nlev, {});
     geom.assign(nlev, Lev{});
@@ -456,6 +889,68 @@ int build_masks(const mac_ctx* c, int nlev, const int* nboxes, const int* box_lo
     return MAC_OK;
 }
 
+// The kernels' bits of a level's mask, kNear and kFull (see the cell kernels), and the list of the
+// region cells without kNear, then of those without kFull; *nrest: how many the first are.
+std::vector<int> classify(int dm, const Lev& V, std::vector<unsigned char>& mask, int* nrest) {
+    const int e0 = V.ext[0], e1 = V.ext[1], e2 = V.ext[2];
+    const long pl = (long)e0 * e1;
+    std::vector<int> far, part;
+    for (int k = 0; k < e2; ++k)
+        for (int j = 0; j < e1; ++j) {
+            unsigned char* m = mask.data() + pl * k + (long)e0 * j;
+            const bool row = (dm < 2 || (j > 0 && j < e1 - 1)) && (dm < 3 || (k > 0 && k < e2 - 1));
+            for (int i = 0; i < e0; ++i) {
+                if (!(m[i] & amr::kIn)) continue;
+                const int idx = (int)(pl * k + (long)e0 * j + i);
+                if (!row || i == 0 || i == e0 - 1) {
+                    far.push_back(idx);
+                    continue;
+                }
+                unsigned char all = m[i - 1] & m[i + 1];
+                if (dm > 1) all &= m[i - e0] & m[i + e0];
+                if (dm > 2) all &= m[i - pl] & m[i + pl];
+                m[i] |= (all & amr::kIn) ? (unsigned char)(kNear | kFull) : kNear;
+                if (!(all & amr::kIn)) part.push_back(idx);
+            }
+        }
+    *nrest = (int)far.size();
+    far.insert(far.end(), part.begin(), part.end());
+    return far;
+}
+
+// Lists of level l >= 1: the valid cells of level l - 1 beside a covered one, the covered ones
+// with their first child.
+void coarse_lists(const mac_ctx* c, const Lev& F, const Lev& K, const std::vector<unsigned char>& mask,
+                  std::vector<int>& reflux, std::vector<int2>& cover) {
+    const int dm = c->dm;
+    std::vector<unsigned char> beside(mask.size(), 0);   // valid cells taken already
+    long idx = 0;
+    for (int k = 0; k < K.ext[2]; ++k)
+        for (int j = 0; j < K.ext[1]; ++j)
+            for (int i = 0; i < K.ext[0]; ++i, ++idx) {
+                if (!(mask[(size_t)idx] & amr::kCov)) continue;
+                const int q[3] = {K.lo[0] + i, K.lo[1] + j, K.lo[2] + k};
+                const int f[3] = {2 * q[0], dm > 1 ? 2 * q[1] : q[1], dm > 2 ? 2 * q[2] : q[2]};
+                cover.push_back(make_int2((int)idx, (int)amr::cix(F, f[0], f[1], f[2])));
+                for (int d = 0; d < dm; ++d)
+                    for (int s = -1; s <= 1; s += 2) {
+                        int p[3] = {q[0], q[1], q[2]};
+                        p[d] += s;
+                        if (p[d] < 0 || p[d] >= K.n[d]) {
+                            if (c->bc_lo[d] != MAC_BC_PER) continue;
+                            p[d] += p[d] < 0 ? K.n[d] : -K.n[d];
+                        }
+                        if (!amr::inside(K, p)) continue;
+                        const size_t n = (size_t)amr::cix(K, p[0], p[1], p[2]);
+                        if ((mask[n] & (amr::kIn | amr::kCov)) == amr::kIn && !beside[n]) {
+                            beside[n] = 1;
+                            reflux.push_back((int)n);
+                        }
+                    }
+            }
+    std::sort(reflux.begin(), reflux.end());
+}
+
 // The executor of amr_solve / amr_project on the context's stream.
 // Level accessors per precision.
 template <typename T> struct AmrAccess;
@@ -484,6 +979,8 @@ struct GpuMl {
     T* buf(int l, int which) const { return AmrAccess<T>::buf(A->L[l], which); }
     long ncell(int l) const { return A->L[l].ncell; }
     int blocks(long n) const { return blocks_for(n, c->sms); }
+    static Plane cell_plane(const amr::LevT<T>& L) { return plane(L.ext[0], L.ext[1]); }
+    static dim3 cell_grid(const amr::LevT<T>& L) { return plane_grid((long)L.ext[0] * L.ext[1], L.ext[2]); }
     void launched() {
         ++c->issued;
         if (!err && cudaPeekAtLastError() != cudaSuccess) {
@@ -495,7 +992,11 @@ struct GpuMl {
 
     void defect(int l, const T* uu, const T* cu, const T* f, T* r) {
         const amr::LevT<T> C = l ? lev(l - 1) : lev(l);
-        k_defect<T><<<blocks(ncell(l)), kThreads, 0, c->stream>>>(geo, lev(l), C, uu, cu, f, r, ncell(l));
+        const amr::LevT<T> L = lev(l);
+        const AmrState::LevelStore& S = A->L[l];
+        const Rest R{S.rest, cu ? S.nrest_cu : S.nrest};
+        k_defect<T><<<plane_grid((long)L.ext[0] * L.ext[1], plane_blocks(L.ext[2]), R.n), kThreads, 0, c->stream>>>(
+            geo, L, C, cell_plane(L), R, uu, cu, f, r);
         launched();
     }
     cudaEvent_t next_event() {
@@ -528,21 +1029,30 @@ struct GpuMl {
     void gsrb_launch(int l, T* uu, const T* f, int nu) {
         for (int s = 0; s < nu; ++s)
             for (int colour = 0; colour < 2; ++colour) {
-                const long nt = amr::colour_threads(lev(l));
-                k_gsrb<T><<<blocks(nt), kThreads, 0, c->stream>>>(geo, lev(l), colour, uu, f, nt);
+                const amr::LevT<T> L = lev(l);
+                const int hw = (L.ext[0] + 1) / 2;
+                const Rest R{A->L[l].rest, A->L[l].nrest};
+                k_gsrb<T><<<plane_grid((long)hw * L.ext[1], plane_blocks(L.ext[2]), R.n), kThreads, 0, c->stream>>>(
+                    geo, L, plane(hw, L.ext[1]), R, colour, uu, f);
                 launched();
             }
     }
     void reflux(int l, const T* uf, const T* uc, T* res) {
-        k_reflux<T><<<blocks(ncell(l - 1)), kThreads, 0, c->stream>>>(geo, lev(l), lev(l - 1), uf, uc, res, ncell(l - 1));
+        const AmrState::LevelStore& S = A->L[l];
+        if (S.nreflux == 0) return;   // (the level covers the whole coarser one)
+        k_reflux<T><<<ceil_div(S.nreflux, kThreads), kThreads, 0, c->stream>>>(
+            geo, lev(l), lev(l - 1), uf, uc, res, S.reflux, S.nreflux);
         launched();
     }
     void restrict_cov(int l, const T* fine, T* crse) {
-        k_restrict<T><<<blocks(ncell(l - 1)), kThreads, 0, c->stream>>>(geo, lev(l), lev(l - 1), fine, crse, ncell(l - 1));
+        const AmrState::LevelStore& S = A->L[l];
+        k_restrict<T><<<ceil_div(S.ncover, kThreads), kThreads, 0, c->stream>>>(geo, lev(l), fine, crse,
+                                                                               S.cover, S.ncover);
         launched();
     }
     void prolong(int l, const T* uc, T* uf) {
-        k_prolong<T><<<blocks(ncell(l)), kThreads, 0, c->stream>>>(geo, lev(l), lev(l - 1), uc, uf, ncell(l));
+        const amr::LevT<T> L = lev(l);
+        k_prolong<T><<<cell_grid(L), kThreads, 0, c->stream>>>(geo, L, lev(l - 1), cell_plane(L), uc, uf);
         launched();
     }
     void axpy3(int l, T* uu, const T* hold, const T* du) {
@@ -571,11 +1081,13 @@ struct GpuMl {
     // Partials of x over the valid cells (valid_only) or the region cells of level l, appended at
     // slot *nparts of A->part.
     template <typename U>
-    void reduce_level(int l, const U* x, int valid_only, int* nparts) {
+    void reduce_level(int l, const U* x, int valid_only, int* nparts, bool sum = true) {
         const amr::LevT<U> L = AmrAccess<U>::lev(A->L[l]);
         const double vol = L.h[0] * (geo.dm > 1 ? L.h[1] : 1.0) * (geo.dm > 2 ? L.h[2] : 1.0);
-        const int nb = std::min(kReduceBlocks, blocks(ncell(l)));
-        k_reduce<U><<<nb, kThreads, 0, c->stream>>>(L, x, vol, valid_only, A->part + 4 * *nparts, ncell(l));
+        // two blocks an SM: the block sums' FP64 instructions are not negligible beside one add a cell
+        const int nb = std::min(std::min(kReduceBlocks, 2 * std::max(1, c->sms)), ceil_div(ncell(l), kThreads * 8));
+        auto kern = sum ? k_reduce<U, true> : k_reduce<U, false>;
+        kern<<<nb, kThreads, 0, c->stream>>>(L, x, vol, valid_only, A->part + 4 * *nparts, ncell(l));
         launched();
         *nparts += nb;
     }
@@ -584,9 +1096,9 @@ struct GpuMl {
         launched();
     }
     // Reduce buf(which) over the valid cells of every level into A->out on the device.
-    void reduce(int which) {
+    void reduce(int which, bool sum) {
         int nparts = 0;
-        for (int l = 0; l < nlev; ++l) reduce_level<T>(l, buf(l, which), 1, &nparts);
+        for (int l = 0; l < nlev; ++l) reduce_level<T>(l, buf(l, which), 1, &nparts, sum);
         finish_reduce(nparts);
     }
     bool fetch() {
@@ -601,12 +1113,12 @@ struct GpuMl {
         return true;
     }
     double valid_max(int which) {
-        reduce(which);
+        reduce(which, false);
         if (!fetch()) return NAN;
         return A->h_out[2] > 0.0 ? NAN : A->h_out[1];
     }
     double valid_mean(int which) {
-        reduce(which);
+        reduce(which, true);
         if (!fetch()) return NAN;
         return A->h_out[4];
     }
@@ -619,76 +1131,42 @@ struct GpuMl {
         }
     }
 
-    // One FP64 V-cycle of the level-0 multigrid on rhs from a zero guess into e (natural layout);
-    // for a singular problem the mean of the right-hand side is removed first and the mean of
-    // the correction after (the constant is in the null space of the composite operator).
-    int level0_fp64(const double* rhs, double* e) {
-        if (err) return err;
-        Level& F = c->lev[0];
-        double* r0 = A->L[0].buf[amr::kTmp];
-        const amr::LevT<double> L0 = A->L[0].lev;
-        if (cudaMemcpyAsync(r0, rhs, sizeof(double) * ncell(0), cudaMemcpyDeviceToDevice, c->stream) != cudaSuccess)
-            err = MAC_ERR_CUDA;
-        if (!err && singular) {
-            int np = 0;
-            reduce_level<double>(0, r0, 0, &np);
-            finish_reduce(np);
-            k_sub_scalar<double><<<blocks(ncell(0)), kThreads, 0, c->stream>>>(L0, r0, A->out + 4, 0, ncell(0));
-            launched();
-        }
-        int rc = err ? err : natural_to_level0(c, r0, F.a64.f);
-        if (!rc && cudaMemsetAsync(F.a64.phi, 0, sizeof(double) * (size_t)F.d.ncell, c->stream) != cudaSuccess)
-            rc = MAC_ERR_CUDA;
-        if (!rc) rc = level0_fp64_vcycle(c);
-        if (!rc) rc = level0_to_natural(c, F.a64.phi, e);
-        if (!rc && singular) {
-            int np = 0;
-            reduce_level<double>(0, e, 0, &np);
-            finish_reduce(np);
-            k_sub_scalar<double><<<blocks(ncell(0)), kThreads, 0, c->stream>>>(L0, e, A->out + 4, 0, ncell(0));
-            launched();
-        }
-        if (rc && !err) err = rc;
-        return err;
-    }
-    // One FP32 V-cycle of the level-0 multigrid (the one-level solver's mixed-precision inner
-    // cycle: over-relaxed half-sweeps, its V-cycle shape and exact bottom) on rhs from a zero
-    // guess into e, natural layout; the means as in level0_fp64.
-    int level0_fp32(const float* rhs, float* e) {
-        if (err) return err;
-        Level& F = c->lev[0];
-        float* r0 = A->L[0].buf32[amr::kTmp];
-        const amr::LevT<float> L0 = A->L[0].lev32;
-        if (cudaMemcpyAsync(r0, rhs, sizeof(float) * ncell(0), cudaMemcpyDeviceToDevice, c->stream) != cudaSuccess)
-            err = MAC_ERR_CUDA;
-        if (!err && singular) {
-            int np = 0;
-            reduce_level<float>(0, r0, 0, &np);
-            finish_reduce(np);
-            k_sub_scalar<float><<<blocks(ncell(0)), kThreads, 0, c->stream>>>(L0, r0, A->out + 4, 0, ncell(0));
-            launched();
-        }
-        int rc = err ? err : natural_to_level0(c, r0, F.a32.f);
-        if (!rc && cudaMemsetAsync(F.a32.phi, 0, sizeof(float) * (size_t)F.d.ncell, c->stream) != cudaSuccess)
-            rc = MAC_ERR_CUDA;
-        if (!rc) rc = level0_fp32_vcycle(c);
-        if (!rc) rc = level0_to_natural(c, F.a32.phi, e);
-        if (!rc && singular) {
-            int np = 0;
-            reduce_level<float>(0, e, 0, &np);
-            finish_reduce(np);
-            k_sub_scalar<float><<<blocks(ncell(0)), kThreads, 0, c->stream>>>(L0, e, A->out + 4, 0, ncell(0));
-            launched();
-        }
-        if (rc && !err) err = rc;
-        return err;
-    }
+    // One V-cycle of the level-0 multigrid (T = float: the one-level solver's mixed-precision inner
+    // cycle -- over-relaxed half-sweeps, its V-cycle shape) on rhs from a zero guess into e, natural
+    // layout; for a singular problem the mean of the right-hand side comes off on the way in and the
+    // mean of the correction on the way out (the constant is in the null space of the composite
+    // operator).
     int level0_correction(const T* rhs, T* e) {
-        if constexpr (std::is_same<T, double>::value) {
-            return level0_fp64(rhs, e);
-        } else {
-            return level0_fp32(rhs, e);
+        if (err) return err;
+        Level& F = c->lev[0];
+        LevelArrays<T>* a;
+        if constexpr (std::is_same<T, double>::value)
+            a = &F.a64;
+        else
+            a = &F.a32;
+        const Grid3 g = grid3(F.d.n0, F.d.n1, F.d.n2);
+        int np = 0;
+        if (singular) {
+            reduce_level<T>(0, rhs, 0, &np);
+            finish_reduce(np);
         }
+        k_level0_in<T><<<g.grid, g.block, 0, c->stream>>>(F.d, rhs, singular ? A->out + 4 : nullptr, a->f, a->phi);
+        launched();
+        int rc = err;
+        if constexpr (std::is_same<T, double>::value) {
+            if (!rc) rc = level0_fp64_vcycle(c);
+        } else {
+            if (!rc) rc = level0_fp32_vcycle(c);
+        }
+        if (!rc && singular) {   // (every cell of level 0 is a region cell, whatever the layout)
+            np = 0;
+            reduce_level<T>(0, a->phi, 0, &np);
+            finish_reduce(np);
+        }
+        k_level0_out<T><<<g.grid, g.block, 0, c->stream>>>(F.d, a->phi, singular ? A->out + 4 : nullptr, e);
+        launched();
+        if (rc && !err) err = rc;
+        return err;
     }
 };
 
@@ -736,29 +1214,30 @@ struct GpuExec : GpuMl<double> {
     void scale_b0(int l, bool mult) {
         if (!b0) return;
         for (int d = 0; d < geo.dm; ++d) {
-            const long nf = amr::nfaces(lev(l), d);
-            k_scale_b0<<<blocks(nf), kThreads, 0, c->stream>>>(geo, lev(l), d, u[3 * l + d], b0[l], b0e[l], mult ? 1 : 0, nf);
+            k_scale_b0<<<face_grid(lev(l), d), kThreads, 0, c->stream>>>(
+                geo, lev(l), d, face_plane(lev(l), d), u[3 * l + d], b0[l], b0e[l], mult ? 1 : 0);
             launched();
         }
     }
     void edge_restrict(int l) {
         for (int d = 0; d < geo.dm; ++d) {
-            const long nf = amr::nfaces(lev(l - 1), d);
-            k_edge_restrict<<<blocks(nf), kThreads, 0, c->stream>>>(geo, lev(l), lev(l - 1), d, u[3 * (l - 1) + d], u[3 * l + d], nf);
+            const Lev K = lev(l - 1);
+            k_edge_restrict<<<face_grid(K, d), kThreads, 0, c->stream>>>(
+                geo, lev(l), K, d, face_plane(K, d), u[3 * (l - 1) + d], u[3 * l + d]);
             launched();
         }
     }
     void divergence(int l) {
-        k_divergence<<<blocks(ncell(l)), kThreads, 0, c->stream>>>(
-            geo, lev(l), u[3 * l], u[3 * l + 1], geo.dm == 3 ? u[3 * l + 2] : nullptr,
-            macrhs ? macrhs[l] : nullptr, buf(l, amr::kRh), ncell(l));
+        k_divergence<<<cell_grid(lev(l)), kThreads, 0, c->stream>>>(
+            geo, lev(l), cell_plane(lev(l)), u[3 * l], u[3 * l + 1], geo.dm == 3 ? u[3 * l + 2] : nullptr,
+            macrhs ? macrhs[l] : nullptr, buf(l, amr::kRh));
         launched();
     }
     void coeffs(int l) {
         for (int d = 0; d < geo.dm; ++d) {
-            const long nf = amr::nfaces(lev(l), d);
-            k_coeff<<<blocks(nf), kThreads, 0, c->stream>>>(geo, lev(l), d, rho[l], b0 ? b0[l] : nullptr,
-                                                            b0 ? b0e[l] : nullptr, alt, A->L[l].beta[d], nf);
+            k_coeff<<<face_grid(lev(l), d), kThreads, 0, c->stream>>>(
+                geo, lev(l), d, face_plane(lev(l), d), rho[l], b0 ? b0[l] : nullptr, b0 ? b0e[l] : nullptr,
+                alt, A->L[l].beta[d]);
             launched();
         }
     }
@@ -766,9 +1245,8 @@ struct GpuExec : GpuMl<double> {
         const Lev C = l ? lev(l - 1) : lev(l);
         const double* cphi = l ? buf(l - 1, amr::kPhi) : nullptr;
         for (int d = 0; d < geo.dm; ++d) {
-            const long nf = amr::nfaces(lev(l), d);
-            k_correct<<<blocks(nf), kThreads, 0, c->stream>>>(geo, lev(l), C, d, buf(l, amr::kPhi), cphi,
-                                                              A->L[l].beta[d], u[3 * l + d], nf);
+            k_correct<<<face_grid(lev(l), d), kThreads, 0, c->stream>>>(
+                geo, lev(l), C, d, face_plane(lev(l), d), buf(l, amr::kPhi), cphi, A->L[l].beta[d], u[3 * l + d]);
             launched();
         }
     }
@@ -810,7 +1288,24 @@ int amr_configure(mac_ctx* c, int nlev, const int* nboxes, const int* box_lo, co
         rc = amr_alloc(A, &S.mask, (size_t)N);
         for (int d = 0; d < c->dm && !rc; ++d) rc = amr_alloc(A, &S.beta[d], (size_t)amr::nfaces(S.lev, d));
         for (int b = 0; b < amr::kNumBufs && !rc; ++b) rc = amr_alloc(A, &S.buf[b], (size_t)N);
+        std::vector<int> reflux;
+        std::vector<int2> cover;
+        if (l > 0) coarse_lists(c, geom[l], geom[l - 1], masks[l - 1], reflux, cover);
+        S.nreflux = (int)reflux.size();
+        S.ncover = (int)cover.size();
+        if (!rc) rc = amr_alloc(A, &S.reflux, reflux.size());
+        if (!rc) rc = amr_alloc(A, &S.cover, cover.size());
+        const std::vector<int> rest = classify(c->dm, geom[l], masks[l], &S.nrest);
+        S.nrest_cu = (int)rest.size();
+        if (!rc) rc = amr_alloc(A, &S.rest, rest.size());
         if (rc) break;
+        if (cudaMemcpy(S.reflux, reflux.data(), reflux.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess ||
+            cudaMemcpy(S.cover, cover.data(), cover.size() * sizeof(int2), cudaMemcpyHostToDevice) != cudaSuccess ||
+            cudaMemcpy(S.rest, rest.data(), rest.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess) {
+            set_last_cuda_error(cudaGetLastError(), "cudaMemcpy(lists)", __FILE__, __LINE__);
+            rc = MAC_ERR_CUDA;
+            break;
+        }
         if (cudaMemcpy(S.mask, masks[l].data(), (size_t)N, cudaMemcpyHostToDevice) != cudaSuccess) {
             set_last_cuda_error(cudaGetLastError(), "cudaMemcpy(mask)", __FILE__, __LINE__);
             rc = MAC_ERR_CUDA;
@@ -1220,19 +1715,20 @@ int ml_dense(mac_ctx* c, double* const* umac, double* const* phi, const double* 
     for (int l = 0; l < nl && !rc; ++l) {
         AmrState::FabArrays& F = A->F[l];
         const Lev L = A->L[l].lev;
-        const long N = A->L[l].ncell;
+        const dim3 cells = plane_grid((long)L.ext[0] * L.ext[1], L.ext[2]);
+        const Plane cp = plane(L.ext[0], L.ext[1]);
         for (int d = 0; d < dm && !rc; ++d) {
-            const long nf = amr::nfaces(L, d);
-            k_full_to_box_faces<<<blocks_for(nf, c->sms), kThreads, 0, c->stream>>>(L, d, umac[3 * l + d], F.u[d], nf);
+            k_full_to_box_faces<<<face_grid(L, d), kThreads, 0, c->stream>>>(
+                L, d, face_plane(L, d), umac[3 * l + d], F.u[d]);
             rc = launched();
             up[3 * l + d] = F.u[d];
         }
-        k_full_to_box_cells<<<blocks_for(N, c->sms), kThreads, 0, c->stream>>>(L, rho[l], F.rho, N);
+        k_full_to_box_cells<<<cells, kThreads, 0, c->stream>>>(L, cp, rho[l], F.rho);
         if (!rc) rc = launched();
-        k_full_to_box_cells<<<blocks_for(N, c->sms), kThreads, 0, c->stream>>>(L, phi[l], F.phi, N);
+        k_full_to_box_cells<<<cells, kThreads, 0, c->stream>>>(L, cp, phi[l], F.phi);
         if (!rc) rc = launched();
         if (macrhs && macrhs[l]) {
-            k_full_to_box_cells<<<blocks_for(N, c->sms), kThreads, 0, c->stream>>>(L, macrhs[l], F.rhs, N);
+            k_full_to_box_cells<<<cells, kThreads, 0, c->stream>>>(L, cp, macrhs[l], F.rhs);
             if (!rc) rc = launched();
             mp[l] = F.rhs;
         }
@@ -1246,13 +1742,14 @@ int ml_dense(mac_ctx* c, double* const* umac, double* const* phi, const double* 
     for (int l = 0; l < nl && !rc; ++l) {
         AmrState::FabArrays& F = A->F[l];
         const Lev L = A->L[l].lev;
-        const long N = A->L[l].ncell;
+        const dim3 cells = plane_grid((long)L.ext[0] * L.ext[1], L.ext[2]);
+        const Plane cp = plane(L.ext[0], L.ext[1]);
         for (int d = 0; d < dm && !rc; ++d) {
-            const long nf = amr::nfaces(L, d);
-            k_box_to_full_faces<<<blocks_for(nf, c->sms), kThreads, 0, c->stream>>>(A->geo, L, d, F.u[d], umac[3 * l + d], nf);
+            k_box_to_full_faces<<<face_grid(L, d), kThreads, 0, c->stream>>>(
+                A->geo, L, d, face_plane(L, d), F.u[d], umac[3 * l + d]);
             rc = launched();
         }
-        k_box_to_full_cells<<<blocks_for(N, c->sms), kThreads, 0, c->stream>>>(L, F.phi, phi[l], N);
+        k_box_to_full_cells<<<cells, kThreads, 0, c->stream>>>(L, cp, F.phi, phi[l]);
         if (!rc) rc = launched();
     }
     if (!rc) MAC_CUDA_TRY(cudaStreamSynchronize(c->stream));

@@ -751,9 +751,9 @@ int ml_vcycle(E& ex, int nu1, int nu2) {
         ex.gsrb(l, ex.buf(l, kUu), ex.buf(l, kRes), nu1);
         ex.defect(l, ex.buf(l, kUu), nullptr, ex.buf(l, kRes), ex.buf(l, kTmp));
         ex.swap_bufs(l, kRes, kTmp);
-        ex.copy(l, ex.buf(l, kHold), ex.buf(l, kUu));
+        ex.swap_bufs(l, kHold, kUu);   // (the way up writes kUu whole)
         ex.restrict_cov(l, ex.buf(l, kRes), ex.buf(l - 1, kRes));
-        ex.reflux(l, ex.buf(l, kUu), nullptr, ex.buf(l - 1, kRes));
+        ex.reflux(l, ex.buf(l, kHold), nullptr, ex.buf(l - 1, kRes));
     }
     int rc = ex.level0_correction(ex.buf(0, kRes), ex.buf(0, kUu));
     if (rc) return rc;
