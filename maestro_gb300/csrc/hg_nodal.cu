@@ -367,23 +367,130 @@ __device__ __forceinline__ void staged_node_op(const hg::LevT<T>& L, const T* ss
 }
 
 constexpr int kTileX = 32, kTileY = 32, kTileH = 4, kTileThreads = 384;
-constexpr int kTRX = kTileX + 2 * kTileH, kTRY = kTileY + 2 * kTileH;           // staged nodes
-constexpr int kTCX = kTileX + 2 * kTileH - 1, kTCY = kTileY + 2 * kTileH - 1;   // staged cells
-constexpr int kTFX = kTileX + 2 * kTileH - 2, kTFY = kTileY + 2 * kTileH - 2;   // right-hand side
+constexpr int kTR = kTileX + 2 * kTileH;         // staged rows and columns (nodes)
+constexpr int kTC = kTR - 1, kTF = kTR - 2;      // rows of cells, of the right-hand side
+// Staged rows keep their even columns in the first half and the odd ones in the second: a colour's
+// nodes are two columns and two rows apart, so half a warp reads 16 consecutive words of a row and
+// the other half those of the second next row, 2 x 40 words on -- the other 16 banks.  (With the
+// columns in order every one of a node's 29 reads took two passes: 64 of the 200 us a launch at 257^3.)
+constexpr int kTP = kTR, kTHalf = kTP / 2;
+static_assert((2 * kTP) % 32 == 16, "rows two apart in the other half of the banks");
+__device__ __forceinline__ constexpr int split_col(int x) { return (x & 1) * kTHalf + (x >> 1); }
 template <typename T>
 constexpr size_t tile_smem() {
-    return sizeof(T) * (3 * kTRX * kTRY + 2 * kTCX * kTCY + kTFX * kTFY);
+    return sizeof(T) * (size_t)(3 * kTR + 2 * kTC + kTF) * kTP;
 }
 
-// (FP32: five blocks an SM, registers capped for it; FP64: two, the staged tile being twice as large)
+// The columns x - 1, x, x + 1 of a staged node of x parity PX relative to half column x >> 1.
+template <int PX>
+__device__ __forceinline__ constexpr int col_of(int o) {
+    return PX == 0 ? (o == 0 ? kTHalf - 1 : o == 1 ? 0 : kTHalf) : (o == 0 ? 0 : o == 1 ? kTHalf : 1);
+}
+
+// node_op_dense3's formula (see staged_node_op) on the split rows.  ss: half column of the node in
+// the cell row y - 1 of layer z - 1; ph: in the node row y - 1 of plane z - 1.
+template <typename T, bool ISO, int PX>
+__device__ __forceinline__ void tile_node_op(const hg::LevT<T>& L, const T* ss, const T* ph, T& dg, T& off) {
+    T s[2][2][2];
+#pragma unroll
+    for (int zz = 0; zz < 2; ++zz)
+#pragma unroll
+        for (int yy = 0; yy < 2; ++yy)
+#pragma unroll
+            for (int xx = 0; xx < 2; ++xx) s[zz][yy][xx] = ss[col_of<PX>(xx) + kTP * (yy + kTC * zz)];
+    T sx[2][2][3];
+#pragma unroll
+    for (int zz = 0; zz < 2; ++zz)
+#pragma unroll
+        for (int yy = 0; yy < 2; ++yy) {
+            sx[zz][yy][0] = s[zz][yy][0];
+            sx[zz][yy][1] = s[zz][yy][0] + s[zz][yy][1];
+            sx[zz][yy][2] = s[zz][yy][1];
+        }
+    T sxy[2][3][3];
+#pragma unroll
+    for (int zz = 0; zz < 2; ++zz)
+#pragma unroll
+        for (int ox = 0; ox < 3; ++ox) {
+            sxy[zz][0][ox] = sx[zz][0][ox];
+            sxy[zz][1][ox] = sx[zz][0][ox] + sx[zz][1][ox];
+            sxy[zz][2][ox] = sx[zz][1][ox];
+        }
+    T am[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    T centre = 0;
+#pragma unroll
+    for (int oz = 0; oz < 3; ++oz)
+#pragma unroll
+        for (int oy = 0; oy < 3; ++oy)
+#pragma unroll
+            for (int ox = 0; ox < 3; ++ox) {
+                const T S = oz == 0 ? sxy[0][oy][ox]
+                                    : (oz == 2 ? sxy[1][oy][ox] : sxy[0][oy][ox] + sxy[1][oy][ox]);
+                const int mask = (ox != 1 ? 1 : 0) | (oy != 1 ? 2 : 0) | (oz != 1 ? 4 : 0);
+                if (mask == 0)
+                    centre = S;
+                else if (!(ISO && (mask == 1 || mask == 2 || mask == 4)))
+                    am[mask] = fma(S, ph[col_of<PX>(ox) + kTP * (oy + kTR * oz)], am[mask]);
+            }
+    T acc = 0;
+#pragma unroll
+    for (int m = 1; m < 8; ++m)
+        if (!(ISO && (m == 1 || m == 2 || m == 4))) acc = fma(L.kw[m], am[m], acc);
+    dg = -L.kw[0] * centre;
+    off = acc;
+}
+
+__device__ __forceinline__ float node_quot(float a, float b) { return a / b; }
+__device__ __forceinline__ double node_quot(double a, double b) { return a * recip_nr(b); }
+
+// Colour K of the slab (x parity K & 1, y parity K >> 1) on the tile grown by 3 - K nodes; the tile
+// starts at even nodes, so the colour's extents are constants.  A half warp takes 16 columns of a
+// row; the up to three columns beyond go to the last warps.  plain: every staged node is an unknown.
+template <typename T, bool ISO, int K>
+__device__ __forceinline__ void tile_colour(const hg::LevT<T>& L, T* sphi, const T* ssig, const T* sf,
+                                            const unsigned char* sux, const unsigned char* suy, bool plain) {
+    constexpr int h = 3 - K, px = K & 1, py = K >> 1;
+    // first staged column / row of the colour: kTileH - h rounded up to its parity
+    constexpr int lx0 = kTileH - h + ((px + kTileH - h) & 1), ly0 = kTileH - h + ((py + kTileH - h) & 1);
+    constexpr int nx = (kTileH + kTileX - 1 + h - lx0) / 2 + 1, ny = (kTileH + kTileY - 1 + h - ly0) / 2 + 1;
+    static_assert(kTileX == 32 && nx >= 16 && nx <= 19, "16 columns and up to three more");
+    constexpr int main = (16 * ny + 31) / 32 * 32, extra = nx - 16;
+    static_assert(main + extra * ny <= kTileThreads, "one node a thread");
+    const int t = threadIdx.x;
+    int ix, iy;
+    bool on;
+    if (t < main) {
+        ix = t & 15;
+        iy = t >> 4;
+        on = iy < ny;
+    } else {
+        const int u = t - main;
+        iy = extra > 0 ? u / (extra > 0 ? extra : 1) : 0;
+        ix = 16 + u - iy * extra;
+        on = extra > 0 && iy < ny;
+    }
+    const int lx = lx0 + 2 * ix, ly = ly0 + 2 * iy;
+    if (on && (plain || (sux[lx] && suy[ly]))) {
+        const int hx = lx >> 1;
+        T dg, off;
+        tile_node_op<T, ISO, px>(L, ssig + hx + kTP * (ly - 1), sphi + hx + kTP * (ly - 1), dg, off);
+        const int own = hx + px * kTHalf;
+        sphi[own + kTP * (ly + kTR)] = node_quot(sf[own + kTP * (ly - 1)] + off, dg);
+    }
+    __syncthreads();
+}
+
+// (FP32: five blocks an SM, registers capped for it -- four or three are 1.5 and 5% slower on a whole
+// 256^3 projection; FP64: two, the staged tile being twice as large.)  257^3 FP32: 146 us a launch,
+// bound by issue (115 instructions a node) and the staging's element copies.
 template <typename T, bool ISO>
 __global__ void __launch_bounds__(kTileThreads, sizeof(T) == 4 ? 5 : 2)
 k_hg_gs_tile(hg::Geo G, hg::LevT<T> L, int sp, int ntx, const T* __restrict__ src,
              const T* __restrict__ srcnb, T* __restrict__ dst, const T* __restrict__ f) {
     extern __shared__ __align__(16) unsigned char hg_tile_smem[];
-    T* sphi = reinterpret_cast<T*>(hg_tile_smem);   // [3][kTRY][kTRX], slabs z-1, z, z+1
-    T* ssig = sphi + 3 * kTRX * kTRY;                // [2][kTCY][kTCX], cell layers z-1, z
-    T* sf = ssig + 2 * kTCX * kTCY;                  // [kTFY][kTFX]
+    T* sphi = reinterpret_cast<T*>(hg_tile_smem);   // [3][kTR] rows, slabs z-1, z, z+1
+    T* ssig = sphi + 3 * kTR * kTP;                  // [2][kTC] rows, cell layers z-1, z
+    T* sf = ssig + 2 * kTC * kTP;                    // [kTF] rows, from node row 1
     const int z = 2 * (int)blockIdx.y + sp;
     const int nzu = G.per[2] ? L.n[2] : L.n[2] + 1;  // slabs with unknown nodes
     if (z >= nzu) return;
@@ -391,102 +498,130 @@ k_hg_gs_tile(hg::Geo G, hg::LevT<T> L, int sp, int ntx, const T* __restrict__ sr
     const int t = threadIdx.x;
     // per staged column / row: folded node and cell coordinates (-1: outside a non-periodic
     // face), whether the folded node is an unknown along that direction
-    __shared__ int sqx[kTRX], sqy[kTRY], scx[kTCX], scy[kTCY];
-    __shared__ unsigned char sux[kTRX], suy[kTRY];
-    if (t < kTRX) {
-        const int raw = x0 - kTileH + t;
-        const int q = hg::node_wrap(G, L, 0, raw);
-        sqx[t] = q;
-        sux[t] = q >= 0 && !(G.per[0] ? q == L.n[0] : ((q == 0 && G.dlo[0]) || (q == L.n[0] && G.dhi[0])));
-        if (t < kTCX) scx[t] = hg::cell_wrap(G, L, 0, raw);
-    } else if (t >= 64 && t < 64 + kTRY) {
-        const int u = t - 64, raw = y0 - kTileH + u;
-        const int q = hg::node_wrap(G, L, 1, raw);
-        sqy[u] = q;
-        suy[u] = q >= 0 && !(G.per[1] ? q == L.n[1] : ((q == 0 && G.dlo[1]) || (q == L.n[1] && G.dhi[1])));
-        if (u < kTCY) scy[u] = hg::cell_wrap(G, L, 1, raw);
-    }
+    __shared__ int sqx[kTR], sqy[kTR], scx[kTC], scy[kTC];
+    __shared__ unsigned char sux[kTR], suy[kTR];
     // (scalars, not arrays: a dynamically indexed array would live in local memory)
     const int qz0 = hg::node_wrap(G, L, 2, z - 1), qz1 = hg::node_wrap(G, L, 2, z),
               qz2 = hg::node_wrap(G, L, 2, z + 1);
     const int cz0 = hg::cell_wrap(G, L, 2, z - 1), cz1 = hg::cell_wrap(G, L, 2, z);
     const bool uz = qz1 >= 0 &&
                     !(G.per[2] ? qz1 == L.n[2] : ((qz1 == 0 && G.dlo[2]) || (qz1 == L.n[2] && G.dhi[2])));
-    __syncthreads();
     const long m01 = (long)L.nn[0] * L.nn[1], c01 = (long)L.n[0] * L.n[1];
-    // stage: nodes x0 - kTileH .. x0 + kTileX + kTileH - 1 (same in y), slabs z - 1 .. z + 1,
-    // the two cell layers and the right-hand side, all copies in flight at once.  A thread keeps
-    // one staged column (its folded x in a register) and walks the rows kPR apart.
-    constexpr int kPR = kTileThreads / kTRX;
-    if (t < kPR * kTRX) {
-        const int lx = t % kTRX, r0 = t / kTRX;
-        const int q0 = sqx[lx];
-        const int im0 = L.nn[0], ic0 = L.n[0];
-#pragma unroll 1
-        for (int lz = 0; lz < 3; ++lz) {
-            const int q2 = lz == 0 ? qz0 : (lz == 1 ? qz1 : qz2);
-            const T* from = lz == 1 ? src : srcnb;
-            const bool zin = q0 >= 0 && q2 >= 0;
-            const T* pb = from + (zin ? q0 + q2 * m01 : 0);
-            T* dst_col = sphi + lz * (kTRX * kTRY) + lx;
-            for (int ly = r0; ly < kTRY; ly += kPR) {
-                const int q1 = sqy[ly];
-                const bool in = zin && q1 >= 0;
-                stage_elem(dst_col + ly * kTRX, in ? pb + (long)q1 * im0 : from, in);
-            }
-        }
-        if (lx < kTCX) {
-            const int c0 = scx[lx];
-#pragma unroll 1
-            for (int lz = 0; lz < 2; ++lz) {
-                const int c2 = lz == 0 ? cz0 : cz1;
-                const bool zin = c0 >= 0 && c2 >= 0;
-                const T* pb = L.sig + (zin ? c0 + c2 * c01 : 0);
-                T* dst_col = ssig + lz * (kTCX * kTCY) + lx;
-                for (int ly = r0; ly < kTCY; ly += kPR) {
-                    const int c1 = scy[ly];
-                    const bool in = zin && c1 >= 0;
-                    stage_elem(dst_col + ly * kTCX, in ? pb + (long)c1 * ic0 : L.sig, in);
+    constexpr int kPR = kTileThreads / kTR;   // staged rows a pass: a column a thread
+    const int lx = t % kTR, r0 = t / kTR;
+    // A tile whose staged nodes all lie inside the domain, away from its faces, in every direction
+    // (most of them) needs no fold and no zero fill: pointers advance by a constant.
+    const bool plain = x0 - kTileH >= 1 && x0 + kTR - kTileH <= L.n[0] && y0 - kTileH >= 1 &&
+                       y0 + kTR - kTileH <= L.n[1] && z >= 1 && z <= L.n[2] - 1;
+    if (plain) {
+        if (t < kPR * kTR) {
+            const int im0 = L.nn[0], ic0 = L.n[0], col = split_col(lx);
+            const long node = (x0 - kTileH + lx) + (long)im0 * (y0 - kTileH + r0) + m01 * z;
+            const long step = (long)kPR * im0;
+            T* d = sphi + r0 * kTP + col;
+            const T* a = srcnb + node - m01;
+            const T* b = src + node;
+            const T* c = srcnb + node + m01;
+#pragma unroll
+            for (int q = 0; q < (kTR + kPR - 1) / kPR; ++q) {
+                if (r0 + q * kPR < kTR) {
+                    stage_elem(d + q * kPR * kTP, a + q * step, true);
+                    stage_elem(d + (q * kPR + kTR) * kTP, b + q * step, true);
+                    stage_elem(d + (q * kPR + 2 * kTR) * kTP, c + q * step, true);
                 }
             }
+            const long cstep = (long)kPR * ic0;
+            const T* g = L.sig + (x0 - kTileH + lx) + (long)ic0 * (y0 - kTileH + r0) + c01 * (z - 1);
+            T* e = ssig + r0 * kTP + col;
+            if (lx < kTC) {
+#pragma unroll
+                for (int q = 0; q < (kTC + kPR - 1) / kPR; ++q) {
+                    if (r0 + q * kPR < kTC) {
+                        stage_elem(e + q * kPR * kTP, g + q * cstep, true);
+                        stage_elem(e + (q * kPR + kTC) * kTP, g + c01 + q * cstep, true);
+                    }
+                }
+            }
+            const T* fr = f + node + im0;
+            T* df = sf + r0 * kTP + col;
+#pragma unroll
+            for (int q = 0; q < (kTF + kPR - 1) / kPR; ++q)
+                if (r0 + q * kPR < kTF) stage_elem(df + q * kPR * kTP, fr + q * step, true);
         }
-        if (lx >= 1 && lx <= kTFX) {
+    } else {
+        if (t < kTR) {
+            const int raw = x0 - kTileH + t;
+            const int q = hg::node_wrap(G, L, 0, raw);
+            sqx[t] = q;
+            sux[t] = uz && q >= 0 &&
+                     !(G.per[0] ? q == L.n[0] : ((q == 0 && G.dlo[0]) || (q == L.n[0] && G.dhi[0])));
+            if (t < kTC) scx[t] = hg::cell_wrap(G, L, 0, raw);
+        } else if (t >= 64 && t < 64 + kTR) {
+            const int u = t - 64, raw = y0 - kTileH + u;
+            const int q = hg::node_wrap(G, L, 1, raw);
+            sqy[u] = q;
+            suy[u] = q >= 0 && !(G.per[1] ? q == L.n[1] : ((q == 0 && G.dlo[1]) || (q == L.n[1] && G.dhi[1])));
+            if (u < kTC) scy[u] = hg::cell_wrap(G, L, 1, raw);
+        }
+        __syncthreads();
+        // nodes x0 - kTileH .. x0 + kTileX + kTileH - 1 (same in y), slabs z - 1 .. z + 1, the two
+        // cell layers and the right-hand side, all copies in flight at once
+        if (t < kPR * kTR) {
+            const int q0 = sqx[lx], col = split_col(lx);
+            const int im0 = L.nn[0], ic0 = L.n[0];
+#pragma unroll 1
+            for (int lz = 0; lz < 3; ++lz) {
+                const int q2 = lz == 0 ? qz0 : (lz == 1 ? qz1 : qz2);
+                const T* from = lz == 1 ? src : srcnb;
+                const bool zin = q0 >= 0 && q2 >= 0;
+                const T* pb = from + (zin ? q0 + q2 * m01 : 0);
+                T* dst_col = sphi + lz * (kTR * kTP) + col;
+                for (int ly = r0; ly < kTR; ly += kPR) {
+                    const int q1 = sqy[ly];
+                    const bool in = zin && q1 >= 0;
+                    stage_elem(dst_col + ly * kTP, in ? pb + (long)q1 * im0 : from, in);
+                }
+            }
+            if (lx < kTC) {
+                const int c0 = scx[lx];
+#pragma unroll 1
+                for (int lz = 0; lz < 2; ++lz) {
+                    const int c2 = lz == 0 ? cz0 : cz1;
+                    const bool zin = c0 >= 0 && c2 >= 0;
+                    const T* pb = L.sig + (zin ? c0 + c2 * c01 : 0);
+                    T* dst_col = ssig + lz * (kTC * kTP) + col;
+                    for (int ly = r0; ly < kTC; ly += kPR) {
+                        const int c1 = scy[ly];
+                        const bool in = zin && c1 >= 0;
+                        stage_elem(dst_col + ly * kTP, in ? pb + (long)c1 * ic0 : L.sig, in);
+                    }
+                }
+            }
             const bool zin = q0 >= 0 && qz1 >= 0;
             const T* pb = f + (zin ? q0 + qz1 * m01 : 0);
-            T* dst_col = sf + (lx - 1);
-            for (int ly = r0; ly < kTFY; ly += kPR) {
+            for (int ly = r0; ly < kTF; ly += kPR) {
                 const int q1 = sqy[ly + 1];
                 const bool in = zin && q1 >= 0;
-                stage_elem(dst_col + ly * kTFX, in ? pb + (long)q1 * im0 : f, in);
+                stage_elem(sf + ly * kTP + col, in ? pb + (long)q1 * im0 : f, in);
             }
         }
     }
     stage_wait();
     __syncthreads();
     // the four in-slab colours, on the tile grown by 3, 2, 1, 0 nodes
-#pragma unroll 1
-    for (int k = 0; k < 4; ++k) {
-        const int h = 3 - k, px = k & 1, py = k >> 1;
-        const int xs = x0 - h + ((px - (x0 - h)) & 1), ys = y0 - h + ((py - (y0 - h)) & 1);
-        const int nx = (x0 + kTileX - 1 + h - xs) / 2 + 1, ny = (y0 + kTileY - 1 + h - ys) / 2 + 1;
-        for (int e = t; e < nx * ny; e += kTileThreads) {
-            const int lx = xs - (x0 - kTileH) + 2 * (e % nx), ly = ys - (y0 - kTileH) + 2 * (e / nx);
-            if (!(sux[lx] && suy[ly] && uz)) continue;
-            T dg, off;
-            staged_node_op<T, ISO, kTRX, kTRX * kTRY, kTCX, kTCX * kTCY>(
-                L, ssig + (lx - 1) + kTCX * (ly - 1), sphi + (lx - 1) + kTRX * (ly - 1), dg, off);
-            const int fi = (lx - 1) + kTFX * (ly - 1);
-            sphi[lx + kTRX * (ly + kTRY)] = (sf[fi] + off) / dg;
-        }
-        __syncthreads();
-    }
+    tile_colour<T, ISO, 0>(L, sphi, ssig, sf, sux, suy, plain);
+    tile_colour<T, ISO, 1>(L, sphi, ssig, sf, sux, suy, plain);
+    tile_colour<T, ISO, 2>(L, sphi, ssig, sf, sux, suy, plain);
+    tile_colour<T, ISO, 3>(L, sphi, ssig, sf, sux, suy, plain);
     // the tile's own unknown nodes
     for (int e = t; e < kTileX * kTileY; e += kTileThreads) {
         const int p[3] = {x0 + e % kTileX, y0 + e / kTileX, z};
-        if (p[0] > L.n[0] - (G.per[0] ? 1 : 0) || p[1] > L.n[1] - (G.per[1] ? 1 : 0)) continue;
-        if (!hg::is_unknown(G, L, p)) continue;
+        if (!plain) {
+            if (p[0] > L.n[0] - (G.per[0] ? 1 : 0) || p[1] > L.n[1] - (G.per[1] ? 1 : 0)) continue;
+            if (!hg::is_unknown(G, L, p)) continue;
+        }
         dst[hg::nix(L, p[0], p[1], p[2])] =
-            sphi[(p[0] - x0 + kTileH) + kTRX * ((p[1] - y0 + kTileH) + kTRY)];
+            sphi[split_col(e % kTileX + kTileH) + kTP * (e / kTileX + kTileH + kTR)];
     }
 }
 
