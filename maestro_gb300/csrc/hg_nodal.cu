@@ -12,6 +12,7 @@
 
 #include "mac_internal.cuh"   // (first: hg_nodal.cuh's device code calls recip_nr)
 #include "hg_nodal.cuh"
+#include "hg_tail.cuh"
 
 namespace mac {
 
@@ -19,6 +20,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kReduceBlocks = 1024;
+constexpr int kSlabThreads = 512;   // most threads of a slab block
 constexpr int kMixedInner = 3;   // FP32 V-cycles per FP64 refinement step of the mixed solve
 
 #define HG_LOOP(N) for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx < (N); \
@@ -718,7 +720,6 @@ k_hg_defect_tile(hg::Geo G, hg::LevT<T> L, int ntx, const T* __restrict__ phi,
     }
 }
 
-constexpr int kSlabThreads = 512;   // most threads of a slab block
 template <typename T, bool DENSE3>
 __global__ void __launch_bounds__(kSlabThreads)
 k_hg_gs_slab(hg::Geo G, hg::LevT<T> L, int sp, T* phi, const T* f) {
@@ -1079,6 +1080,9 @@ struct HgState {
         int key[4] = {-1, -1, -1, -1};   // count, nu1, nu2, dense stencil
         long long kernels = 0;
     } graph[2];
+    // first level the cluster tail runs (-1: none) per precision: [0] FP64, [1] FP32
+    int tail[2] = {-1, -1};
+    int tail_nc = 16;
     int bM = 0;
     int* bnode = nullptr;
     int* bmap = nullptr;
@@ -1264,6 +1268,55 @@ struct HgMg {
         }
     }
     bool dense3() const { return geo.dense && geo.dm == 3; }
+    // The cluster tail of the dense 3-D cycles (hg_tail.cu)
+    static constexpr int kSlot = std::is_same<T, float>::value ? 1 : 0;
+    bool tail_level(int l) const { return dense3() && l == H->tail[kSlot]; }
+    HgTailParams<T> tail_params(int l, int nu1, int nu2) const {
+        HgTailParams<T> P;
+        P.geo = geo;
+        P.nlev = nlev - 1 - l;
+        for (int q = 0; q < P.nlev; ++q) {
+            P.lev[q] = lev(l + q);
+            P.iso[q] = iso(l + q);
+        }
+        P.f0 = buf(l, hg::kF);
+        P.e0 = buf(l, hg::kPhi);
+        P.nu1 = nu1;
+        P.nu2 = nu2;
+        P.singular = singular;
+        P.bot = lev(nlev - 1);
+        P.M = H->bM;
+        P.node = H->bnode;
+        P.map = H->bmap;
+        P.binv = H->binv;
+        return P;
+    }
+    void tail(int l, int nu1, int nu2) {
+        HgTailParams<T> P = tail_params(l, nu1, nu2);
+        const size_t smem = hg_tail_plan<T>(P, H->tail_nc);
+        launch_hg_tail<T>(P, smem, H->tail_nc, c->stream);
+        launched();
+    }
+    // The first level >= 1 whose slabs fit one block a colour and whose tail fits the cluster's
+    // shared memory (33^3 nodes in FP32, 25 x 20 x 17 and below in FP64 typically).
+    void plan_tail() {
+        int& at = H->tail[kSlot];
+        at = -1;
+        if (err || !dense3() || !H->binv || nlev < 3) return;
+        if (prepare_hg_tail_kernels(&H->tail_nc)) {
+            set_last_cuda_error(cudaGetLastError(), "nodal tail kernels", __FILE__, __LINE__);
+            err = MAC_ERR_CUDA;
+            return;
+        }
+        for (int l = 1; l < nlev - 1; ++l) {
+            const hg::LevT<T> L = lev(l);
+            if ((L.nn[0] + 1) / 2 * ((L.nn[1] + 1) / 2) > kSlabThreads || nlev - 1 - l > kHgTailLevels) continue;
+            HgTailParams<T> P = tail_params(l, 0, 0);
+            if (!hg_tail_plan<T>(P, H->tail_nc)) continue;
+            at = l;
+            return;
+        }
+    }
     // isotropic level spacing: the dense 3-D weights of the axis neighbours are exactly 0
     bool iso(int l) const {
         const hg::LevT<T>& L = lev(l);
@@ -1274,6 +1327,7 @@ struct HgMg {
     // most of them small, and needs no host value inside
     void run_cycles(int count, int nu1, int nu2) {
         prepare_tiles();
+        plan_tail();
         if (err) return;
         if (c->o.timing) {   // events around the level-0 launches: no capture
             for (int v = 0; v < count; ++v) hg::vcycle(*this, 0, nu1, nu2);

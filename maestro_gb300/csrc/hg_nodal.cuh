@@ -745,8 +745,21 @@ HG_HD inline long fab_target(const Geo& G, const Lev& L, const Fab& B, long e) {
 enum { kPhi = 0, kF = 1, kR = 2, kNumBufs = 3 };
 constexpr int kBottomSweeps = 60;
 
+// An executor with members tail_level(l) and tail(l, nu1, nu2) runs the V-cycle from such a level
+// down itself (the GPU executor: one kernel).
+template <class E, class = void>
+struct HasTail : std::false_type {};
+template <class E>
+struct HasTail<E, std::void_t<decltype(std::declval<E&>().tail_level(0))>> : std::true_type {};
+
 template <class E>
 void vcycle(E& ex, int l, int nu1, int nu2) {
+    if constexpr (HasTail<E>::value) {
+        if (ex.tail_level(l)) {
+            ex.tail(l, nu1, nu2);
+            return;
+        }
+    }
     if (l == ex.nlev - 1) {
         if (ex.singular) ex.sub_unknown_mean(l, ex.buf(l, kF));
         ex.bottom_gs(l, ex.buf(l, kPhi), ex.buf(l, kF), kBottomSweeps);

@@ -21,12 +21,12 @@
 // 7.1 ms, 256^3 mixed 6.99 -> 6.87 ms.
 #include "mac_internal.cuh"
 #include "mac_bottom.cuh"
+#include "mac_cluster.cuh"
 
 namespace mac {
 namespace {
 
 constexpr int kInvThreads = 1024;
-constexpr int kClusterMax = 16;          // CTAs of the tail cluster (16: opt-in size; fallback 8)
 constexpr int kTailMaxThreads = 512;
 constexpr int kTailItems = 2;            // pairs of cells a thread at most
 constexpr int kOps = 17;                 // operator values of a pair in shared memory
@@ -36,57 +36,6 @@ constexpr int kReplCells = sizeof(T) == 4 ? 512 : 128;
 __device__ __forceinline__ double fmaT2(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float fmaT2(float a, float b, float c) { return fmaf(a, b, c); }
 
-// x / d for x d < 2^32 with m = floor(2^32 / d) + 1 (d > 1; d == 1 is m = 0)
-__host__ __device__ __forceinline__ unsigned div_magic(unsigned d) {
-    return d > 1 ? (unsigned)(0x100000000ull / d) + 1u : 0u;
-}
-__device__ __forceinline__ unsigned fdiv(unsigned x, unsigned m) { return m ? __umulhi(x, m) : x; }
-
-// ---- cluster primitives -----------------------------------------------------------------------
-__device__ __forceinline__ unsigned cluster_rank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ unsigned cluster_size() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::
-                     : "memory");
-}
-__device__ __forceinline__ void cluster_arrive() {
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait() {
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ unsigned smem_u32(const void* p) {
-    return (unsigned)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ unsigned mapa(unsigned a, unsigned cta) {
-    unsigned r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(cta));
-    return r;
-}
-__device__ __forceinline__ float ld_cluster(unsigned a, float) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ double ld_cluster(unsigned a, double) {
-    double v;
-    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ void st_cluster(unsigned a, float v) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
-}
-__device__ __forceinline__ void st_cluster(unsigned a, double v) {
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
-}
 __device__ __forceinline__ void sync_level(bool repl) {
     if (repl)
         __syncthreads();
@@ -194,17 +143,6 @@ __device__ __forceinline__ void load_pair(Pair<T>& q, const Geo& g, const T* ops
     }
 }
 
-template <typename T>
-__device__ __forceinline__ void sts(unsigned a, T v);
-template <>
-__device__ __forceinline__ void sts<float>(unsigned a, float v) {
-    asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
-}
-template <>
-__device__ __forceinline__ void sts<double>(unsigned a, double v) {
-    asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
-}
-
 // acc + the six arms (x-, x+, y-, y+, z-, z+) of the pair's colour-s cell; a 2-D level has no z arm
 template <typename T, bool Z3>
 __device__ __forceinline__ T arms(T acc, const Pair<T>& q, int s) {
@@ -229,7 +167,7 @@ __device__ __forceinline__ T arms(T acc, const Pair<T>& q, int s) {
 
 template <typename T>
 __device__ __forceinline__ void store_e(const Pair<T>& q, int s) {
-    sts<T>(q.own + (s ? 1 - q.p : q.p) * (unsigned)sizeof(T), q.e[s]);
+    lds_store(q.own + (s ? 1 - q.p : q.p) * (unsigned)sizeof(T), q.e[s]);
 }
 
 // nu sweeps.  zero: from e = 0 -- the first colour-0 half-sweep has no arm that contributes.
@@ -289,7 +227,7 @@ __device__ __forceinline__ void visit_down(const TailParams<T>& P, int l, unsign
             const T e = s ? q[m].e[1] : q[m].e[0], f = s ? q[m].f[1] : q[m].f[0];
             const T r0 = fmaT2(-dg, e, f);
             const T r = s ? arms<T, Z3>(r0, q[m], 1) : arms<T, Z3>(r0, q[m], 0);
-            sts<T>(q[m].own + dr + a * (unsigned)sizeof(T), r);
+            lds_store(q[m].own + dr + a * (unsigned)sizeof(T), r);
         }
     }
     sync_level(g.repl);
@@ -529,7 +467,7 @@ __device__ __forceinline__ double cl_gsrb(const ClBottom& B, double fi, double x
         const bool act = B.on && B.colour == (it & 1);
         if (act) x = cl_gsum(B, 0, fi, false);
         if (B.odd) cluster_sync();
-        if (act) sts<double>(B.xa, x);
+        if (act) lds_store(B.xa, x);
         cluster_sync();
     }
     return x;
@@ -581,7 +519,7 @@ __device__ __noinline__ double cl_solve(const ClBottom& bottom, ClReduce& R, dou
             if (B.on) {
                 p = fma(beta, fma(-omega, vv, p), r);
                 y = p * B.id;
-                sts<double>(ya, y);
+                lds_store(ya, y);
             }
             cluster_sync();
             if (B.on) vv = B.dg * cl_gsum(B, B.yoff, y, true);
@@ -599,7 +537,7 @@ __device__ __noinline__ double cl_solve(const ClBottom& bottom, ClReduce& R, dou
                 s = fma(-alpha, vv, r);
                 x = fma(alpha, y, x);
                 y = s * B.id;
-                sts<double>(ya, y);
+                lds_store(ya, y);
             }
             cluster_sync();
             if (B.on) t = B.dg * cl_gsum(B, B.yoff, y, true);
@@ -630,13 +568,12 @@ __device__ __noinline__ double cl_solve(const ClBottom& bottom, ClReduce& R, dou
             if (omega == 0.0) break;
         }
     }
-    if (B.on) sts<double>(B.xa, x);
+    if (B.on) lds_store(B.xa, x);
     cluster_sync();
     *iters = count;
     return cl_gsrb(B, fi, x, nub);
 }
 
-__host__ __device__ __forceinline__ size_t pad16(size_t b) { return (b + 15) & ~(size_t)15; }
 // bottom cells per CTA (even: pairs of cells) and the threads they take (colours in warps of
 // their own)
 __host__ __device__ __forceinline__ int bottom_cells(int N, int nc) { return 2 * ((N + 2 * nc - 1) / (2 * nc)); }
@@ -808,9 +745,9 @@ k_tail(const __grid_constant__ TailParams<T> P) {
                             st_cluster(mapa(a, c), (double)v);
                     }
                 } else if (lev) {
-                    sts<T>(a, v);
+                    lds_store(a, v);
                 } else {
-                    sts<double>(a, (double)v);
+                    lds_store(a, (double)v);
                 }
             }
             sync_level(!push);
@@ -857,7 +794,7 @@ k_tail(const __grid_constant__ TailParams<T> P) {
         }
         cluster_sync();
     } else {
-        if (B.on) sts<double>(B.xa, bx);
+        if (B.on) lds_store(B.xa, bx);
         bx = cl_solve(B, R, bf, bx, bottom_threads(M) / 32, P.singular, P.nub, P.bottom_eps,
                       P.bottom_max_iter, &count);
         if (B.on) eb[bc - (int)rank * M] = (T)bx;
@@ -1073,32 +1010,11 @@ void launch_tail(TailParams<T>& P, int nc, cudaStream_t s) {
 
 // Opts the tail kernels into their shared memory and cluster size; *nc: the CTAs of a cluster.
 int prepare_tail_kernels(int* nc) {
-    const void* kern[2] = {(const void*)k_tail<float>, (const void*)k_tail<double>};
     *nc = kClusterMax;
-    for (const void* k : kern) {
-        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmemMax) != cudaSuccess ||
-            cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-            cudaGetLastError();
-            return MAC_ERR_CUDA;
-        }
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(kClusterMax);
-        cfg.blockDim = dim3(kTailMaxThreads);
-        cfg.dynamicSmemBytes = kTailSmemMax;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = kClusterMax;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 1) {
-            cudaGetLastError();
-            *nc = 8;   // the portable size
-        }
-    }
-    return MAC_OK;
+    return cluster_opt_in((const void*)k_tail<float>, kTailMaxThreads, kTailSmemMax, nc) &&
+                   cluster_opt_in((const void*)k_tail<double>, kTailMaxThreads, kTailSmemMax, nc)
+               ? MAC_OK
+               : MAC_ERR_CUDA;
 }
 
 template bool tail_fits<float>(const Dims*, int, const Dims&, bool, int);
