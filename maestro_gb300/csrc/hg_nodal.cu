@@ -776,79 +776,158 @@ __global__ void k_hg_defect3(hg::Geo G, hg::LevT<T> L, const T* phi, const T* f,
 }
 
 // ---- exact coarsest-level solve --------------------------------------------------------------
-constexpr int kExactMax = 128;   // unknown nodes of a coarsest level solved by its dense inverse
+// The operator of the coarsest level on its M unknown nodes (FP64, rows by node_row), plus sigma 1
+// 1^T for the singular problem (sigma = a diagonal / M: B^-1 f = A^+ f for a mean-free f), inverted
+// by Gauss-Jordan elimination without pivoting (B is definite) in blocks of kInvB rows: one launch
+// a block over kInvT x kInvT tiles, each tile from the old matrix into the new one, the tile with
+// the next diagonal block inverting it on the way.  The matrix is padded to whole blocks by the
+// identity.  A pivot at a time in one block of 256 threads M = 120 took 890 us; this is bound by the
+// 16 dependent pivots of a diagonal block (~6 us) and 15 us a launch of 576 unknowns.  A coarsest
+// level without the inverse costs 60 colour-ordered sweeps in one block, and where an odd periodic
+// extent couples nodes of one colour they are serial: two seconds for a 256 x 160 x 192 projection
+// (8 x 5 x 7 unknowns), so kExactMax covers every level whose extents are at most 8.
+constexpr int kExactMax = kHgTailBottom;   // unknown nodes of a coarsest level solved by its inverse
 constexpr int kExactThreads = 256;
+constexpr int kInvB = 16, kInvT = 32;
+inline int inv_pitch(int M) { return (M + kInvB - 1) / kInvB * kInvB; }
 
-// One block: the operator of the coarsest level (FP64, rows by node_row) on its M unknown
-// nodes, plus sigma 1 1^T for the singular problem (sigma = mean diagonal / M: B^-1 f = A^+ f
-// for a mean-free f), inverted in place by Gauss-Jordan elimination without pivoting (B is
-// definite).  A: M x M, row-major.
-__global__ void __launch_bounds__(kExactThreads)
-k_hg_bottom_inverse(hg::Geo G, hg::Lev L, int M, const int* __restrict__ node,
-                    const int* __restrict__ map, int singular, double* __restrict__ A) {
-    __shared__ double col[kExactMax];
-    __shared__ double piv;
-    const int t = threadIdx.x;
-    for (int e = t; e < M * M; e += kExactThreads) A[e] = 0.0;
+// Row blockIdx.x of the padded operator.
+__global__ void __launch_bounds__(64)
+k_hg_bottom_row(hg::Geo G, hg::Lev L, int M, int pitch, const int* __restrict__ node,
+                const int* __restrict__ map, int singular, double* __restrict__ A) {
+    __shared__ double row[kExactMax];
+    __shared__ double sg;
+    const int u = blockIdx.x, t = threadIdx.x;
+    for (int j = t; j < pitch; j += 64) row[j] = u >= M && j == u ? 1.0 : 0.0;
+    if (t == 0) sg = 0.0;
     __syncthreads();
-    for (int u = t; u < M; u += kExactThreads) {
+    if (u < M && t == 0) {
         int p[3];
         hg::node_coords(L, node[u], p);
-        double* row = A + (long)u * M;
         hg::node_row(G, L, p, [&](long m, double w) {
             const int v = map[m];
             if (v >= 0) row[v] += w;
         });
     }
-    __syncthreads();
-    if (singular) {
-        if (t == 0) {
-            double s = 0.0;
-            for (int u = 0; u < M; ++u) s += A[(long)u * M + u];
-            piv = s / M / M;
-        }
-        __syncthreads();
-        const double sg = piv;
-        for (int e = t; e < M * M; e += kExactThreads) A[e] += sg;
-        __syncthreads();
+    if (u < M && t == 32 && singular) {
+        int p[3];
+        hg::node_coords(L, node[0], p);
+        double d = 0.0;
+        hg::node_row(G, L, p, [&](long m, double w) {
+            if (map[m] == 0) d += w;
+        });
+        sg = d / M;
     }
-    for (int k = 0; k < M; ++k) {
-        if (t == 0) {
-            piv = 1.0 / A[(long)k * M + k];
-            A[(long)k * M + k] = 1.0;
-        }
+    __syncthreads();
+    for (int j = t; j < pitch; j += 64) A[(size_t)u * pitch + j] = row[j] + (j < M ? sg : 0.0);
+}
+
+// S (kInvB x kInvB, shared) replaced by its inverse; kExactThreads = kInvB^2 threads.
+__device__ __forceinline__ void invert_block(double (&S)[kInvB][kInvB + 1], double& ip) {
+    const int r = threadIdx.x / kInvB, c = threadIdx.x % kInvB;
+    for (int k = 0; k < kInvB; ++k) {
+        if (threadIdx.x == 0) ip = 1.0 / S[k][k];
+        const double ark = S[r][k], akc = S[k][c], a = S[r][c];
         __syncthreads();
-        const double ip = piv;
-        for (int j = t; j < M; j += kExactThreads) A[(long)k * M + j] *= ip;
-        for (int i = t; i < M; i += kExactThreads) {
-            if (i == k) continue;
-            col[i] = A[(long)i * M + k];
-            A[(long)i * M + k] = 0.0;
-        }
-        __syncthreads();
-        for (int e = t; e < M * M; e += kExactThreads) {
-            const int i = e / M, j = e - i * M;
-            if (i != k) A[e] -= col[i] * A[(long)k * M + j];
-        }
+        const double q = ip;
+        double v;
+        if (r == k)
+            v = c == k ? q : akc * q;
+        else
+            v = c == k ? -ark * q : fma(-ark * q, akc, a);
+        S[r][c] = v;
         __syncthreads();
     }
 }
 
+__global__ void __launch_bounds__(kExactThreads)
+k_hg_inv_first(int pitch, const double* __restrict__ A, double* __restrict__ P) {
+    __shared__ double S[kInvB][kInvB + 1];
+    __shared__ double ip;
+    const int r = threadIdx.x / kInvB, c = threadIdx.x % kInvB;
+    S[r][c] = A[(size_t)r * pitch + c];
+    __syncthreads();
+    invert_block(S, ip);
+    P[threadIdx.x] = S[r][c];
+}
+
+// Block step k: B = the sweep of A by its diagonal block k, whose inverse is P; Pn: the inverse of
+// B's diagonal block k + 1 (where there is one).
+__global__ void __launch_bounds__(kExactThreads)
+k_hg_inv_step(int pitch, int k, const double* __restrict__ A, const double* __restrict__ P,
+              double* __restrict__ B, double* __restrict__ Pn) {
+    __shared__ double aik[kInvT][kInvB + 1], akj[kInvB][kInvT], tj[kInvB][kInvT], p[kInvB][kInvB + 1];
+    __shared__ double ip;
+    const int t = threadIdx.x, i0 = blockIdx.y * kInvT, j0 = blockIdx.x * kInvT, K = k * kInvB;
+    p[t / kInvB][t % kInvB] = P[t];
+    for (int q = t; q < kInvT * kInvB; q += kExactThreads) {
+        const int r = q / kInvB, s = q % kInvB, i = i0 + r;
+        aik[r][s] = i < pitch ? A[(size_t)i * pitch + K + s] : 0.0;
+        const int s2 = q / kInvT, j = j0 + q % kInvT;
+        akj[s2][q % kInvT] = j < pitch ? A[(size_t)(K + s2) * pitch + j] : 0.0;
+    }
+    __syncthreads();
+    // the pivot rows: P A_K,j (the pivot columns: P itself)
+    for (int q = t; q < kInvT * kInvB; q += kExactThreads) {
+        const int r = q / kInvT, c = q % kInvT, j = j0 + c;
+        double v = 0.0;
+        if (j >= K && j < K + kInvB) {
+            v = p[r][j - K];
+        } else {
+#pragma unroll
+            for (int s = 0; s < kInvB; ++s) v = fma(p[r][s], akj[s][c], v);
+        }
+        tj[r][c] = v;
+    }
+    __syncthreads();
+    const int c = t % kInvT, j = j0 + c;
+    double out[kInvT * kInvT / kExactThreads];
+#pragma unroll
+    for (int q = 0; q < kInvT * kInvT / kExactThreads; ++q) {
+        const int r = t / kInvT + q * (kExactThreads / kInvT), i = i0 + r;
+        double v = 0.0;
+        if (i < pitch && j < pitch) {
+            if (i >= K && i < K + kInvB) {
+                v = tj[i - K][c];
+            } else {
+                v = j >= K && j < K + kInvB ? 0.0 : A[(size_t)i * pitch + j];
+#pragma unroll
+                for (int s = 0; s < kInvB; ++s) v = fma(-aik[r][s], tj[s][c], v);
+            }
+            B[(size_t)i * pitch + j] = v;
+        }
+        out[q] = v;
+    }
+    // the tile that holds the next diagonal block
+    const int N = K + kInvB;
+    if (N >= pitch || N / kInvT != (int)blockIdx.x || blockIdx.x != blockIdx.y) return;
+    __syncthreads();   // (p is free now)
+#pragma unroll
+    for (int q = 0; q < kInvT * kInvT / kExactThreads; ++q) {
+        const int i = i0 + t / kInvT + q * (kExactThreads / kInvT);
+        if (i >= N && i < N + kInvB && j >= N && j < N + kInvB) p[i - N][j - N] = out[q];
+    }
+    __syncthreads();
+    invert_block(p, ip);
+    Pn[t] = p[t / kInvB][t % kInvB];
+}
+
 // phi = B^-1 f on the unknown nodes of the coarsest level (FP64 arithmetic; phi elsewhere
-// untouched).
+// untouched), a row a warp.
 template <typename T>
 __global__ void __launch_bounds__(kExactThreads)
-k_hg_bottom_exact(int M, const int* __restrict__ node, const double* __restrict__ Binv,
+k_hg_bottom_exact(int M, int pitch, const int* __restrict__ node, const double* __restrict__ Binv,
                   const T* __restrict__ f, T* __restrict__ phi) {
     __shared__ double fs[kExactMax];
     for (int v = threadIdx.x; v < M; v += kExactThreads) fs[v] = (double)f[node[v]];
     __syncthreads();
-    for (int u = threadIdx.x; u < M; u += kExactThreads) {
-        const double* row = Binv + (long)u * M;
-        double x = 0.0;
-        for (int v = 0; v < M; ++v) x = fma(row[v], fs[v], x);
-        phi[node[u]] = (T)x;
-    }
+    const int u = blockIdx.x * (kExactThreads / 32) + threadIdx.x / 32;
+    if (u >= M) return;
+    const double* row = Binv + (size_t)u * pitch;
+    double x = 0.0;
+    for (int v = threadIdx.x & 31; v < M; v += 32) x = fma(row[v], fs[v], x);
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if ((threadIdx.x & 31) == 0) phi[node[u]] = (T)x;
 }
 
 // nu colour-ordered Gauss-Seidel sweeps of the coarsest level in one block.  An odd periodic
@@ -1086,7 +1165,8 @@ struct HgState {
     int bM = 0;
     int* bnode = nullptr;
     int* bmap = nullptr;
-    double* binv = nullptr;
+    double* binv = nullptr;    // rows of inv_pitch(bM)
+    double* bwork = nullptr;   // the elimination's second matrix and diagonal blocks
     double* part = nullptr;
     double* out = nullptr;
     double* h_out = nullptr;
@@ -1207,9 +1287,11 @@ int hg_ensure(mac_ctx* c) {
         }
         if (!nodes.empty() && (int)nodes.size() <= kExactMax) {
             H->bM = (int)nodes.size();
+            const size_t pitch = (size_t)inv_pitch(H->bM);
             rc = hg_alloc(H, &H->bnode, nodes.size());
             if (!rc) rc = hg_alloc(H, &H->bmap, map.size());
-            if (!rc) rc = hg_alloc(H, &H->binv, nodes.size() * nodes.size());
+            if (!rc) rc = hg_alloc(H, &H->binv, pitch * pitch);
+            if (!rc) rc = hg_alloc(H, &H->bwork, pitch * pitch + 2 * kInvB * kInvB);
             if (!rc && (cudaMemcpy(H->bnode, nodes.data(), nodes.size() * sizeof(int),
                                    cudaMemcpyHostToDevice) != cudaSuccess ||
                         cudaMemcpy(H->bmap, map.data(), map.size() * sizeof(int),
@@ -1289,6 +1371,7 @@ struct HgMg {
         P.node = H->bnode;
         P.map = H->bmap;
         P.binv = H->binv;
+        P.ldb = inv_pitch(H->bM);
         return P;
     }
     void tail(int l, int nu1, int nu2) {
@@ -1527,7 +1610,8 @@ struct HgMg {
     void bottom_gs(int l, T* phi, const T* f, int nu) {
         if (H->binv && l == (int)H->L.size() - 1) {
             // the exact solve replaces the sweeps (the inverse is built with the coefficients)
-            k_hg_bottom_exact<T><<<1, kExactThreads, 0, c->stream>>>(H->bM, H->bnode, H->binv, f, phi);
+            k_hg_bottom_exact<T><<<ceil_div(H->bM, kExactThreads / 32), kExactThreads, 0, c->stream>>>(
+                H->bM, inv_pitch(H->bM), H->bnode, H->binv, f, phi);
         } else {
             k_hg_bottom<T><<<1, 1024, 0, c->stream>>>(geo, lev(l), phi, f, nu, nn(l));
         }
@@ -1606,9 +1690,21 @@ struct HgExec : HgMg<double> {
             launched();
         }
         if (H->binv) {
-            k_hg_bottom_inverse<<<1, kExactThreads, 0, c->stream>>>(
-                geo, lev((int)H->L.size() - 1), H->bM, H->bnode, H->bmap, singular ? 1 : 0, H->binv);
+            const int pitch = inv_pitch(H->bM), steps = pitch / kInvB;
+            const dim3 tiles((unsigned)ceil_div(pitch, kInvT), (unsigned)ceil_div(pitch, kInvT));
+            double* m[2] = {H->binv, H->bwork};
+            double* P[2] = {H->bwork + (size_t)pitch * pitch, H->bwork + (size_t)pitch * pitch + kInvB * kInvB};
+            int at = steps & 1;   // (the last step writes binv)
+            k_hg_bottom_row<<<pitch, 64, 0, c->stream>>>(geo, lev((int)H->L.size() - 1), H->bM, pitch, H->bnode,
+                                                        H->bmap, singular ? 1 : 0, m[at]);
             launched();
+            k_hg_inv_first<<<1, kExactThreads, 0, c->stream>>>(pitch, m[at], P[0]);
+            launched();
+            for (int k = 0; k < steps; ++k, at ^= 1) {
+                k_hg_inv_step<<<tiles, kExactThreads, 0, c->stream>>>(pitch, k, m[at], P[k & 1], m[at ^ 1],
+                                                                     P[(k + 1) & 1]);
+                launched();
+            }
         }
         return err;
     }

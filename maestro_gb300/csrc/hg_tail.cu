@@ -276,7 +276,6 @@ __device__ __forceinline__ double warp_mean(const T* v, int M) {
     return s / M;
 }
 
-constexpr int kHgTailBottom = 128;   // unknown nodes of the bottom at most
 constexpr int kSeg = 16;             // lanes a row of its inverse
 
 }  // namespace
@@ -366,7 +365,7 @@ k_hg_tail(const __grid_constant__ HgTailParams<T> P) {
                 if (u0 + (tid & ~31) / kSeg >= last) continue;   // (whole warps)
                 double x = 0.0;
                 if (u < last)
-                    for (int v = sg; v < M; v += kSeg) x = fma(__ldg(P.binv + (size_t)u * M + v), (double)fb[v], x);
+                    for (int v = sg; v < M; v += kSeg) x = fma(__ldg(P.binv + (size_t)u * P.ldb + v), (double)fb[v], x);
                 for (int o = kSeg / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
                 if (u < last && sg < (int)nc) st_cluster(mapa(smem_u32(eb + u), sg), (T)x);
             }

@@ -9,6 +9,7 @@ namespace mac {
 constexpr int kHgTailLevels = 8;
 constexpr int kHgTailThreads = 512;
 constexpr int kHgTailSmem = 200 * 1024;
+constexpr int kHgTailBottom = 640;   // unknown nodes of an exactly solved bottom at most
 
 template <typename T>
 struct HgTailParams {
@@ -25,6 +26,7 @@ struct HgTailParams {
     const int* node;
     const int* map;
     const double* binv;
+    int ldb;                          // its row pitch
     // plan (hg_tail_plan)
     int spc[kHgTailLevels];           // slabs a CTA
     int off[kHgTailLevels];           // byte offset of the level's arrays

@@ -54,3 +54,40 @@ def test_tail_matches_levels_and_oracle(cuda_lib, name, precision):
     for u, phi in ((u1, phi1), (u2, phi2)):
         assert phi_rel_err(phi, phi_o, top != BC_DIR) <= 1e-9
         assert u_rel_err(u, u_o) <= 1e-9
+
+
+NODAL = {
+    # name: (cells, top face, precision): the cluster tail's slab split and the blocked inverse
+    "two_slabs_a_cta": ((32, 32, 32), BC_NEU, "mixed"),      # 17 slabs over 16 CTAs: two a CTA
+    "three_slabs_a_cta": ((64, 64, 64), BC_NEU, "mixed"),   # 33 slabs, isotropic
+    "uneven_extents": ((24, 20, 36), BC_DIR, "fp64"),       # bottom 6 x 5 x 9: odd periodic extent
+    "periodic_vertical": ((32, 16, 48), BC_PER, "fp64"),
+    "bottom_one_block": ((16, 16, 16), BC_NEU, "fp64"),     # 12 unknowns: less than one block
+    "bottom_576": ((32, 24, 44), BC_NEU, "mixed"),          # 8 x 6 x 12 nodes: 36 whole blocks
+}
+
+
+@pytest.mark.parametrize("dense", [True, False])
+@pytest.mark.parametrize("name", list(NODAL))
+def test_nodal_tail_and_bottom_match_oracle(cuda_lib, name, dense):
+    from tests.test_gpu_zz_hg import _run
+    n, top, precision = NODAL[name]
+    rng = np.random.default_rng(29)
+    dx = tuple(1.0 / v for v in n)
+    lo, hi = (BC_PER, BC_PER, BC_NEU), (BC_PER, BC_PER, top)
+    if top == BC_PER:
+        lo = hi
+    z = np.exp(-np.arange(n[2]) / n[2])
+    unew = rng.standard_normal(n + (3,))
+    gpi = rng.standard_normal(n + (3,))
+    rho = z * np.exp(0.2 * rng.standard_normal(n))
+    pi = np.zeros(tuple(v + 1 for v in n))
+    u, g, p, st = _run(n, dx, lo, hi, O.HG_REGULAR, 0.01, unew, unew, gpi, rho, pi, dense=dense,
+                       rel_eps=O.EPS_HG, precision=precision)
+    assert st["status"] == 0 and st["rel_resid"] <= O.EPS_HG
+    uo, go, po, pho, so = O.hgproject(unew, unew, gpi, rho, pi, dx, lo, hi, proj_type=O.HG_REGULAR,
+                                      dt=0.01, dense=dense, rel_eps=O.EPS_HG)
+    assert so["status"] == 0
+    # eps_hg = 1e-12 on operators of contrast below 20: three orders under the 1e-9 bar
+    assert np.max(np.abs(u - uo)) <= 1e-9 * np.max(np.abs(uo))
+    assert np.max(np.abs(g - go)) <= 1e-9 * np.max(np.abs(go))
