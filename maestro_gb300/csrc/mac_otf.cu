@@ -999,10 +999,31 @@ void plan_fused_tile(const Dims& d, int sms, OtfParams& P) {
     P.fthreads = nt;
 }
 
+// Planes a block of a staged kernel marches through: the chunk length (a multiple of `unit`, at least
+// 4) for which waves x (planes + 4) is least, a wave being all resident blocks and 4 planes what a
+// block's start costs (two halo planes and the first copies' latency).  One chunk a resident block
+// leaves a sixth of them idle where the tiles do not divide them: 512^3 (128 tiles, 304 blocks) took
+// 432 us a half-sweep with 2 chunks a tile and takes 363 with 7, 384^3 (96 tiles, 456 blocks) 181 with
+// 4 and 157 with 14; 256^3 (32 tiles, 456 blocks) keeps 14, 43.3 us (28: 46.7).
+static int plane_chunk(long tiles, long resident, int n2, int unit) {
+    int best = n2;
+    double least = 0.0;
+    for (int chunks = 1; chunks <= n2 / 4 || chunks == 1; ++chunks) {
+        int zc = ceil_div(n2, chunks);
+        zc = ceil_div(zc, unit) * unit;
+        const long blocks = tiles * ceil_div(n2, zc);
+        const double t = (double)ceil_div(blocks, (int)resident) * (zc + 4);
+        if (chunks == 1 || t < least) {
+            least = t;
+            best = zc;
+        }
+    }
+    return best;
+}
+
 // Tile plan of the staged half-sweep: ty = the largest power of two with ty * hn0 <= 1024 cells
 // that divides n1 (one float4 group of 4 cells per thread, at most 256 threads); whole rows of
-// 16-byte multiples (hn0 % 4 == 0); chunks of planes so that the blocks fill the resident slots
-// of every SM once.  Sets ty = 0 where the staged kernel does not apply.
+// 16-byte multiples (hn0 % 4 == 0); chunks of plane_chunk planes.  Sets ty = 0 where the staged kernel does not apply.
 void plan_otf_tile(const Dims& d, int dm, int sms, OtfParams& P) {
     static std::mutex mu;
     static int smem_set = 0;
@@ -1051,10 +1072,7 @@ void plan_otf_tile(const Dims& d, int dm, int sms, OtfParams& P) {
         return;
     }
     const long tiles = d.n1 / ty;
-    long chunks = ((long)sms * per_sm) / tiles;
-    if (chunks < 1) chunks = 1;
-    int zc = ceil_div(d.n2, (int)std::min<long>(chunks, d.n2));
-    if (zc < 4) zc = std::min(4, d.n2);
+    const int zc = plane_chunk(tiles, (long)sms * per_sm, d.n2, 1);
     P.ty = ty;
     P.zc = zc;
     P.nz = ceil_div(d.n2, zc);
@@ -1093,11 +1111,7 @@ void plan_otf_tile(const Dims& d, int dm, int sms, OtfParams& P) {
         cudaGetLastError();
         return;
     }
-    long rchunks = ((long)sms * rper_sm) / tiles;
-    if (rchunks < 1) rchunks = 1;
-    int rzc = ceil_div(d.n2, (int)std::min<long>(rchunks, d.n2 / 2));
-    rzc += rzc & 1;
-    if (rzc < 4) rzc = std::min(4, d.n2);
+    const int rzc = plane_chunk(tiles, (long)sms * rper_sm, d.n2, 2);
     P.rty = ty;
     P.rzc = rzc;
     P.rnz = ceil_div(d.n2, rzc);
