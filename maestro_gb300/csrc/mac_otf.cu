@@ -35,7 +35,7 @@ k_gsrb_otf(Dims d, OtfParams P, int colour, float* __restrict__ es, const float*
     otf_cell<DM>(P, nb, i, j, k, rhos[q], rhoo, eo, acc, diag);
     if (SOR) {
         const float old = es[q];
-        es[q] = fmaf(P.omega, acc * rcp_approx(diag) - old, old);
+        es[q] = fmaf(P.omega, __fmul_rn(acc, rcp_approx(diag)) - old, old);
     } else {
         es[q] = acc * rcp_approx(diag);
     }
@@ -176,31 +176,31 @@ __device__ __forceinline__ void update_group(float ex, float rx, const FV<V>& Ec
             fh = m == V - 1 ? fxhV : fx;
         }
         float acc = Fo.v[m];
-        float b = fl * rcp_approx(rc + rl);
+        float b = __fmul_rn(fl, rcp_approx(rc + rl));
         acc = fmaf(b, el, acc);
         float dg = b;
-        b = fh * rcp_approx(rc + rh);
+        b = __fmul_rn(fh, rcp_approx(rc + rh));
         acc = fmaf(b, eh, acc);
-        dg += b;
-        b = fyl * rcp_approx(rc + Rym.v[m]);
+        dg = __fadd_rn(dg, b);
+        b = __fmul_rn(fyl, rcp_approx(rc + Rym.v[m]));
         acc = fmaf(b, Eym.v[m], acc);
-        dg += b;
-        b = fyh * rcp_approx(rc + Ryp.v[m]);
+        dg = __fadd_rn(dg, b);
+        b = __fmul_rn(fyh, rcp_approx(rc + Ryp.v[m]));
         acc = fmaf(b, Eyp.v[m], acc);
-        dg += b;
-        b = fzl * rcp_approx(rc + Rb.v[m]);
+        dg = __fadd_rn(dg, b);
+        b = __fmul_rn(fzl, rcp_approx(rc + Rb.v[m]));
         acc = fmaf(b, Eb.v[m], acc);
-        dg += b;
-        b = fzh * rcp_approx(rc + Ra.v[m]);
+        dg = __fadd_rn(dg, b);
+        b = __fmul_rn(fzh, rcp_approx(rc + Ra.v[m]));
         acc = fmaf(b, Ea.v[m], acc);
-        dg += b;
+        dg = __fadd_rn(dg, b);
         if (DIR) {
             const float w = (SP == 0 && m == 0) ? wx0 : (SP == 1 && m == V - 1) ? wxV : wmid;
-            dg += w * rcp_approx(rc);
+            dg = fmaf(w, rcp_approx(rc), dg);
         }
         // RES: the defect f - L e of the own cell instead of its Gauss-Seidel update; KEEP: also
         // hand back f + sum(arms) and the diagonal (the defect after an over-relaxed update)
-        out[m] = RES ? fmaf(-dg, eown[m], acc) : acc * rcp_approx(dg);
+        out[m] = RES ? fmaf(-dg, eown[m], acc) : __fmul_rn(acc, rcp_approx(dg));
         if (KEEP) {
             accv[m] = acc;
             dgv[m] = dg;
@@ -869,13 +869,15 @@ k_resid_restrict_otf(Dims F, Dims C, OtfParams P, const float* __restrict__ e,
     const int K = blockIdx.z;
     if (I >= C.n0 || J >= C.n1) return;
     const int rz = DM == 3 ? 2 : 1;
-    float sum = 0.f;
+    float sum = 0.f;   // colour pairs, then plane pairs, then rows: the staged kernel's order
 #pragma unroll
-    for (int b = 0; b < rz; ++b) {
+    for (int a = 0; a < 2; ++a) {
+        float row = 0.f;
 #pragma unroll
-        for (int a = 0; a < 2; ++a) {
+        for (int b = 0; b < rz; ++b) {
             const int j = 2 * J + a;
             const int k = DM == 3 ? 2 * K + b : K;
+            float pair = 0.f;
 #pragma unroll
             for (int colour = 0; colour < (RED_ONLY ? 1 : 2); ++colour) {
                 const int off = colour * F.half, oth = (colour ^ 1) * F.half;
@@ -885,9 +887,11 @@ k_resid_restrict_otf(Dims F, Dims C, OtfParams P, const float* __restrict__ e,
                 const int me = (j + F.n1 * k) * F.hn0 + I;
                 float acc = r[off + me], diag;
                 otf_cell<DM>(P, nb, i, j, k, P.rho[off + me], P.rho + oth, e + oth, acc, diag);
-                sum += fmaf(-diag, e[off + me], acc);
+                pair += fmaf(-diag, e[off + me], acc);
             }
+            row += pair;
         }
+        sum += row;
     }
     int ci;
     if (C.split)

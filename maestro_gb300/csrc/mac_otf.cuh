@@ -41,7 +41,9 @@ __device__ __forceinline__ void nbrs(const Dims& d, int colour, int h, int j, in
 // Adds sum_arms beta'_f e_n to acc and returns the diagonal of cell (i, j, k) (colour half
 // index via nb; ro/eo = the other colour's rho and e, rc = own rho).  Branch-free: a face on a
 // non-periodic wall gets a zero factor (horizontal walls by position, vertical walls through the
-// wall-zeroed layer tables), and its wrapped neighbour index stays a valid address.
+// wall-zeroed layer tables), and its wrapped neighbour index stays a valid address.  Every rounding
+// is spelled out (here and in update_group): the staged, fused and per-cell kernels agree bitwise,
+// whatever the compiler would have contracted in each.
 template <int DM>
 __device__ __forceinline__ void otf_cell(const OtfParams& P, const Nb& nb, int i, int j, int k,
                                          float rc, const float* __restrict__ ro,
@@ -62,35 +64,31 @@ __device__ __forceinline__ void otf_cell(const OtfParams& P, const Nb& nb, int i
         fyl = P.fac[2 * st + r];
         fyh = P.fac[3 * st + r];
     }
-    float b = fxl * rcp_approx(rc + ro[nb.xm]);
+    float b = __fmul_rn(fxl, rcp_approx(rc + ro[nb.xm]));
     acc = fmaf(b, eo[nb.xm], acc);
     float dg = b;
-    b = fxh * rcp_approx(rc + ro[nb.xp]);
+    b = __fmul_rn(fxh, rcp_approx(rc + ro[nb.xp]));
     acc = fmaf(b, eo[nb.xp], acc);
-    dg += b;
-    b = fyl * rcp_approx(rc + ro[nb.ym]);
+    dg = __fadd_rn(dg, b);
+    b = __fmul_rn(fyl, rcp_approx(rc + ro[nb.ym]));
     acc = fmaf(b, eo[nb.ym], acc);
-    dg += b;
-    b = fyh * rcp_approx(rc + ro[nb.yp]);
+    dg = __fadd_rn(dg, b);
+    b = __fmul_rn(fyh, rcp_approx(rc + ro[nb.yp]));
     acc = fmaf(b, eo[nb.yp], acc);
-    dg += b;
+    dg = __fadd_rn(dg, b);
     if (DM == 3) {
-        b = fzl * rcp_approx(rc + ro[nb.zm]);
+        b = __fmul_rn(fzl, rcp_approx(rc + ro[nb.zm]));
         acc = fmaf(b, eo[nb.zm], acc);
-        dg += b;
-        b = fzh * rcp_approx(rc + ro[nb.zp]);
+        dg = __fadd_rn(dg, b);
+        b = __fmul_rn(fzh, rcp_approx(rc + ro[nb.zp]));
         acc = fmaf(b, eo[nb.zp], acc);
-        dg += b;
+        dg = __fadd_rn(dg, b);
     }
     if (P.has_dir) {   // Dirichlet walls add fac / rho to the diagonal
         float w = P.fac[4 * st + r];
-        if (DM == 3) {
-            w += (i == 0 && P.dlo[0]) || (i == P.n[0] - 1 && P.dhi[0]) ? fx : 0.f;
-            w += (j == 0 && P.dlo[1]) || (j == P.n[1] - 1 && P.dhi[1]) ? P.fac[st + r] : 0.f;
-        } else {
-            w += (i == 0 && P.dlo[0]) || (i == P.n[0] - 1 && P.dhi[0]) ? fx : 0.f;
-        }
-        dg += w * rcp_approx(rc);
+        if (DM == 3) w += (j == 0 && P.dlo[1]) || (j == P.n[1] - 1 && P.dhi[1]) ? P.fac[st + r] : 0.f;
+        w += (i == 0 && P.dlo[0]) || (i == P.n[0] - 1 && P.dhi[0]) ? fx : 0.f;
+        dg = fmaf(w, rcp_approx(rc), dg);
     }
     diag = dg;
 }

@@ -125,6 +125,11 @@ OtfParams otf_params(const mac_ctx* c) {
     P.fst = c->otf_tile.fst;
     P.fsmem = c->otf_tile.fsmem;
     P.fthreads = c->otf_tile.fthreads;
+    // The staged kernels pay off where their blocks fill the chip: up to 2^21 cells one thread a cell
+    // is faster (whole mixed solves, staged -> per cell: 32^3 875 -> 607 us, 64^3 1124 -> 848, 96^3
+    // 1906 -> 1755, 128^3 1831 -> 1736; 160 x 128 x 128 2530 -> 2930).  The fused sweep and the
+    // wait's fault injection are the staged kernels' own.
+    if (c->lev[0].d.ncell <= (1 << 21) && !c->o.fused_sweep && !c->o.inject_wait_expiry) P.ty = P.rty = 0;
     return P;
 }
 

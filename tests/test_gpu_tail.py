@@ -91,3 +91,21 @@ def test_nodal_tail_and_bottom_match_oracle(cuda_lib, name, dense):
     # eps_hg = 1e-12 on operators of contrast below 20: three orders under the 1e-9 bar
     assert np.max(np.abs(u - uo)) <= 1e-9 * np.max(np.abs(uo))
     assert np.max(np.abs(g - go)) <= 1e-9 * np.max(np.abs(go))
+
+
+@pytest.mark.parametrize("n,top", [((128, 128, 128), BC_NEU), ((160, 128, 112), BC_DIR),
+                                   ((192, 112, 128), BC_NEU)])
+def test_finest_level_paths_match_oracle(cuda_lib, n, top):
+    # 2^21 cells (one thread a cell) and just above it (staged planes, rows that are no power of
+    # two, plane chunks that do not divide the extent)
+    box = tuple(v // 2 for v in n)
+    c = make_case(name="paths", dm=3, n=n, box=box, H_frac=0.25, noise=0.02, kmax=8, seed=23)
+    c.bc_hi = (BC_PER, BC_PER, top)
+    u, phi, st = gpu_project(c, "mixed", rel_eps=1e-12)
+    assert st["status"] == 0 and st["rel_resid"] <= 1e-12
+    u_o, phi_o, st_o = O.macproject(c.umac, c.phi0, c.rho, c.dx, c.bc_lo, c.bc_hi,
+                                    macrhs=c.macrhs, beta0=c.beta0, beta0_edge=c.beta0_edge,
+                                    nlevels=O.nlevels_for_boxes([box]), rel_eps=1e-12)
+    assert st_o["status"] == 0
+    assert phi_rel_err(phi, phi_o, top != BC_DIR) <= 1e-9
+    assert u_rel_err(u, u_o) <= 1e-9
