@@ -32,261 +32,265 @@ constexpr int kB = 256;
 
 struct AdjGeom {
     int n[3];
-    int dm, va, p;
+    int dm, p;      // p: beta0 exponent (0: no beta0)
     int per[3];
     double idx[3];
     Dims d0;
 };
 
-__device__ __forceinline__ double ipow(double b, int e) {
-    return e == 0 ? 1.0 : (e == 1 ? b : b * b);
-}
-
-__device__ __forceinline__ int nat(const AdjGeom& G, int i, int j, int k) {
-    return i + G.n[0] * (j + G.n[1] * k);
-}
-
-__device__ __forceinline__ int face_nat(const AdjGeom& G, int d, int i, int j, int k) {
-    const int m0 = G.n[0] + (d == 0), m1 = G.n[1] + (d == 1);
-    return i + m0 * (j + m1 * k);
-}
-
-// beta0 on a face entry of direction d whose cell/face coordinate along the vertical is r.
-__device__ __forceinline__ double b0_face(const AdjGeom& G, const double* b0, const double* b0e,
-                                          int d, int r) {
-    if (G.p == 0) return 1.0;
-    return d == G.va ? b0e[r] : b0[r];
-}
+// All kernels below are bound by the FP64 pipe (one warp instruction per 16 cycles of an SM: an
+// operation on every cell of 256^3 is 29 us, a pass over an array of 256^3 doubles 20 us), so they
+// divide nowhere: the stored coefficient of the finest level is beta'_f = beta0^p h_f / dx^2, and the
+// per-layer tables of the forward setup turn it into whatever multiple of h_f is wanted.
 
 // lambda_a = sum over the face entries touching cell a of c_e w_e (+1/dx on the low entry,
-// -1/dx on the high entry), walls excluded.
+// -1/dx on the high entry), walls excluded;  c_e / dx = beta'_f dx / beta0.  A thread marches
+// kAdjPlanes planes up and hands the upper face's product to the next plane: 8 FP64 operations a
+// cell (with a division for each of the six faces: 2399 us at 256^3; now 346).
+constexpr int kAdjPlanes = 8;
+
+template <int DM>
 __global__ void __launch_bounds__(kB)
-k_adj_rhs(AdjGeom G, const double* __restrict__ rho, const double* __restrict__ b0,
-          const double* __restrict__ b0e, const double* __restrict__ wx,
-          const double* __restrict__ wy, const double* __restrict__ wz,
-          double* __restrict__ lam) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= G.d0.ncell) return;
-    const int i = q % G.n[0], row = q / G.n[0], j = row % G.n[1], k = row / G.n[1];
-    const int c[3] = {i, j, k};
-    const double* w[3] = {wx, wy, wz};
-    const double rc = rho[q];
-    double s = 0.0;
-    for (int d = 0; d < G.dm; ++d) {
-        const int n = G.n[d];
-        // low physical face
-        if (c[d] > 0 || G.per[d]) {
-            int nb[3] = {i, j, k};
-            nb[d] = c[d] > 0 ? c[d] - 1 : n - 1;
-            const double h = 2.0 / (rc + rho[nat(G, nb[0], nb[1], nb[2])]);
-            int e[3] = {i, j, k};
-            double wl = w[d][face_nat(G, d, e[0], e[1], e[2])];
-            if (c[d] == 0) {   // periodic: entry n is the same physical face
-                e[d] = n;
-                wl += w[d][face_nat(G, d, e[0], e[1], e[2])];
-            }
-            const int r = d == G.va ? c[G.va] : c[G.va];
-            const double cc = ipow(b0_face(G, b0, b0e, d, r), G.p > 0 ? G.p - 1 : 0) * h;
-            s -= cc * wl * G.idx[d];
-        }
-        // high physical face
-        if (c[d] < n - 1 || G.per[d]) {
-            int nb[3] = {i, j, k};
-            nb[d] = c[d] < n - 1 ? c[d] + 1 : 0;
-            const double h = 2.0 / (rc + rho[nat(G, nb[0], nb[1], nb[2])]);
-            int e[3] = {i, j, k};
-            e[d] = c[d] + 1;
-            double wh = w[d][face_nat(G, d, e[0], e[1], e[2])];
-            if (c[d] == n - 1) {   // periodic: entry 0 is the same physical face
-                e[d] = 0;
-                wh += w[d][face_nat(G, d, e[0], e[1], e[2])];
-            }
-            const int r = d == G.va ? c[G.va] + 1 : c[G.va];
-            const double cc = ipow(b0_face(G, b0, b0e, d, r), G.p > 0 ? G.p - 1 : 0) * h;
-            s += cc * wh * G.idx[d];
-        }
+k_adj_rhs(AdjGeom G, const double* __restrict__ bx, const double* __restrict__ by,
+          const double* __restrict__ bz, const double* __restrict__ tab,
+          const double* __restrict__ wx, const double* __restrict__ wy,
+          const double* __restrict__ wz, double* __restrict__ lam) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k0 = blockIdx.z * kAdjPlanes;
+    const int n0 = G.n[0], n1 = G.n[1], n2 = G.n[2];
+    if (i >= n0 || j >= n1) return;
+    const Dims& d = G.d0;
+    const int st = G.n[DM - 1] + 1;
+    const double* K0 = tab + kTabK0 * st;
+    const double* K1 = K0 + st;
+    const double* K2 = K1 + st;
+    const int plane = n0 * n1;
+    double zl = 0.0;   // beta' dx/beta0 w of the cell's lower z face
+    if (DM == 3) {
+        const int q = i + n0 * j + plane * k0;
+        double w = wz[q];
+        if (k0 == 0) w = G.per[2] ? w + wz[q + plane * n2] : 0.0;
+        zl = bz[level_index(d, i, j, k0)] * w * K2[k0];
     }
-    lam[q] = s;
+    for (int k = k0; k < min(k0 + kAdjPlanes, n2); ++k) {
+        const int c = level_index(d, i, j, k);
+        const int fx = i + (n0 + 1) * (j + n1 * k), fy = i + n0 * (j + (n1 + 1) * k);
+        const int fz = i + n0 * j + plane * (k + 1);
+        double xl = wx[fx], xh = wx[fx + 1], yl = wy[fy], yh = wy[fy + n0];
+        double zw = DM == 3 ? wz[fz] : 0.0;
+        const bool ex = i == 0 || i == n0 - 1, ey = j == 0 || j == n1 - 1;
+        const bool ez = DM == 3 && k == n2 - 1;
+        if (ex || ey || ez) {   // entries 0 and n of a periodic direction are one face; walls: none
+            if (i == 0) xl = G.per[0] ? xl + wx[fx + n0] : 0.0;
+            if (i == n0 - 1) xh = G.per[0] ? xh + wx[fx + 1 - n0] : 0.0;
+            if (j == 0) yl = G.per[1] ? yl + wy[fy + n0 * n1] : 0.0;
+            if (j == n1 - 1) yh = G.per[1] ? yh + wy[fy + n0 - n0 * n1] : 0.0;
+            if (ez) zw = G.per[2] ? zw + wz[fz - plane * n2] : 0.0;
+        }
+        const double bxh = bx[level_index(d, i < n0 - 1 ? i + 1 : 0, j, k)];
+        const double byh = by[level_index(d, i, j < n1 - 1 ? j + 1 : 0, k)];
+        double s = fma(bxh, xh, -(bx[c] * xl)) * K0[DM == 3 ? k : j];
+        if (DM == 3) {
+            s = fma(fma(byh, yh, -(by[c] * yl)), K1[k], s);
+            const double zh = bz[level_index(d, i, j, k < n2 - 1 ? k + 1 : 0)] * zw * K2[k + 1];
+            s += zh - zl;
+            zl = zh;
+        } else {
+            s = fma(byh * yh, K1[j + 1], s);
+            s = fma(-(by[c] * yl), K1[j], s);
+        }
+        lam[i + n0 * (j + n1 * k)] = s;
+    }
 }
 
-// Deterministic block partial sums of a level-0 array (for the mean of mu).
+// Sum of a level-0 array for the mean of mu, in a fixed order: kMeanBlocks blocks, each thread
+// four running sums (a shared-memory tree for every 256 elements took 247 us at 256^3; now 30).
+constexpr int kMeanBlocks = 608;
+
+__device__ __forceinline__ double block_sum(double v) {   // result in thread 0
+    __shared__ double sm[32];
+    const int t = threadIdx.x + blockDim.x * threadIdx.y;
+    const int nw = (blockDim.x * blockDim.y) >> 5;
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((t & 31) == 0) sm[t >> 5] = v;
+    __syncthreads();
+    if (t == 0)
+        for (int w = 1; w < nw; ++w) v += sm[w];
+    return v;
+}
+
 __global__ void __launch_bounds__(kB)
 k_partial_sum(int n, const double* __restrict__ a, double* __restrict__ part) {
-    __shared__ double sm[kB];
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    sm[threadIdx.x] = q < n ? a[q] : 0.0;
-    __syncthreads();
-    for (int o = kB / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
-        __syncthreads();
+    const int step = kMeanBlocks * kB;
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    long q = blockIdx.x * kB + threadIdx.x;
+    for (; q + 3L * step < n; q += 4L * step) {
+        s0 += a[q];
+        s1 += a[q + step];
+        s2 += a[q + 2L * step];
+        s3 += a[q + 3L * step];
     }
-    if (threadIdx.x == 0) part[blockIdx.x] = sm[0];
+    for (; q < n; q += step) s0 += a[q];
+    const double s = block_sum((s0 + s1) + (s2 + s3));
+    if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-__global__ void k_final_mean(int nb, int n, const double* __restrict__ part, double* __restrict__ out) {
-    __shared__ double sm[1024];
+__global__ void k_final_mean(int n, const double* __restrict__ part, double* __restrict__ out) {
     double s = 0.0;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) s += part[b];
-    sm[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[0] = sm[0] / n;
+    for (int b = threadIdx.x; b < kMeanBlocks; b += blockDim.x) s += part[b];
+    s = block_sum(s);
+    if (threadIdx.x == 0) out[0] = s / n;
 }
 
-struct FaceOut {
-    double* du;     // dL/dU entries (natural face layout)
-    double* dh;     // per-entry share of dL/dh_f
-    double* db0;    // per-entry dL/dbeta0_e
+// nu = mu - mean(mu) in the natural layout.
+__global__ void __launch_bounds__(kB)
+k_mu_to_nat(Dims d, const double* __restrict__ mu, const double* __restrict__ mean,
+            double* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = blockIdx.z;
+    if (i >= d.n0 || j >= d.n1) return;
+    out[i + d.n0 * (j + d.n1 * k)] = mu[level_index(d, i, j, k)] - mean[0];
+}
+
+struct FaceIo {
+    const double* beta;   // beta' of this direction, level-0 layout
+    const double* u;
+    const double* w;
+    const double* phi;    // natural
+    const double* nu;     // natural
+    double* du;           // dL/dU entries (natural face layout)
+    double* g;            // -dL/dh_f h_f^2 / 2 shares per entry (null: not wanted)
+    double* part;         // [layer][tile] sums of the dL/dbeta0_e shares (null: not wanted)
+    int cols, tiles;      // tiles of a layer's plane: along x, in all
 };
 
-// Per face entry of direction d: dU, dh share, dbeta0 share.
+// Per face entry of direction D, all in one pass: dU, the share of dL/d(1/rho) and the layer sums
+// of dL/dbeta0_e.  With t = beta' dphi, dmu = nu_hi - nu_lo (nu = 0 outside the domain), b = beta0:
+//   dU = w + (b/dx) dmu,   g = -(1/2) h^2 dL/dh = beta' t (A dmu + C w),
+//   dL/dbeta0_e = u dmu / dx - t (p/b dmu + (p-1) dx/b^2 w)
+// with A and C constant on a layer, like every factor of the last line, which is therefore summed
+// as three plain products.  A block covers blockDim.x columns and kFaceRows rows a thread of one
+// layer's plane, so that its reduction costs about one FP64 operation an entry.  11 of them an entry:
+// 256^3 took 1012 us a direction (division, general index arrays, an array of shares and 470 us to
+// sum it), now 393 to 459.
+constexpr int kFaceRows = 8;
+
+template <int D, bool ALT>   // ALT: p = 2
 __global__ void __launch_bounds__(kB)
-k_adj_face(AdjGeom G, int d, const double* __restrict__ rho, const double* __restrict__ b0,
-           const double* __restrict__ b0e, const double* __restrict__ u,
-           const double* __restrict__ w, const double* __restrict__ phi,
-           const double* __restrict__ mu, const double* __restrict__ mean_mu, FaceOut out) {
-    const int m0 = G.n[0] + (d == 0), m1 = G.n[1] + (d == 1), m2 = G.n[2] + (d == 2);
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= m0 * m1 * m2) return;
-    const int i = q % m0, row = q / m0, j = row % m1, k = row / m1;
-    const int f[3] = {i, j, k};
-    const int n = G.n[d];
-    const int qd = f[d];
-    const double mm = *mean_mu;
-    const double dx1 = G.idx[d];
-    // cells on either side (may be outside the domain)
-    int lo[3] = {i, j, k}, hi[3] = {i, j, k};
-    lo[d] = qd - 1;
-    const bool lo_in = qd > 0, hi_in = qd < n;
-    // -(D^T nu)_e = (nu_hi - nu_lo)/dx with nu = 0 outside the domain
-    const double nu_hi = hi_in ? mu[level_index(G.d0, hi[0], hi[1], hi[2])] - mm : 0.0;
-    const double nu_lo = lo_in ? mu[level_index(G.d0, lo[0], lo[1], lo[2])] - mm : 0.0;
-    const double dtnu = (nu_hi - nu_lo) * dx1;
-    const int r = d == G.va ? qd : f[G.va];
-    const double bb = b0_face(G, b0, b0e, d, r);
-    const double ue = u[q], we = w[q];
-    double du = we + bb * dtnu;
-    double dh = 0.0, db0 = u[q] * dtnu;
-    // physical face: interior, or a periodic boundary entry (0 or n)
-    const bool interior = qd > 0 && qd < n;
-    const bool per_entry = G.per[d] && (qd == 0 || qd == n);
-    if (interior || per_entry) {
-        int a[3] = {i, j, k}, b[3] = {i, j, k};
-        a[d] = interior ? qd - 1 : n - 1;
-        b[d] = interior ? qd : 0;
-        const int ia = level_index(G.d0, a[0], a[1], a[2]);
-        const int ib = level_index(G.d0, b[0], b[1], b[2]);
-        const double gphi = (phi[ib] - phi[ia]) * dx1;
-        const double gnu = (mu[ib] - mu[ia]) * dx1;
-        const double h = 2.0 / (rho[nat(G, a[0], a[1], a[2])] + rho[nat(G, b[0], b[1], b[2])]);
-        const double dc = -we * gphi;
-        // the solve uses each physical face once: entry n of a periodic direction is the duplicate
-        const double dbeta = (qd == n) ? 0.0 : -gnu * gphi;
-        const int p = G.p > 0 ? G.p : 1;
-        dh = ipow(bb, p) * dbeta + ipow(bb, p - 1) * dc;
-        if (G.p > 0) db0 += p * ipow(bb, p - 1) * h * dbeta + (p - 1) * h * dc;
-    }
-    (void)ue;
-    out.du[q] = du;
-    out.dh[q] = dh;
-    out.db0[q] = db0;
+k_adj_face(AdjGeom G, const double* __restrict__ tab, FaceIo io) {
+    const int n0 = G.n[0], n1 = G.n[1];
+    const int m0 = n0 + (D == 0), m1 = n1 + (D == 1);
+    const bool v3 = G.dm == 3;
+    const int r = blockIdx.x / io.tiles;      // vertical index: z in 3-D, y in 2-D
+    const int tile = blockIdx.x - r * io.tiles;
+    const int st = G.n[G.dm - 1] + 1;
+    const int rows = v3 ? m1 : 1;             // rows of the layer's plane
+    const int i = tile % io.cols * blockDim.x + threadIdx.x;
+    const int row0 = tile / io.cols * blockDim.y * kFaceRows;
+    const int row1 = min(rows, row0 + (int)blockDim.y * kFaceRows);
+    const double gd = tab[(kTabG0 + D) * st + r], kd = tab[(kTabK0 + D) * st + r];
+    const double A = -recip_nr(tab[(kTabFac0 + D) * st + r]), C = kd * A;
+    const int sd = D == 0 ? 1 : (D == 1 ? n0 : n0 * n1);
+    const int nd = G.n[D];
+    const bool sums = io.part != nullptr;
+    double a1 = 0.0, a2 = 0.0, a3 = 0.0;
+    if (i < m0)
+        for (int row = row0 + threadIdx.y; row < row1; row += blockDim.y) {
+            const int j = v3 ? row : r, k = v3 ? r : 0;
+            const int q = i + m0 * (j + m1 * k);
+            const int c = i + n0 * (j + n1 * k);   // the cell above the face
+            const int qd = D == 0 ? i : (D == 1 ? j : k);
+            const double we = io.w[q];
+            // dmu: over the entry, nu = 0 outside; dmf: over the physical face, which the solve uses
+            // once (entry n of a periodic direction is the duplicate)
+            double dmu, dmf = 0.0, dphi = 0.0, b = 0.0;
+            if (qd > 0 && qd < nd) {
+                dmu = io.nu[c] - io.nu[c - sd];
+                dphi = io.phi[c] - io.phi[c - sd];
+                b = io.beta[level_index(G.d0, i, j, k)];
+                dmf = dmu;
+            } else {
+                dmu = qd == 0 ? io.nu[c] : -io.nu[c - sd];
+                if (G.per[D]) {
+                    const int lo = qd == 0 ? c + (nd - 1) * sd : c - sd;
+                    const int hi = qd == 0 ? c : c - nd * sd;
+                    dphi = io.phi[hi] - io.phi[lo];
+                    b = io.beta[level_index(G.d0, D == 0 ? 0 : i, D == 1 ? 0 : j, D == 2 ? 0 : k)];
+                    if (qd == 0) dmf = io.nu[hi] - io.nu[lo];
+                }
+            }
+            const double ue = sums ? io.u[q] : 0.0;
+            const double t = b * dphi;
+            io.du[q] = fma(gd, dmu, we);
+            if (io.g) io.g[q] = t * fma(A, dmf, C * we) * b;
+            if (sums) {
+                a1 = fma(ue, dmu, a1);
+                a2 = fma(t, dmf, a2);
+                if (ALT) a3 = fma(t, we, a3);
+            }
+        }
+    if (!sums) return;
+    const double ib = kd * G.idx[D];   // 1 / beta0
+    double v = a1 * G.idx[D];
+    v = fma(ALT ? -2.0 * ib : -ib, a2, v);
+    if (ALT) v = fma(-ib * kd, a3, v);
+    v = block_sum(v);
+    if (threadIdx.x == 0 && threadIdx.y == 0)
+        io.part[blockIdx.x] = v;
 }
 
-// dL/d(1/rho_a) = sum over the physical faces of a of dL/dh_f * h_f^2 rho_a^2 / 2.
+// dL/d(1/rho_a) = sum over the physical faces of a of dL/dh_f * h_f^2 rho_a^2 / 2: the faces'
+// shares g carry the factors of dL/dh_f (zero on walls), so 7 FP64 operations a cell remain
+// (2300 us at 256^3 with a division a face; now 246).
 __global__ void __launch_bounds__(kB)
-k_adj_sigma(AdjGeom G, const double* __restrict__ rho, const double* __restrict__ dhx,
-            const double* __restrict__ dhy, const double* __restrict__ dhz,
+k_adj_sigma(AdjGeom G, const double* __restrict__ rho, const double* __restrict__ gx,
+            const double* __restrict__ gy, const double* __restrict__ gz,
             double* __restrict__ ds) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= G.d0.ncell) return;
-    const int i = q % G.n[0], row = q / G.n[0], j = row % G.n[1], k = row / G.n[1];
-    const int c[3] = {i, j, k};
-    const double* dh[3] = {dhx, dhy, dhz};
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = blockIdx.z;
+    const int n0 = G.n[0], n1 = G.n[1], n2 = G.n[2];
+    if (i >= n0 || j >= n1) return;
+    const int q = i + n0 * (j + n1 * k);
     const double rc = rho[q];
-    double s = 0.0;
-    for (int d = 0; d < G.dm; ++d) {
-        const int n = G.n[d];
-        if (c[d] > 0 || G.per[d]) {
-            int nb[3] = {i, j, k};
-            nb[d] = c[d] > 0 ? c[d] - 1 : n - 1;
-            const double h = 2.0 / (rc + rho[nat(G, nb[0], nb[1], nb[2])]);
-            int e[3] = {i, j, k};
-            double g = dh[d][face_nat(G, d, e[0], e[1], e[2])];
-            if (c[d] == 0) {
-                e[d] = n;
-                g += dh[d][face_nat(G, d, e[0], e[1], e[2])];
-            }
-            s += g * h * h;
-        }
-        if (c[d] < n - 1 || G.per[d]) {
-            int nb[3] = {i, j, k};
-            nb[d] = c[d] < n - 1 ? c[d] + 1 : 0;
-            const double h = 2.0 / (rc + rho[nat(G, nb[0], nb[1], nb[2])]);
-            int e[3] = {i, j, k};
-            e[d] = c[d] + 1;
-            double g = dh[d][face_nat(G, d, e[0], e[1], e[2])];
-            if (c[d] == n - 1) {
-                e[d] = 0;
-                g += dh[d][face_nat(G, d, e[0], e[1], e[2])];
-            }
-            s += g * h * h;
-        }
+    const int fx = i + (n0 + 1) * (j + n1 * k), fy = i + n0 * (j + (n1 + 1) * k);
+    double s = (gx[fx] + gx[fx + 1]) + (gy[fy] + gy[fy + n0]);
+    const int pl = n0 * n1;
+    if (G.dm == 3) s += gz[q] + gz[q + pl];
+    // periodic: the other entry of a boundary face (one branch, no predicated FP64 adds inside)
+    const bool ex = i == 0 || i == n0 - 1, ey = j == 0 || j == n1 - 1;
+    const bool ez = G.dm == 3 && (k == 0 || k == n2 - 1);
+    if (ex || ey || ez) {
+        if (ex) s += gx[i == 0 ? fx + n0 : fx + 1 - n0];
+        if (ey) s += gy[j == 0 ? fy + n0 * n1 : fy + n0 - n0 * n1];
+        if (ez) s += gz[k == 0 ? q + pl * n2 : q + pl - pl * n2];
     }
-    ds[q] = s * rc * rc * 0.5;
+    ds[q] = s * (rc * rc);
 }
 
-// One CTA per vertical index r: sum of the per-entry dbeta0 shares of the horizontal faces in
-// layer r (r < nr) into sh[r], of the vertical faces in plane r (r <= nr) into sv[r].
-__global__ void __launch_bounds__(kB)
-k_layer_sums(AdjGeom G, const double* __restrict__ bx, const double* __restrict__ by,
-             const double* __restrict__ bz, double* __restrict__ sh, double* __restrict__ sv) {
-    __shared__ double s1[kB], s2[kB];
+// One warp per vertical index r: the block sums of the horizontal faces of layer r (r < nr) into
+// sh[r], of the vertical faces of plane r (r <= nr) into sv[r].
+__global__ void k_layer_sums(int dm, int nr, int t0, int t1, int t2, const double* __restrict__ p0,
+                             const double* __restrict__ p1, const double* __restrict__ p2,
+                             double* __restrict__ sh, double* __restrict__ sv) {
     const int r = blockIdx.x;
-    const int nr = G.n[G.va];
-    const double* b[3] = {bx, by, bz};
+    const int nb[3] = {t0, t1, t2};
+    const double* p[3] = {p0, p1, p2};
     double a = 0.0, v = 0.0;
-    for (int d = 0; d < G.dm; ++d) {
-        const int m[3] = {G.n[0] + (d == 0), G.n[1] + (d == 1), G.n[2] + (d == 2)};
-        if (d == G.va && r > nr) continue;
-        if (d != G.va && r >= nr) continue;
-        // entries with vertical coordinate r: iterate over the other two directions
-        const int o0 = G.va == 0 ? 1 : 0, o1 = G.va == 2 ? 1 : 2;
-        const int cnt = m[o0] * m[o1];
-        for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
-            int e[3];
-            e[o0] = t % m[o0];
-            e[o1] = t / m[o0];
-            e[G.va] = r;
-            const double x = b[d][e[0] + m[0] * (e[1] + m[1] * e[2])];
-            if (d == G.va) v += x;
-            else a += x;
-        }
-    }
-    s1[threadIdx.x] = a;
-    s2[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = kB / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) {
-            s1[threadIdx.x] += s1[threadIdx.x + o];
-            s2[threadIdx.x] += s2[threadIdx.x + o];
-        }
-        __syncthreads();
+    if (r < nr)
+        for (int d = 0; d < dm - 1; ++d)
+            for (int t = threadIdx.x; t < nb[d]; t += 32) a += p[d][(long)r * nb[d] + t];
+    for (int t = threadIdx.x; t < nb[dm - 1]; t += 32) v += p[dm - 1][(long)r * nb[dm - 1] + t];
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, o);
+        v += __shfl_down_sync(0xffffffffu, v, o);
     }
     if (threadIdx.x == 0) {
-        if (r < nr) sh[r] = s1[0];
-        sv[r] = s2[0];
+        if (r < nr) sh[r] = a;
+        sv[r] = v;
     }
-}
-
-__global__ void k_mu_to_nat(Dims d, const double* __restrict__ mu, const double* __restrict__ mean,
-                            double* __restrict__ out) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= d.ncell) return;
-    const int i = q % d.n0, row = q / d.n0, j = row % d.n1, k = row / d.n1;
-    out[q] = mu[level_index(d, i, j, k)] - mean[0];
 }
 
 // Transpose of cell_to_edge (Source/cell_to_edge.f90:39-60) applied to the edge sensitivities sv:
@@ -322,15 +326,8 @@ void cell_to_edge_vjp(int nr, const double* c, const double* sv, double* g) {
     }
 }
 
-struct AdjBuffers {
-    double* phiF = nullptr;     // forward phi, level-0 layout
-    double* part = nullptr;     // partial sums
-    double* mean = nullptr;     // [1]
-    double* dh[3] = {nullptr, nullptr, nullptr};
-    double* db0[3] = {nullptr, nullptr, nullptr};
-    double* layer = nullptr;    // sh[nr], sv[nr+1]
-    bool ready = false;
-};
+// Block of k_adj_face: (32, 8) threads over a plane in 3-D, a single row in 2-D.
+dim3 face_block(const mac_ctx* c) { return c->dm == 3 ? dim3(32, 8) : dim3(kB, 1); }
 
 }  // namespace
 }  // namespace mac
@@ -359,45 +356,48 @@ extern "C" int mac_macproject_adjoint_dense(mac_ctx* c, const double* ux, const 
         if (c->bc_lo[d] == MAC_BC_DIR || c->bc_hi[d] == MAC_BC_DIR) return st->status = MAC_ERR_UNSUPPORTED;
     const auto t0 = std::chrono::steady_clock::now();
     begin_call_stats(c, st);
-    // adjoint buffers live with the context's allocations (freed by mac_ctx_destroy)
     const size_t N = (size_t)c->n[0] * c->n[1] * c->n[2];
     const int nr = c->n[c->va];
-    const int nbp = ceil_div((long)N, kB);
-    AdjBuffers B;
-    int rc = MAC_OK;
-    rc |= alloc_device(c, (void**)&B.phiF, N * sizeof(double));
-    rc |= alloc_device(c, (void**)&B.part, (size_t)nbp * sizeof(double));
-    rc |= alloc_device(c, (void**)&B.mean, sizeof(double));
-    rc |= alloc_device(c, (void**)&B.layer, (size_t)(2 * nr + 2) * sizeof(double));
+    // sums of this call: [mean, kMeanBlocks partials, sh[nr], sv[nr + 1], layer partials of each d];
+    // everything of the size of a field uses solver arrays that are idle at the time
+    size_t off[4] = {(size_t)(1 + kMeanBlocks + 2 * nr + 1), 0, 0, 0};
+    const dim3 fb = face_block(c);
+    int cols[3], tiles[3] = {0, 0, 0}, layers[3];
     for (int d = 0; d < c->dm; ++d) {
-        const size_t nf = (size_t)(c->n[0] + (d == 0)) * (c->n[1] + (d == 1)) * (c->n[2] + (d == 2));
-        rc |= alloc_device(c, (void**)&B.dh[d], nf * sizeof(double));
-        rc |= alloc_device(c, (void**)&B.db0[d], nf * sizeof(double));
+        cols[d] = ceil_div(c->n[0] + (d == 0), fb.x);
+        tiles[d] = cols[d] * ceil_div(c->dm == 3 ? c->n[1] + (d == 1) : 1, fb.y * kFaceRows);
+        layers[d] = nr + (d == c->va);
+        off[d + 1] = off[d] + (size_t)tiles[d] * layers[d];
     }
-    if (rc) return st->status = MAC_ERR_ALLOC;
+    if (!c->adj_sums && alloc_device(c, (void**)&c->adj_sums, off[c->dm] * sizeof(double)))
+        return st->status = MAC_ERR_ALLOC;
+    double* mean = c->adj_sums;
+    double* part = mean + 1;
+    double* layer = part + kMeanBlocks;
     cudaStream_t s = c->stream;
     Level& F = c->lev[0];
     const double* uin[3] = {ux, uy, uz};
     const double* win[3] = {wx, wy, wz};
     double* dout[3] = {dux, duy, duz};
-    // ---- forward: phi of the projection (U copied; the caller's arrays stay untouched)
-    for (int d = 0; d < c->dm; ++d) {
-        const size_t nf = (size_t)(c->n[0] + (d == 0)) * (c->n[1] + (d == 1)) * (c->n[2] + (d == 2));
-        MAC_CUDA_TRY(cudaMemcpyAsync(c->u[d], uin[d], nf * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    }
+    // ---- forward: phi of the projection, in c->phin.  The velocities are read where they are and
+    // not corrected (the gradient does not need the projected ones).
     double* saved_rho = c->rho;
+    double* saved_u[3] = {c->u[0], c->u[1], c->u[2]};
     c->rho = const_cast<double*>(rho);
-    MAC_CUDA_TRY(cudaMemsetAsync(c->phin, 0, N * sizeof(double), s));
-    if (beta0) rc = load_beta0(c, MAC_PTR_DEVICE, beta0, beta0_edge);
+    for (int d = 0; d < c->dm; ++d) c->u[d] = const_cast<double*>(uin[d]);
     mac_stats fst;
     std::memset(&fst, 0, sizeof(fst));
-    if (!rc) rc = forward_projection(c, macrhs, beta0 != nullptr, &fst);
+    auto forward = [&]() -> int {
+        MAC_CUDA_TRY(cudaMemsetAsync(c->phin, 0, N * sizeof(double), s));
+        const int r = beta0 ? load_beta0(c, MAC_PTR_DEVICE, beta0, beta0_edge) : MAC_OK;
+        return r ? r : forward_phi(c, macrhs, beta0 != nullptr, &fst);
+    };
+    int rc = forward();
+    for (int d = 0; d < c->dm; ++d) c->u[d] = saved_u[d];
     if (rc != MAC_OK) {
         c->rho = saved_rho;
         return st->status = rc;
     }
-    MAC_CUDA_TRY(cudaMemcpyAsync(B.phiF, F.a64.phi, N * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    if (phi_out) MAC_CUDA_TRY(cudaMemcpyAsync(phi_out, c->phin, N * sizeof(double), cudaMemcpyDeviceToDevice, s));
 
     AdjGeom G;
     for (int d = 0; d < 3; ++d) {
@@ -406,78 +406,71 @@ extern "C" int mac_macproject_adjoint_dense(mac_ctx* c, const double* ux, const 
         G.idx[d] = 1.0 / c->dx[d];
     }
     G.dm = c->dm;
-    G.va = c->va;
     G.p = beta0 ? (c->o.use_alt_energy_fix ? 2 : 1) : 0;
     G.d0 = F.d;
-    const double* b0 = beta0 ? c->beta0 : nullptr;
-    const double* b0e = beta0 ? c->beta0e : nullptr;
+    const Grid3 g = grid3(c->n[0], c->n[1], c->n[2]);
 
     // ---- adjoint right-hand side and solve with the same hierarchy
-    k_adj_rhs<<<ceil_div((long)N, kB), kB, 0, s>>>(G, rho, b0, b0e, wx, wy, c->dm == 3 ? wz : wy,
-                                                   c->scratch);
-    MAC_CUDA_TRY(cudaGetLastError());
-    rc = setup_rhs_from(c, c->scratch);
+    auto adjoint_rhs = [&]() -> int {
+        if (phi_out)
+            MAC_CUDA_TRY(cudaMemcpyAsync(phi_out, c->phin, N * sizeof(double), cudaMemcpyDeviceToDevice, s));
+        const dim3 rg(g.grid.x, g.grid.y, ceil_div(c->n[2], kAdjPlanes));
+        auto kern = c->dm == 3 ? k_adj_rhs<3> : k_adj_rhs<2>;
+        kern<<<rg, g.block, 0, s>>>(G, F.a64.bx, F.a64.by, F.a64.bz, c->b0tab, wx, wy,
+                                    c->dm == 3 ? wz : wy, c->scratch);
+        MAC_CUDA_TRY(cudaGetLastError());
+        const int r = setup_rhs_from(c, c->scratch);
+        if (r) return r;
+        MAC_CUDA_TRY(cudaMemsetAsync(F.a64.phi, 0, N * sizeof(double), s));
+        return MAC_OK;
+    };
+    rc = adjoint_rhs();
     if (rc) {
         c->rho = saved_rho;
         return st->status = rc;
     }
-    MAC_CUDA_TRY(cudaMemsetAsync(F.a64.phi, 0, N * sizeof(double), s));
     const int solve_rc = run_solve(c, st);
     c->rho = saved_rho;
     if (solve_rc != MAC_OK && solve_rc != MAC_ERR_NOT_CONVERGED) return st->status = solve_rc;
     // nu = mu - mean(mu)
-    k_partial_sum<<<nbp, kB, 0, s>>>((int)N, F.a64.phi, B.part);
-    k_final_mean<<<1, 1024, 0, s>>>(nbp, (int)N, B.part, B.mean);
+    double* nu = dmacrhs ? dmacrhs : c->scratch;
+    k_partial_sum<<<kMeanBlocks, kB, 0, s>>>((int)N, F.a64.phi, part);
+    k_final_mean<<<1, 1024, 0, s>>>((int)N, part, mean);
+    k_mu_to_nat<<<g.grid, g.block, 0, s>>>(F.d, F.a64.phi, mean, nu);
     MAC_CUDA_TRY(cudaGetLastError());
 
-    // ---- per-face gradients
+    // ---- per-face gradients (the faces' shares of dL/d(1/rho) go to the solver's velocity arrays)
+    const double* beta[3] = {F.a64.bx, F.a64.by, F.a64.bz};
     for (int d = 0; d < c->dm; ++d) {
-        const long nf = (long)(c->n[0] + (d == 0)) * (c->n[1] + (d == 1)) * (c->n[2] + (d == 2));
-        FaceOut fo{dout[d], B.dh[d], B.db0[d]};
-        k_adj_face<<<ceil_div(nf, kB), kB, 0, s>>>(G, d, rho, b0, b0e, uin[d], win[d], B.phiF,
-                                                   F.a64.phi, B.mean, fo);
+        const FaceIo io{beta[d], uin[d], win[d], c->phin, nu, dout[d], drinv ? c->u[d] : nullptr,
+                        dbeta0 ? c->adj_sums + off[d] : nullptr, cols[d], tiles[d]};
+        auto kern = G.p == 2 ? (d == 0   ? k_adj_face<0, true>
+                                : d == 1 ? k_adj_face<1, true>
+                                         : k_adj_face<2, true>)
+                             : (d == 0   ? k_adj_face<0, false>
+                                : d == 1 ? k_adj_face<1, false>
+                                         : k_adj_face<2, false>);
+        kern<<<tiles[d] * layers[d], fb, 0, s>>>(G, c->b0tab, io);
         MAC_CUDA_TRY(cudaGetLastError());
     }
     if (drinv) {
-        k_adj_sigma<<<ceil_div((long)N, kB), kB, 0, s>>>(G, rho, B.dh[0], B.dh[1],
-                                                         c->dm == 3 ? B.dh[2] : B.dh[1], drinv);
-        MAC_CUDA_TRY(cudaGetLastError());
-    }
-    if (dmacrhs) {
-        k_mu_to_nat<<<ceil_div((long)N, kB), kB, 0, s>>>(F.d, F.a64.phi, B.mean, dmacrhs);
+        k_adj_sigma<<<g.grid, g.block, 0, s>>>(G, rho, c->u[0], c->u[1], c->u[2], drinv);
         MAC_CUDA_TRY(cudaGetLastError());
     }
     if (dbeta0) {
-        k_layer_sums<<<nr + 1, kB, 0, s>>>(G, B.db0[0], B.db0[1], c->dm == 3 ? B.db0[2] : B.db0[1],
-                                           B.layer, B.layer + nr);
+        k_layer_sums<<<nr + 1, 32, 0, s>>>(c->dm, nr, tiles[0], tiles[1], tiles[2],
+                                           c->adj_sums + off[0], c->adj_sums + off[1],
+                                           c->adj_sums + off[2], layer, layer + nr);
         MAC_CUDA_TRY(cudaGetLastError());
-        std::vector<double> h(2 * nr + 1), cb(nr), g(nr);
-        MAC_CUDA_TRY(cudaMemcpyAsync(h.data(), B.layer, (2 * nr + 1) * sizeof(double), cudaMemcpyDeviceToHost, s));
+        std::vector<double> h(2 * nr + 1), cb(nr), gb(nr);
+        MAC_CUDA_TRY(cudaMemcpyAsync(h.data(), layer, (2 * nr + 1) * sizeof(double), cudaMemcpyDeviceToHost, s));
         MAC_CUDA_TRY(cudaMemcpyAsync(cb.data(), beta0, nr * sizeof(double), cudaMemcpyDeviceToHost, s));
         MAC_CUDA_TRY(cudaStreamSynchronize(s));
-        for (int k = 0; k < nr; ++k) g[k] = h[k];
-        cell_to_edge_vjp(nr, cb.data(), h.data() + nr, g.data());
-        MAC_CUDA_TRY(cudaMemcpyAsync(dbeta0, g.data(), nr * sizeof(double), cudaMemcpyHostToDevice, s));
+        for (int k = 0; k < nr; ++k) gb[k] = h[k];
+        cell_to_edge_vjp(nr, cb.data(), h.data() + nr, gb.data());
+        MAC_CUDA_TRY(cudaMemcpyAsync(dbeta0, gb.data(), nr * sizeof(double), cudaMemcpyHostToDevice, s));
     }
     MAC_CUDA_TRY(cudaStreamSynchronize(s));
-    // the temporaries go back to the device now (the context keeps only its solver arrays)
-    auto release = [&](void* p) {
-        if (!p) return;
-        for (size_t a = 0; a < c->allocations.size(); ++a)
-            if (c->allocations[a] == p) {
-                c->allocations.erase(c->allocations.begin() + (long)a);
-                break;
-            }
-        cudaFree(p);
-    };
-    release(B.phiF);
-    release(B.part);
-    release(B.mean);
-    release(B.layer);
-    for (int d = 0; d < 3; ++d) {
-        release(B.dh[d]);
-        release(B.db0[d]);
-    }
     st->vcycles += fst.vcycles;
     st->setup_ms += fst.setup_ms;
     st->solve_ms += fst.solve_ms;

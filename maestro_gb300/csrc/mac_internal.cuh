@@ -266,6 +266,7 @@ struct mac_ctx {
     // per vertical index r: the kTab* factor tables, (nr+1) doubles each
     double* b0tab = nullptr;
     double* scratch = nullptr;                    // generic FP64 scratch (ncell)
+    double* adj_sums = nullptr;                   // the adjoint's sums (allocated on first use)
     double* base1d = nullptr;                     // 4 x (nr + 1) base-state values
     // caller-layout staging (host-pointer calls): one region per array of a call, filled and
     // drained by the copy engines on the transfer stream
@@ -500,9 +501,9 @@ int amr_configure(mac_ctx* c, int nlev, const int* nboxes, const int* box_lo, co
 void amr_release(mac_ctx* c);
 // ---- nodal projection (hg_nodal.cu) -----------------------------------------------------------
 void hg_release(mac_ctx* c);
-// Forward projection on the whole-domain arrays already in c->u / c->rho / c->phin; leaves the
-// level-0 coefficients and phi (level-0 layout) in place.
-int forward_projection(mac_ctx* c, const double* macrhs, bool have_beta0, mac_stats* st);
+// Solve of the forward projection on the whole-domain arrays in c->u / c->rho / c->phin, without the
+// velocity correction; leaves the level-0 coefficients and phi (both layouts) in place.
+int forward_phi(mac_ctx* c, const double* macrhs, bool have_beta0, mac_stats* st);
 int set_call_state(mac_ctx* c, bool with_alpha);
 // finest FP32 level with coefficients from rho on the fly (mixed MAC projection) or stored
 int set_otf_mode(mac_ctx* c, bool on);

@@ -864,12 +864,13 @@ int set_call_state_impl(mac_ctx* c, bool with_alpha) {
     return MAC_OK;
 }
 
-// The projection on whole-domain device arrays already in c->u / c->rho / rhs / phin.
+// The projection on whole-domain device arrays already in c->u / c->rho / rhs / phin; `correct`
+// false leaves the velocities as they are and only returns phi.
 int core_macproject(mac_ctx* c, const double* macrhs, bool have_beta0, mac_stats* st,
                     const std::function<int()>* before_rhs = nullptr,
                     const std::function<int()>* before_phi = nullptr,
                     const std::function<int()>* after_phi = nullptr,
-                    const std::function<int(int)>* after_dir = nullptr) {
+                    const std::function<int(int)>* after_dir = nullptr, bool correct = true) {
     Level& F = c->lev[0];
     cudaEventRecord(c->ev[0], c->stream);
     int rc = set_call_state_impl(c, false);
@@ -897,7 +898,8 @@ int core_macproject(mac_ctx* c, const double* macrhs, bool have_beta0, mac_stats
         if (!r && after_dir) r = (*after_dir)(d);
         return r;
     };
-    rc = correct_velocity(c, have_beta0, &dir_hook, c->phin);
+    rc = correct ? correct_velocity(c, have_beta0, &dir_hook, c->phin)
+                 : level0_to_natural(c, F.a64.phi, c->phin);
     if (rc) return rc;
     c->ktime_launches[MAC_KT_CORRECT] += (int)(c->issued - before_corr);
     c->ktime_launches[MAC_KT_SETUP] += (int)setup_kernels;
@@ -962,8 +964,8 @@ int level0_fp32_vcycle(mac_ctx* c) {
     MAC_CUDA_TRY(cudaGetLastError());
     return MAC_OK;
 }
-int forward_projection(mac_ctx* c, const double* macrhs, bool have_beta0, mac_stats* st) {
-    return core_macproject(c, macrhs, have_beta0, st);
+int forward_phi(mac_ctx* c, const double* macrhs, bool have_beta0, mac_stats* st) {
+    return core_macproject(c, macrhs, have_beta0, st, nullptr, nullptr, nullptr, nullptr, false);
 }
 int set_call_state(mac_ctx* c, bool with_alpha) { return set_call_state_impl(c, with_alpha); }
 int set_otf_mode(mac_ctx* c, bool on) { return set_otf(c, on); }
