@@ -127,6 +127,17 @@ __device__ __forceinline__ bool positive_finite(double v) {
     return b > 0 && b < 0x7FF0000000000000LL;
 }
 
+// Coarse correction of cell ci that a restriction hands on, v its defect: zero, or, given the coarse
+// level's inverse diagonal (idc), what that level's first colour-0 half-sweep makes of zero, so that it
+// needs no launch of its own.  Bitwise the half-sweep's result: its six arms add b * 0 to v.
+template <typename T>
+__device__ __forceinline__ T coarse_start(T v, int ci, const Dims& C, const T* __restrict__ idc,
+                                          T omega) {
+    if (!idc || ci >= C.half) return T(0);
+    const T e = v * idc[ci];
+    return sizeof(T) == 8 ? e : omega * e;   // (FP64 half-sweeps are never over-relaxed)
+}
+
 // Per-layer factor tables (k_beta0_tables), nr+1 entries each, vertical index r:
 enum {
     kTabFac0 = 0,   // beta0_f^p * 2 / h_d^2 of the low face along d (3 tables: d = 0, 1, 2)
@@ -337,7 +348,7 @@ template <typename T>
 void launch_gsrb(const Dims& d, int colour, LevelArrays<T>& a, cudaStream_t s, T omega = T(1));
 template <typename T>
 void launch_resid_restrict(const Dims& fine, const Dims& coarse, const LevelArrays<T>& a,
-                           T* fc, T* ec, bool red_only, cudaStream_t s);
+                           T* fc, T* ec, bool red_only, cudaStream_t s, const T* idc, T omega);
 // phi_in (optional): read the fine values from phi_in instead of phi_fine (out of place; the
 // cells the kernel does not update keep phi_fine's values)
 template <typename T>
@@ -373,7 +384,8 @@ void launch_gsrb_otf(const Dims& d, const OtfParams& P, int colour, float* e, co
 // with red_only false the staged kernel then forms only the colour-0 defects and adds them
 void launch_resid_restrict_otf(const Dims& fine, const Dims& coarse, const OtfParams& P,
                                const float* e, const float* r, float* fc, float* ec,
-                               bool red_only, cudaStream_t s, const float* blk = nullptr);
+                               bool red_only, cudaStream_t s, const float* idc, float omega,
+                               const float* blk = nullptr);
 // whether the staged half-sweep and defect kernels run on this level (then dout/blk apply)
 inline bool otf_staged(const OtfParams& P) { return P.dm == 3 && P.ty > 0 && P.rty > 0; }
 // one whole red/black sweep of the finest FP32 level, ein -> eout (both colours; ein != eout);

@@ -192,7 +192,8 @@ template <typename T, bool RED_ONLY>
 __global__ void __launch_bounds__(kBlock)
 k_resid_restrict(Dims F, Dims C, const T* __restrict__ u, const T* __restrict__ f,
                  const T* __restrict__ bx, const T* __restrict__ by, const T* __restrict__ bz,
-                 const T* __restrict__ dg, T* __restrict__ fc, T* __restrict__ ec) {
+                 const T* __restrict__ dg, T* __restrict__ fc, T* __restrict__ ec,
+                 const T* __restrict__ idc, T omega) {
     pdl_wait();
     pdl_trigger();
     const int I = blockIdx.x * blockDim.x + threadIdx.x;
@@ -223,8 +224,9 @@ k_resid_restrict(Dims F, Dims C, const T* __restrict__ u, const T* __restrict__ 
         ci = ((I + J + K) & 1) * C.half + (J + C.n1 * K) * C.hn0 + (I >> 1);
     else
         ci = I + C.n0 * (J + C.n1 * K);
-    fc[ci] = sum * (T)(1.0 / (4 * F.rz));
-    ec[ci] = T(0);   // the coarse correction starts from zero (no separate memset in the chain)
+    const T v = sum * (T)(1.0 / (4 * F.rz));
+    fc[ci] = v;
+    ec[ci] = coarse_start(v, ci, C, idc, omega);
 }
 
 // ---- prolongation: u_fine += (bi/tri)linear interpolation of the coarse correction ----------
@@ -686,16 +688,16 @@ void launch_gsrb(const Dims& d, int colour, LevelArrays<T>& a, cudaStream_t s, T
 
 template <typename T>
 void launch_resid_restrict(const Dims& fine, const Dims& coarse, const LevelArrays<T>& a, T* fc,
-                           T* ec, bool red_only, cudaStream_t s) {
+                           T* ec, bool red_only, cudaStream_t s, const T* idc, T omega) {
     const Grid3 g = grid3(coarse.n0, coarse.n1, coarse.n2);
     if (red_only)
         launch_chain(k_resid_restrict<T, true>, g.grid, g.block, 0, s, fine, coarse,
                    (const T*)a.phi, (const T*)a.f, (const T*)a.bx, (const T*)a.by, (const T*)a.bz,
-                   (const T*)a.diag, fc, ec);
+                   (const T*)a.diag, fc, ec, idc, omega);
     else
         launch_chain(k_resid_restrict<T, false>, g.grid, g.block, 0, s, fine, coarse,
                    (const T*)a.phi, (const T*)a.f, (const T*)a.bx, (const T*)a.by, (const T*)a.bz,
-                   (const T*)a.diag, fc, ec);
+                   (const T*)a.diag, fc, ec, idc, omega);
 }
 
 template <typename T>
@@ -796,9 +798,9 @@ void launch_bottom(const Dims& d, const LevelArrays<double>& a64, Tio* x, const 
 template void launch_gsrb<double>(const Dims&, int, LevelArrays<double>&, cudaStream_t, double);
 template void launch_gsrb<float>(const Dims&, int, LevelArrays<float>&, cudaStream_t, float);
 template void launch_resid_restrict<double>(const Dims&, const Dims&, const LevelArrays<double>&,
-                                            double*, double*, bool, cudaStream_t);
+                                            double*, double*, bool, cudaStream_t, const double*, double);
 template void launch_resid_restrict<float>(const Dims&, const Dims&, const LevelArrays<float>&,
-                                            float*, float*, bool, cudaStream_t);
+                                            float*, float*, bool, cudaStream_t, const float*, float);
 template void launch_prolong_add<double>(const Dims&, const Dims&, const BcDesc&, const double*,
                                          double*, bool, cudaStream_t, const double*);
 template void launch_prolong_add<float>(const Dims&, const Dims&, const BcDesc&, const float*,

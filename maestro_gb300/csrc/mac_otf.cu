@@ -438,6 +438,7 @@ k_resid_restrict_staged(Dims d, Dims C, OtfParams P, const float* __restrict__ e
                         const float* __restrict__ eown, const float* __restrict__ rs,
                         const float* __restrict__ rhos, const float* __restrict__ rhoo,
                         float* __restrict__ fc, float* __restrict__ ec,
+                        const float* __restrict__ idc, float omega,
                         const float* __restrict__ blk = nullptr) {
     constexpr int V = kCellsPerThread;
     constexpr int colour = 0;
@@ -594,8 +595,14 @@ k_resid_restrict_staged(Dims d, Dims C, OtfParams P, const float* __restrict__ e
                 const long base = (long)(J + C.n1 * K) * C.hn0 + (c0 >> 1);
                 *reinterpret_cast<float2*>(fc + pc * C.half + base) = make_float2(v0, v2);
                 *reinterpret_cast<float2*>(fc + (pc ^ 1) * C.half + base) = make_float2(v1, v3);
-                *reinterpret_cast<float2*>(ec + pc * C.half + base) = make_float2(0.f, 0.f);
-                *reinterpret_cast<float2*>(ec + (pc ^ 1) * C.half + base) = make_float2(0.f, 0.f);
+                float2 red = make_float2(0.f, 0.f);   // coarse_start of the two colour-0 cells
+                if (idc) {
+                    const float2 id = *reinterpret_cast<const float2*>(idc + base);
+                    red.x = omega * __fmul_rn(pc ? v1 : v0, id.x);
+                    red.y = omega * __fmul_rn(pc ? v3 : v2, id.y);
+                }
+                *reinterpret_cast<float2*>(ec + base) = red;
+                *reinterpret_cast<float2*>(ec + C.half + base) = make_float2(0.f, 0.f);
             }
         }
         Eb = Ec;
@@ -861,7 +868,8 @@ k_sweep_otf_fused(Dims d, OtfParams P, const float* __restrict__ ein, float* __r
 template <int DM, bool RED_ONLY>
 __global__ void __launch_bounds__(kB)
 k_resid_restrict_otf(Dims F, Dims C, OtfParams P, const float* __restrict__ e,
-                     const float* __restrict__ r, float* __restrict__ fc, float* __restrict__ ec) {
+                     const float* __restrict__ r, float* __restrict__ fc, float* __restrict__ ec,
+                     const float* __restrict__ idc, float omega) {
     pdl_wait();
     pdl_trigger();
     const int I = blockIdx.x * blockDim.x + threadIdx.x;
@@ -898,8 +906,9 @@ k_resid_restrict_otf(Dims F, Dims C, OtfParams P, const float* __restrict__ e,
         ci = ((I + J + K) & 1) * C.half + (J + C.n1 * K) * C.hn0 + (I >> 1);
     else
         ci = I + C.n0 * (J + C.n1 * K);
-    fc[ci] = sum * (DM == 3 ? 0.125f : 0.25f);
-    ec[ci] = 0.f;   // the coarse correction starts from zero (no separate memset in the chain)
+    const float v = sum * (DM == 3 ? 0.125f : 0.25f);
+    fc[ci] = v;
+    ec[ci] = coarse_start(v, ci, C, idc, omega);
 }
 
 }  // namespace
@@ -1027,7 +1036,8 @@ static int plane_chunk(long tiles, long resident, int n2, int unit) {
 
 // Tile plan of the staged half-sweep: ty = the largest power of two with ty * hn0 <= 1024 cells
 // that divides n1 (one float4 group of 4 cells per thread, at most 256 threads); whole rows of
-// 16-byte multiples (hn0 % 4 == 0); chunks of plane_chunk planes.  Sets ty = 0 where the staged kernel does not apply.
+// 16-byte multiples (hn0 % 4 == 0); chunks of plane_chunk planes.  Sets ty = 0 where the staged
+// kernel does not apply.
 void plan_otf_tile(const Dims& d, int dm, int sms, OtfParams& P) {
     static std::mutex mu;
     static int smem_set = 0;
@@ -1137,7 +1147,8 @@ void launch_sweep_otf_fused(const Dims& d, const OtfParams& P, const float* ein,
 
 void launch_resid_restrict_otf(const Dims& fine, const Dims& coarse, const OtfParams& P,
                                const float* e, const float* r, float* fc, float* ec,
-                               bool red_only, cudaStream_t s, const float* blk) {
+                               bool red_only, cudaStream_t s, const float* idc, float omega,
+                               const float* blk) {
     if (P.dm == 3 && P.rty > 0 && (red_only || blk) && coarse.split) {
         // colour 0 is "own": its e, f and rho; colour 1 the other colour's e and rho (and, after
         // an over-relaxed colour-1 half-sweep, its defects in blk)
@@ -1150,24 +1161,24 @@ void launch_resid_restrict_otf(const Dims& fine, const Dims& coarse, const OtfPa
                              : (P.has_dir ? k_resid_restrict_staged<true, true>
                                           : k_resid_restrict_staged<false, true>);
         launch_chain(kern, grid, dim3(nt), (size_t)P.rsmem, s, fine, coarse, P, eo, e, r,
-                     (const float*)P.rho, rhoo, fc, ec, red_only ? (const float*)nullptr : blk);
+                     (const float*)P.rho, rhoo, fc, ec, idc, omega, red_only ? (const float*)nullptr : blk);
         return;
     }
     const Grid3 g = grid3(coarse.n0, coarse.n1, coarse.n2);
     if (P.dm == 3) {
         if (red_only)
             launch_chain(k_resid_restrict_otf<3, true>, g.grid, g.block, 0, s, fine, coarse, P, e, r,
-                       fc, ec);
+                       fc, ec, idc, omega);
         else
             launch_chain(k_resid_restrict_otf<3, false>, g.grid, g.block, 0, s, fine, coarse, P, e,
-                       r, fc, ec);
+                       r, fc, ec, idc, omega);
     } else {
         if (red_only)
             launch_chain(k_resid_restrict_otf<2, true>, g.grid, g.block, 0, s, fine, coarse, P, e, r,
-                       fc, ec);
+                       fc, ec, idc, omega);
         else
             launch_chain(k_resid_restrict_otf<2, false>, g.grid, g.block, 0, s, fine, coarse, P, e,
-                       r, fc, ec);
+                       r, fc, ec, idc, omega);
     }
 }
 

@@ -165,8 +165,10 @@ int sweeps_up(const mac_ctx* c, bool fp32) {
     return fp32 && c->o.inner_nu2 >= 0 ? c->o.inner_nu2 : c->o.nu2;
 }
 
+// One V-cycle from level l down; red_done: the level's first colour-0 half-sweep has been done
+// (coarse_start).
 template <typename T>
-void vcycle(mac_ctx* c, int l) {
+void vcycle(mac_ctx* c, int l, bool red_done = false) {
     Level& L = c->lev[l];
     LevelArrays<T>& a = arrays<T>(L);
     const mac_opts& o = c->o;
@@ -225,6 +227,11 @@ void vcycle(mac_ctx* c, int l) {
     const OtfParams P = otf ? otf_params(c) : OtfParams{};
     Level& C = c->lev[l + 1];
     LevelArrays<T>& ac = arrays<T>(C);
+    // a coarse level that is swept here, not in the tail or the bottom solve, gets its first colour-0
+    // half-sweep from the restriction
+    const bool next_red = nu1 > 0 && l + 1 < c->nlevels - 1 &&
+                          !(o.coarse_tail && l + 1 == c->tail_start[tslot]);
+    const T* idc = next_red ? ac.invdiag : nullptr;
     // over-relaxed finest level with the staged kernels: the last pre-smoothing colour-1
     // half-sweep writes its cells' defects, and the staged restriction forms only the colour-0
     // ones (instead of both colours cell by cell)
@@ -247,10 +254,11 @@ void vcycle(mac_ctx* c, int l) {
         }
         mark(c, tm, 1);
         launch_resid_restrict_otf(L.d, C.d, P, cur, f, reinterpret_cast<float*>(ac.f),
-                                  reinterpret_cast<float*>(ac.phi), gs && nu1 > 0, c->stream, blk);
+                                  reinterpret_cast<float*>(ac.phi), gs && nu1 > 0, c->stream,
+                                  reinterpret_cast<const float*>(idc), (float)omega, blk);
         ++c->issued;
         mark(c, tm, 2);
-        vcycle<T>(c, l + 1);
+        vcycle<T>(c, l + 1, next_red);
         mark(c, tm, 3);
         float* tgt = nu2 % 2 ? B : A;
         launch_prolong_add<float>(L.d, C.d, bc_desc(c), reinterpret_cast<const float*>(ac.phi),
@@ -267,36 +275,37 @@ void vcycle(mac_ctx* c, int l) {
         mark(c, tm, 5);
         return;
     }
-    auto sweep = [&](bool last_down) {
-        for (int colour = 0; colour < 2; ++colour) {
+    auto sweep = [&](bool last_down, bool first) {
+        for (int colour = first && red_done ? 1 : 0; colour < 2; ++colour) {
             if (otf)
                 launch_gsrb_otf(L.d, P, colour, reinterpret_cast<float*>(a.phi),
                                 reinterpret_cast<const float*>(a.f), c->stream,
                                 last_down && colour == 1 ? blk : nullptr);
             else
                 launch_gsrb<T>(L.d, colour, a, c->stream, omega);
+            ++c->issued;
         }
-        c->issued += 2;
     };
     mark(c, tm, 0);
-    for (int s = 0; s < nu1; ++s) sweep(s == nu1 - 1);
+    for (int s = 0; s < nu1; ++s) sweep(s == nu1 - 1, s == 0);
     mark(c, tm, 1);
     if (otf)
         launch_resid_restrict_otf(L.d, C.d, P, reinterpret_cast<const float*>(a.phi),
                                   reinterpret_cast<const float*>(a.f),
                                   reinterpret_cast<float*>(ac.f), reinterpret_cast<float*>(ac.phi),
-                                  gs && nu1 > 0, c->stream, blk);
+                                  gs && nu1 > 0, c->stream, reinterpret_cast<const float*>(idc),
+                                  (float)omega, blk);
     else
-        launch_resid_restrict<T>(L.d, C.d, a, ac.f, ac.phi, gs && nu1 > 0, c->stream);
+        launch_resid_restrict<T>(L.d, C.d, a, ac.f, ac.phi, gs && nu1 > 0, c->stream, idc, omega);
     ++c->issued;
-    mark(c, tm, 2);   // (the restriction also zeroed the coarse correction ac.phi)
-    vcycle<T>(c, l + 1);
+    mark(c, tm, 2);   // (the restriction also set the coarse correction ac.phi)
+    vcycle<T>(c, l + 1, next_red);
     mark(c, tm, 3);
     // with post-smoothing, only colour-1 cells need the correction (see k_prolong_add)
     launch_prolong_add<T>(L.d, C.d, bc_desc(c), ac.phi, a.phi, gs && nu2 > 0, c->stream);
     ++c->issued;
     mark(c, tm, 4);
-    for (int s = 0; s < nu2; ++s) sweep(false);
+    for (int s = 0; s < nu2; ++s) sweep(false, false);
     mark(c, tm, 5);
 }
 
