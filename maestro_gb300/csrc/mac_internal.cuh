@@ -359,6 +359,9 @@ void launch_resid_norm(const Dims& d, const LevelArrays<T>& a, bool red_only,
                        unsigned long long* maxbits, cudaStream_t s);
 // r32 = f - L phi (FP64 arithmetic, FP32 result) and its max-norm; e32 (optional) is zeroed in
 // the same pass (the next inner solve starts from e = 0)
+// colour-0 half-sweep and the residual max-norm before it; keep[half]: the values before it
+void launch_gsrb_norm(const Dims& d, LevelArrays<double>& a, double* keep,
+                      unsigned long long* maxbits, cudaStream_t s);
 void launch_resid64_to32(const Dims& d, const LevelArrays<double>& a, float* r32,
                          unsigned long long* maxbits, cudaStream_t s, float* e32 = nullptr);
 // the initial residual of a zero guess: f -= mean (mean non-null), r32 = f, e32 = 0, max |f|

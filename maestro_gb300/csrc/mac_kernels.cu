@@ -520,6 +520,38 @@ k_resid_norm(Dims F, const T* __restrict__ u, const T* __restrict__ f, const T* 
     if (threadIdx.x == 0 && threadIdx.y == 0 && m) atomicMax(maxbits, m);
 }
 
+// The residual max-norm after a V-cycle (colour 1 has none: its half-sweep came last) and the next
+// cycle's first colour-0 half-sweep in one pass: both need the six arms of every colour-0 cell, which
+// are 6 of the half-sweep's 7 FP64 operations (a kernel each: 127 + 105 us at 256^3; together 117).
+// keep receives the values before the update, to be put back if the norm ends the iteration.
+__global__ void __launch_bounds__(kBlock)
+k_gsrb_norm(Dims d, double* __restrict__ us, const double* __restrict__ uo,
+            const double* __restrict__ fs, const double* __restrict__ bxs,
+            const double* __restrict__ bys, const double* __restrict__ bzs,
+            const double* __restrict__ bxo, const double* __restrict__ byo,
+            const double* __restrict__ bzo, const double* __restrict__ dgs,
+            const double* __restrict__ ids, double* __restrict__ keep,
+            unsigned long long* __restrict__ maxbits) {
+    pdl_wait();
+    pdl_trigger();
+    const int h = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = blockIdx.z;
+    unsigned long long m = 0ull;
+    if (h < d.hn0 && j < d.n1) {
+        const int q = (j + d.n1 * k) * d.hn0 + h;
+        Nbr nb;
+        split_nbrs(d, 0, h, j, k, nb);
+        const double old = us[q];
+        const double acc = arms<double>(fs[q], q, nb, uo, bxs, bys, bzs, bxo, byo, bzo);
+        m = abs_bits(fma(-dgs[q], old, acc));
+        keep[q] = old;
+        us[q] = acc * ids[q];
+    }
+    m = block_max_u64(m);
+    if (threadIdx.x == 0 && threadIdx.y == 0 && m) atomicMax(maxbits, m);
+}
+
 // FP64 residual of the whole fine level, stored as FP32 (the refinement right-hand side).  Where
 // phi is +0 on a cell and its six neighbours (the usual zero initial guess) the residual is f
 // itself, except that -0 becomes +0 as (-0) + (+0) does in the FMA chain: that branch issues no
@@ -752,6 +784,16 @@ void launch_resid_norm(const Dims& d, const LevelArrays<T>& a, bool red_only,
         launch_chain(k_resid_norm<T, false>, g.grid, g.block, 0, s, d, (const T*)a.phi,
                    (const T*)a.f, (const T*)a.bx, (const T*)a.by, (const T*)a.bz,
                    (const T*)a.diag, maxbits);
+}
+
+void launch_gsrb_norm(const Dims& d, LevelArrays<double>& a, double* keep,
+                      unsigned long long* maxbits, cudaStream_t s) {
+    const Grid3 g = grid3(d.hn0, d.n1, d.n2);
+    launch_chain(k_gsrb_norm, g.grid, g.block, 0, s, d, a.phi, (const double*)(a.phi + d.half),
+                 (const double*)a.f, (const double*)a.bx, (const double*)a.by, (const double*)a.bz,
+                 (const double*)(a.bx + d.half), (const double*)(a.by + d.half),
+                 (const double*)(a.bz + d.half), (const double*)a.diag, (const double*)a.invdiag,
+                 keep, maxbits);
 }
 
 void launch_resid64_to32(const Dims& d, const LevelArrays<double>& a, float* r32,

@@ -309,6 +309,14 @@ void vcycle(mac_ctx* c, int l, bool red_done = false) {
     mark(c, tm, 5);
 }
 
+// FP64 iterations whose closing residual norm and next first half-sweep are one kernel
+// (k_gsrb_norm): level 0 smoothed by its own launches before and after the coarse correction.
+// c->scratch (idle during a solve) holds the colour-0 half before the sweep ahead.
+bool sweep_ahead(const mac_ctx* c, int prec) {
+    return prec == MAC_PREC_FP64 && c->o.nu1 > 0 && c->o.nu2 > 0 && c->nlevels > 1 &&
+           !(c->o.coarse_tail && c->tail_start[0] == 0);
+}
+
 // Flexible CG around the inner V-cycles: mixed precision with post-smoothing (after its last
 // colour-1 half-sweep the V-cycle output satisfies L z = r on colour 1, which the Krylov kernels
 // use).
@@ -354,10 +362,14 @@ void issue_iteration(mac_ctx* c, int prec) {
     cudaMemsetAsync(c->red.maxbits, 0, sizeof(unsigned long long), c->stream);
     if (prec == MAC_PREC_FP64) {
         c->vtimer = 0;
-        vcycle<double>(c, 0);
+        const bool ahead = sweep_ahead(c, prec);
+        vcycle<double>(c, 0, ahead);
         if (tm) cudaEventRecordWithFlags(c->tail[0], c->stream, cudaEventRecordExternal);
         if (tm) cudaEventRecordWithFlags(c->tail[1], c->stream, cudaEventRecordExternal);
-        launch_resid_norm<double>(F.d, F.a64, c->o.nu2 > 0, c->red.maxbits, c->stream);
+        if (ahead)
+            launch_gsrb_norm(F.d, F.a64, c->scratch, c->red.maxbits, c->stream);
+        else
+            launch_resid_norm<double>(F.d, F.a64, c->o.nu2 > 0, c->red.maxbits, c->stream);
         ++c->issued;
     } else {
         // e (F.a32.phi) enters at zero: the residual kernel that formed this step's right-hand
@@ -409,7 +421,8 @@ void collect_timing(mac_ctx* c, int prec) {
         c->ktime_ms[MAC_KT_SMOOTH] += t[0] + t[4];
         c->ktime_launches[MAC_KT_SMOOTH] +=
             (prec == MAC_PREC_MIXED && fused_sweeps(c) ? 1 : 2) *
-            (sweeps_down(c, prec == MAC_PREC_MIXED) + sweeps_up(c, prec == MAC_PREC_MIXED));
+                (sweeps_down(c, prec == MAC_PREC_MIXED) + sweeps_up(c, prec == MAC_PREC_MIXED)) -
+            (sweep_ahead(c, prec) ? 1 : 0);
         c->ktime_ms[MAC_KT_RESTRICT] += t[1];
         c->ktime_launches[MAC_KT_RESTRICT] += 1;
         c->ktime_ms[MAC_KT_COARSE] += t[2];
@@ -575,6 +588,11 @@ int run_solve(mac_ctx* c, mac_stats* st) {
     const int inner_max = o.inner_vcycles > 1 ? o.inner_vcycles : 1;
     const double target = std::max(o.rel_eps * fnorm, o.abs_eps > 0.0 ? o.abs_eps : 0.0);
     c->cur_inner = inner_max;
+    const bool ahead = sweep_ahead(c, prec);
+    if (ahead && !converged(res) && o.max_vcycles > 0) {
+        launch_gsrb<double>(F.d, 0, F.a64, c->stream);
+        ++c->issued;
+    }
     while (!converged(res) && it < o.max_vcycles) {
         const double res_prev = res;
         const int nv = inner_cycles(c, prec);
@@ -595,6 +613,9 @@ int run_solve(mac_ctx* c, mac_stats* st) {
         if (prec == MAC_PREC_MIXED && o.adaptive_inner)
             c->cur_inner = next_inner(res_prev, res, nv, target, inner_max);
     }
+    if (ahead && it > 0)   // the sweep ahead of a cycle that does not come
+        MAC_CUDA_TRY(cudaMemcpyAsync(F.a64.phi, c->scratch, (size_t)F.d.half * sizeof(double),
+                                     cudaMemcpyDeviceToDevice, c->stream));
     st->vcycles = nv_total;
     st->refine_iters = prec == MAC_PREC_MIXED ? it : 0;
     st->rel_resid = res / fnorm;
