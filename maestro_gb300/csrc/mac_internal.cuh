@@ -461,12 +461,11 @@ int setup_rhs(mac_ctx* c, const double* macrhs, bool have_beta0, const double* p
 int finish_rhs_stats(mac_ctx* c, double* fnorm_out, bool* finite_out);
 // f -= mean on level 0 (red.scalars[0]); the solve issues it for singular problems
 void launch_sub_mean(mac_ctx* c);
-// after_dir (optional) runs after the direction's correction kernel is queued (host-pointer
-// calls start that direction's copy-back there); phi_nat_out (optional) receives phi in natural
-// layout from the x-direction pass.
-int correct_velocity(mac_ctx* c, bool have_beta0,
-                     const std::function<int(int)>* after_dir = nullptr,
-                     double* phi_nat_out = nullptr);
+// after_dir (optional) runs once the direction's correction is queued.  by_direction: a launch a
+// direction instead of one for all (host-pointer calls, which copy each direction back while the next
+// is corrected).  phi_nat_out receives phi in natural layout before the first after_dir.
+int correct_velocity(mac_ctx* c, const std::function<int(int)>* after_dir, bool by_direction,
+                     double* phi_nat_out);
 // reset_flags: clear the device flags (bad density, ...) first; false when a kernel of the same
 // setup already raised one
 int setup_fine_from_faces(mac_ctx* c, const double* fx, const double* fy, const double* fz,

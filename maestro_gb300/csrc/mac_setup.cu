@@ -81,13 +81,12 @@ __device__ __forceinline__ void fine_face(const FineParams& P, int dd, int cd, i
                                           int stride, double rc, const double* __restrict__ rho,
                                           double fac, double fhi, double* out, int li,
                                           double* wl, double* wh, int plane) {
-    double v = 0.0;
+    // one select of the neighbour instead of a reciprocal a case (476 -> 458 us at 256^3, where 430
+    // are the FP64 pipe's 15 operations a cell)
     const bool per = P.bc_lo[dd] == MAC_BC_PER;
-    if (cd > 0)
-        v = fac * recip_nr(rc + rho[q - stride]);
-    else if (per)
-        v = fac * recip_nr(rc + rho[q + (nd - 1) * stride]);
-    out[li] = v;
+    const int lo = cd > 0 ? q - stride : (per ? q + (nd - 1) * stride : q);
+    const double v = fac * recip_nr(rc + rho[lo]);
+    out[li] = cd > 0 || per ? v : 0.0;
     if (cd == 0 && P.bc_lo[dd] == MAC_BC_DIR) wl[plane] = fac * recip_nr(rc + rc);
     if (cd == nd - 1 && P.bc_hi[dd] == MAC_BC_DIR) wh[plane] = fhi * recip_nr(rc + rc);
 }
@@ -390,60 +389,77 @@ __global__ void k_sub_mean(int n, double* __restrict__ f, const double* __restri
 
 struct CorrParams {
     int n[3];
-    int dir, va, have_beta0;
-    int bc_lo, bc_hi;
-    double idx;  // 1/dx
-    double h2;   // h_dir^2 (beta = beta' * h2)
+    int va;
+    int d0, d1;              // directions d0 .. d1 - 1
+    int bc_lo[3], bc_hi[3];
+    double* u[3];
+    const double* bd[3];     // beta' of the low faces, level-0 layout
+    const double* wlo[3];    // Dirichlet wall planes
+    const double* whi[3];
+    double* phi_nat;         // phi in the natural layout (null: not wanted)
 };
 
 // U = (beta0 U - beta_f G phi) / beta0 = U - beta' (h / beta0) (phi_hi - phi_lo) on every face
-// normal to P.dir (natural face layout); beta' = beta_f / h^2 is the stored coefficient, h/beta0 a
-// per-layer factor.  Neumann walls keep U; Dirichlet walls use the ghost -phi_boundary.
+// normal to the wanted directions (natural face layout); beta' = beta_f / h^2 is the stored
+// coefficient, h/beta0 a per-layer factor.  Neumann walls keep U; Dirichlet walls use the ghost
+// -phi_boundary.  One thread per cell does its low faces, the last cell of a row its high face as
+// well: phi is read once for all directions and, being in hand, returned to the natural layout.
+// Bound by the FP64 pipe (9 operations a cell, 258 us at 256^3): a launch a direction, with one
+// thread a face, took 426 us, all in one 404 (499 with a subtraction for each kind of face).
 __global__ void __launch_bounds__(kBlock)
-k_correct(CorrParams P, Dims d, double* __restrict__ u, const double* __restrict__ phi,
-          const double* __restrict__ bd, const double* __restrict__ wlo,
-          const double* __restrict__ whi, const double* __restrict__ tab,
-          double* __restrict__ phi_nat) {
-    const int dir = P.dir;
-    const int m0 = P.n[0] + (dir == 0), m1 = P.n[1] + (dir == 1);
+k_correct(const __grid_constant__ CorrParams P, Dims d, const double* __restrict__ phi,
+          const double* __restrict__ tab) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = blockIdx.z;
-    if (i >= m0 || j >= m1) return;
-    const int q = i + m0 * (j + m1 * k);
-    const int qd = dir == 0 ? i : (dir == 1 ? j : k);
-    const int nd = dir == 0 ? P.n[0] : (dir == 1 ? P.n[1] : P.n[2]);
-    const bool v2 = P.va == 2;
-    const int r = v2 ? k : j;
-    const int st = (v2 ? P.n[2] : P.n[1]) + 1;
-    const double kap = tab[(kTabK0 + dir) * st + r];
-    const int plane = dir == 0 ? (j + P.n[1] * k) : dir == 1 ? (i + P.n[0] * k) : (i + P.n[0] * j);
-    // cells on the low (a) and high (b) side of the face, periodic wrap at the boundary faces
-    const int di = dir == 0, dj = dir == 1, dk = dir == 2;
-    double beta = 0.0, dphi = 0.0;
-    if (qd > 0 && qd < nd) {
-        const int chi = lidx(d, i, j, k);
-        beta = bd[chi];
-        dphi = phi[chi] - phi[lidx(d, i - di, j - dj, k - dk)];
-    } else if ((qd == 0 && P.bc_lo == MAC_BC_PER) || (qd == nd && P.bc_hi == MAC_BC_PER)) {
-        const int chi = lidx(d, di ? 0 : i, dj ? 0 : j, dk ? 0 : k);
-        beta = bd[chi];
-        dphi = phi[chi] - phi[lidx(d, di ? nd - 1 : i, dj ? nd - 1 : j, dk ? nd - 1 : k)];
-    } else if (qd == 0) {
-        if (P.bc_lo == MAC_BC_DIR) {
-            beta = wlo[plane];
-            dphi = 2.0 * phi[lidx(d, i, j, k)];
+    if (i >= P.n[0] || j >= P.n[1]) return;
+    const int cell[3] = {i, j, k};
+    const int c = lidx(d, i, j, k);
+    const double pc = phi[c];
+    if (P.phi_nat) P.phi_nat[i + P.n[0] * (j + P.n[1] * k)] = pc;
+    const int r = P.va == 2 ? k : j;
+    const int st = P.n[P.va] + 1;
+    // the low faces; a wall's outer value is the negative of the cell's (Dirichlet), a sign bit, so that
+    // one subtraction serves every case: predicated-off FP64 instructions cost as much as executed ones
+#pragma unroll
+    for (int dir = 0; dir < 3; ++dir) {
+        if (dir < P.d0 || dir >= P.d1) continue;
+        const int nd = P.n[dir], cd = cell[dir];
+        const int q = i + (P.n[0] + (dir == 0)) * (j + (P.n[1] + (dir == 1)) * k);
+        const bool per = P.bc_lo[dir] == MAC_BC_PER, wall = cd == 0 && !per;
+        const int lo = cd > 0 ? cd - 1 : (per ? nd - 1 : 0);
+        long long pl = __double_as_longlong(
+            phi[lidx(d, dir == 0 ? lo : i, dir == 1 ? lo : j, dir == 2 ? lo : k)]);
+        double beta = P.bd[dir][c];
+        if (wall && P.bc_lo[dir] == MAC_BC_DIR) {
+            beta = P.wlo[dir][dir == 0 ? (j + P.n[1] * k) : dir == 1 ? (i + P.n[0] * k) : (i + P.n[0] * j)];
+            pl ^= (long long)(1ull << 63);
         }
-    } else if (P.bc_hi == MAC_BC_DIR) {
-        beta = whi[plane];
-        dphi = -2.0 * phi[lidx(d, i - di, j - dj, k - dk)];
+        // beta == 0 (a wall face without Dirichlet) leaves the face alone; tested on the bit pattern
+        // so that no FP64 comparison occupies the FP64 pipe
+        if ((unsigned long long)__double_as_longlong(beta) << 1)
+            P.u[dir][q] = fma(-(beta * tab[(kTabK0 + dir) * st + r]), pc - __longlong_as_double(pl),
+                              P.u[dir][q]);
     }
-    // beta == 0 (a wall face without Dirichlet) leaves the face alone; tested on the bit pattern
-    // so that no FP64 comparison occupies the FP64 pipe
-    if ((unsigned long long)__double_as_longlong(beta) << 1) u[q] = fma(-(beta * kap), dphi, u[q]);
-    // the x-direction pass also returns phi to the natural layout (one cell per x face but the
-    // last; this kernel is bound by the FP64 pipe, the copy rides along)
-    if (phi_nat && i < P.n[0]) phi_nat[i + P.n[0] * (j + P.n[1] * k)] = phi[lidx(d, i, j, k)];
+    // the high faces of the last cells
+    if (i < P.n[0] - 1 && j < P.n[1] - 1 && k < P.n[2] - 1) return;
+#pragma unroll 1
+    for (int dir = P.d0; dir < P.d1; ++dir) {
+        if (cell[dir] != P.n[dir] - 1) continue;
+        const int m0 = P.n[0] + (dir == 0), m1 = P.n[1] + (dir == 1);
+        const int q = i + m0 * (j + m1 * k) + (dir == 0 ? 1 : dir == 1 ? m0 : m0 * m1);
+        const int ch = lidx(d, dir == 0 ? 0 : i, dir == 1 ? 0 : j, dir == 2 ? 0 : k);
+        double beta = 0.0, ph = -pc;
+        if (P.bc_hi[dir] == MAC_BC_PER) {
+            beta = P.bd[dir][ch];
+            ph = phi[ch];
+        } else if (P.bc_hi[dir] == MAC_BC_DIR) {
+            beta = P.whi[dir][dir == 0 ? (j + P.n[1] * k) : dir == 1 ? (i + P.n[0] * k) : (i + P.n[0] * j)];
+        }
+        if ((unsigned long long)__double_as_longlong(beta) << 1)
+            P.u[dir][q] = fma(-(beta * tab[(kTabK0 + dir) * st + r + (dir == P.va)]), ph - pc,
+                              P.u[dir][q]);
+    }
 }
 
 template <typename T>
@@ -778,26 +794,31 @@ int setup_rhs(mac_ctx* c, const double* macrhs, bool have_beta0, const double* p
     return launch_rhs(c, macrhs, false, phi_nat);
 }
 
-int correct_velocity(mac_ctx* c, bool have_beta0, const std::function<int(int)>* after_dir,
+int correct_velocity(mac_ctx* c, const std::function<int(int)>* after_dir, bool by_direction,
                      double* phi_nat_out) {
     Level& L = c->lev[0];
     const double* bd[3] = {L.a64.bx, L.a64.by, L.a64.bz};
+    CorrParams P;
+    for (int d = 0; d < 3; ++d) {
+        P.n[d] = c->n[d];
+        P.bc_lo[d] = c->bc_lo[d];
+        P.bc_hi[d] = c->bc_hi[d];
+        P.u[d] = c->u[d];
+        P.bd[d] = bd[d];
+        P.wlo[d] = L.wall[d][0];
+        P.whi[d] = L.wall[d][1];
+    }
+    P.va = c->va;
+    const Grid3 g = grid3(c->n[0], c->n[1], c->n[2]);
     for (int d = 0; d < c->dm; ++d) {
-        CorrParams P;
-        for (int e = 0; e < 3; ++e) P.n[e] = c->n[e];
-        P.dir = d;
-        P.va = c->va;
-        P.have_beta0 = have_beta0 ? 1 : 0;
-        P.bc_lo = c->bc_lo[d];
-        P.bc_hi = c->bc_hi[d];
-        P.idx = 1.0 / c->dx[d];
-        P.h2 = c->dx[d] * c->dx[d];
-        const Grid3 g = grid3(c->n[0] + (d == 0), c->n[1] + (d == 1), c->n[2] + (d == 2));
-        k_correct<<<g.grid, g.block, 0, c->stream>>>(P, L.d, c->u[d], L.a64.phi, bd[d],
-                                                     L.wall[d][0], L.wall[d][1], c->b0tab,
-                                                     d == 0 ? phi_nat_out : nullptr);
-        MAC_CUDA_TRY(cudaGetLastError());
-        ++c->issued;
+        if (by_direction || d == 0) {
+            P.d0 = d;
+            P.d1 = by_direction ? d + 1 : c->dm;
+            P.phi_nat = d == 0 ? phi_nat_out : nullptr;
+            k_correct<<<g.grid, g.block, 0, c->stream>>>(P, L.d, L.a64.phi, c->b0tab);
+            MAC_CUDA_TRY(cudaGetLastError());
+            ++c->issued;
+        }
         if (after_dir) {
             int rc = (*after_dir)(d);
             if (rc) return rc;

@@ -894,13 +894,17 @@ int set_call_state_impl(mac_ctx* c, bool with_alpha) {
     return MAC_OK;
 }
 
-// The projection on whole-domain device arrays already in c->u / c->rho / rhs / phin; `correct`
-// false leaves the velocities as they are and only returns phi.
+// What a projection does to the velocities: all directions in one launch, a launch a direction, or
+// nothing (only phi is returned).
+enum class Correct { kAtOnce, kByDirection, kNone };
+
+// The projection on whole-domain device arrays already in c->u / c->rho / rhs / phin.
 int core_macproject(mac_ctx* c, const double* macrhs, bool have_beta0, mac_stats* st,
                     const std::function<int()>* before_rhs = nullptr,
                     const std::function<int()>* before_phi = nullptr,
                     const std::function<int()>* after_phi = nullptr,
-                    const std::function<int(int)>* after_dir = nullptr, bool correct = true) {
+                    const std::function<int(int)>* after_dir = nullptr,
+                    Correct correct = Correct::kAtOnce) {
     Level& F = c->lev[0];
     cudaEventRecord(c->ev[0], c->stream);
     int rc = set_call_state_impl(c, false);
@@ -920,7 +924,7 @@ int core_macproject(mac_ctx* c, const double* macrhs, bool have_beta0, mac_stats
     if (solve_rc != MAC_OK && solve_rc != MAC_ERR_NOT_CONVERGED) return solve_rc;
     cudaEventRecord(c->ev[2], c->stream);
     const long long before_corr = c->issued;
-    // the x-direction correction also returns phi to the natural layout; phi's copy-back (host
+    // the first correction launch also returns phi to the natural layout; phi's copy-back (host
     // pointers) starts right after it
     const std::function<int(int)> dir_hook = [&](int d) {
         int r = MAC_OK;
@@ -928,8 +932,9 @@ int core_macproject(mac_ctx* c, const double* macrhs, bool have_beta0, mac_stats
         if (!r && after_dir) r = (*after_dir)(d);
         return r;
     };
-    rc = correct ? correct_velocity(c, have_beta0, &dir_hook, c->phin)
-                 : level0_to_natural(c, F.a64.phi, c->phin);
+    rc = correct == Correct::kNone
+             ? level0_to_natural(c, F.a64.phi, c->phin)
+             : correct_velocity(c, &dir_hook, correct == Correct::kByDirection, c->phin);
     if (rc) return rc;
     c->ktime_launches[MAC_KT_CORRECT] += (int)(c->issued - before_corr);
     c->ktime_launches[MAC_KT_SETUP] += (int)setup_kernels;
@@ -995,7 +1000,7 @@ int level0_fp32_vcycle(mac_ctx* c) {
     return MAC_OK;
 }
 int forward_phi(mac_ctx* c, const double* macrhs, bool have_beta0, mac_stats* st) {
-    return core_macproject(c, macrhs, have_beta0, st, nullptr, nullptr, nullptr, nullptr, false);
+    return core_macproject(c, macrhs, have_beta0, st, nullptr, nullptr, nullptr, nullptr, Correct::kNone);
 }
 int set_call_state(mac_ctx* c, bool with_alpha) { return set_call_state_impl(c, with_alpha); }
 int set_otf_mode(mac_ctx* c, bool on) { return set_otf(c, on); }
@@ -1270,7 +1275,8 @@ int mac_macproject(mac_ctx* c, int ptr_kind, double* const* umac, int ng_u, doub
     int solve_rc = MAC_OK;
     if (!rc) {
         solve_rc = core_macproject(c, macrhs ? c->rhs : nullptr, beta0_1d != nullptr, st,
-                                   &before_rhs, &before_phi, &after_phi, &after_dir);
+                                   &before_rhs, &before_phi, &after_phi, &after_dir,
+                                   ptr_kind == MAC_PTR_HOST ? Correct::kByDirection : Correct::kAtOnce);
         if (solve_rc != MAC_OK && solve_rc != MAC_ERR_NOT_CONVERGED) rc = solve_rc;
     }
     {
