@@ -391,25 +391,28 @@ k_prolong_add(Dims F, Dims C, BcDesc bc, const T* __restrict__ ec, T* u, const T
         }
     if (!valid) return;
     const int lane = (threadIdx.x + blockDim.x * threadIdx.y) & 31;
+    const bool has_l = xs[0] == I - 1 && lane > 0 && threadIdx.x > 0;
+    const bool has_r = xs[2] == I + 1 && lane < 31 && threadIdx.x + 1 < blockDim.x;
 #pragma unroll
-    for (int side = 0; side < 2; ++side) {
-        const int a = side ? 2 : 0;
-        const int X = xs[a];
-        const bool from_lane = side ? (X == I + 1 && lane < 31 && threadIdx.x + 1 < blockDim.x)
-                                    : (X == I - 1 && lane > 0 && threadIdx.x > 0);
-        if (from_lane) {
+    for (int yc = 0; yc < 2; ++yc)
 #pragma unroll
-            for (int yc = 0; yc < 2; ++yc)
-#pragma unroll
-                for (int zc = 0; zc < 2; ++zc) Yv[a][yc][zc] = side ? rgt[yc][zc] : lft[yc][zc];
-        } else if (X == I) {
-#pragma unroll
-            for (int yc = 0; yc < 2; ++yc)
-#pragma unroll
-                for (int zc = 0; zc < 2; ++zc) Yv[a][yc][zc] = Yv[1][yc][zc];
-        } else {
-            column(X, Yv[a]);
+        for (int zc = 0; zc < 2; ++zc) {
+            Yv[0][yc][zc] = has_l ? lft[yc][zc] : Yv[1][yc][zc];
+            Yv[2][yc][zc] = has_r ? rgt[yc][zc] : Yv[1][yc][zc];
         }
+    // the first and the last lane of a warp need different sides: one pass serves both
+    const bool need_l = !has_l && xs[0] != I, need_r = !has_r && xs[2] != I;
+    if (need_l || need_r) {
+        T Yn[2][2];
+        column(need_l ? xs[0] : xs[2], Yn);
+#pragma unroll
+        for (int yc = 0; yc < 2; ++yc)
+#pragma unroll
+            for (int zc = 0; zc < 2; ++zc) {
+                if (need_l) Yv[0][yc][zc] = Yn[yc][zc];
+                else Yv[2][yc][zc] = Yn[yc][zc];
+            }
+        if (need_l && need_r) column(xs[2], Yv[2]);   // (rows of one lane)
     }
 #pragma unroll
     for (int zc = 0; zc < kNz; ++zc) {
@@ -569,7 +572,8 @@ k_resid_norm(Dims F, const T* __restrict__ u, const T* __restrict__ f, const T* 
 
 // The residual max-norm after a V-cycle (colour 1 has none: its half-sweep came last) and the next
 // cycle's first colour-0 half-sweep in one pass: both need the six arms of every colour-0 cell, which
-// are 6 of the half-sweep's 7 FP64 operations (a kernel each: 127 + 105 us at 256^3; together 117).
+// are 6 of the half-sweep's 7 FP64 operations (a kernel each: 127 + 105 us at 256^3; together 143, by then
+// HBM as much as FP64: 13 arrays of half the cells).
 // keep receives the values before the update, to be put back if the norm ends the iteration.
 __global__ void __launch_bounds__(kBlock)
 k_gsrb_norm(Dims d, double* __restrict__ us, const double* __restrict__ uo,
