@@ -681,13 +681,18 @@ k_hg_gs_tile(hg::Geo G, hg::LevT<T> L, int sp, int ntx, const T* __restrict__ sr
 // (folded through the periodic wrap, 0 outside the domain) and forms each node's defect with
 // staged_node_op -- the arithmetic of node_op_dense3 for every node, so interior nodes get
 // k_hg_defect3's result bitwise and nodes next to a face its terms in another order -- instead
-// of one thread per node reading its 35 operands through the cache.
+// of one thread per node reading its 35 operands through the cache.  In FP32 a block does two slabs,
+// which share two of their four staged slabs and one of their three cell layers, and tiles away from the
+// faces are staged by constant pointer steps (257^3: 190 us with a slab a block and a folded index
+// looked up for every element, now 127); the FP64 form is bound by its FP64 operations and keeps one.
 constexpr int kDefX = 32, kDefY = 32, kDefThreads = 256;
 constexpr int kDRX = kDefX + 2, kDRY = kDefY + 2;   // staged nodes
 constexpr int kDCX = kDefX + 1, kDCY = kDefY + 1;   // staged cells
 template <typename T>
+constexpr int kDefZ = sizeof(T) == 4 ? 2 : 1;   // slabs a block
+template <typename T>
 constexpr size_t deftile_smem() {
-    return sizeof(T) * (3 * kDRX * kDRY + 2 * kDCX * kDCY);
+    return sizeof(T) * ((kDefZ<T> + 2) * kDRX * kDRY + (kDefZ<T> + 1) * kDCX * kDCY);
 }
 
 template <typename T, bool ISO>
@@ -695,75 +700,78 @@ __global__ void __launch_bounds__(kDefThreads)
 k_hg_defect_tile(hg::Geo G, hg::LevT<T> L, int ntx, const T* __restrict__ phi,
                  const T* __restrict__ f, T* __restrict__ r) {
     extern __shared__ __align__(16) unsigned char hg_deftile_smem[];
-    T* sphi = reinterpret_cast<T*>(hg_deftile_smem);   // [3][kDRY][kDRX], slabs z-1, z, z+1
-    T* ssig = sphi + 3 * kDRX * kDRY;                   // [2][kDCY][kDCX], cell layers z-1, z
-    const int z = (int)blockIdx.y;                      // 0 .. the slabs with unknown nodes - 1
+    constexpr int NZ = kDefZ<T>;
+    T* sphi = reinterpret_cast<T*>(hg_deftile_smem);   // [NZ + 2][kDRY][kDRX], slabs z-1 .. z+NZ
+    T* ssig = sphi + (NZ + 2) * kDRX * kDRY;            // [NZ + 1][kDCY][kDCX], cell layers z-1 ..
+    const int z = NZ * (int)blockIdx.y;                 // (of the slabs with unknown nodes)
     const int x0 = kDefX * ((int)blockIdx.x % ntx), y0 = kDefY * ((int)blockIdx.x / ntx);
     const int t = threadIdx.x;
-    __shared__ int sqx[kDRX], sqy[kDRY], scx[kDCX], scy[kDCY];
-    if (t < kDRX) {
-        const int raw = x0 - 1 + t;
-        sqx[t] = hg::node_wrap(G, L, 0, raw);
-        if (t < kDCX) scx[t] = hg::cell_wrap(G, L, 0, raw);
-    } else if (t >= 64 && t < 64 + kDRY) {
-        const int u = t - 64, raw = y0 - 1 + u;
-        sqy[u] = hg::node_wrap(G, L, 1, raw);
-        if (u < kDCY) scy[u] = hg::cell_wrap(G, L, 1, raw);
-    }
-    const int qz0 = hg::node_wrap(G, L, 2, z - 1), qz1 = hg::node_wrap(G, L, 2, z),
-              qz2 = hg::node_wrap(G, L, 2, z + 1);
-    const int cz0 = hg::cell_wrap(G, L, 2, z - 1), cz1 = hg::cell_wrap(G, L, 2, z);
-    __syncthreads();
     const long m01 = (long)L.nn[0] * L.nn[1], c01 = (long)L.n[0] * L.n[1];
-    // stage, one column a thread (its folded x in a register), rows kPR apart
+    const int im0 = L.nn[0], ic0 = L.n[0];
+    // one staged column a thread, rows kPR apart
     constexpr int kPR = kDefThreads / kDRX;
-    if (t < kPR * kDRX) {
-        const int lx = t % kDRX, r0 = t / kDRX;
-        const int q0 = sqx[lx];
-        const int im0 = L.nn[0], ic0 = L.n[0];
-#pragma unroll 1
-        for (int lz = 0; lz < 3; ++lz) {
-            const int q2 = lz == 0 ? qz0 : (lz == 1 ? qz1 : qz2);
-            const bool zin = q0 >= 0 && q2 >= 0;
-            const T* pb = phi + (zin ? q0 + q2 * m01 : 0);
-            T* dst_col = sphi + lz * (kDRX * kDRY) + lx;
-            for (int ly = r0; ly < kDRY; ly += kPR) {
-                const int q1 = sqy[ly];
-                const bool in = zin && q1 >= 0;
-                stage_elem(dst_col + ly * kDRX, in ? pb + (long)q1 * im0 : phi, in);
+    const int lx = t % kDRX, r0 = t / kDRX;
+    const bool plain = x0 >= 1 && x0 + kDefX < L.n[0] && y0 >= 1 && y0 + kDefY < L.n[1] && z >= 1 &&
+                       z + NZ < L.n[2];
+    if (plain) {   // every staged node and cell exists unfolded, every node of the tile is an unknown
+        if (t < kPR * kDRX) {
+            const T* pb = phi + (x0 - 1 + lx) + (long)im0 * (y0 - 1 + r0) + m01 * (z - 1);
+            const T* gb = L.sig + (x0 - 1 + lx) + (long)ic0 * (y0 - 1 + r0) + c01 * (z - 1);
+            T* dp = sphi + lx + kDRX * r0;
+            T* dg = ssig + lx + kDCX * r0;
+#pragma unroll
+            for (int q = 0; q < (kDRY + kPR - 1) / kPR; ++q) {
+                if (r0 + q * kPR >= kDRY) break;
+#pragma unroll
+                for (int lz = 0; lz < NZ + 2; ++lz)
+                    stage_elem(dp + (q * kPR + lz * kDRY) * kDRX, pb + (long)q * kPR * im0 + lz * m01, true);
+                if (lx >= kDCX || r0 + q * kPR >= kDCY) continue;
+#pragma unroll
+                for (int lz = 0; lz < NZ + 1; ++lz)
+                    stage_elem(dg + (q * kPR + lz * kDCY) * kDCX, gb + (long)q * kPR * ic0 + lz * c01, true);
             }
         }
-        if (lx < kDCX) {
-            const int c0 = scx[lx];
-#pragma unroll 1
-            for (int lz = 0; lz < 2; ++lz) {
-                const int c2 = lz == 0 ? cz0 : cz1;
-                const bool zin = c0 >= 0 && c2 >= 0;
-                const T* pb = L.sig + (zin ? c0 + c2 * c01 : 0);
-                T* dst_col = ssig + lz * (kDCX * kDCY) + lx;
-                for (int ly = r0; ly < kDCY; ly += kPR) {
-                    const int c1 = scy[ly];
-                    const bool in = zin && c1 >= 0;
-                    stage_elem(dst_col + ly * kDCX, in ? pb + (long)c1 * ic0 : L.sig, in);
-                }
+    } else if (t < kPR * kDRX) {
+        const int q0 = hg::node_wrap(G, L, 0, x0 - 1 + lx), c0 = hg::cell_wrap(G, L, 0, x0 - 1 + lx);
+        for (int ly = r0; ly < kDRY; ly += kPR) {
+            const int q1 = hg::node_wrap(G, L, 1, y0 - 1 + ly), c1 = hg::cell_wrap(G, L, 1, y0 - 1 + ly);
+#pragma unroll
+            for (int lz = 0; lz < NZ + 2; ++lz) {
+                const int q2 = hg::node_wrap(G, L, 2, z - 1 + lz);
+                const bool in = q0 >= 0 && q1 >= 0 && q2 >= 0;
+                stage_elem(sphi + lx + kDRX * (ly + kDRY * lz), in ? phi + q0 + (long)q1 * im0 + q2 * m01 : phi,
+                           in);
+            }
+            if (lx >= kDCX || ly >= kDCY) continue;
+#pragma unroll
+            for (int lz = 0; lz < NZ + 1; ++lz) {
+                const int c2 = hg::cell_wrap(G, L, 2, z - 1 + lz);
+                const bool in = c0 >= 0 && c1 >= 0 && c2 >= 0;
+                stage_elem(ssig + lx + kDCX * (ly + kDCY * lz),
+                           in ? L.sig + c0 + (long)c1 * ic0 + c2 * c01 : L.sig, in);
             }
         }
     }
     stage_wait();
     __syncthreads();
-    for (int e = t; e < kDefX * kDefY; e += kDefThreads) {
-        const int lx = 1 + e % kDefX, ly = 1 + e / kDefX;
-        const int p[3] = {x0 + lx - 1, y0 + ly - 1, z};
-        if (p[0] > L.n[0] - (G.per[0] ? 1 : 0) || p[1] > L.n[1] - (G.per[1] ? 1 : 0)) continue;
+    const int last[3] = {L.n[0] - (G.per[0] ? 1 : 0), L.n[1] - (G.per[1] ? 1 : 0),
+                         L.n[2] - (G.per[2] ? 1 : 0)};
+    for (int e = t; e < NZ * kDefX * kDefY; e += kDefThreads) {
+        const int nx = 1 + e % kDefX, ny = 1 + e / kDefX % kDefY, nz = e / (kDefX * kDefY);
+        const int p[3] = {x0 + nx - 1, y0 + ny - 1, z + nz};
         const long i = hg::nix(L, p[0], p[1], p[2]);
-        if (!hg::is_unknown(G, L, p)) {
-            r[i] = 0;
-            continue;
+        if (!plain) {
+            if (p[0] > last[0] || p[1] > last[1] || p[2] > last[2]) continue;
+            if (!hg::is_unknown(G, L, p)) {
+                r[i] = 0;
+                continue;
+            }
         }
         T dg, off;
         staged_node_op<T, ISO, kDRX, kDRX * kDRY, kDCX, kDCX * kDCY>(
-            L, ssig + (lx - 1) + kDCX * (ly - 1), sphi + (lx - 1) + kDRX * (ly - 1), dg, off);
-        r[i] = f[i] - (dg * sphi[lx + kDRX * (ly + kDRY)] - off);
+            L, ssig + (nx - 1) + kDCX * (ny - 1 + kDCY * nz), sphi + (nx - 1) + kDRX * (ny - 1 + kDRY * nz), dg,
+            off);
+        r[i] = f[i] - (dg * sphi[nx + kDRX * (ny + kDRY * (nz + 1))] - off);
     }
 }
 
@@ -1550,7 +1558,7 @@ struct HgMg {
             const int ntx = (L.n[0] + (geo.per[0] ? 0 : 1) + kDefX - 1) / kDefX;
             const int nty = (L.n[1] + (geo.per[1] ? 0 : 1) + kDefY - 1) / kDefY;
             const int nzu = L.n[2] + (geo.per[2] ? 0 : 1);
-            const dim3 grid((unsigned)(ntx * nty), (unsigned)nzu);
+            const dim3 grid((unsigned)(ntx * nty), (unsigned)ceil_div(nzu, kDefZ<T>));
             auto kern = iso(l) ? k_hg_defect_tile<T, true> : k_hg_defect_tile<T, false>;
             kern<<<grid, kDefThreads, deftile_smem<T>(), c->stream>>>(geo, L, ntx, phi, f, r);
         } else if (dense3() && iso(l))
