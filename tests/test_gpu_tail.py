@@ -57,13 +57,17 @@ def test_tail_matches_levels_and_oracle(cuda_lib, name, precision):
 
 
 NODAL = {
-    # name: (cells, top face, precision): the cluster tail's slab split and the blocked inverse
+    # name: (cells, top face, precision): the cluster tail's slab split, the blocked inverse, and the
+    # tiled levels (tiles off the faces, slab pairs of an odd number of slabs, restriction at faces)
     "two_slabs_a_cta": ((32, 32, 32), BC_NEU, "mixed"),      # 17 slabs over 16 CTAs: two a CTA
     "three_slabs_a_cta": ((64, 64, 64), BC_NEU, "mixed"),   # 33 slabs, isotropic
     "uneven_extents": ((24, 20, 36), BC_DIR, "fp64"),       # bottom 6 x 5 x 9: odd periodic extent
     "periodic_vertical": ((32, 16, 48), BC_PER, "fp64"),
     "bottom_one_block": ((16, 16, 16), BC_NEU, "fp64"),     # 12 unknowns: less than one block
     "bottom_576": ((32, 24, 44), BC_NEU, "mixed"),          # 8 x 6 x 12 nodes: 36 whole blocks
+    "tiles_odd_slabs": ((96, 104, 28), BC_NEU, "mixed"),    # 29 slabs, one tile off the faces
+    "tiles_periodic": ((96, 96, 20), BC_PER, "mixed"),
+    "tiles_outflow": ((104, 96, 12), BC_DIR, "fp64"),
 }
 
 
