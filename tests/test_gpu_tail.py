@@ -65,9 +65,9 @@ NODAL = {
     "periodic_vertical": ((32, 16, 48), BC_PER, "fp64"),
     "bottom_one_block": ((16, 16, 16), BC_NEU, "fp64"),     # 12 unknowns: less than one block
     "bottom_576": ((32, 24, 44), BC_NEU, "mixed"),          # 8 x 6 x 12 nodes: 36 whole blocks
-    "tiles_odd_slabs": ((96, 104, 28), BC_NEU, "mixed"),    # 29 slabs, one tile off the faces
-    "tiles_periodic": ((96, 96, 20), BC_PER, "mixed"),
-    "tiles_outflow": ((104, 96, 12), BC_DIR, "fp64"),
+    "tiles_odd_slabs": ((96, 112, 32), BC_NEU, "mixed"),    # 33 slabs, tiles off the faces
+    "tiles_periodic": ((96, 96, 48), BC_PER, "mixed"),
+    "tiles_outflow": ((96, 80, 48), BC_DIR, "fp64"),
 }
 
 
