@@ -559,9 +559,10 @@ k_hg_gs_tile(hg::Geo G, hg::LevT<T> L, int sp, int ntx, const T* __restrict__ sr
     constexpr int kPR = kTileThreads / kTR;   // staged rows a pass: a column a thread
     const int lx = t % kTR, r0 = t / kTR;
     // A tile whose staged nodes all lie inside the domain, away from its faces, in every direction
-    // (most of them) needs no fold and no zero fill: pointers advance by a constant.
+    // (most of them) needs no fold and no zero fill: pointers advance by a constant.  (A periodic z
+    // excludes its last slab too: the slab above it is an image, which the sweeps leave stale.)
     const bool plain = x0 - kTileH >= 1 && x0 + kTR - kTileH <= L.n[0] && y0 - kTileH >= 1 &&
-                       y0 + kTR - kTileH <= L.n[1] && z >= 1 && z <= L.n[2] - 1;
+                       y0 + kTR - kTileH <= L.n[1] && z >= 1 && z + 1 <= L.n[2] - (G.per[2] ? 1 : 0);
     if (plain) {
         if (t < kPR * kTR) {
             const int im0 = L.nn[0], ic0 = L.n[0], col = split_col(lx);
