@@ -374,6 +374,11 @@ __device__ __forceinline__ void cp_async_wait() {
 // BiCGStab reducing ||f - A x||_inf by eps, nub sweeps (FBoxLib's bottom, Docs/mg/mg.tex:221-249)
 // with f_c / diag_c + sum_n gc_n x_n as the Gauss-Seidel update (gc_n = a_n / diag).  A warp's
 // cells have one colour (odd rows excepted), so a half-sweep issues half the FP64 instructions.
+// Up to kOneBottom cells belong to one CTA (ONE), four warps on its four FP64 units: spread out they
+// issue no faster, and every step waits for the cluster's barrier and remote loads (whole FP64
+// calls, 16 CTAs -> one: 40^3 with 125 cells 1701 -> 1270 us, 24 x 40 x 56 with 105 cells 4011 ->
+// 2841).  Above that the units are shared by more warps: 26 x 22 with 143 cells takes 1457 us spread
+// out and took 1784 in a tail of one CTA.
 struct ClBottom {
     int N;
     bool on, odd;            // a cell here; a periodic extent is odd (same-colour neighbours)
@@ -394,17 +399,34 @@ struct ClReduce {
     double tot[5];
     double out[4];
 };
-template <int NS, class Fin>
+// The CTAs' barrier, or that of the one CTA's first kOneBottom threads.
+constexpr int kOneBottom = 128;
+template <bool ONE>
+__device__ __forceinline__ void bot_sync() {
+    if (ONE)
+        asm volatile("bar.sync 1, %0;" ::"n"(kOneBottom) : "memory");
+    else
+        cluster_sync();
+}
+template <bool ONE>
+__device__ __forceinline__ void cta_sync() {
+    if (ONE)
+        bot_sync<true>();
+    else
+        __syncthreads();
+}
+
+template <bool ONE, int NS, class Fin>
 __device__ __forceinline__ void cl_reduce(ClReduce& R, int& parity, const double (&v)[NS],
                                           unsigned long long key, int nw, Fin fin) {
-    static_assert(NS <= 4, "four sums");
+    static_assert(NS <= 4 && kOneBottom >= 4 * 32, "four sums, a warp each");
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (w < nw) {
 #pragma unroll
         for (int s = 0; s < NS; ++s) R.ws[s][threadIdx.x] = v[s];
         R.wk[threadIdx.x] = key;
     }
-    __syncthreads();
+    cta_sync<ONE>();
     const unsigned nc = cluster_size(), rank = cluster_rank();
     constexpr int kw = NS < 4 ? NS : 0;   // the warp that takes the key
     if (w < NS) {
@@ -412,7 +434,11 @@ __device__ __forceinline__ void cl_reduce(ClReduce& R, int& parity, const double
         for (int i = 1; i < nw; ++i) s += R.ws[w][32 * i + lane];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane < (int)nc) st_cluster(mapa(smem_u32(&R.slot[parity][w][rank]), lane), s);
+        if (ONE) {
+            if (lane == 0) R.tot[w] = s;
+        } else if (lane < (int)nc) {
+            st_cluster(mapa(smem_u32(&R.slot[parity][w][rank]), lane), s);
+        }
     }
     if (w == kw) {
         unsigned long long k = R.wk[lane];
@@ -425,17 +451,20 @@ __device__ __forceinline__ void cl_reduce(ClReduce& R, int& parity, const double
             const unsigned long long q = __shfl_xor_sync(0xffffffffu, k, o);
             k = q > k ? q : k;
         }
-        if (lane < (int)nc)
+        if (ONE) {
+            if (lane == 0) R.tot[4] = __longlong_as_double((long long)k);
+        } else if (lane < (int)nc) {
             st_cluster(mapa(smem_u32(&R.slot[parity][4][rank]), lane), __longlong_as_double((long long)k));
+        }
     }
-    cluster_sync();
-    if (w < NS) {
+    bot_sync<ONE>();
+    if (!ONE && w < NS) {
         double s = lane < (int)nc ? R.slot[parity][w][lane] : 0.0;
 #pragma unroll
         for (int o = kClusterMax / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0) R.tot[w] = s;
     }
-    if (w == kw) {
+    if (!ONE && w == kw) {
         unsigned long long k =
             lane < (int)nc ? (unsigned long long)__double_as_longlong(R.slot[parity][4][lane]) : 0ull;
 #pragma unroll
@@ -445,9 +474,9 @@ __device__ __forceinline__ void cl_reduce(ClReduce& R, int& parity, const double
         }
         if (lane == 0) R.tot[4] = __longlong_as_double((long long)k);
     }
-    __syncthreads();
+    if (!ONE) __syncthreads();
     if (threadIdx.x == 0) fin(R.tot, R.tot[4], R.out);
-    __syncthreads();
+    cta_sync<ONE>();
     parity ^= 1;
 }
 
@@ -462,19 +491,22 @@ __device__ __forceinline__ double cl_gsum(const ClBottom& B, unsigned off, doubl
 
 // nu red/black sweeps on x (register x, published).  Where a periodic extent is odd, same-colour
 // cells neighbour each other: they are updated from each other's old values.
+template <bool ONE>
 __device__ __forceinline__ double cl_gsrb(const ClBottom& B, double fi, double x, int nu) {
     for (int it = 0; it < 2 * nu; ++it) {
         const bool act = B.on && B.colour == (it & 1);
         if (act) x = cl_gsum(B, 0, fi, false);
-        if (B.odd) cluster_sync();
+        if (B.odd) bot_sync<ONE>();
         if (act) lds_store(B.xa, x);
-        cluster_sync();
+        bot_sync<ONE>();
     }
     return x;
 }
 
 // Solves for x (in: the guess, already published at B.xa by every owner); f's mean comes off when
-// singular.  Every CTA of the cluster runs the same control flow.
+// singular.  Every CTA of the cluster runs the same control flow (ONE: the first kOneBottom threads of
+// the one CTA).
+template <bool ONE>
 __device__ __noinline__ double cl_solve(const ClBottom& bottom, ClReduce& R, double f, double x, int nw,
                                         int singular, int nub, double eps, int max_iter, int* iters) {
     const ClBottom B = bottom;   // (registers)
@@ -482,13 +514,13 @@ __device__ __noinline__ double cl_solve(const ClBottom& bottom, ClReduce& R, dou
     const unsigned ya = B.xa + B.yoff;
     {
         const double v[1] = {B.on ? f : 0.0};
-        cl_reduce<1>(R, parity, v, 0ull, nw, [&](const double* t, double, double* o) {
+        cl_reduce<ONE>(R, parity, v, 0ull, nw, [&](const double* t, double, double* o) {
             o[0] = singular ? t[0] / B.N : 0.0;
         });   // (its barrier also publishes x)
     }
     if (singular && B.on) f -= R.out[0];
     const double fi = B.on ? f * B.id : 0.0;
-    x = cl_gsrb(B, fi, x, nub);
+    x = cl_gsrb<ONE>(B, fi, x, nub);
     double r = 0.0, dx = 0.0;
     if (B.on) {
         r = f - B.dg * cl_gsum(B, 0, x, true);
@@ -502,7 +534,7 @@ __device__ __noinline__ double cl_solve(const ClBottom& bottom, ClReduce& R, dou
         // rounding level of f - A x: a residual that small (the sweeps alone solved the bottom, or
         // a singular one's right-hand side keeps a rounded mean) cannot be reduced further, and
         // iterating on it only adds noise to x
-        cl_reduce<2>(R, parity, v, abs_key(r), nw, [&](const double* t, double k, double* o) {
+        cl_reduce<ONE>(R, parity, v, abs_key(r), nw, [&](const double* t, double k, double* o) {
             o[0] = t[0];
             o[1] = k;
             o[2] = 2e-15 * sqrt(t[1]);
@@ -521,12 +553,12 @@ __device__ __noinline__ double cl_solve(const ClBottom& bottom, ClReduce& R, dou
                 y = p * B.id;
                 lds_store(ya, y);
             }
-            cluster_sync();
+            bot_sync<ONE>();
             if (B.on) vv = B.dg * cl_gsum(B, B.yoff, y, true);
             // (rh, v); ||r|| of the step before: its test costs one operator application after
             // convergence instead of a reduction every iteration
             const double v1[1] = {B.on ? rh * vv : 0.0};
-            cl_reduce<1>(R, parity, v1, abs_key(r), nw, [&](const double* q, double k, double* o) {
+            cl_reduce<ONE>(R, parity, v1, abs_key(r), nw, [&](const double* q, double k, double* o) {
                 o[0] = q[0] == 0.0 ? 0.0 : rho * recip_nr(q[0]);
                 o[1] = k;
                 o[2] = q[0];
@@ -539,7 +571,7 @@ __device__ __noinline__ double cl_solve(const ClBottom& bottom, ClReduce& R, dou
                 y = s * B.id;
                 lds_store(ya, y);
             }
-            cluster_sync();
+            bot_sync<ONE>();
             if (B.on) t = B.dg * cl_gsum(B, B.yoff, y, true);
             double v4[4] = {0.0, 0.0, 0.0, 0.0};
             if (B.on) {
@@ -549,7 +581,7 @@ __device__ __noinline__ double cl_solve(const ClBottom& bottom, ClReduce& R, dou
                 v4[3] = rh * t;
             }
             // omega = (t, s) / (t, t); (rh, r_new) = (rh, s) - omega (rh, t); the next beta
-            cl_reduce<4>(R, parity, v4, abs_key(s), nw, [&](const double* q, double k, double* o) {
+            cl_reduce<ONE>(R, parity, v4, abs_key(s), nw, [&](const double* q, double k, double* o) {
                 const double w = q[1] > 0.0 ? q[0] * recip_nr(q[1]) : 0.0;
                 const double rn = fma(-w, q[3], q[2]);
                 o[0] = w;
@@ -569,14 +601,17 @@ __device__ __noinline__ double cl_solve(const ClBottom& bottom, ClReduce& R, dou
         }
     }
     if (B.on) lds_store(B.xa, x);
-    cluster_sync();
+    bot_sync<ONE>();
     *iters = count;
-    return cl_gsrb(B, fi, x, nub);
+    return cl_gsrb<ONE>(B, fi, x, nub);
 }
 
 // bottom cells per CTA (even: pairs of cells) and the threads they take (colours in warps of
 // their own)
-__host__ __device__ __forceinline__ int bottom_cells(int N, int nc) { return 2 * ((N + 2 * nc - 1) / (2 * nc)); }
+__host__ __device__ __forceinline__ int bottom_cells(int N, int nc) {
+    const int ctas = N <= kOneBottom ? 1 : nc;
+    return 2 * ((N + 2 * ctas - 1) / (2 * ctas));
+}
 __host__ __device__ __forceinline__ int bottom_threads(int M) { return 2 * ((M / 2 + 31) / 32 * 32); }
 
 }  // namespace
@@ -795,8 +830,12 @@ k_tail(const __grid_constant__ TailParams<T> P) {
         cluster_sync();
     } else {
         if (B.on) lds_store(B.xa, bx);
-        bx = cl_solve(B, R, bf, bx, bottom_threads(M) / 32, P.singular, P.nub, P.bottom_eps,
-                      P.bottom_max_iter, &count);
+        if (NB > kOneBottom)
+            bx = cl_solve<false>(B, R, bf, bx, bottom_threads(M) / 32, P.singular, P.nub, P.bottom_eps,
+                                 P.bottom_max_iter, &count);
+        else if (rank == 0 && tid < kOneBottom)
+            bx = cl_solve<true>(B, R, bf, bx, kOneBottom / 32, P.singular, P.nub, P.bottom_eps,
+                                P.bottom_max_iter, &count);
         if (B.on) eb[bc - (int)rank * M] = (T)bx;
         cluster_sync();
     }
