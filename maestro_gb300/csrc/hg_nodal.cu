@@ -1229,7 +1229,9 @@ struct HgState {
         int key[4] = {-1, -1, -1, -1};   // count, nu1, nu2, dense stencil
         long long kernels = 0;
     } graph[2];
-    // first level the cluster tail runs (-1: none) per precision: [0] FP64, [1] FP32
+    // per precision, [0] FP64, [1] FP32: the dense 3-D cycles have been prepared; the first level the
+    // cluster tail runs in them (-1: none)
+    bool ready[2] = {false, false};
     int tail[2] = {-1, -1};
     int tail_nc = 16;
     int bM = 0;
@@ -1454,8 +1456,7 @@ struct HgMg {
     // shared memory (33^3 nodes in FP32, 25 x 20 x 17 and below in FP64 typically).
     void plan_tail() {
         int& at = H->tail[kSlot];
-        at = -1;
-        if (err || !dense3() || !H->binv || nlev < 3) return;
+        if (err || !H->binv || nlev < 3) return;
         if (prepare_hg_tail_kernels(&H->tail_nc)) {
             set_last_cuda_error(cudaGetLastError(), "nodal tail kernels", __FILE__, __LINE__);
             err = MAC_ERR_CUDA;
@@ -1479,8 +1480,11 @@ struct HgMg {
     // stencil) and replayed: the cycle issues one launch per colour, level and kernel kind,
     // most of them small, and needs no host value inside
     void run_cycles(int count, int nu1, int nu2) {
-        prepare_tiles();
-        plan_tail();
+        if (dense3() && !H->ready[kSlot]) {   // once a context: it is bound to one device and hierarchy
+            prepare_tiles();
+            plan_tail();
+            H->ready[kSlot] = !err;
+        }
         if (err) return;
         if (c->o.timing) {   // events around the level-0 launches: no capture
             for (int v = 0; v < count; ++v) hg::vcycle(*this, 0, nu1, nu2);
@@ -1647,8 +1651,8 @@ struct HgMg {
     // Levels that sweep with the tiled kernel: their second phi array (zeroed) and the kernel's
     // shared-memory limit, set up outside any stream capture.
     void prepare_tiles() {
-        if (err || !dense3()) return;
-        {   // (per call, a few host calls: a process-wide flag would skip a second device)
+        if (err) return;
+        {
             // the largest shared-memory carveout (a hint; the kernel runs with any)
             cudaFuncSetAttribute(k_hg_gs_tile<T, false>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  (int)cudaSharedmemCarveoutMaxShared);
