@@ -1,4 +1,4 @@
-// Multi-level (AMR) MAC projection on the GPU: the composite cell functions of mac_amr.cuh as
+// Multi-level (AMR) MAC projection on the GPU: the cell and face functions of mac_amr.cuh as
 // kernels, the executor that runs amr_solve / amr_project on device arrays, and the C ABI
 // (mac_ctx_set_amr, mac_macproject_ml_dense).
 //
@@ -15,8 +15,8 @@
 #include <type_traits>
 #include <vector>
 
+#include "mac_internal.cuh"   // (first: mac_amr.cuh's device code calls recip_nr)
 #include "mac_amr.cuh"
-#include "mac_internal.cuh"
 
 namespace mac {
 
@@ -34,35 +34,14 @@ constexpr int kMixedInner = 2;        // FP32 multi-level V-cycles per FP64 step
 #define AMR_LOOP(N) for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx < (N); \
                          idx += (long)gridDim.x * blockDim.x)
 
-// ---- cell kernels of one level ---------------------------------------------------------------
-//
-// One thread per cell (or cell of one colour) of a plane of the array box, planes along
-// blockIdx.z, the row by one multiplication (Plane).  Two more bits of the level's mask, set with
-// the hierarchy, choose the cell function: kFull (a region cell whose neighbours are all region
-// cells: the plain stencil at constant offsets), kNear (a region cell whose neighbours lie in the
-// array box without a wrap; without coarse data a coarse-fine side only adds to the diagonal).  The
-// other region cells (at domain faces; with coarse data also the kNear ones) take the general
-// functions of mac_amr.cuh, by list in extra planes of the grid: inline, one or two of them in
-// every row made half of all warps run both forms (53 us a defect of 130^3 cells).  They run the same operations in the same order, except
-// that the FP64 stencil takes differences, which needs 15 instead of 20 FP64 instructions (the
-// FP64 pipe binds it: 2.2 M cells took 127 us, with 40 us of memory traffic) and FP64 Gauss-Seidel
-// multiplies by recip_nr.  With the general function for every cell (64-bit indices, divisions,
-// six mask tests) the FP32 sweep ran at 0.23 of HBM, 38 us a colour, the defect 83 us.
-constexpr unsigned char kFull = 4;
-constexpr unsigned char kNear = 8;
-
-struct Plane {
-    unsigned m0;   // reciprocal of the row length (0: divide)
-};
-__device__ __forceinline__ unsigned row_of(unsigned t, unsigned e, Plane P) {
-    return P.m0 ? __umulhi(t, P.m0) : t / e;
-}
-// floor(2^32 / e) + 1 is exact for t e < 2^32, t < e rows
-inline Plane plane(long e, long rows) {
-    Plane P;
-    P.m0 = e > 1 && e * e * rows < (1L << 32) ? (unsigned)(0x100000000ull / (unsigned long long)e) + 1u : 0u;
-    return P;
-}
+// (cells, colours and faces of a plane: see the functions in mac_amr.cuh)
+using amr::Cell;
+using amr::Child;
+using amr::Face;
+using amr::Plane;
+using amr::plane;
+using amr::face_plane;
+__device__ __forceinline__ unsigned plane_thread() { return blockIdx.x * kThreads + threadIdx.x; }
 inline dim3 plane_grid(long cells, int planes) {
     return dim3((unsigned)((cells + kThreads - 1) / kThreads), 1, (unsigned)planes);
 }
@@ -73,153 +52,13 @@ struct Rest {
     int n;
 };
 __device__ __forceinline__ int rest_index(int planes, const Rest& R) {
-    const unsigned t = ((blockIdx.z - (unsigned)planes) * gridDim.x + blockIdx.x) * kThreads + threadIdx.x;
-    return t < (unsigned)R.n ? R.list[t] : -1;
+    return amr::rest_entry(R.list, R.n, (blockIdx.z - (unsigned)planes) * gridDim.x * kThreads + plane_thread());
 }
 inline dim3 plane_grid(long cells, int planes, int rest) {
     dim3 g = plane_grid(cells, planes);
     const long slice = (long)g.x * kThreads;
-    g.z += (unsigned)((rest + slice - 1) / slice);
+    g.z += (unsigned)amr::rest_planes(rest, slice);
     return g;
-}
-
-// A cell of plane k of the box: index, row r = j + ext1 k, and whether the plane has it.
-struct Cell {
-    unsigned q, r, i, j, k;
-};
-template <typename T>
-__device__ __forceinline__ bool plane_cell(const amr::LevT<T>& L, Plane P, unsigned k, Cell& c) {
-    const unsigned e0 = L.ext[0], e1 = L.ext[1], t = blockIdx.x * kThreads + threadIdx.x;
-    c.j = row_of(t, e0, P);
-    c.i = t - c.j * e0;
-    c.k = k;
-    c.r = c.j + e1 * k;
-    c.q = c.i + e0 * c.r;
-    return t < e0 * e1 && k < (unsigned)L.ext[2];
-}
-// One cell of the colour a thread: half a row each.
-template <typename T>
-__device__ __forceinline__ bool colour_plane_cell(const amr::LevT<T>& L, Plane P, int colour, unsigned k,
-                                                  Cell& c) {
-    const unsigned e0 = L.ext[0], e1 = L.ext[1], hw = (e0 + 1) / 2;
-    const unsigned t = blockIdx.x * kThreads + threadIdx.x;
-    c.j = row_of(t, hw, P);
-    c.k = k;
-    c.r = c.j + e1 * k;
-    c.i = 2 * (t - c.j * hw) + ((colour + L.lo[0] + L.lo[1] + c.j + L.lo[2] + k) & 1);
-    c.q = c.i + e0 * c.r;
-    return t < hw * e1 && c.i < e0 && k < (unsigned)L.ext[2];
-}
-
-// (Explicit rounding: the FP32 cycles give the general functions' results bit for bit, and with
-// them the constant that a closed domain's phi picks up from FP32 rounding.)
-__device__ __forceinline__ float mulT(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mulT(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float addT(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ double addT(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ float fmaT(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double fmaT(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float recip(float x) { return 1.f / x; }
-__device__ __forceinline__ double recip(double x) { return recip_nr(x); }
-
-// A cell's stencil, loaded before its mask is known (one memory latency a cell instead of two; a
-// neighbour index outside the box is clamped, its value unused): face coefficients and neighbours
-// x-, x+, y-, y+, z-, z+.
-template <typename T>
-struct Stencil {
-    T b[6], u[6], uc, f;
-    unsigned n[6];
-    unsigned char m;
-};
-template <typename T>
-__device__ __forceinline__ void load_stencil(const Geo& G, const amr::LevT<T>& L, const Cell& c, const T* u,
-                                             const T* __restrict__ f, Stencil<T>& A) {
-    const unsigned e0 = L.ext[0], pl = e0 * (unsigned)L.ext[1], last = pl * (unsigned)L.ext[2] - 1;
-    const unsigned f0 = c.q + c.r, f1 = c.q + e0 * c.k;
-    A.m = L.mask[c.q];
-    A.n[0] = c.q - (c.q >= 1u);
-    A.n[1] = min(c.q + 1, last);
-    A.n[2] = c.q >= e0 ? c.q - e0 : 0u;
-    A.n[3] = min(c.q + e0, last);
-    A.b[0] = L.b[0][f0];
-    A.b[1] = L.b[0][f0 + 1];
-    A.b[2] = L.b[1][f1];
-    A.b[3] = L.b[1][f1 + e0];
-    A.uc = u[c.q];
-    A.f = f[c.q];
-#pragma unroll
-    for (int n = 0; n < 4; ++n) A.u[n] = u[A.n[n]];
-    if (G.dm > 2) {
-        A.n[4] = c.q >= pl ? c.q - pl : 0u;
-        A.n[5] = min(c.q + pl, last);
-        A.b[4] = L.b[2][c.q];
-        A.b[5] = L.b[2][c.q + pl];
-        A.u[4] = u[A.n[4]];
-        A.u[5] = u[A.n[5]];
-    }
-}
-
-// cell_op with zero coarse data on a kFull or kNear cell (see amr::cell_op).
-template <typename T>
-__device__ __forceinline__ void near_op(const Geo& G, const amr::LevT<T>& L, const Stencil<T>& A, T& diag,
-                                        T& off) {
-    diag = 0;
-    off = 0;
-#pragma unroll
-    for (int n = 0; n < 6; ++n) {
-        if (n >= 2 * G.dm) break;
-        const T w = mulT(A.b[n], (T)L.ih2[n >> 1]);
-        if ((A.m & kFull) || (L.mask[A.n[n]] & amr::kIn)) {
-            diag = addT(diag, w);
-            off = fmaT(w, A.u[n], off);
-        } else {
-            diag = fmaT((T)(2.0 / 3.0), w, diag);
-        }
-    }
-}
-
-template <typename T>
-__device__ __forceinline__ void defect_near(const Geo& G, const amr::LevT<T>& L, const Stencil<T>& A,
-                                            unsigned q, bool cu, T* __restrict__ r) {
-    if (!(A.m & amr::kIn)) {
-        r[q] = 0;
-    } else if (std::is_same<T, double>::value && (A.m & kFull)) {
-        T s = A.f;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            if (d >= G.dm) break;
-            T t = A.b[2 * d] * (A.u[2 * d] - A.uc);
-            t = fma(A.b[2 * d + 1], A.u[2 * d + 1] - A.uc, t);
-            s = fma((T)L.ih2[d], t, s);
-        }
-        r[q] = s;
-    } else if ((A.m & kFull) || ((A.m & kNear) && !cu)) {
-        T dg, off;
-        near_op(G, L, A, dg, off);
-        r[q] = addT(A.f, -fmaT(dg, A.uc, -off));
-    }
-}
-
-template <typename T>
-__device__ __forceinline__ void gsrb_near(const Geo& G, const amr::LevT<T>& L, const Stencil<T>& A,
-                                          unsigned q, T* u) {
-    if (!(A.m & amr::kIn)) return;
-    if (std::is_same<T, double>::value && (A.m & kFull)) {
-        T dg = 0, s = A.f;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            if (d >= G.dm) break;
-            T t = A.b[2 * d] * A.u[2 * d];
-            t = fma(A.b[2 * d + 1], A.u[2 * d + 1], t);
-            dg = fma((T)L.ih2[d], A.b[2 * d] + A.b[2 * d + 1], dg);
-            s = fma((T)L.ih2[d], t, s);
-        }
-        u[q] = s * recip(dg);
-    } else if (A.m & (kFull | kNear)) {
-        T dg, off;
-        near_op<T>(G, L, A, dg, off);
-        u[q] = (A.f + off) / dg;
-    }
 }
 
 // Two planes a thread: twice the loads in flight.
@@ -237,16 +76,16 @@ k_defect(Geo G, amr::LevT<T> L, amr::LevT<T> C, Plane P, Rest R, const T* __rest
         return;
     }
     Cell c[kPlanes];
-    Stencil<T> A[kPlanes];
+    amr::Stencil<T> A[kPlanes];
     bool on[kPlanes];
 #pragma unroll
     for (int p = 0; p < kPlanes; ++p) {
-        on[p] = plane_cell(L, P, kPlanes * blockIdx.z + p, c[p]);
-        if (on[p]) load_stencil(G, L, c[p], u, f, A[p]);
+        on[p] = amr::plane_cell(L, P, plane_thread(), kPlanes * blockIdx.z + p, c[p]);
+        if (on[p]) amr::load_stencil(G, L, c[p], u, f, A[p]);
     }
 #pragma unroll
     for (int p = 0; p < kPlanes; ++p)
-        if (on[p]) defect_near(G, L, A[p], c[p].q, cu != nullptr, r);
+        if (on[p]) amr::defect_near(G, L, A[p], c[p].q, cu != nullptr, r);
 }
 
 // One colour of a sweep, zero coarse data.
@@ -260,16 +99,16 @@ k_gsrb(Geo G, amr::LevT<T> L, Plane P, Rest R, int colour, T* u, const T* __rest
         return;
     }
     Cell c[kPlanes];
-    Stencil<T> A[kPlanes];
+    amr::Stencil<T> A[kPlanes];
     bool on[kPlanes];
 #pragma unroll
     for (int p = 0; p < kPlanes; ++p) {
-        on[p] = colour_plane_cell(L, P, colour, kPlanes * blockIdx.z + p, c[p]);
-        if (on[p]) load_stencil(G, L, c[p], u, f, A[p]);
+        on[p] = amr::colour_plane_cell(L, P, colour, plane_thread(), kPlanes * blockIdx.z + p, c[p]);
+        if (on[p]) amr::load_stencil(G, L, c[p], u, f, A[p]);
     }
 #pragma unroll
     for (int p = 0; p < kPlanes; ++p)
-        if (on[p]) gsrb_near(G, L, A[p], c[p].q, u);
+        if (on[p]) amr::gsrb_near(G, L, A[p], c[p].q, u);
 }
 
 // The coarse cells that take a reflux, by list (a scan of the coarse level's mask took 67 us at
@@ -281,67 +120,19 @@ k_reflux(Geo G, amr::LevT<T> F, amr::LevT<T> C, const T* uf, const T* uc, T* res
     if (t < n) amr::reflux_cell(G, F, C, (long)list[t], uf, uc, res);
 }
 
-// Covered coarse cells, by list (coarse cell, first child): the mean of the children.
+// Covered coarse cells, by list.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 k_restrict(Geo G, amr::LevT<T> F, const T* __restrict__ fine, T* __restrict__ crse,
-           const int2* __restrict__ list, int n) {
+           const Child* __restrict__ list, int n) {
     const int t = blockIdx.x * kThreads + threadIdx.x;
-    if (t >= n) return;
-    const int2 q = list[t];
-    const unsigned e0 = F.ext[0], pl = e0 * F.ext[1];
-    T s = 0;
-#pragma unroll
-    for (int a = 0; a < 8; ++a) {
-        if (a >= (1 << G.dm)) break;
-        s += fine[(unsigned)q.y + (a & 1) + (a & 2 ? e0 : 0u) + (a & 4 ? pl : 0u)];
-    }
-    crse[q.x] = s / (T)(1 << G.dm);
+    if (t < n) amr::restrict_child(G, F, list[t], fine, crse);
 }
 
-// Multilinear interpolation to the region cells, 0 elsewhere (amr::prolong_cell): the coarse
-// neighbours of a cell away from the domain faces at constant offsets.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 k_prolong(Geo G, amr::LevT<T> F, amr::LevT<T> C, Plane P, const T* __restrict__ uc, T* __restrict__ uf) {
-    Cell c;
-    if (!plane_cell(F, P, blockIdx.z, c)) return;
-    const unsigned char m = F.mask[c.q];
-    if (!(m & amr::kIn)) {
-        uf[c.q] = 0;
-        return;
-    }
-    const int g[3] = {F.lo[0] + (int)c.i, F.lo[1] + (int)c.j, F.lo[2] + (int)blockIdx.z};
-    bool in = true;
-    int at[3], st[3];
-    const int sz[3] = {1, C.ext[0], C.ext[0] * C.ext[1]};
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        at[d] = d < G.dm ? (g[d] >> 1) - C.lo[d] : 0;
-        const int o = d < G.dm ? (g[d] & 1 ? 1 : -1) : 0;
-        st[d] = o * sz[d];
-        in = in && at[d] + o >= 0 && at[d] + o < C.ext[d];
-    }
-    if (!in) {
-        amr::prolong_cell(G, F, C, (long)c.q, uc, uf);
-        return;
-    }
-    const T* b = uc + (at[0] + at[1] * sz[1] + at[2] * sz[2]);
-    T s = 0;
-#pragma unroll
-    for (int a = 0; a < 8; ++a) {
-        if (a >= (1 << G.dm)) break;
-        T w = 1;
-        int o = 0;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            if (d >= G.dm) break;
-            w *= (a >> d) & 1 ? (T)0.25 : (T)0.75;
-            o += (a >> d) & 1 ? st[d] : 0;
-        }
-        s += w * b[o];
-    }
-    uf[c.q] = s;
+    amr::prolong_plane(G, F, C, P, plane_thread(), blockIdx.z, uc, uf);
 }
 
 template <typename T>
@@ -511,110 +302,36 @@ __global__ void k_level0_out(Dims d, const T* __restrict__ phi, const double* me
 }
 
 // ---- face kernels: one thread per face of a plane of the array box, planes along blockIdx.z ----
-struct Face {
-    unsigned q, f[3];     // index; box coordinates
-    unsigned hi, lo;      // the cells on either side, when both are in the box (two)
-    bool two;
-};
-__device__ __forceinline__ bool plane_face(const Lev& L, int d, Plane P, Face& c) {
-    const unsigned m0 = L.ext[0] + (d == 0), m1 = L.ext[1] + (d == 1);
-    const unsigned t = blockIdx.x * kThreads + threadIdx.x;
-    if (t >= m0 * m1) return false;
-    c.f[1] = row_of(t, m0, P);
-    c.f[0] = t - c.f[1] * m0;
-    c.f[2] = blockIdx.z;
-    c.q = t + m0 * m1 * c.f[2];
-    const unsigned e0 = L.ext[0], e1 = L.ext[1];
-    c.hi = c.f[0] + e0 * (c.f[1] + e1 * c.f[2]);
-    c.lo = c.hi - (d == 0 ? 1u : d == 1 ? e0 : e0 * e1);
-    c.two = c.f[d] >= 1 && c.f[d] < (unsigned)L.ext[d];
-    return true;
-}
 inline dim3 face_grid(const Lev& L, int d) {
     return plane_grid((long)(L.ext[0] + (d == 0)) * (L.ext[1] + (d == 1)), L.ext[2] + (d == 2));
-}
-inline Plane face_plane(const Lev& L, int d) { return plane(L.ext[0] + (d == 0), L.ext[1] + (d == 1)); }
-
-// Whether the face borders a region cell (amr::face_in_level).
-__device__ __forceinline__ bool face_used(const Geo& G, const Lev& L, int d, const Face& c) {
-    if (c.two) return (L.mask[c.hi] | L.mask[c.lo]) & amr::kIn;
-    int f[3];
-    amr::face_coords(L, d, (long)c.q, f);
-    return amr::face_in_level(G, L, d, f);
 }
 
 __global__ void __launch_bounds__(kThreads)
 k_scale_b0(Geo G, Lev L, int d, Plane P, double* u, const double* b0, const double* b0e, int mult) {
-    Face c;
-    if (!plane_face(L, d, P, c)) return;
-    const int r = L.lo[G.va] + (int)(G.va == 2 ? c.f[2] : c.f[1]);
-    const double bb = d == G.va ? b0e[r] : b0[r];
-    u[c.q] *= mult ? bb : recip_nr(bb);
+    amr::scale_b0_plane(G, L, d, P, plane_thread(), blockIdx.z, u, b0, b0e, mult);
 }
 
-// Coarse faces away from covered cells keep their values.
 __global__ void __launch_bounds__(kThreads)
 k_edge_restrict(Geo G, Lev F, Lev C, int d, Plane P, double* uc, const double* uf) {
-    Face c;
-    if (!plane_face(C, d, P, c)) return;
-    if (c.two && !((C.mask[c.hi] | C.mask[c.lo]) & amr::kCov)) return;
-    amr::edge_restrict_face(G, F, C, d, (long)c.q, uc, uf);
+    amr::edge_restrict_plane(G, F, C, d, P, plane_thread(), blockIdx.z, uc, uf);
 }
 
-// rh = -(div(beta0 U) - macrhs) on region cells (U already holds beta0 U), 0 elsewhere.
 __global__ void __launch_bounds__(kThreads)
 k_divergence(Geo G, Lev L, Plane P, const double* __restrict__ u0, const double* __restrict__ u1,
              const double* __restrict__ u2, const double* __restrict__ macrhs, double* __restrict__ rh) {
-    Cell c;
-    if (!plane_cell(L, P, blockIdx.z, c)) return;
-    if (!(L.mask[c.q] & amr::kIn)) {
-        rh[c.q] = 0.0;
-        return;
-    }
-    const unsigned e0 = L.ext[0], f0 = c.q + c.r, f1 = c.q + e0 * blockIdx.z;
-    double s = macrhs ? macrhs[c.q] : 0.0;
-    s = fma(-L.ih[0], u0[f0 + 1] - u0[f0], s);
-    s = fma(-L.ih[1], u1[f1 + e0] - u1[f1], s);
-    if (G.dm > 2) s = fma(-L.ih[2], u2[c.q + e0 * L.ext[1]] - u2[c.q], s);
-    rh[c.q] = s;
+    amr::divergence_plane(G, L, P, plane_thread(), blockIdx.z, u0, u1, u2, macrhs, rh);
 }
 
-// Solver coefficient of a face of the level (amr::coeff_face).
 __global__ void __launch_bounds__(kThreads)
 k_coeff(Geo G, Lev L, int d, Plane P, const double* __restrict__ rho, const double* __restrict__ b0,
         const double* __restrict__ b0e, int alt, double* __restrict__ beta) {
-    Face c;
-    if (!plane_face(L, d, P, c)) return;
-    if (!c.two) {
-        amr::coeff_face(G, L, d, (long)c.q, rho, b0, b0e, alt, beta);
-        return;
-    }
-    if (!((L.mask[c.hi] | L.mask[c.lo]) & amr::kIn)) return;
-    double v = 2.0 * recip_nr(rho[c.hi] + rho[c.lo]);
-    if (b0) {
-        const int r = L.lo[G.va] + (int)(G.va == 2 ? c.f[2] : c.f[1]);
-        const double bb = d == G.va ? b0e[r] : b0[r];
-        v *= bb;
-        if (alt) v *= bb;
-    }
-    beta[c.q] = v;
+    amr::coeff_plane(G, L, d, P, plane_thread(), blockIdx.z, rho, b0, b0e, alt, beta);
 }
 
-// beta0 U -= beta G phi on a face of the level (amr::correct_face).
 __global__ void __launch_bounds__(kThreads)
 k_correct(Geo G, Lev L, Lev C, int d, Plane P, const double* phi, const double* cphi,
           const double* beta, double* u) {
-    Face c;
-    if (!plane_face(L, d, P, c)) return;
-    if (c.two) {
-        const int n = (L.mask[c.hi] & amr::kIn) + (L.mask[c.lo] & amr::kIn);
-        if (n == 0) return;
-        if (n == 2 * amr::kIn) {
-            u[c.q] = fma(-beta[c.q] * L.ih[d], phi[c.hi] - phi[c.lo], u[c.q]);
-            return;
-        }
-    }
-    amr::correct_face(G, L, C, d, (long)c.q, phi, cphi, beta, u);
+    amr::correct_plane(G, L, C, d, P, plane_thread(), blockIdx.z, phi, cphi, beta, u);
 }
 
 // A density that is not positive and finite on a cell the level's faces read (its region and
@@ -640,32 +357,27 @@ __global__ void k_check_rho(Geo G, Lev L, const double* rho, int* flag, long N) 
 
 // The caller's whole-level-domain arrays <-> the level's box arrays (back: the level's own faces
 // and region cells only).
-__device__ __forceinline__ size_t full_face(const Lev& L, int d, const Face& c) {
-    const size_t m0 = L.n[0] + (d == 0), m1 = L.n[1] + (d == 1);
-    return (c.f[0] + L.lo[0]) + m0 * ((c.f[1] + L.lo[1]) + m1 * (size_t)(c.f[2] + L.lo[2]));
-}
-__device__ __forceinline__ size_t full_cell(const Lev& L, const Cell& c) {
-    return (c.i + L.lo[0]) + (size_t)L.n[0] * ((c.j + L.lo[1]) + (size_t)L.n[1] * (blockIdx.z + L.lo[2]));
-}
 __global__ void __launch_bounds__(kThreads)
 k_full_to_box_faces(Lev L, int d, Plane P, const double* __restrict__ full, double* __restrict__ box) {
     Face c;
-    if (plane_face(L, d, P, c)) box[c.q] = full[full_face(L, d, c)];
+    if (amr::plane_face(L, d, P, plane_thread(), blockIdx.z, c)) box[c.q] = full[amr::full_face(L, d, c)];
 }
 __global__ void __launch_bounds__(kThreads)
 k_full_to_box_cells(Lev L, Plane P, const double* __restrict__ full, double* __restrict__ box) {
     Cell c;
-    if (plane_cell(L, P, blockIdx.z, c)) box[c.q] = full[full_cell(L, c)];
+    if (amr::plane_cell(L, P, plane_thread(), blockIdx.z, c)) box[c.q] = full[amr::full_cell(L, c)];
 }
 __global__ void __launch_bounds__(kThreads)
 k_box_to_full_faces(Geo G, Lev L, int d, Plane P, const double* __restrict__ box, double* __restrict__ full) {
     Face c;
-    if (plane_face(L, d, P, c) && face_used(G, L, d, c)) full[full_face(L, d, c)] = box[c.q];
+    if (amr::plane_face(L, d, P, plane_thread(), blockIdx.z, c) && amr::face_used(G, L, d, c))
+        full[amr::full_face(L, d, c)] = box[c.q];
 }
 __global__ void __launch_bounds__(kThreads)
 k_box_to_full_cells(Lev L, Plane P, const double* __restrict__ box, double* __restrict__ full) {
     Cell c;
-    if (plane_cell(L, P, blockIdx.z, c) && (L.mask[c.q] & amr::kIn)) full[full_cell(L, c)] = box[c.q];
+    if (amr::plane_cell(L, P, plane_thread(), blockIdx.z, c) && (L.mask[c.q] & amr::kIn))
+        full[amr::full_cell(L, c)] = box[c.q];
 }
 
 __global__ void k_sync_periodic_faces(Geo G, Lev L, int d, double* u, long N) {
@@ -741,7 +453,7 @@ struct AmrState {
         // cells of the next coarser level: those that take this level's reflux; the covered ones
         // with their first child
         int* reflux = nullptr;
-        int2* cover = nullptr;
+        Child* cover = nullptr;
         int nreflux = 0, ncover = 0;
         // this level's region cells that are not kNear (nrest), then those that are not kFull
         int* rest = nullptr;
@@ -887,68 +599,6 @@ int build_masks(const mac_ctx* c, int nlev, const int* nboxes, const int* box_lo
         }
     }
     return MAC_OK;
-}
-
-// The kernels' bits of a level's mask, kNear and kFull (see the cell kernels), and the list of the
-// region cells without kNear, then of those without kFull; *nrest: how many the first are.
-std::vector<int> classify(int dm, const Lev& V, std::vector<unsigned char>& mask, int* nrest) {
-    const int e0 = V.ext[0], e1 = V.ext[1], e2 = V.ext[2];
-    const long pl = (long)e0 * e1;
-    std::vector<int> far, part;
-    for (int k = 0; k < e2; ++k)
-        for (int j = 0; j < e1; ++j) {
-            unsigned char* m = mask.data() + pl * k + (long)e0 * j;
-            const bool row = (dm < 2 || (j > 0 && j < e1 - 1)) && (dm < 3 || (k > 0 && k < e2 - 1));
-            for (int i = 0; i < e0; ++i) {
-                if (!(m[i] & amr::kIn)) continue;
-                const int idx = (int)(pl * k + (long)e0 * j + i);
-                if (!row || i == 0 || i == e0 - 1) {
-                    far.push_back(idx);
-                    continue;
-                }
-                unsigned char all = m[i - 1] & m[i + 1];
-                if (dm > 1) all &= m[i - e0] & m[i + e0];
-                if (dm > 2) all &= m[i - pl] & m[i + pl];
-                m[i] |= (all & amr::kIn) ? (unsigned char)(kNear | kFull) : kNear;
-                if (!(all & amr::kIn)) part.push_back(idx);
-            }
-        }
-    *nrest = (int)far.size();
-    far.insert(far.end(), part.begin(), part.end());
-    return far;
-}
-
-// Lists of level l >= 1: the valid cells of level l - 1 beside a covered one, the covered ones
-// with their first child.
-void coarse_lists(const mac_ctx* c, const Lev& F, const Lev& K, const std::vector<unsigned char>& mask,
-                  std::vector<int>& reflux, std::vector<int2>& cover) {
-    const int dm = c->dm;
-    std::vector<unsigned char> beside(mask.size(), 0);   // valid cells taken already
-    long idx = 0;
-    for (int k = 0; k < K.ext[2]; ++k)
-        for (int j = 0; j < K.ext[1]; ++j)
-            for (int i = 0; i < K.ext[0]; ++i, ++idx) {
-                if (!(mask[(size_t)idx] & amr::kCov)) continue;
-                const int q[3] = {K.lo[0] + i, K.lo[1] + j, K.lo[2] + k};
-                const int f[3] = {2 * q[0], dm > 1 ? 2 * q[1] : q[1], dm > 2 ? 2 * q[2] : q[2]};
-                cover.push_back(make_int2((int)idx, (int)amr::cix(F, f[0], f[1], f[2])));
-                for (int d = 0; d < dm; ++d)
-                    for (int s = -1; s <= 1; s += 2) {
-                        int p[3] = {q[0], q[1], q[2]};
-                        p[d] += s;
-                        if (p[d] < 0 || p[d] >= K.n[d]) {
-                            if (c->bc_lo[d] != MAC_BC_PER) continue;
-                            p[d] += p[d] < 0 ? K.n[d] : -K.n[d];
-                        }
-                        if (!amr::inside(K, p)) continue;
-                        const size_t n = (size_t)amr::cix(K, p[0], p[1], p[2]);
-                        if ((mask[n] & (amr::kIn | amr::kCov)) == amr::kIn && !beside[n]) {
-                            beside[n] = 1;
-                            reflux.push_back((int)n);
-                        }
-                    }
-            }
-    std::sort(reflux.begin(), reflux.end());
 }
 
 // The executor of amr_solve / amr_project on the context's stream.
@@ -1289,18 +939,18 @@ int amr_configure(mac_ctx* c, int nlev, const int* nboxes, const int* box_lo, co
         for (int d = 0; d < c->dm && !rc; ++d) rc = amr_alloc(A, &S.beta[d], (size_t)amr::nfaces(S.lev, d));
         for (int b = 0; b < amr::kNumBufs && !rc; ++b) rc = amr_alloc(A, &S.buf[b], (size_t)N);
         std::vector<int> reflux;
-        std::vector<int2> cover;
-        if (l > 0) coarse_lists(c, geom[l], geom[l - 1], masks[l - 1], reflux, cover);
+        std::vector<Child> cover;
+        if (l > 0) amr::coarse_lists(A->geo, geom[l], geom[l - 1], masks[l - 1], reflux, cover);
         S.nreflux = (int)reflux.size();
         S.ncover = (int)cover.size();
         if (!rc) rc = amr_alloc(A, &S.reflux, reflux.size());
         if (!rc) rc = amr_alloc(A, &S.cover, cover.size());
-        const std::vector<int> rest = classify(c->dm, geom[l], masks[l], &S.nrest);
+        const std::vector<int> rest = amr::classify(c->dm, geom[l], masks[l], &S.nrest);
         S.nrest_cu = (int)rest.size();
         if (!rc) rc = amr_alloc(A, &S.rest, rest.size());
         if (rc) break;
         if (cudaMemcpy(S.reflux, reflux.data(), reflux.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(S.cover, cover.data(), cover.size() * sizeof(int2), cudaMemcpyHostToDevice) != cudaSuccess ||
+            cudaMemcpy(S.cover, cover.data(), cover.size() * sizeof(Child), cudaMemcpyHostToDevice) != cudaSuccess ||
             cudaMemcpy(S.rest, rest.data(), rest.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess) {
             set_last_cuda_error(cudaGetLastError(), "cudaMemcpy(lists)", __FILE__, __LINE__);
             rc = MAC_ERR_CUDA;

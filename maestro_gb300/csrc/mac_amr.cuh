@@ -25,14 +25,18 @@
 // a level (see GpuExec in mac_amr.cu).
 #pragma once
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <type_traits>
+#include <vector>
 
 #if defined(__CUDACC__)
 #define AMR_HD __host__ __device__
+#define AMR_FI __host__ __device__ __forceinline__
 #else
 #define AMR_HD
+#define AMR_FI inline
 #endif
 #if defined(__CUDA_ARCH__)
 #define AMR_UNROLL _Pragma("unroll")
@@ -546,6 +550,432 @@ AMR_HD inline long full_face(const LevT<T>& L, int d, long idx) {
     face_coords(L, d, idx, f);
     const long m0 = L.n[0] + (d == 0), m1 = L.n[1] + (d == 1);
     return (long)f[0] + m0 * ((long)f[1] + m1 * f[2]);
+}
+
+// ---- what the kernels run --------------------------------------------------------------------
+//
+// One thread per cell (or cell of one colour) or face of a plane k of the array box, thread t of the
+// plane; the row by one multiplication (Plane).  Two more bits of the level's mask, set with the
+// hierarchy (classify), choose the cell function: kFull (a region cell whose neighbours are all region
+// cells: the plain stencil at constant offsets), kNear (a region cell whose neighbours lie in the
+// array box without a wrap; without coarse data a coarse-fine side only adds to the diagonal).  The
+// other region cells (at domain faces; with coarse data also the kNear ones) take the general
+// functions above, by list in extra planes of the grid: inline, one or two of them in every row made
+// half of all warps run both forms (53 us a defect of 130^3 cells).  They run the same operations in
+// the same order, except that the FP64 stencil takes differences, which needs 15 instead of 20 FP64
+// instructions (the FP64 pipe binds it: 2.2 M cells took 127 us, with 40 us of memory traffic) and
+// FP64 Gauss-Seidel multiplies by a reciprocal.  With the general function for every cell (64-bit
+// indices, divisions, six mask tests) the FP32 sweep ran at 0.23 of HBM, 38 us a colour, the defect 83
+// us.  The general functions are also what these are tested against, cell by cell, on the host.
+constexpr unsigned char kFull = 4;
+constexpr unsigned char kNear = 8;
+
+struct Plane {
+    unsigned m0;   // reciprocal of the row length (0: divide)
+};
+AMR_FI unsigned mul_hi(unsigned a, unsigned b) {
+#if defined(__CUDA_ARCH__)
+    return __umulhi(a, b);
+#else
+    return (unsigned)(((unsigned long long)a * b) >> 32);
+#endif
+}
+AMR_FI unsigned least(unsigned a, unsigned b) { return b < a ? b : a; }
+AMR_FI unsigned row_of(unsigned t, unsigned e, Plane P) { return P.m0 ? mul_hi(t, P.m0) : t / e; }
+// floor(2^32 / e) + 1 is exact for t e < 2^32, t < e rows
+inline Plane plane(long e, long rows) {
+    Plane P;
+    P.m0 = e > 1 && e * e * rows < (1L << 32) ? (unsigned)(0x100000000ull / (unsigned long long)e) + 1u : 0u;
+    return P;
+}
+
+// A cell of plane k of the box: index, row r = j + ext1 k, and whether the plane has it.
+struct Cell {
+    unsigned q, r, i, j, k;
+};
+template <typename T>
+AMR_FI bool plane_cell(const LevT<T>& L, Plane P, unsigned t, unsigned k, Cell& c) {
+    const unsigned e0 = L.ext[0], e1 = L.ext[1];
+    c.j = row_of(t, e0, P);
+    c.i = t - c.j * e0;
+    c.k = k;
+    c.r = c.j + e1 * k;
+    c.q = c.i + e0 * c.r;
+    return t < e0 * e1 && k < (unsigned)L.ext[2];
+}
+// One cell of the colour a thread: half a row each.
+template <typename T>
+AMR_FI bool colour_plane_cell(const LevT<T>& L, Plane P, int colour, unsigned t, unsigned k, Cell& c) {
+    const unsigned e0 = L.ext[0], e1 = L.ext[1], hw = (e0 + 1) / 2;
+    c.j = row_of(t, hw, P);
+    c.k = k;
+    c.r = c.j + e1 * k;
+    c.i = 2 * (t - c.j * hw) + ((colour + L.lo[0] + L.lo[1] + c.j + L.lo[2] + k) & 1);
+    c.q = c.i + e0 * c.r;
+    return t < hw * e1 && c.i < e0 && k < (unsigned)L.ext[2];
+}
+
+// Cells taken by list, in extra planes of `slice` threads: how many of them, and thread t's cell.
+AMR_FI long rest_planes(long rest, long slice) { return (rest + slice - 1) / slice; }
+AMR_FI int rest_entry(const int* list, int n, unsigned t) { return t < (unsigned)n ? list[t] : -1; }
+
+// (Explicit rounding: the FP32 cycles give the general functions' results bit for bit, and with
+// them the constant that a closed domain's phi picks up from FP32 rounding.)
+#if defined(__CUDA_ARCH__)
+AMR_FI float mulT(float a, float b) { return __fmul_rn(a, b); }
+AMR_FI double mulT(double a, double b) { return __dmul_rn(a, b); }
+AMR_FI float addT(float a, float b) { return __fadd_rn(a, b); }
+AMR_FI double addT(double a, double b) { return __dadd_rn(a, b); }
+AMR_FI float fmaT(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+AMR_FI double fmaT(double a, double b, double c) { return __fma_rn(a, b, c); }
+AMR_FI double recip(double x) { return recip_nr(x); }
+#else
+AMR_FI float mulT(float a, float b) { return a * b; }
+AMR_FI double mulT(double a, double b) { return a * b; }
+AMR_FI float addT(float a, float b) { return a + b; }
+AMR_FI double addT(double a, double b) { return a + b; }
+AMR_FI float fmaT(float a, float b, float c) { return std::fma(a, b, c); }
+AMR_FI double fmaT(double a, double b, double c) { return std::fma(a, b, c); }
+AMR_FI double recip(double x) { return 1.0 / x; }
+#endif
+AMR_FI float recip(float x) { return 1.f / x; }
+
+// A cell's stencil, loaded before its mask is known (one memory latency a cell instead of two; a
+// neighbour index outside the box is clamped, its value unused): face coefficients and neighbours
+// x-, x+, y-, y+, z-, z+.
+template <typename T>
+struct Stencil {
+    T b[6], u[6], uc, f;
+    unsigned n[6];
+    unsigned char m;
+};
+template <typename T>
+AMR_FI void load_stencil(const Geo& G, const LevT<T>& L, const Cell& c, const T* u,
+                                             const T* __restrict__ f, Stencil<T>& A) {
+    const unsigned e0 = L.ext[0], pl = e0 * (unsigned)L.ext[1], last = pl * (unsigned)L.ext[2] - 1;
+    const unsigned f0 = c.q + c.r, f1 = c.q + e0 * c.k;
+    A.m = L.mask[c.q];
+    A.n[0] = c.q - (c.q >= 1u);
+    A.n[1] = least(c.q + 1, last);
+    A.n[2] = c.q >= e0 ? c.q - e0 : 0u;
+    A.n[3] = least(c.q + e0, last);
+    A.b[0] = L.b[0][f0];
+    A.b[1] = L.b[0][f0 + 1];
+    A.b[2] = L.b[1][f1];
+    A.b[3] = L.b[1][f1 + e0];
+    A.uc = u[c.q];
+    A.f = f[c.q];
+    AMR_UNROLL
+    for (int n = 0; n < 4; ++n) A.u[n] = u[A.n[n]];
+    if (G.dm > 2) {
+        A.n[4] = c.q >= pl ? c.q - pl : 0u;
+        A.n[5] = least(c.q + pl, last);
+        A.b[4] = L.b[2][c.q];
+        A.b[5] = L.b[2][c.q + pl];
+        A.u[4] = u[A.n[4]];
+        A.u[5] = u[A.n[5]];
+    }
+}
+
+// cell_op with zero coarse data on a kFull or kNear cell (see cell_op).
+template <typename T>
+AMR_FI void near_op(const Geo& G, const LevT<T>& L, const Stencil<T>& A, T& diag,
+                                        T& off) {
+    diag = 0;
+    off = 0;
+    AMR_UNROLL
+    for (int n = 0; n < 6; ++n) {
+        if (n >= 2 * G.dm) break;
+        const T w = mulT(A.b[n], (T)L.ih2[n >> 1]);
+        if ((A.m & kFull) || (L.mask[A.n[n]] & kIn)) {
+            diag = addT(diag, w);
+            off = fmaT(w, A.u[n], off);
+        } else {
+            diag = fmaT((T)(2.0 / 3.0), w, diag);
+        }
+    }
+}
+
+template <typename T>
+AMR_FI void defect_near(const Geo& G, const LevT<T>& L, const Stencil<T>& A,
+                                            unsigned q, bool cu, T* __restrict__ r) {
+    if (!(A.m & kIn)) {
+        r[q] = 0;
+    } else if (std::is_same<T, double>::value && (A.m & kFull)) {
+        T s = A.f;
+        AMR_UNROLL
+        for (int d = 0; d < 3; ++d) {
+            if (d >= G.dm) break;
+            T t = A.b[2 * d] * (A.u[2 * d] - A.uc);
+            t = fma(A.b[2 * d + 1], A.u[2 * d + 1] - A.uc, t);
+            s = fma((T)L.ih2[d], t, s);
+        }
+        r[q] = s;
+    } else if ((A.m & kFull) || ((A.m & kNear) && !cu)) {
+        T dg, off;
+        near_op(G, L, A, dg, off);
+        r[q] = addT(A.f, -fmaT(dg, A.uc, -off));
+    }
+}
+
+template <typename T>
+AMR_FI void gsrb_near(const Geo& G, const LevT<T>& L, const Stencil<T>& A,
+                                          unsigned q, T* u) {
+    if (!(A.m & kIn)) return;
+    if (std::is_same<T, double>::value && (A.m & kFull)) {
+        T dg = 0, s = A.f;
+        AMR_UNROLL
+        for (int d = 0; d < 3; ++d) {
+            if (d >= G.dm) break;
+            T t = A.b[2 * d] * A.u[2 * d];
+            t = fma(A.b[2 * d + 1], A.u[2 * d + 1], t);
+            dg = fma((T)L.ih2[d], A.b[2 * d] + A.b[2 * d + 1], dg);
+            s = fma((T)L.ih2[d], t, s);
+        }
+        u[q] = s * recip(dg);
+    } else if (A.m & (kFull | kNear)) {
+        T dg, off;
+        near_op<T>(G, L, A, dg, off);
+        u[q] = (A.f + off) / dg;
+    }
+}
+
+
+// A covered coarse cell and its first child.
+struct alignas(8) Child {
+    int coarse, fine;
+};
+// The covered cell's value: the mean of its children (restrict_cell).
+template <typename T>
+AMR_FI void restrict_child(const Geo& G, const LevT<T>& F, Child q, const T* __restrict__ fine,
+                           T* __restrict__ crse) {
+    const unsigned e0 = F.ext[0], pl = e0 * F.ext[1];
+    T s = 0;
+    AMR_UNROLL
+    for (int a = 0; a < 8; ++a) {
+        if (a >= (1 << G.dm)) break;
+        s += fine[(unsigned)q.fine + (a & 1) + (a & 2 ? e0 : 0u) + (a & 4 ? pl : 0u)];
+    }
+    crse[q.coarse] = s / (T)(1 << G.dm);
+}
+
+// Multilinear interpolation to the region cells, 0 elsewhere (prolong_cell): the coarse neighbours of a
+// cell away from the domain faces at constant offsets.
+template <typename T>
+AMR_FI void prolong_plane(const Geo& G, const LevT<T>& F, const LevT<T>& C, Plane P, unsigned t, unsigned k,
+                          const T* __restrict__ uc, T* __restrict__ uf) {
+    Cell c;
+    if (!plane_cell(F, P, t, k, c)) return;
+    const unsigned char m = F.mask[c.q];
+    if (!(m & kIn)) {
+        uf[c.q] = 0;
+        return;
+    }
+    const int g[3] = {F.lo[0] + (int)c.i, F.lo[1] + (int)c.j, F.lo[2] + (int)k};
+    bool in = true;
+    int at[3], st[3];
+    const int sz[3] = {1, C.ext[0], C.ext[0] * C.ext[1]};
+    AMR_UNROLL
+    for (int d = 0; d < 3; ++d) {
+        at[d] = d < G.dm ? (g[d] >> 1) - C.lo[d] : 0;
+        const int o = d < G.dm ? (g[d] & 1 ? 1 : -1) : 0;
+        st[d] = o * sz[d];
+        in = in && at[d] + o >= 0 && at[d] + o < C.ext[d];
+    }
+    if (!in) {
+        prolong_cell(G, F, C, (long)c.q, uc, uf);
+        return;
+    }
+    const T* b = uc + (at[0] + at[1] * sz[1] + at[2] * sz[2]);
+    T s = 0;
+    AMR_UNROLL
+    for (int a = 0; a < 8; ++a) {
+        if (a >= (1 << G.dm)) break;
+        T w = 1;
+        int o = 0;
+        AMR_UNROLL
+        for (int d = 0; d < 3; ++d) {
+            if (d >= G.dm) break;
+            w *= (a >> d) & 1 ? (T)0.25 : (T)0.75;
+            o += (a >> d) & 1 ? st[d] : 0;
+        }
+        s += w * b[o];
+    }
+    uf[c.q] = s;
+}
+
+// ---- faces: one thread per face of a plane of the array box
+struct Face {
+    unsigned q, f[3];     // index; box coordinates
+    unsigned hi, lo;      // the cells on either side, when both are in the box (two)
+    bool two;
+};
+AMR_FI bool plane_face(const Lev& L, int d, Plane P, unsigned t, unsigned k, Face& c) {
+    const unsigned m0 = L.ext[0] + (d == 0), m1 = L.ext[1] + (d == 1);
+    if (t >= m0 * m1) return false;
+    c.f[1] = row_of(t, m0, P);
+    c.f[0] = t - c.f[1] * m0;
+    c.f[2] = k;
+    c.q = t + m0 * m1 * c.f[2];
+    const unsigned e0 = L.ext[0], e1 = L.ext[1];
+    c.hi = c.f[0] + e0 * (c.f[1] + e1 * c.f[2]);
+    c.lo = c.hi - (d == 0 ? 1u : d == 1 ? e0 : e0 * e1);
+    c.two = c.f[d] >= 1 && c.f[d] < (unsigned)L.ext[d];
+    return true;
+}
+inline Plane face_plane(const Lev& L, int d) { return plane(L.ext[0] + (d == 0), L.ext[1] + (d == 1)); }
+
+// Whether the face borders a region cell (face_in_level).
+AMR_FI bool face_used(const Geo& G, const Lev& L, int d, const Face& c) {
+    if (c.two) return ((L.mask[c.hi] | L.mask[c.lo]) & kIn) != 0;
+    int f[3];
+    face_coords(L, d, (long)c.q, f);
+    return face_in_level(G, L, d, f);
+}
+
+AMR_FI void scale_b0_plane(const Geo& G, const Lev& L, int d, Plane P, unsigned t, unsigned k, double* u,
+                           const double* b0, const double* b0e, int mult) {
+    Face c;
+    if (!plane_face(L, d, P, t, k, c)) return;
+    const int r = L.lo[G.va] + (int)(G.va == 2 ? c.f[2] : c.f[1]);
+    const double bb = d == G.va ? b0e[r] : b0[r];
+    u[c.q] *= mult ? bb : recip(bb);
+}
+
+// Coarse faces away from covered cells keep their values.
+AMR_FI void edge_restrict_plane(const Geo& G, const Lev& F, const Lev& C, int d, Plane P, unsigned t, unsigned k,
+                                double* uc, const double* uf) {
+    Face c;
+    if (!plane_face(C, d, P, t, k, c)) return;
+    if (c.two && !((C.mask[c.hi] | C.mask[c.lo]) & kCov)) return;
+    edge_restrict_face(G, F, C, d, (long)c.q, uc, uf);
+}
+
+// rh = -(div(beta0 U) - macrhs) on region cells (U already holds beta0 U), 0 elsewhere.
+AMR_FI void divergence_plane(const Geo& G, const Lev& L, Plane P, unsigned t, unsigned k,
+                             const double* __restrict__ u0, const double* __restrict__ u1,
+                             const double* __restrict__ u2, const double* __restrict__ macrhs,
+                             double* __restrict__ rh) {
+    Cell c;
+    if (!plane_cell(L, P, t, k, c)) return;
+    if (!(L.mask[c.q] & kIn)) {
+        rh[c.q] = 0.0;
+        return;
+    }
+    const unsigned e0 = L.ext[0], f0 = c.q + c.r, f1 = c.q + e0 * k;
+    double s = macrhs ? macrhs[c.q] : 0.0;
+    s = fma(-L.ih[0], u0[f0 + 1] - u0[f0], s);
+    s = fma(-L.ih[1], u1[f1 + e0] - u1[f1], s);
+    if (G.dm > 2) s = fma(-L.ih[2], u2[c.q + e0 * L.ext[1]] - u2[c.q], s);
+    rh[c.q] = s;
+}
+
+// Solver coefficient of a face of the level (coeff_face).
+AMR_FI void coeff_plane(const Geo& G, const Lev& L, int d, Plane P, unsigned t, unsigned k,
+                        const double* __restrict__ rho, const double* __restrict__ b0,
+                        const double* __restrict__ b0e, int alt, double* __restrict__ beta) {
+    Face c;
+    if (!plane_face(L, d, P, t, k, c)) return;
+    if (!c.two) {
+        coeff_face(G, L, d, (long)c.q, rho, b0, b0e, alt, beta);
+        return;
+    }
+    if (!((L.mask[c.hi] | L.mask[c.lo]) & kIn)) return;
+    double v = 2.0 * recip(rho[c.hi] + rho[c.lo]);
+    if (b0) {
+        const int r = L.lo[G.va] + (int)(G.va == 2 ? c.f[2] : c.f[1]);
+        const double bb = d == G.va ? b0e[r] : b0[r];
+        v *= bb;
+        if (alt) v *= bb;
+    }
+    beta[c.q] = v;
+}
+
+// beta0 U -= beta G phi on a face of the level (correct_face).
+AMR_FI void correct_plane(const Geo& G, const Lev& L, const Lev& C, int d, Plane P, unsigned t, unsigned k,
+                          const double* phi, const double* cphi, const double* beta, double* u) {
+    Face c;
+    if (!plane_face(L, d, P, t, k, c)) return;
+    if (c.two) {
+        const int n = (L.mask[c.hi] & kIn) + (L.mask[c.lo] & kIn);
+        if (n == 0) return;
+        if (n == 2 * kIn) {
+            u[c.q] = fma(-beta[c.q] * L.ih[d], phi[c.hi] - phi[c.lo], u[c.q]);
+            return;
+        }
+    }
+    correct_face(G, L, C, d, (long)c.q, phi, cphi, beta, u);
+}
+
+// Index of a face or cell of the box in the caller's whole-level-domain arrays.
+AMR_FI size_t full_face(const Lev& L, int d, const Face& c) {
+    const size_t m0 = L.n[0] + (d == 0), m1 = L.n[1] + (d == 1);
+    return (c.f[0] + L.lo[0]) + m0 * ((c.f[1] + L.lo[1]) + m1 * (size_t)(c.f[2] + L.lo[2]));
+}
+AMR_FI size_t full_cell(const Lev& L, const Cell& c) {
+    return (c.i + L.lo[0]) + (size_t)L.n[0] * ((c.j + L.lo[1]) + (size_t)L.n[1] * (c.k + L.lo[2]));
+}
+
+// A level's mask bits kNear and kFull, and the list of the
+// region cells without kNear, then of those without kFull; *nrest: how many the first are.
+inline std::vector<int> classify(int dm, const Lev& V, std::vector<unsigned char>& mask, int* nrest) {
+    const int e0 = V.ext[0], e1 = V.ext[1], e2 = V.ext[2];
+    const long pl = (long)e0 * e1;
+    std::vector<int> far, part;
+    for (int k = 0; k < e2; ++k)
+        for (int j = 0; j < e1; ++j) {
+            unsigned char* m = mask.data() + pl * k + (long)e0 * j;
+            const bool row = (dm < 2 || (j > 0 && j < e1 - 1)) && (dm < 3 || (k > 0 && k < e2 - 1));
+            for (int i = 0; i < e0; ++i) {
+                if (!(m[i] & kIn)) continue;
+                const int idx = (int)(pl * k + (long)e0 * j + i);
+                if (!row || i == 0 || i == e0 - 1) {
+                    far.push_back(idx);
+                    continue;
+                }
+                unsigned char all = m[i - 1] & m[i + 1];
+                if (dm > 1) all &= m[i - e0] & m[i + e0];
+                if (dm > 2) all &= m[i - pl] & m[i + pl];
+                m[i] |= (all & kIn) ? (unsigned char)(kNear | kFull) : kNear;
+                if (!(all & kIn)) part.push_back(idx);
+            }
+        }
+    *nrest = (int)far.size();
+    far.insert(far.end(), part.begin(), part.end());
+    return far;
+}
+
+// Lists of level l >= 1: the valid cells of level l - 1 beside a covered one, the covered ones
+// with their first child.
+inline void coarse_lists(const Geo& G, const Lev& F, const Lev& K, const std::vector<unsigned char>& mask,
+                  std::vector<int>& reflux, std::vector<Child>& cover) {
+    const int dm = G.dm;
+    std::vector<unsigned char> beside(mask.size(), 0);   // valid cells taken already
+    long idx = 0;
+    for (int k = 0; k < K.ext[2]; ++k)
+        for (int j = 0; j < K.ext[1]; ++j)
+            for (int i = 0; i < K.ext[0]; ++i, ++idx) {
+                if (!(mask[(size_t)idx] & kCov)) continue;
+                const int q[3] = {K.lo[0] + i, K.lo[1] + j, K.lo[2] + k};
+                const int f[3] = {2 * q[0], dm > 1 ? 2 * q[1] : q[1], dm > 2 ? 2 * q[2] : q[2]};
+                cover.push_back(Child{(int)idx, (int)cix(F, f[0], f[1], f[2])});
+                for (int d = 0; d < dm; ++d)
+                    for (int s = -1; s <= 1; s += 2) {
+                        int p[3] = {q[0], q[1], q[2]};
+                        p[d] += s;
+                        if (p[d] < 0 || p[d] >= K.n[d]) {
+                            if (!G.per[d]) continue;
+                            p[d] += p[d] < 0 ? K.n[d] : -K.n[d];
+                        }
+                        if (!inside(K, p)) continue;
+                        const size_t n = (size_t)cix(K, p[0], p[1], p[2]);
+                        if ((mask[n] & (kIn | kCov)) == kIn && !beside[n]) {
+                            beside[n] = 1;
+                            reflux.push_back((int)n);
+                        }
+                    }
+            }
+    std::sort(reflux.begin(), reflux.end());
 }
 
 // ---- caller fabs <-> level arrays -------------------------------------------------------------
