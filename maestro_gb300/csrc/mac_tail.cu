@@ -1,9 +1,11 @@
 // Cluster "tail" of the V-cycle: every level from the first one small enough down to the bottom
 // solve runs inside one kernel, on one thread-block cluster whose CTAs share the levels through
 // distributed shared memory, so the small levels pay a cluster barrier instead of a kernel launch
-// per half-sweep.  The arithmetic is the multi-kernel V-cycle's, operation for operation (same
-// fused-multiply-add order per cell, same child order in the restriction, same separable
-// trilinear prolongation, the same bottom solver), so the result is bitwise the same.
+// per half-sweep.  The levels' arithmetic is the multi-kernel V-cycle's, operation for operation
+// (same fused-multiply-add order per cell, same child order in the restriction, same separable
+// trilinear prolongation), so the result is bitwise that of the levels launched one by one with this
+// kernel for the bottom alone (coarse_tail = 0).  The bottom solver has reductions and a stopping test
+// of its own: it agrees with the one-CTA solver of larger bottoms (mac_kernels.cu) to its tolerance.
 //
 // What bounds it: latency.  On GB300 a cluster barrier takes ~380 cycles (256 threads a CTA), a
 // dependent distributed-shared-memory load ~240, a block barrier 20-80, and an SM sub-partition
