@@ -46,77 +46,84 @@ inline dim3 plane_grid(long cells, int planes) {
     return dim3((unsigned)((cells + kThreads - 1) / kThreads), 1, (unsigned)planes);
 }
 
-// Cells taken by list: the extra planes' threads in order.
+// Cells taken by list: the first `per` threads of every block of the extra planes, in order.  They are
+// long in FP64, so a list that leaves SMs without a block is spread over four times as many.
+constexpr int kListThreads = 64;
 struct Rest {
     const int* list;
-    int n;
+    int n, per;
 };
+inline Rest rest_of(const int* list, int n, int sms) { return Rest{list, n, n < kThreads * sms ? kListThreads : kThreads}; }
 __device__ __forceinline__ int rest_index(int planes, const Rest& R) {
-    return amr::rest_entry(R.list, R.n, (blockIdx.z - (unsigned)planes) * gridDim.x * kThreads + plane_thread());
+    if ((int)threadIdx.x >= R.per) return -1;
+    return amr::rest_entry(R.list, R.n,
+                           ((blockIdx.z - (unsigned)planes) * gridDim.x + blockIdx.x) * R.per + threadIdx.x);
 }
-inline dim3 plane_grid(long cells, int planes, int rest) {
+inline dim3 plane_grid(long cells, int planes, const Rest& R) {
     dim3 g = plane_grid(cells, planes);
-    const long slice = (long)g.x * kThreads;
-    g.z += (unsigned)amr::rest_planes(rest, slice);
+    g.z += (unsigned)amr::rest_planes(R.n, (long)g.x * R.per);
     return g;
 }
 
-// Two planes a thread: twice the loads in flight.
-constexpr int kPlanes = 2;
-inline int plane_blocks(int planes) { return (planes + kPlanes - 1) / kPlanes; }
+// NP planes a thread: two, with twice the loads in flight, where that leaves every SM a block; small
+// levels, which FP64 issue on the SMs they reach binds, take one (26^3 cells, FP64: 10.9 -> 7.3 us a
+// colour).
+inline int planes_a_thread(long cells, int planes, int sms) {
+    return (cells + kThreads - 1) / kThreads * ((planes + 1) / 2) < sms ? 1 : 2;
+}
 
-template <typename T>
+template <typename T, int NP>
 __global__ void __launch_bounds__(kThreads)
 k_defect(Geo G, amr::LevT<T> L, amr::LevT<T> C, Plane P, Rest R, const T* __restrict__ u,
          const T* __restrict__ cu, const T* __restrict__ f, T* __restrict__ r) {
-    const int nz = (L.ext[2] + kPlanes - 1) / kPlanes;
+    const int nz = (L.ext[2] + NP - 1) / NP;
     if (blockIdx.z >= (unsigned)nz) {
         const int q = rest_index(nz, R);
         if (q >= 0) amr::defect_cell(G, L, C, (long)q, u, cu, f, r);
         return;
     }
-    Cell c[kPlanes];
-    amr::Stencil<T> A[kPlanes];
-    bool on[kPlanes];
+    Cell c[NP];
+    amr::Stencil<T> A[NP];
+    bool on[NP];
 #pragma unroll
-    for (int p = 0; p < kPlanes; ++p) {
-        on[p] = amr::plane_cell(L, P, plane_thread(), kPlanes * blockIdx.z + p, c[p]);
+    for (int p = 0; p < NP; ++p) {
+        on[p] = amr::plane_cell(L, P, plane_thread(), NP * blockIdx.z + p, c[p]);
         if (on[p]) amr::load_stencil(G, L, c[p], u, f, A[p]);
     }
 #pragma unroll
-    for (int p = 0; p < kPlanes; ++p)
+    for (int p = 0; p < NP; ++p)
         if (on[p]) amr::defect_near(G, L, A[p], c[p].q, cu != nullptr, r);
 }
 
 // One colour of a sweep, zero coarse data.
-template <typename T>
+template <typename T, int NP>
 __global__ void __launch_bounds__(kThreads)
 k_gsrb(Geo G, amr::LevT<T> L, Plane P, Rest R, int colour, T* u, const T* __restrict__ f) {
-    const int nz = (L.ext[2] + kPlanes - 1) / kPlanes;
+    const int nz = (L.ext[2] + NP - 1) / NP;
     if (blockIdx.z >= (unsigned)nz) {
         const int q = rest_index(nz, R);
         if (q >= 0) amr::gsrb_cell(G, L, (long)q, colour, u, f);
         return;
     }
-    Cell c[kPlanes];
-    amr::Stencil<T> A[kPlanes];
-    bool on[kPlanes];
+    Cell c[NP];
+    amr::Stencil<T> A[NP];
+    bool on[NP];
 #pragma unroll
-    for (int p = 0; p < kPlanes; ++p) {
-        on[p] = amr::colour_plane_cell(L, P, colour, plane_thread(), kPlanes * blockIdx.z + p, c[p]);
+    for (int p = 0; p < NP; ++p) {
+        on[p] = amr::colour_plane_cell(L, P, colour, plane_thread(), NP * blockIdx.z + p, c[p]);
         if (on[p]) amr::load_stencil(G, L, c[p], u, f, A[p]);
     }
 #pragma unroll
-    for (int p = 0; p < kPlanes; ++p)
+    for (int p = 0; p < NP; ++p)
         if (on[p]) amr::gsrb_near(G, L, A[p], c[p].q, u);
 }
 
 // The coarse cells that take a reflux, by list (a scan of the coarse level's mask took 67 us at
 // 128^3 for 25 thousand cells).
 template <typename T>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kListThreads)
 k_reflux(Geo G, amr::LevT<T> F, amr::LevT<T> C, const T* uf, const T* uc, T* res, const int* list, int n) {
-    const int t = blockIdx.x * kThreads + threadIdx.x;
+    const int t = blockIdx.x * kListThreads + threadIdx.x;
     if (t < n) amr::reflux_cell(G, F, C, (long)list[t], uf, uc, res);
 }
 
@@ -644,9 +651,12 @@ struct GpuMl {
         const amr::LevT<T> C = l ? lev(l - 1) : lev(l);
         const amr::LevT<T> L = lev(l);
         const AmrState::LevelStore& S = A->L[l];
-        const Rest R{S.rest, cu ? S.nrest_cu : S.nrest};
-        k_defect<T><<<plane_grid((long)L.ext[0] * L.ext[1], plane_blocks(L.ext[2]), R.n), kThreads, 0, c->stream>>>(
-            geo, L, C, cell_plane(L), R, uu, cu, f, r);
+        const Rest R = rest_of(S.rest, cu ? S.nrest_cu : S.nrest, c->sms);
+        const long cells = (long)L.ext[0] * L.ext[1];
+        const int np = planes_a_thread(cells, L.ext[2], c->sms);
+        auto kern = np == 2 ? k_defect<T, 2> : k_defect<T, 1>;
+        kern<<<plane_grid(cells, ceil_div(L.ext[2], np), R), kThreads, 0, c->stream>>>(geo, L, C, cell_plane(L), R,
+                                                                                      uu, cu, f, r);
         launched();
     }
     cudaEvent_t next_event() {
@@ -681,8 +691,11 @@ struct GpuMl {
             for (int colour = 0; colour < 2; ++colour) {
                 const amr::LevT<T> L = lev(l);
                 const int hw = (L.ext[0] + 1) / 2;
-                const Rest R{A->L[l].rest, A->L[l].nrest};
-                k_gsrb<T><<<plane_grid((long)hw * L.ext[1], plane_blocks(L.ext[2]), R.n), kThreads, 0, c->stream>>>(
+                const Rest R = rest_of(A->L[l].rest, A->L[l].nrest, c->sms);
+                const long cells = (long)hw * L.ext[1];
+                const int np = planes_a_thread(cells, L.ext[2], c->sms);
+                auto kern = np == 2 ? k_gsrb<T, 2> : k_gsrb<T, 1>;
+                kern<<<plane_grid(cells, ceil_div(L.ext[2], np), R), kThreads, 0, c->stream>>>(
                     geo, L, plane(hw, L.ext[1]), R, colour, uu, f);
                 launched();
             }
@@ -690,7 +703,7 @@ struct GpuMl {
     void reflux(int l, const T* uf, const T* uc, T* res) {
         const AmrState::LevelStore& S = A->L[l];
         if (S.nreflux == 0) return;   // (the level covers the whole coarser one)
-        k_reflux<T><<<ceil_div(S.nreflux, kThreads), kThreads, 0, c->stream>>>(
+        k_reflux<T><<<ceil_div(S.nreflux, kListThreads), kListThreads, 0, c->stream>>>(
             geo, lev(l), lev(l - 1), uf, uc, res, S.reflux, S.nreflux);
         launched();
     }

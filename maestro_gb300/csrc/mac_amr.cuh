@@ -25,7 +25,6 @@
 // a level (see GpuExec in mac_amr.cu).
 #pragma once
 
-#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <type_traits>
@@ -916,41 +915,56 @@ AMR_FI size_t full_cell(const Lev& L, const Cell& c) {
     return (c.i + L.lo[0]) + (size_t)L.n[0] * ((c.j + L.lo[1]) + (size_t)L.n[1] * (c.k + L.lo[2]));
 }
 
-// A level's mask bits kNear and kFull, and the list of the
-// region cells without kNear, then of those without kFull; *nrest: how many the first are.
+// The lists below are in order of the sides that need attention, then of the index: lanes of a warp
+// that go through different sides run them one after the other (sorted by the index alone, a reflux of
+// 24^3 fine cells took 37 us in FP64; 21).
+struct BySide {
+    std::vector<int> of[64];
+    void put(unsigned sides, long cell) { of[sides & 63u].push_back((int)cell); }
+    void append_to(std::vector<int>& list) const {
+        for (const std::vector<int>& v : of) list.insert(list.end(), v.begin(), v.end());
+    }
+};
+
+// A level's mask bits kNear and kFull, and the list of the region cells without kNear, then of those
+// without kFull; *nrest: how many the first are.
 inline std::vector<int> classify(int dm, const Lev& V, std::vector<unsigned char>& mask, int* nrest) {
     const int e0 = V.ext[0], e1 = V.ext[1], e2 = V.ext[2];
     const long pl = (long)e0 * e1;
-    std::vector<int> far, part;
+    BySide far, part;
     for (int k = 0; k < e2; ++k)
         for (int j = 0; j < e1; ++j) {
             unsigned char* m = mask.data() + pl * k + (long)e0 * j;
-            const bool row = (dm < 2 || (j > 0 && j < e1 - 1)) && (dm < 3 || (k > 0 && k < e2 - 1));
             for (int i = 0; i < e0; ++i) {
                 if (!(m[i] & kIn)) continue;
-                const int idx = (int)(pl * k + (long)e0 * j + i);
-                if (!row || i == 0 || i == e0 - 1) {
-                    far.push_back(idx);
+                const long idx = pl * k + (long)e0 * j + i;
+                unsigned edge = (i == 0 ? 1u : 0u) | (i == e0 - 1 ? 2u : 0u);
+                if (dm > 1) edge |= (j == 0 ? 4u : 0u) | (j == e1 - 1 ? 8u : 0u);
+                if (dm > 2) edge |= (k == 0 ? 16u : 0u) | (k == e2 - 1 ? 32u : 0u);
+                if (edge) {
+                    far.put(edge, idx);
                     continue;
                 }
-                unsigned char all = m[i - 1] & m[i + 1];
-                if (dm > 1) all &= m[i - e0] & m[i + e0];
-                if (dm > 2) all &= m[i - pl] & m[i + pl];
-                m[i] |= (all & kIn) ? (unsigned char)(kNear | kFull) : kNear;
-                if (!(all & kIn)) part.push_back(idx);
+                unsigned out = (m[i - 1] & kIn ? 0u : 1u) | (m[i + 1] & kIn ? 0u : 2u);
+                if (dm > 1) out |= (m[i - e0] & kIn ? 0u : 4u) | (m[i + e0] & kIn ? 0u : 8u);
+                if (dm > 2) out |= (m[i - pl] & kIn ? 0u : 16u) | (m[i + pl] & kIn ? 0u : 32u);
+                m[i] |= out ? kNear : (unsigned char)(kNear | kFull);
+                if (out) part.put(out, idx);
             }
         }
-    *nrest = (int)far.size();
-    far.insert(far.end(), part.begin(), part.end());
-    return far;
+    std::vector<int> list;
+    far.append_to(list);
+    *nrest = (int)list.size();
+    part.append_to(list);
+    return list;
 }
 
 // Lists of level l >= 1: the valid cells of level l - 1 beside a covered one, the covered ones
 // with their first child.
 inline void coarse_lists(const Geo& G, const Lev& F, const Lev& K, const std::vector<unsigned char>& mask,
-                  std::vector<int>& reflux, std::vector<Child>& cover) {
+                         std::vector<int>& reflux, std::vector<Child>& cover) {
     const int dm = G.dm;
-    std::vector<unsigned char> beside(mask.size(), 0);   // valid cells taken already
+    std::vector<unsigned char> beside(mask.size(), 0);   // a valid cell's covered sides
     long idx = 0;
     for (int k = 0; k < K.ext[2]; ++k)
         for (int j = 0; j < K.ext[1]; ++j)
@@ -969,13 +983,13 @@ inline void coarse_lists(const Geo& G, const Lev& F, const Lev& K, const std::ve
                         }
                         if (!inside(K, p)) continue;
                         const size_t n = (size_t)cix(K, p[0], p[1], p[2]);
-                        if ((mask[n] & (kIn | kCov)) == kIn && !beside[n]) {
-                            beside[n] = 1;
-                            reflux.push_back((int)n);
-                        }
+                        if ((mask[n] & (kIn | kCov)) == kIn) beside[n] |= (unsigned char)(1u << (2 * d + (s < 0)));
                     }
             }
-    std::sort(reflux.begin(), reflux.end());
+    BySide sides;
+    for (size_t n = 0; n < beside.size(); ++n)
+        if (beside[n]) sides.put(beside[n], (long)n);
+    sides.append_to(reflux);
 }
 
 // ---- caller fabs <-> level arrays -------------------------------------------------------------

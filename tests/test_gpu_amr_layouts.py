@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 import oracle as O
-from maestro_gb300.inputs import BC_DIR, cell_to_edge
+from maestro_gb300.inputs import BC_DIR, BC_NEU, BC_PER, cell_to_edge
 from tests.test_amr_planes import LAYOUTS
 from tests.test_oracle_amr import G, phi_err, u_err
 
@@ -13,8 +13,13 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 
+# two planes a thread, lists longer than a block on every SM (the other layouts: one plane, short lists)
+LARGE = {"large": ((64, 56, 48), (BC_PER, BC_PER, BC_NEU), (BC_PER, BC_PER, BC_DIR),
+                   [[((12, 12, 8), (115, 103, 87))]])}
+
+
 def make_case(name):
-    n0, lo, hi, fine = LAYOUTS[name]
+    n0, lo, hi, fine = {**LAYOUTS, **LARGE}[name]
     dm, boxes = len(n0), [[]] + fine
     rng = np.random.default_rng(19)
     c = dict(n0=n0, dm=dm, nlev=len(boxes), boxes=boxes, bc_lo=lo, bc_hi=hi,
@@ -41,7 +46,7 @@ def make_case(name):
 
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
-@pytest.mark.parametrize("name", list(LAYOUTS))
+@pytest.mark.parametrize("name", [*LAYOUTS, *LARGE])
 def test_layouts_match_oracle(cuda_lib, name, precision):
     from tests.test_gpu_zz_amr import _run
     c = make_case(name)
