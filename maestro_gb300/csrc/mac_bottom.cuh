@@ -14,68 +14,44 @@ struct BotView {
     const double *bx, *by, *bz, *dg, *idg;
 };
 
-// Synchronisation policy of the one-CTA bottom solver: any CTA size, natural item order.
-struct CtaSync {
-    static __device__ __forceinline__ void sync() { __syncthreads(); }
-    static __device__ __forceinline__ int tid() { return threadIdx.x; }
-    static __device__ __forceinline__ int nt() { return blockDim.x; }
-    static __device__ double sum(double v, double* sm) {
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-        if (lane == 0) sm[wid] = v;
-        __syncthreads();
-        if (wid == 0) {
-            double r = lane < nw ? sm[lane] : 0.0;
-            for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
-            if (lane == 0) sm[32] = r;
-        }
-        __syncthreads();
-        const double r = sm[32];
-        __syncthreads();
-        return r;
+// Sum and maximum key over the CTA in a fixed order; every thread gets the result.
+__device__ double cta_sum(double v, double* sm) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    if (lane == 0) sm[wid] = v;
+    __syncthreads();
+    if (wid == 0) {
+        double r = lane < nw ? sm[lane] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
+        if (lane == 0) sm[32] = r;
     }
-    static __device__ double max(double v, double* sm) {
-        for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-        if (lane == 0) sm[wid] = v;
-        __syncthreads();
-        if (wid == 0) {
-            double r = lane < nw ? sm[lane] : 0.0;
-            for (int o = 16; o > 0; o >>= 1) r = fmax(r, __shfl_down_sync(0xffffffffu, r, o));
-            if (lane == 0) sm[32] = r;
-        }
-        __syncthreads();
-        const double r = sm[32];
-        __syncthreads();
-        return r;
+    __syncthreads();
+    const double r = sm[32];
+    __syncthreads();
+    return r;
+}
+__device__ unsigned long long cta_umax(unsigned long long v, double* sm) {
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long w = __shfl_down_sync(0xffffffffu, v, o);
+        v = w > v ? w : v;
     }
-    static __device__ void sum2(double& a, double& b, double* sm) {
-        a = sum(a, sm);
-        b = sum(b, sm);
-    }
-    static __device__ unsigned long long umax(unsigned long long v, double* sm) {
+    unsigned long long* u = reinterpret_cast<unsigned long long*>(sm);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    if (lane == 0) u[wid] = v;
+    __syncthreads();
+    if (wid == 0) {
+        unsigned long long r = lane < nw ? u[lane] : 0ull;
         for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long w = __shfl_down_sync(0xffffffffu, v, o);
-            v = w > v ? w : v;
+            const unsigned long long w = __shfl_down_sync(0xffffffffu, r, o);
+            r = w > r ? w : r;
         }
-        unsigned long long* u = reinterpret_cast<unsigned long long*>(sm);
-        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-        if (lane == 0) u[wid] = v;
-        __syncthreads();
-        if (wid == 0) {
-            unsigned long long r = lane < nw ? u[lane] : 0ull;
-            for (int o = 16; o > 0; o >>= 1) {
-                const unsigned long long w = __shfl_down_sync(0xffffffffu, r, o);
-                r = w > r ? w : r;
-            }
-            if (lane == 0) u[32] = r;
-        }
-        __syncthreads();
-        const unsigned long long r = u[32];
-        __syncthreads();
-        return r;
+        if (lane == 0) u[32] = r;
     }
-};
+    __syncthreads();
+    const unsigned long long r = u[32];
+    __syncthreads();
+    return r;
+}
 
 // |v| as an order-preserving integer key (the bit pattern of a non-negative double).
 __device__ __forceinline__ unsigned long long abs_key(double v) {
@@ -100,10 +76,9 @@ struct BotTables {
     double* fi;    // N doubles: f / diag
 };
 
-template <class S>
 __device__ void bot_prepare(const BotView& v, const BotTables& T) {
     const int N = v.N;
-    for (int c = S::tid(); c < N; c += S::nt()) {
+    for (int c = (int)threadIdx.x; c < N; c += (int)blockDim.x) {
         const int i = c % v.n0;
         const int row = c / v.n0;
         const int j = row % v.n1;
@@ -129,7 +104,7 @@ __device__ void bot_prepare(const BotView& v, const BotTables& T) {
         T.gc[4 * N + c] = v.bz[c] * id;
         T.gc[5 * N + c] = v.bz[czp] * id;
     }
-    S::sync();
+    __syncthreads();
 }
 
 __device__ __forceinline__ double bot_gsum(const BotTables& T, int N, const double* __restrict__ x,
@@ -140,27 +115,25 @@ __device__ __forceinline__ double bot_gsum(const BotTables& T, int N, const doub
 }
 
 // One red/black sweep.
-template <class S>
 __device__ __noinline__ void bot_gsrb(const BotView& v, const BotTables& T, double* x) {
     const int N = v.N;
     for (int colour = 0; colour < 2; ++colour) {
-        for (int c = S::tid(); c < N; c += S::nt())
+        for (int c = (int)threadIdx.x; c < N; c += (int)blockDim.x)
             if (T.nb[6 * N + c] == colour) x[c] = bot_gsum(T, N, x, c, T.fi[c]);
-        S::sync();
+        __syncthreads();
     }
 }
 
 // y = A x
-template <class S>
 __device__ __noinline__ void bot_apply(const BotView& v, const BotTables& T, const double* x, double* y) {
     const int N = v.N;
-    for (int c = S::tid(); c < N; c += S::nt()) {
+    for (int c = (int)threadIdx.x; c < N; c += (int)blockDim.x) {
         double t = x[c];
 #pragma unroll
         for (int n = 0; n < 6; ++n) t = fma(-T.gc[n * N + c], x[T.nb[n * N + c]], t);
         y[c] = v.dg[c] * t;
     }
-    S::sync();
+    __syncthreads();
 }
 
 // The bottom solve on FP64 arrays x (in/out) and f (in; mean removed here when singular):
@@ -168,11 +141,10 @@ __device__ __noinline__ void bot_apply(const BotView& v, const BotTables& T, con
 // scr holds kBotScrPerCell doubles per cell (14 N doubles, then 7 N ints).  Returns the BiCGStab
 // iteration count.
 
-template <class S>
 __device__ int bottom_body(const BotView& v, double* x, double* f, double* scr, double* sm,
                            int singular, int nub, double eps, int max_iter) {
     const int N = v.N;
-    const int tid = S::tid(), nt = S::nt();
+    const int tid = (int)threadIdx.x, nt = (int)blockDim.x;
     double* r = scr;
     double* rh = scr + N;
     double* p = scr + 2 * N;
@@ -184,17 +156,17 @@ __device__ int bottom_body(const BotView& v, double* x, double* f, double* scr, 
     T.gc = scr + 7 * N;
     T.fi = scr + 13 * N;
     T.nb = reinterpret_cast<int*>(scr + 14 * N);
-    bot_prepare<S>(v, T);
+    bot_prepare(v, T);
     double loc = 0.0;
     for (int c = tid; c < N; c += nt) loc += f[c];
-    const double mean = S::sum(loc, sm) / N;
+    const double mean = cta_sum(loc, sm) / N;
     for (int c = tid; c < N; c += nt) {
         if (singular) f[c] -= mean;
         T.fi[c] = f[c] * v.idg[c];
     }
-    S::sync();
-    for (int it = 0; it < nub; ++it) bot_gsrb<S>(v, T, x);
-    bot_apply<S>(v, T, x, t);
+    __syncthreads();
+    for (int it = 0; it < nub; ++it) bot_gsrb(v, T, x);
+    bot_apply(v, T, x, t);
     unsigned long long kmax = 0;
     loc = 0.0;
     for (int c = tid; c < N; c += nt) {
@@ -207,8 +179,8 @@ __device__ int bottom_body(const BotView& v, double* x, double* f, double* scr, 
         kmax = key > kmax ? key : kmax;
         loc = fma(rc, rc, loc);
     }
-    const double r0 = key_value(S::umax(kmax, sm));
-    double rho = S::sum(loc, sm);   // (rh, r) of the first iteration
+    const double r0 = key_value(cta_umax(kmax, sm));
+    double rho = cta_sum(loc, sm);   // (rh, r) of the first iteration
     int count = 0;
     if (r0 > 0.0) {
         const double tol = eps * r0;
@@ -222,11 +194,11 @@ __device__ int bottom_body(const BotView& v, double* x, double* f, double* scr, 
                 p[c] = pc;
                 y[c] = pc * v.idg[c];
             }
-            S::sync();
-            bot_apply<S>(v, T, y, vv);
+            __syncthreads();
+            bot_apply(v, T, y, vv);
             loc = 0.0;
             for (int c = tid; c < N; c += nt) loc = fma(rh[c], vv[c], loc);
-            const double rv = S::sum(loc, sm);
+            const double rv = cta_sum(loc, sm);
             if (rv == 0.0) break;
             alpha = rho * recip_nr(rv);
             kmax = 0;
@@ -237,17 +209,18 @@ __device__ int bottom_body(const BotView& v, double* x, double* f, double* scr, 
                 const unsigned long long key = abs_key(sc);
                 kmax = key > kmax ? key : kmax;
             }
-            const double sn = key_value(S::umax(kmax, sm));
+            const double sn = key_value(cta_umax(kmax, sm));
             if (sn <= tol) break;
             for (int c = tid; c < N; c += nt) y[c] = s[c] * v.idg[c];
-            S::sync();
-            bot_apply<S>(v, T, y, t);
+            __syncthreads();
+            bot_apply(v, T, y, t);
             double l1 = 0.0, l2 = 0.0;
             for (int c = tid; c < N; c += nt) {
                 l1 = fma(t[c], s[c], l1);
                 l2 = fma(t[c], t[c], l2);
             }
-            S::sum2(l1, l2, sm);
+            l1 = cta_sum(l1, sm);
+            l2 = cta_sum(l2, sm);
             omega = l2 > 0.0 ? l1 * recip_nr(l2) : 0.0;
             kmax = 0;
             loc = 0.0;
@@ -259,14 +232,14 @@ __device__ int bottom_body(const BotView& v, double* x, double* f, double* scr, 
                 kmax = key > kmax ? key : kmax;
                 loc = fma(rh[c], rc, loc);
             }
-            const double rn = key_value(S::umax(kmax, sm));
+            const double rn = key_value(cta_umax(kmax, sm));
             rho_old = rho;
-            rho = S::sum(loc, sm);
+            rho = cta_sum(loc, sm);
             if (rn <= tol || omega == 0.0) break;
         }
     }
-    S::sync();
-    for (int it = 0; it < nub; ++it) bot_gsrb<S>(v, T, x);
+    __syncthreads();
+    for (int it = 0; it < nub; ++it) bot_gsrb(v, T, x);
     return count;
 }
 

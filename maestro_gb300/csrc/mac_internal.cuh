@@ -471,10 +471,7 @@ int correct_velocity(mac_ctx* c, const std::function<int(int)>* after_dir, bool 
 int setup_fine_from_faces(mac_ctx* c, const double* fx, const double* fy, const double* fz,
                           const double* alpha_nat, bool reset_flags = true);
 int setup_rhs_from(mac_ctx* c, const double* rh_nat, const double* phi_nat = nullptr);
-int natural_to_level0(mac_ctx* c, const double* src, double* dst);
 int level0_to_natural(mac_ctx* c, const double* src, double* dst);
-int natural_to_level0(mac_ctx* c, const float* src, float* dst);
-int level0_to_natural(mac_ctx* c, const float* src, float* dst);
 int check_density(mac_ctx* c, bool* ok);
 
 // caller box layout

@@ -734,7 +734,7 @@ k_bottom(BotView v, Tio* __restrict__ xio, const Tio* __restrict__ fio, double* 
         f[c] = (double)fio[c];
     }
     __syncthreads();
-    const int count = bottom_body<CtaSync>(v, x, f, scr + 2 * N, sm, singular, nub, eps, max_iter);
+    const int count = bottom_body(v, x, f, scr + 2 * N, sm, singular, nub, eps, max_iter);
     __syncthreads();
     for (int c = tid; c < N; c += nt) xio[c] = (Tio)x[c];
     if (tid == 0 && iters) atomicAdd(iters, count);

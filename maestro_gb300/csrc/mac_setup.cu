@@ -462,17 +462,7 @@ k_correct(const __grid_constant__ CorrParams P, Dims d, const double* __restrict
     }
 }
 
-template <typename T>
-__global__ void k_nat_to_l0(Dims d, const T* __restrict__ src, T* __restrict__ dst) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z;
-    if (i >= d.n0 || j >= d.n1) return;
-    dst[lidx(d, i, j, k)] = src[i + d.n0 * (j + d.n1 * k)];
-}
-
-template <typename T>
-__global__ void k_l0_to_nat(Dims d, const T* __restrict__ src, T* __restrict__ dst) {
+__global__ void k_l0_to_nat(Dims d, const double* __restrict__ src, double* __restrict__ dst) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = blockIdx.z;
@@ -622,7 +612,6 @@ k_fine_coef_faces(FineParams P, Dims d, const double* __restrict__ fx,
     }
 }
 
-Dims level0_dims(const mac_ctx* c) { return c->lev[0].d; }
 
 }  // namespace
 
@@ -827,31 +816,14 @@ int correct_velocity(mac_ctx* c, const std::function<int(int)>* after_dir, bool 
     return MAC_OK;
 }
 
-namespace {
-template <typename T>
-int nat_to_l0(mac_ctx* c, const T* src, T* dst) {
-    const Dims d = level0_dims(c);
+int level0_to_natural(mac_ctx* c, const double* src, double* dst) {
+    const Dims& d = c->lev[0].d;
     const Grid3 g = grid3(d.n0, d.n1, d.n2);
-    k_nat_to_l0<T><<<g.grid, g.block, 0, c->stream>>>(d, src, dst);
+    k_l0_to_nat<<<g.grid, g.block, 0, c->stream>>>(d, src, dst);
     MAC_CUDA_TRY(cudaGetLastError());
     ++c->issued;
     return MAC_OK;
 }
-template <typename T>
-int l0_to_nat(mac_ctx* c, const T* src, T* dst) {
-    const Dims d = level0_dims(c);
-    const Grid3 g = grid3(d.n0, d.n1, d.n2);
-    k_l0_to_nat<T><<<g.grid, g.block, 0, c->stream>>>(d, src, dst);
-    MAC_CUDA_TRY(cudaGetLastError());
-    ++c->issued;
-    return MAC_OK;
-}
-}  // namespace
-
-int natural_to_level0(mac_ctx* c, const double* src, double* dst) { return nat_to_l0(c, src, dst); }
-int level0_to_natural(mac_ctx* c, const double* src, double* dst) { return l0_to_nat(c, src, dst); }
-int natural_to_level0(mac_ctx* c, const float* src, float* dst) { return nat_to_l0(c, src, dst); }
-int level0_to_natural(mac_ctx* c, const float* src, float* dst) { return l0_to_nat(c, src, dst); }
 
 // ---- box tables ----------------------------------------------------------------------------
 namespace {
