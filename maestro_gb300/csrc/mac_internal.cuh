@@ -405,10 +405,10 @@ void launch_bottom(const Dims& d, const LevelArrays<double>& a64, Tio* x, const 
 // ---- cluster tail V-cycle (mac_tail.cu) -----------------------------------------------------
 // nlev == 0: the bottom alone (f0 and e0 in its natural layout, e0 the initial guess)
 constexpr int kTailMaxLevels = 8;
+constexpr int kTailCells = 4096;   // cells of the first level of a tail at most
 constexpr int kTailSmemMax = 200 * 1024;
 struct TailGeo {
     int repl, rpc;                        // held whole by every CTA; rows a CTA
-    int two;                              // two pairs of cells a thread
     int off;                              // byte offset in shared memory
     unsigned mcpc, mn1, mhn0;             // reciprocals of rpc n0, n1, n0 / 2
 };

@@ -11,12 +11,13 @@
 // dependent distributed-shared-memory load ~240, a block barrier 20-80, and an SM sub-partition
 // issues one FP64 warp instruction per 64 cycles; a launch-chained half-sweep kernel takes 2-3 us.
 // So
-//  * a level's rows are spread over all CTAs; a thread owns one or two pairs of x-neighbours (one
-//    cell of each colour) for a whole visit of the level, their operator, right-hand side and
-//    neighbour addresses in registers; only e and the defects are in (distributed) shared memory;
+//  * a level's rows are spread over all CTAs; a thread owns a pair of x-neighbours (one cell of each
+//    colour) for a whole visit of the level, their operator, right-hand side and neighbour addresses in
+//    registers; only e and the defects are in (distributed) shared memory;
 //  * levels of at most kReplCells<T> cells and the exactly solved bottom are computed by every CTA
-//    alone: block barriers only (above that the FP64 rate, or the work, of one SM costs more than
-//    the cluster barriers saved);
+//    alone: block barriers only.  Above that the FP64 rate, or the work, of one SM costs more than
+//    the cluster barriers saved (whole calls against 512 / 128 cells: none 128^2 mixed +9%, 64^3 +5%;
+//    2048 / 256 and 4096 / 512 96 x 112 x 96 mixed +16%);
 //  * the first red half-sweep of a level starts from a zero correction, so it reads no neighbour.
 // Measured against the one-CTA tail and bottom it replaces (whole calls): 128^2 FP64 1427 -> 1116
 // us, 64^3 mixed 1316 -> 1131 us, 160x96x112 FP64 (a bottom of 3360 cells, 14 bottom solves) 20.8 ->
@@ -30,7 +31,6 @@ namespace {
 
 constexpr int kInvThreads = 1024;
 constexpr int kTailMaxThreads = 512;
-constexpr int kTailItems = 2;            // pairs of cells a thread at most
 constexpr int kOps = 17;                 // operator values of a pair in shared memory
 template <typename T>
 constexpr int kReplCells = sizeof(T) == 4 ? 512 : 128;
@@ -175,33 +175,28 @@ __device__ __forceinline__ void store_e(const Pair<T>& q, int s) {
 // nu sweeps.  zero: from e = 0 -- the first colour-0 half-sweep has no arm that contributes.
 // (A predicated-off FP64 instruction still takes its pipe's 64 cycles: the dimension is a template
 // parameter, and FP64 levels are never over-relaxed.)
-template <typename T, int K, bool Z3>
-__device__ __forceinline__ void sweeps(Pair<T> (&q)[K], const Geo& g, int nu, T omega, bool zero) {
+template <typename T, bool Z3>
+__device__ __forceinline__ void sweeps(Pair<T>& q, const Geo& g, int nu, T omega, bool zero) {
     const bool sor = sizeof(T) == 4 && omega != T(1);
     if (zero) {
-#pragma unroll
-        for (int m = 0; m < K; ++m) {
-            q[m].e[0] = q[m].e[1] = T(0);
-            if (nu == 0 && q[m].on) {
-                store_e(q[m], 0);
-                store_e(q[m], 1);
-            }
+        q.e[0] = q.e[1] = T(0);
+        if (nu == 0 && q.on) {
+            store_e(q, 0);
+            store_e(q, 1);
         }
         if (nu == 0) sync_level(g.repl);
     }
     for (int it = 0; it < nu; ++it) {
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
-#pragma unroll
-            for (int m = 0; m < K; ++m) {
-                if (!q[m].on) continue;
-                T acc = q[m].f[s];
-                if (!(zero && it == 0 && s == 0)) acc = arms<T, Z3>(acc, q[m], s);
+            if (q.on) {
+                T acc = q.f[s];
+                if (!(zero && it == 0 && s == 0)) acc = arms<T, Z3>(acc, q, s);
                 if (sor)
-                    q[m].e[s] = fmaT2(omega, fmaT2(acc, q[m].id[s], -q[m].e[s]), q[m].e[s]);
+                    q.e[s] = fmaT2(omega, fmaT2(acc, q.id[s], -q.e[s]), q.e[s]);
                 else
-                    q[m].e[s] = acc * q[m].id[s];
-                store_e(q[m], s);
+                    q.e[s] = acc * q.id[s];
+                store_e(q, s);
             }
             sync_level(g.repl);
         }
@@ -210,26 +205,23 @@ __device__ __forceinline__ void sweeps(Pair<T> (&q)[K], const Geo& g, int nu, T 
 
 // One level down: sweeps from e = 0 and the defects (colour 0 only after a plain Gauss-Seidel
 // black half-sweep) into r.
-template <typename T, int K, bool Z3>
+template <typename T, bool Z3>
 __device__ __forceinline__ void visit_down(const TailParams<T>& P, int l, unsigned rank, unsigned char* sm,
                                         bool red_only) {
     const Geo g = geo_of<T>(P, l, rank, smem_u32(sm));
     const T* ops = reinterpret_cast<const T*>(sm + g.nops);
-    Pair<T> q[K];
-#pragma unroll
-    for (int m = 0; m < K; ++m) load_pair<T, Z3>(q[m], g, ops, threadIdx.x + m * blockDim.x);
-    sweeps<T, K, Z3>(q, g, P.nu1, P.omega, true);
+    Pair<T> q;
+    load_pair<T, Z3>(q, g, ops, threadIdx.x);
+    sweeps<T, Z3>(q, g, P.nu1, P.omega, true);
     const unsigned dr = g.ra - g.ea;
-#pragma unroll
-    for (int m = 0; m < K; ++m) {
-        if (!q[m].on) continue;
+    if (q.on) {
         for (int s = 0; s < (red_only ? 1 : 2); ++s) {
-            const int a = s ? 1 - q[m].p : q[m].p;
-            const T dg = ops[(kDg + a) * g.pairs + threadIdx.x + m * blockDim.x];
-            const T e = s ? q[m].e[1] : q[m].e[0], f = s ? q[m].f[1] : q[m].f[0];
+            const int a = s ? 1 - q.p : q.p;
+            const T dg = ops[(kDg + a) * g.pairs + threadIdx.x];
+            const T e = s ? q.e[1] : q.e[0], f = s ? q.f[1] : q.f[0];
             const T r0 = fmaT2(-dg, e, f);
-            const T r = s ? arms<T, Z3>(r0, q[m], 1) : arms<T, Z3>(r0, q[m], 0);
-            lds_store(q[m].own + dr + a * (unsigned)sizeof(T), r);
+            const T r = s ? arms<T, Z3>(r0, q, 1) : arms<T, Z3>(r0, q, 0);
+            lds_store(q.own + dr + a * (unsigned)sizeof(T), r);
         }
     }
     sync_level(g.repl);
@@ -288,7 +280,7 @@ struct Coarse {
 
 // One level up: e += trilinear interpolation of the coarse correction, then the sweeps.
 // black_only: colour-1 cells only (plain Gauss-Seidel post-smoothing follows; see k_prolong_add).
-template <typename T, int K, bool Z3>
+template <typename T, bool Z3>
 __device__ __forceinline__ void visit_up(const TailParams<T>& P, int l, unsigned rank, unsigned char* sm,
                                       const Coarse<T>& ec, int cn1, int cn2, bool black_only) {
     const Geo g = geo_of<T>(P, l, rank, smem_u32(sm));
@@ -296,65 +288,63 @@ __device__ __forceinline__ void visit_up(const TailParams<T>& P, int l, unsigned
     const int cn0 = g.hn0;
     // a row's pairs lie in one warp: the neighbouring coarse columns come from its lanes
     const bool lanes = cn0 <= 32 && (cn0 & (cn0 - 1)) == 0;
-    Pair<T> q[K];
-#pragma unroll
-    for (int m = 0; m < K; ++m) {
-        const int t = threadIdx.x + m * blockDim.x;
-        load_pair<T, Z3>(q[m], g, ops, t);
-        const int tt = q[m].on ? t : 0;   // (idle lanes stay for the shuffles)
-        const int lr = fdiv(tt, g.mhn0), I = tt - lr * g.hn0;
-        const int row = min(g.row0 + lr, g.n1 * g.n2 - 1);   // (a CTA may own no row)
-        const int k = fdiv(row, g.mn1), j = row - k * g.n1;
-        const int J = j >> 1, Kc = Z3 ? k >> 1 : k;
-        int xs[3], qq[2];
-        T wx[2], w[2];
-        xs[1] = I;
-        nb_w<T>(I, cn0, P.bc.lo[0], P.bc.hi[0], xs[0], xs[2], wx[0], wx[1]);
-        nb_w<T>(J, cn1, P.bc.lo[1], P.bc.hi[1], qq[0], qq[1], w[0], w[1]);
-        const int Yn = j & 1 ? qq[1] : qq[0];
-        const T wy = j & 1 ? w[1] : w[0];
-        int Zn = Kc;
-        T wz = T(0);
+    Pair<T> q;
+    const int t = threadIdx.x;
+    load_pair<T, Z3>(q, g, ops, t);
+    const int tt = q.on ? t : 0;   // (idle lanes stay for the shuffles)
+    const int lr = fdiv(tt, g.mhn0), I = tt - lr * g.hn0;
+    const int row = min(g.row0 + lr, g.n1 * g.n2 - 1);   // (a CTA may own no row)
+    const int k = fdiv(row, g.mn1), j = row - k * g.n1;
+    const int J = j >> 1, Kc = Z3 ? k >> 1 : k;
+    int xs[3], qq[2];
+    T wx[2], w[2];
+    xs[1] = I;
+    nb_w<T>(I, cn0, P.bc.lo[0], P.bc.hi[0], xs[0], xs[2], wx[0], wx[1]);
+    nb_w<T>(J, cn1, P.bc.lo[1], P.bc.hi[1], qq[0], qq[1], w[0], w[1]);
+    const int Yn = j & 1 ? qq[1] : qq[0];
+    const T wy = j & 1 ? w[1] : w[0];
+    int Zn = Kc;
+    T wz = T(0);
+    if (Z3) {
+        nb_w<T>(Kc, cn2, P.bc.lo[2], P.bc.hi[2], qq[0], qq[1], w[0], w[1]);
+        Zn = k & 1 ? qq[1] : qq[0];
+        wz = k & 1 ? w[1] : w[0];
+    }
+    const int r00 = cn0 * (J + cn1 * Kc), r10 = cn0 * (Yn + cn1 * Kc);
+    const int r01 = cn0 * (J + cn1 * Zn), r11 = cn0 * (Yn + cn1 * Zn);
+    // coarse column X interpolated in z, then y
+    auto column = [&](int X) -> T {
+        T zc = ec(X + r00), zn = ec(X + r10);
         if (Z3) {
-            nb_w<T>(Kc, cn2, P.bc.lo[2], P.bc.hi[2], qq[0], qq[1], w[0], w[1]);
-            Zn = k & 1 ? qq[1] : qq[0];
-            wz = k & 1 ? w[1] : w[0];
+            const T pc = ec(X + r01), pn = ec(X + r11);
+            zc = fmaT2(wz, pc, T(0.75) * zc);
+            zn = fmaT2(wz, pn, T(0.75) * zn);
         }
-        const int r00 = cn0 * (J + cn1 * Kc), r10 = cn0 * (Yn + cn1 * Kc);
-        const int r01 = cn0 * (J + cn1 * Zn), r11 = cn0 * (Yn + cn1 * Zn);
-        // coarse column X interpolated in z, then y
-        auto column = [&](int X) -> T {
-            T zc = ec(X + r00), zn = ec(X + r10);
-            if (Z3) {
-                const T pc = ec(X + r01), pn = ec(X + r11);
-                zc = fmaT2(wz, pc, T(0.75) * zc);
-                zn = fmaT2(wz, pn, T(0.75) * zn);
-            }
-            return fmaT2(wy, zn, T(0.75) * zc);
-        };
-        T Y[3];
-        Y[1] = column(I);
-        if (lanes) {
-            const int l0 = (threadIdx.x & 31) - I;
-            Y[0] = __shfl_sync(0xffffffffu, Y[1], l0 + xs[0]);
-            Y[2] = __shfl_sync(0xffffffffu, Y[1], l0 + xs[2]);
-        } else {
-            Y[0] = column(xs[0]);
-            Y[2] = column(xs[2]);
-        }
-        if (!q[m].on) continue;
+        return fmaT2(wy, zn, T(0.75) * zc);
+    };
+    T Y[3];
+    Y[1] = column(I);
+    if (lanes) {
+        const int l0 = (threadIdx.x & 31) - I;
+        Y[0] = __shfl_sync(0xffffffffu, Y[1], l0 + xs[0]);
+        Y[2] = __shfl_sync(0xffffffffu, Y[1], l0 + xs[2]);
+    } else {
+        Y[0] = column(xs[0]);
+        Y[2] = column(xs[2]);
+    }
+    if (q.on) {
         const T mid = T(0.75) * Y[1];
         const T d0 = fmaT2(wx[0], Y[0], mid), d1 = fmaT2(wx[1], Y[2], mid);   // cells 2I, 2I + 1
-        const int p = q[m].p;
+        const int p = q.p;
         const unsigned z = sizeof(T);
-        const T e0 = ld_cluster(q[m].own + p * z, T(0)), e1 = ld_cluster(q[m].own + (1 - p) * z, T(0));
-        q[m].e[0] = black_only ? e0 : e0 + (p ? d1 : d0);
-        q[m].e[1] = e1 + (p ? d0 : d1);
-        if (!black_only) store_e(q[m], 0);
-        store_e(q[m], 1);
+        const T e0 = ld_cluster(q.own + p * z, T(0)), e1 = ld_cluster(q.own + (1 - p) * z, T(0));
+        q.e[0] = black_only ? e0 : e0 + (p ? d1 : d0);
+        q.e[1] = e1 + (p ? d0 : d1);
+        if (!black_only) store_e(q, 0);
+        store_e(q, 1);
     }
     sync_level(g.repl);
-    sweeps<T, K, Z3>(q, g, P.nu2, P.omega, false);
+    sweeps<T, Z3>(q, g, P.nu2, P.omega, false);
 }
 
 // Asynchronous 4/8-byte global -> shared copy (cp.async); completed by cp_async_wait().
@@ -746,12 +736,9 @@ k_tail(const __grid_constant__ TailParams<T> P) {
     const bool red = gs && P.nu1 > 0, black = gs && P.nu2 > 0;
     for (int l = 0; l < nl; ++l) {
         if (z3) {
-            if (P.geo[l].two)
-                visit_down<T, 2, true>(P, l, rank, tail_smem, red);
-            else
-                visit_down<T, 1, true>(P, l, rank, tail_smem, red);
+            visit_down<T, true>(P, l, rank, tail_smem, red);
         } else {
-            visit_down<T, 1, false>(P, l, rank, tail_smem, red);
+            visit_down<T, false>(P, l, rank, tail_smem, red);
         }
         const Geo F = geo_of<T>(P, l, rank, sbase);
         auto coarse_f = [&](int I, int J, int K) -> T {
@@ -852,12 +839,9 @@ k_tail(const __grid_constant__ TailParams<T> P) {
             cn2 = ec.g.n2;
         }
         if (z3) {
-            if (P.geo[l].two)
-                visit_up<T, 2, true>(P, l, rank, tail_smem, ec, cn1, cn2, black);
-            else
-                visit_up<T, 1, true>(P, l, rank, tail_smem, ec, cn1, cn2, black);
+            visit_up<T, true>(P, l, rank, tail_smem, ec, cn1, cn2, black);
         } else {
-            visit_up<T, 1, false>(P, l, rank, tail_smem, ec, cn1, cn2, black);
+            visit_up<T, false>(P, l, rank, tail_smem, ec, cn1, cn2, black);
         }
     }
     // hand the correction back: of the first tail level (its split layout), or the bottom's
@@ -994,7 +978,7 @@ static size_t plan_tail(TailParams<T>& P, int nc, int* threads) {
         const int pairs = q.rpc * (D.n0 >> 1);
         most = pairs > most ? pairs : most;
         off += pad16((size_t)(2 * q.rpc * D.n0 + kOps * pairs) * sizeof(T));
-        if (off > (size_t)kTailSmemMax || pairs > (D.n2 > 1 ? kTailItems : 1) * kTailMaxThreads) return 0;
+        if (off > (size_t)kTailSmemMax || pairs > kTailMaxThreads) return 0;
     }
     const size_t N = P.bottom.ncell;
     P.bottom_off = (int)off;
@@ -1007,11 +991,9 @@ static size_t plan_tail(TailParams<T>& P, int nc, int* threads) {
         off += P.bottom_m * (2 * sizeof(double) + sizeof(T));
     const int need = exact ? 256 : bottom_threads(P.bottom_m);
     if (off > (size_t)kTailSmemMax || need > kTailMaxThreads) return 0;
-    // a pair a thread up to 512 threads (a cluster barrier costs 380 cycles with 256 threads, 470
-    // with 512, 600 with 1024), then two
+    // a pair a thread (a cluster barrier costs 380 cycles with 256 threads, 470 with 512)
     int t = 128;
     while (t < kTailMaxThreads && (t < most || t < need)) t *= 2;
-    for (int l = 0; l < P.nlev; ++l) P.geo[l].two = P.geo[l].rpc * (P.lev[l].n0 >> 1) > t;
     *threads = t;
     return off;
 }
