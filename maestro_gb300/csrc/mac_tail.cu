@@ -608,7 +608,9 @@ __host__ __device__ __forceinline__ int bottom_threads(int M) { return 2 * ((M /
 
 }  // namespace
 
-template <typename T>
+// ONE: a bottom of at most kOneBottom cells, solved by one CTA or by its inverse (an instantiation of its
+// own: with both solvers in one kernel the spread one lost 1% of a 3360-cell call).
+template <typename T, bool ONE>
 __global__ void __launch_bounds__(kTailMaxThreads)
 k_tail(const __grid_constant__ TailParams<T> P) {
     extern __shared__ __align__(16) unsigned char tail_smem[];
@@ -620,7 +622,7 @@ k_tail(const __grid_constant__ TailParams<T> P) {
     const int nl = P.nlev;   // non-bottom tail levels
     const Dims& BD = P.bottom;
     const int NB = BD.ncell;
-    const bool exact = P.binv != nullptr;
+    const bool exact = ONE && P.binv != nullptr;
     const unsigned sbase = smem_u32(tail_smem);
     cluster_arrive();   // (waited for below: every CTA runs before another touches its memory)
     // bottom's shared memory.  exact: the inverse, f, then the solution as T; else x, y (M cells
@@ -819,12 +821,9 @@ k_tail(const __grid_constant__ TailParams<T> P) {
         cluster_sync();
     } else {
         if (B.on) lds_store(B.xa, bx);
-        if (NB > kOneBottom)
-            bx = cl_solve<false>(B, R, bf, bx, bottom_threads(M) / 32, P.singular, P.nub, P.bottom_eps,
-                                 P.bottom_max_iter, &count);
-        else if (rank == 0 && tid < kOneBottom)
-            bx = cl_solve<true>(B, R, bf, bx, kOneBottom / 32, P.singular, P.nub, P.bottom_eps,
-                                P.bottom_max_iter, &count);
+        if (!ONE || (rank == 0 && tid < kOneBottom))
+            bx = cl_solve<ONE>(B, R, bf, bx, (ONE ? kOneBottom : bottom_threads(M)) / 32, P.singular, P.nub,
+                               P.bottom_eps, P.bottom_max_iter, &count);
         if (B.on) eb[bc - (int)rank * M] = (T)bx;
         cluster_sync();
     }
@@ -1028,16 +1027,16 @@ void launch_tail(TailParams<T>& P, int nc, cudaStream_t s) {
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    cudaLaunchKernelEx(&cfg, k_tail<T>, P);
+    cudaLaunchKernelEx(&cfg, P.bottom.ncell <= kOneBottom ? k_tail<T, true> : k_tail<T, false>, P);
 }
 
 // Opts the tail kernels into their shared memory and cluster size; *nc: the CTAs of a cluster.
 int prepare_tail_kernels(int* nc) {
     *nc = kClusterMax;
-    return cluster_opt_in((const void*)k_tail<float>, kTailMaxThreads, kTailSmemMax, nc) &&
-                   cluster_opt_in((const void*)k_tail<double>, kTailMaxThreads, kTailSmemMax, nc)
-               ? MAC_OK
-               : MAC_ERR_CUDA;
+    for (const void* k : {(const void*)k_tail<float, true>, (const void*)k_tail<float, false>,
+                          (const void*)k_tail<double, true>, (const void*)k_tail<double, false>})
+        if (!cluster_opt_in(k, kTailMaxThreads, kTailSmemMax, nc)) return MAC_ERR_CUDA;
+    return MAC_OK;
 }
 
 template bool tail_fits<float>(const Dims*, int, const Dims&, bool, int);
