@@ -232,7 +232,8 @@ k_resid_restrict(Dims F, Dims C, const T* __restrict__ u, const T* __restrict__ 
 // The same with a thread a row of children, summed in the same order over the lanes: a small level has
 // too few coarse cells to hide the latency of eight children a thread, a large one only pays for the
 // additions done by every lane.  Per launch, a thread a cell -> a row: 32^3 coarse cells 11.5 -> 7.1 us
-// (FP32), 11.8 -> 8.1 (FP64), 16^3 FP64 11.2 -> 6.0;  64^3 21.8 -> 26.4 and 23.7 -> 29.7.
+// (FP32), 11.8 -> 8.1 (FP64), 16^3 FP64 11.2 -> 6.0;  64^3 21.8 -> 26.4 and 23.7 -> 29.7.  Between those
+// the line hardly matters: whole calls with it at 2^15 or 2^19 are within 1%.
 constexpr int kRowsMax = 1 << 17;   // coarse cells below which rows are split
 template <typename T, bool RED_ONLY, int RZ>
 __global__ void __launch_bounds__(kBlock)

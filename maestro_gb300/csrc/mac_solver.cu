@@ -126,9 +126,10 @@ OtfParams otf_params(const mac_ctx* c) {
     P.fsmem = c->otf_tile.fsmem;
     P.fthreads = c->otf_tile.fthreads;
     // The staged kernels pay off where their blocks fill the chip: up to 2^21 cells one thread a cell
-    // is faster (whole mixed solves, staged -> per cell: 32^3 875 -> 607 us, 64^3 1124 -> 848, 96^3
-    // 1906 -> 1755, 128^3 1831 -> 1736; 160 x 128 x 128 2530 -> 2930).  The fused sweep and the
-    // wait's fault injection are the staged kernels' own.
+    // is faster (whole mixed solves, staged against per cell: 64^3 +33%, 96^3 +15%, 128 x 128 x 96 +14%,
+    // 128^3 +6%; long rows the other way, 512 x 64 x 64 -8%), above it slower (per cell against
+    // staged: 160 x 128 x 128 +20%, 192 x 128 x 96 +8%, 256 x 96 x 96 +5%, 192^3 +31%; 128 x 144 x 128
+    // -1%).  The fused sweep and the wait's fault injection are the staged kernels' own.
     if (c->lev[0].d.ncell <= (1 << 21) && !c->o.fused_sweep && !c->o.inject_wait_expiry) P.ty = P.rty = 0;
     return P;
 }

@@ -19,9 +19,9 @@
 //    the cluster barriers saved (whole calls against 512 / 128 cells: none 128^2 mixed +9%, 64^3 +5%;
 //    2048 / 256 and 4096 / 512 96 x 112 x 96 mixed +16%);
 //  * the first red half-sweep of a level starts from a zero correction, so it reads no neighbour.
-// Measured against the one-CTA tail and bottom it replaces (whole calls): 128^2 FP64 1427 -> 1116
-// us, 64^3 mixed 1316 -> 1131 us, 160x96x112 FP64 (a bottom of 3360 cells, 14 bottom solves) 20.8 ->
-// 7.1 ms, 256^3 mixed 6.99 -> 6.87 ms.
+// A V-cycle's tail of a 256^3 call (16^3, 8^3 and an exact 4^3 bottom) takes 19 us in FP32 (54 in the
+// one-CTA tail it replaces) and 33 in FP64, of which the first execution of every instruction is the
+// largest part; a bottom of 3360 cells about 380 us (1358 in one CTA).
 #include "mac_internal.cuh"
 #include "mac_bottom.cuh"
 #include "mac_cluster.cuh"
@@ -495,8 +495,8 @@ __device__ __forceinline__ double cl_gsrb(const ClBottom& B, double fi, double x
     return x;
 }
 
-// Solves for x (in: the guess, already published at B.xa by every owner); f's mean comes off when
-// singular.  Every CTA of the cluster runs the same control flow (ONE: the first kOneBottom threads of
+// Solves for x (in: zero, already published at B.xa by every owner: a bottom is a coarse correction,
+// one-level contexts are refused); f's mean comes off when singular.  Every CTA of the cluster runs the same control flow (ONE: the first kOneBottom threads of
 // the one CTA).
 template <bool ONE>
 __device__ __noinline__ double cl_solve(const ClBottom& bottom, ClReduce& R, double f, double x, int nw,
@@ -525,7 +525,9 @@ __device__ __noinline__ double cl_solve(const ClBottom& bottom, ClReduce& R, dou
         // [0] rho = (rh, r) and the first beta (rho_old = alpha = omega = 1); [1] ||r||;  [2] the
         // rounding level of f - A x: a residual that small (the sweeps alone solved the bottom, or
         // a singular one's right-hand side keeps a rounded mean) cannot be reduced further, and
-        // iterating on it only adds noise to x
+        // iterating on it only adds noise to x.  A 2-norm, so larger than the largest residual's level
+        // by up to 10 sqrt(N): harmless from x = 0, decades under what a cycle needs of its bottom, but
+        // it would stall a solver that called this again on its own result
         cl_reduce<ONE>(R, parity, v, abs_key(r), nw, [&](const double* t, double k, double* o) {
             o[0] = t[0];
             o[1] = k;

@@ -8,7 +8,9 @@ import numpy as np
 import pytest
 
 import oracle as O
+from maestro_gb300 import capi
 from maestro_gb300.inputs import BC_DIR, BC_NEU, BC_PER, make_case
+from maestro_gb300.macproject import BcTower, Layout, MacError, MacProjector
 from tests._util import phi_rel_err, u_rel_err
 from tests.test_gpu_parity import gpu_project
 
@@ -87,3 +89,12 @@ def test_cluster_bottom_matches_the_one_cta_solver(bottom_check, n, dm, top, per
     if not per and all(v % 2 == 0 for v in n[:dm - 1]):
         # no cells of one colour side by side: the same iteration up to the order of its sums
         assert abs(its[0] - its[1]) <= 3 + its[0] // 5, r.stdout
+
+
+@pytest.mark.parametrize("n,box", [((25, 325), (25, 325)), ((45, 90), (45, 45)), ((9, 7, 6), (9, 7, 6))])
+def test_one_level_contexts_are_refused(cuda_lib, n, box):
+    # the cluster's bottom solver relies on it: a bottom always starts from a zero correction
+    with pytest.raises(MacError) as e:
+        MacProjector(Layout.tiled(n, box), (1.0 / max(n),) * len(n),
+                     BcTower((BC_PER,) * len(n), (BC_PER,) * len(n)))
+    assert e.value.code == capi.MAC_ERR_UNSUPPORTED
