@@ -405,7 +405,7 @@ void launch_bottom(const Dims& d, const LevelArrays<double>& a64, Tio* x, const 
 // ---- cluster tail V-cycle (mac_tail.cu) -----------------------------------------------------
 // nlev == 0: the bottom alone (f0 and e0 in its natural layout, e0 the initial guess)
 constexpr int kTailMaxLevels = 8;
-constexpr int kTailCells = 4096;   // cells of the first level of a tail at most
+constexpr int kTailCells2 = 16384, kTailCells3 = 4096;   // cells of a tail's first level at most, 2-D / 3-D
 constexpr int kTailSmemMax = 200 * 1024;
 struct TailGeo {
     int repl, rpc;                        // held whole by every CTA; rows a CTA

@@ -750,18 +750,20 @@ int ctx_alloc(mac_ctx* c) {
         }
     const Level& B = c->lev[c->nlevels - 1];
     if (B.d.ncell > kBottomMaxCells) return MAC_ERR_UNSUPPORTED;
-    // Cluster tail plans: from the first level >= 1 with at most 4096 cells that fits the cluster.  Larger
-    // levels are as fast or faster by launches over the whole chip, whose restriction also does the next
-    // level's first half-sweep (whole calls, 32768 cells in FP32 and 16384 in FP64 -> 4096: 64^3 mixed 770
-    // -> 734 us, 112^3 mixed 2392 -> 2069, 96 x 112 x 96 FP64 3772 -> 3413, 512^2 FP64 1505 -> 1410; 8192
-    // the same; 2048: 32^3 FP64 847 -> 964, 256^2 FP64 1104 -> 1143).
+    // Cluster tail plans: from the first level >= 1 that fits the cluster and has at most 4096 cells in
+    // 3-D, 16384 in 2-D.  Larger 3-D levels are as fast or faster by launches over the whole chip, whose
+    // restriction also does the next level's first half-sweep (whole calls, 32768 cells in FP32 and
+    // 16384 in FP64 -> 4096: 64^3 mixed 770 -> 734 us, 112^3 mixed 2392 -> 2069, 96 x 112 x 96 FP64 3772 ->
+    // 3413; 8192: 72^3 FP64 +3%; 2048: 32^3 FP64 847 -> 964).  A 2-D half-sweep has two arms less, the
+    // launch costs the same (4096 cells -> 16384: 160^2 FP64 909 -> 820, 96 x 320 FP64 2742 -> 2443, 320^2
+    // mixed 784 -> 747, 512^2 the same).
     c->bottom_cluster = tail_fits<double>(nullptr, 0, B.d, false, c->tail_nc);
     const bool small_bottom = B.d.ncell <= kDenseBottomMax;
     for (int slot = 0; slot < 2; ++slot) {
         c->tail_start[slot] = -1;
         for (int l = 1; l < c->nlevels - 1; ++l) {
             const int nl = c->nlevels - 1 - l;
-            if (c->lev[l].d.ncell > kTailCells || nl > kTailMaxLevels) continue;
+            if (c->lev[l].d.ncell > (c->dm == 2 ? kTailCells2 : kTailCells3) || nl > kTailMaxLevels) continue;
             Dims ds[kTailMaxLevels];
             for (int q = 0; q < nl; ++q) ds[q] = c->lev[l + q].d;
             bool fits = true;
